@@ -641,8 +641,8 @@ int slu_gemm_batched(slu_handle_t h, int transa, int transb, int M, int N, int K
                      long long sB, double beta, double* C, int ldc, long long sC, int nb) {
   return guard(h, [&] {
     SLU_REQUIRE(h && A && B && C, "null argument");
-    slu::gemm_batched<double>(h->h.stream, transa != 0, transb != 0, M, N, K, alpha, A, lda, sA,
-                              0, B, ldb, sB, 0, beta, C, ldc, sC, 0, nb, 1);
+    slu::gemm_f64(h->h, transa != 0, transb != 0, M, N, K, alpha, A, lda, sA, 0, B, ldb, sB, 0,
+                  beta, C, ldc, sC, 0, nb, 1);
   });
 }
 

@@ -1,0 +1,845 @@
+// Float64-accurate GEMM on the tensor cores (tcgen05) by residue arithmetic.
+//
+// The dense products of the float64 path -- sampling a dense interface block
+// (matAssembly/HBS/HBSnew.py:211-227), the Schur complements, pivot-block
+// inverses and block products of the red-black and Thomas eliminations
+// (direct_solve/omsdirectsolve.py:89-94, 238-277, 316-324) -- are bound by
+// GB300's float64 pipe (2 FMA per clock and SM, ~1.05 TFLOP/s measured).
+// Here such a product runs as 16 bfloat16 products on the tensor cores whose
+// results are exact, after the method published as "Ozaki scheme II"
+// (K. Ozaki, Y. Uchino, T. Imamura, 2025): scale each row of op(A) and each
+// column of op(B) to t-bit integers, multiply modulo pairwise coprime
+// moduli, and rebuild the integer product by the Chinese remainder theorem.
+//
+//   1. crt_convert_kernel: row r of op(A) (column of op(B)) with largest
+//      exponent field F becomes the integers a' = rint(a 2^(t - F + 1022)),
+//      |a'| <= 2^t, and their balanced residues modulo p_0 .. p_15, |r| <=
+//      128: exact in bfloat16.  B's residues carry the factor (P/p)^-1 mod p
+//      of the reconstruction.
+//   2. crt_gemm_kernel: per modulus a bfloat16 GEMM with float32 accumulation
+//      in TMEM.  The sum of 1024 products of two residues is at most 2^24,
+//      so every accumulator holds the exact integer; deeper products are
+//      drained every 960 terms.  The epilogue reduces each sum modulo p and
+//      stores it as one byte.
+//   3. crt_combine_kernel: X = sum_l y_l P/p_l - k P as a 128-bit integer
+//      (byte dot products, __dp4a), rounded once to float64, scaled by the
+//      row and column powers of two, then alpha and beta.
+//
+// With t = (123 - log2 K) / 2 (56 at K = 1024) the only errors are the
+// rounding of the inputs at 2^-(t+1) of their row's (column's) largest entry
+// and the final rounding; a float64 FMA chain rounds once per term.  Measured
+// against exact products the result is no further off than the float64
+// kernel's at every tested shape.  Rows or columns that hold an infinity or a
+// NaN take float64 dot products in step 3, with the float64 kernel's result.
+//
+// Work per element of A and B: 16 residues at ~9 integer / float32 slots;
+// per element of C: 16 x 2K bfloat16 flops, 16 bytes and ~220 slots of step
+// 3.  At 1024^3 that is 34 tensor GFLOP (~25 us) beside ~8 us of conversion
+// and ~6 us of reconstruction, against 2.1 ms on the float64 pipe.
+#include <cuda.h>
+#include <cuda_bf16.h>
+
+#include <algorithm>
+#include <mutex>
+
+#include "hbs.cuh"
+
+namespace slu {
+namespace {
+
+constexpr int NM = 16;   // moduli
+struct Tables {
+  int p[NM];
+  float pf[NM], inv[NM];
+  uint32_t ca[2][NM], cb[2][NM];   // balanced 2^(8 i) mod p (A), times (P/p)^-1 (B), packed bytes
+  int ba[NM], bb[NM];              // -(2^59) mod p (A), times (P/p)^-1 (B)
+  uint32_t w[15][NM / 4];          // byte i of P/p_l, four moduli packed
+  int p16[8];                      // P in 16-bit pieces
+  float top;                       // 2^112 / P
+};
+
+constexpr unsigned long long mod_pow2(int e, int p) {
+  unsigned long long r = 1;
+  for (int i = 0; i < e; ++i) r = r * 2 % p;
+  return r;
+}
+constexpr int balanced(int v, int p) { return 2 * v > p ? v - p : v; }
+
+constexpr Tables make_tables() {
+  Tables T{};
+  const int p[NM] = {256, 253, 251, 249, 247, 245, 241, 239, 233, 229, 227, 223, 211, 199, 197, 193};
+  unsigned __int128 P = 1;
+  for (int l = 0; l < NM; ++l) P *= (unsigned)p[l];
+  for (int l = 0; l < NM; ++l) {
+    T.p[l] = p[l];
+    T.pf[l] = (float)p[l];
+    T.inv[l] = 1.0f / (float)p[l];
+    const unsigned __int128 W = P / (unsigned)p[l];
+    const int wm = (int)(W % (unsigned)p[l]);
+    int m = 1;   // inverse of P/p modulo p
+    while (m * wm % p[l] != 1) ++m;
+    for (int i = 0; i < 8; ++i) {
+      const int c = (int)mod_pow2(8 * i, p[l]);
+      // p = 256: 128 is its own balanced form's limit; store -128
+      int a = balanced(c, p[l]), b = balanced(c * m % p[l], p[l]);
+      if (a == 128) a = -128;
+      if (b == 128) b = -128;
+      T.ca[i / 4][l] |= (uint32_t)(uint8_t)a << (8 * (i % 4));
+      T.cb[i / 4][l] |= (uint32_t)(uint8_t)b << (8 * (i % 4));
+    }
+    const int h = (int)mod_pow2(59, p[l]);
+    T.ba[l] = -h;
+    T.bb[l] = -(h * m % p[l]);
+    for (int i = 0; i < 15; ++i)
+      T.w[i][l / 4] |= (uint32_t)(uint8_t)(W >> (8 * i)) << (8 * (l % 4));
+  }
+  for (int i = 0; i < 8; ++i) T.p16[i] = (int)(uint16_t)(P >> (16 * i));
+  T.top = (float)(5192296858534827628530496329220096.0 / (double)P);   // 2^112 / P
+  return T;
+}
+__constant__ Tables c_tab = make_tables();
+
+// Largest |a'| exponent for products of depth K: |X| <= K 2^(2t) <= 2^123 < P / 4.
+int bits_for(int K) {
+  int lg = 0;
+  while ((1LL << lg) < K) ++lg;
+  return (123 - lg) / 2;
+}
+
+// dp4a of unsigned bytes of a with signed bytes of b, and the reverse
+__device__ __forceinline__ int dp4a_us(uint32_t a, uint32_t b, int c) {
+  int d;
+  asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  return d;
+}
+__device__ __forceinline__ int dp4a_su(uint32_t a, uint32_t b, int c) {
+  int d;
+  asm("dp4a.s32.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  return d;
+}
+
+// ---------------------------------------------------------------- conversion
+struct CrtOperand {
+  const double* x;
+  int ld;
+  long long s0, s1;
+  int rows;              // rows of op(A), columns of op(B)
+  int kcontig;           // consecutive k adjacent in memory
+  __nv_bfloat16* out;    // residues [modulus][batch][row][Kp]
+  int* ex;               // exponent field per [batch][row]; 2047 = not finite
+};
+
+constexpr int kStrip = 8;                     // rows per CTA
+constexpr int kChunkK = 256;                  // k per staged chunk
+constexpr int kPitch = kChunkK + kChunkK / 8; // one pad every 8 values: conflict-free
+
+// a CTA converts kStrip rows over the whole depth: exponents first (one
+// pass), then residues chunk by chunk through shared memory, which also
+// turns k-strided operands around.  Eight k per thread and modulus: 16-byte
+// stores.  Bound by the ~150 integer / float32 slots per element.
+__global__ void __launch_bounds__(256)
+crt_convert_kernel(CrtOperand a, CrtOperand b, int strips_a, int K, int Kp, int t, int batch0,
+                   int batch) {
+  __shared__ long long tile[kStrip * kPitch];
+  __shared__ int s_ex[kStrip];
+  __shared__ int s_red[8][kStrip];
+  const bool second = (int)blockIdx.x >= strips_a;
+  const CrtOperand& o = second ? b : a;
+  const int r0 = (second ? blockIdx.x - strips_a : blockIdx.x) * kStrip;
+  const int bt = blockIdx.y, b0 = bt % batch0, b1 = bt / batch0;
+  const long long* x = reinterpret_cast<const long long*>(o.x + b0 * o.s0 + b1 * o.s1);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int nr = min(kStrip, o.rows - r0);
+  // ---- exponent field of every row
+  int f = 0;
+  if (o.kcontig) {
+    if (warp < nr) {
+      const long long* row = x + (long long)(r0 + warp) * o.ld;
+      for (int k = lane; k < K; k += 32) f = max(f, (int)((row[k] >> 52) & 0x7ff));
+    }
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) f = max(f, __shfl_xor_sync(0xffffffffu, f, s));
+    if (lane == 0) s_ex[warp] = f;
+  } else {
+    const int r = tid & 7;
+    if (r < nr) {
+      const long long* col = x + r0 + r;
+      for (int k = tid >> 3; k < K; k += 32)
+        f = max(f, (int)((col[(long long)k * o.ld] >> 52) & 0x7ff));
+    }
+    f = max(f, __shfl_xor_sync(0xffffffffu, f, 8));
+    f = max(f, __shfl_xor_sync(0xffffffffu, f, 16));
+    if (lane < 8) s_red[warp][lane] = f;
+    __syncthreads();
+    if (tid < 8) {
+      int g = 0;
+      for (int w = 0; w < 8; ++w) g = max(g, s_red[w][tid]);
+      s_ex[tid] = g;
+    }
+  }
+  __syncthreads();
+  if (tid < nr) o.ex[(long long)bt * o.rows + r0 + tid] = s_ex[tid];
+  // ---- residues
+  const int row = warp, k8 = 8 * lane;
+  const int F = max(s_ex[row], 1);
+  const bool live = row < nr, finite = s_ex[row] != 0x7ff;
+  const long long plane = (long long)batch * o.rows * Kp;
+  __nv_bfloat16* dst = o.out + ((long long)bt * o.rows + r0 + row) * Kp + k8;
+  for (int kc = 0; kc < Kp; kc += kChunkK) {
+    const int kn = min(kChunkK, K - kc);   // may be <= 0 in the padding
+    __syncthreads();
+    if (o.kcontig) {
+      for (int k = lane; k < kChunkK; k += 32)
+        tile[warp * kPitch + k + (k >> 3)] =
+            (live && k < kn) ? x[(long long)(r0 + warp) * o.ld + kc + k] : 0;
+    } else {
+      const int r = tid & 7;
+      for (int k = tid >> 3; k < kChunkK; k += 32)
+        tile[r * kPitch + k + (k >> 3)] =
+            (r < nr && k < kn) ? x[(long long)(kc + k) * o.ld + r0 + r] : 0;
+    }
+    __syncthreads();
+    if (!live || kc + k8 >= Kp) continue;
+    uint32_t lo[8], hi[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const long long v = tile[row * kPitch + 9 * lane + u];
+      const int fe = (int)((v >> 52) & 0x7ff);
+      unsigned long long m = (unsigned long long)v & 0xfffffffffffffULL;
+      if (fe) m |= 1ULL << 52;
+      // a' = m 2^(t - 53 - (F - max(fe, 1))), rounded to nearest
+      const int sh = t - 53 - (F - max(fe, 1));
+      unsigned long long q;
+      if (sh >= 0) q = m << sh;
+      else if (sh > -55) q = (m + (1ULL << (-sh - 1))) >> -sh;
+      else q = 0;
+      if (!finite) q = 0;
+      // shifted by 2^59 to be non-negative (the tables take it off again)
+      const unsigned long long z = v < 0 ? (1ULL << 59) - q : (1ULL << 59) + q;
+      lo[u] = (uint32_t)z;
+      hi[u] = (uint32_t)(z >> 32);
+    }
+#pragma unroll
+    for (int l = 0; l < NM; ++l) {
+      const uint32_t c0 = second ? c_tab.cb[0][l] : c_tab.ca[0][l];
+      const uint32_t c1 = second ? c_tab.cb[1][l] : c_tab.ca[1][l];
+      const int bias = 0x4B400000 + (second ? c_tab.bb[l] : c_tab.ba[l]);
+      const float p = c_tab.pf[l], ip = c_tab.inv[l];
+      uint32_t w[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        float r[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          // |s| < 2^19: exact as the low bits of a float of magnitude 1.5 2^23
+          const int s = dp4a_us(lo[2 * u + e], c0, dp4a_us(hi[2 * u + e], c1, bias));
+          const float g = __int_as_float(s) - 12582912.f;
+          const float q = fmaf(g, ip, 12582912.f) - 12582912.f;
+          r[e] = fmaf(-p, q, g);
+        }
+        const __nv_bfloat162 h = __floats2bfloat162_rn(r[0], r[1]);
+        w[u] = *reinterpret_cast<const uint32_t*>(&h);
+      }
+      *reinterpret_cast<uint4*>(dst + l * plane + kc) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+  }
+}
+
+// ---------------------------------------------------------------- tcgen05 GEMM
+constexpr int BM = 128, BK = 64;
+constexpr int A_BYTES = BM * BK * 2;
+constexpr int kEpiWarps = 8;
+constexpr int kThreads = 32 * (kEpiWarps + 2);   // warps 0-7 epilogue, 8 TMA, 9 MMA
+constexpr int kMaxStages = 8;
+constexpr int kRing = 208 * 1024;
+constexpr long long kWaitLimit = 1LL << 22;
+constexpr int kTmemCols = 512;                   // two accumulators of up to 256 columns
+constexpr int kChunkOne = 16, kChunkMany = 15;   // k-tiles per exact float32 sum
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) {
+  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count)
+               : "memory");
+}
+__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
+               "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+// Bounded wait for the phase with the given parity; gives up early once
+// another role has.
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* fail) {
+  const uint32_t addr = smem_u32(bar);
+  for (long long i = 0; i < kWaitLimit; ++i) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(addr), "r"(parity)
+        : "memory");
+    if (done) return true;
+    if (fail && *fail) return false;
+  }
+  return false;
+}
+__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y,
+                                            uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar))
+      : "memory");
+}
+// K-major, 128B swizzle, 8-row groups 1024 B apart
+__device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
+  return (uint64_t)((addr >> 4) & 0x3FFFu) | (uint64_t)1 << 16 | (uint64_t)(1024 >> 4) << 32 |
+         (uint64_t)1 << 46 | (uint64_t)2 << 61;
+}
+__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
+                                         uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void mma_commit(uint64_t* bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+          smem_u32(bar))
+      : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
+        "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+}
+
+struct CrtGemm {
+  int M, N, batch;
+  int tm, tn;            // tiles
+  int BN;                // tile columns, a multiple of 16, at most 256
+  int KT, chunks, per;   // k-tiles; chunks of `per` k-tiles
+  int stages;
+  long long items;       // NM * batch * tm * tn
+  int8_t* R;             // residues [modulus][batch][M][pitch]
+  int pitch;
+  unsigned int* err;
+};
+
+// Persistent: each CTA runs every gridDim-th (modulus, batch, tile) item.
+//   warp 8: TMA into a ring of (A 128 x 64, B BN x 64) slabs
+//   warp 9: tcgen05.mma, the items' chunks alternating between the two TMEM
+//           accumulators
+//   warps 0-7: drain the other accumulator meanwhile (lanes 32 (w % 4) ..,
+//           columns of half w / 4): reduce modulo p, pack, 16-byte stores
+// Tiles of 128 x up to 256 columns: a smaller one doubles the operand
+// traffic per flop, and 256 is the widest the instruction takes.
+__global__ void __maxnreg__(168)
+crt_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                const __grid_constant__ CrtGemm g) {
+  extern __shared__ unsigned char smem_raw[];
+  __shared__ __align__(8) uint64_t full_bar[kMaxStages];
+  __shared__ __align__(8) uint64_t empty_bar[kMaxStages];
+  __shared__ __align__(8) uint64_t ready_bar[2];
+  __shared__ __align__(8) uint64_t drained_bar[2];
+  __shared__ __align__(8) uint64_t quiet_bar;
+  __shared__ uint32_t tmem_slot;
+  __shared__ volatile int s_fail;
+  __shared__ volatile long long s_issued;
+  unsigned char* smem = reinterpret_cast<unsigned char*>(
+      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int S = g.stages, BN = g.BN;
+  const uint32_t stage_bytes = A_BYTES + BN * BK * 2;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < S; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
+    }
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(&ready_bar[a], 1);
+      mbar_init(&drained_bar[a], 32 * kEpiWarps);
+    }
+    mbar_init(&quiet_bar, 1);
+    s_fail = 0;
+    s_issued = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == kEpiWarps + 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(&tmem_slot)),
+                 "r"(kTmemCols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_slot;
+  const int tiles = g.tm * g.tn;
+
+  if (warp == kEpiWarps) {
+    if (lane == 0) {
+      long long it = 0;
+      bool ok = true;
+      for (long long id = blockIdx.x; id < g.items && ok; id += gridDim.x) {
+        const long long mb = id / tiles;              // modulus * batch + batch index
+        const int tile = (int)(id - mb * tiles);
+        const int m0 = (tile / g.tn) * BM, n0 = (tile % g.tn) * BN;
+        const int ya = (int)(mb * g.M) + m0, yb = (int)(mb * g.N) + n0;
+        for (int kt = 0; kt < g.KT; ++kt, ++it) {
+          const int s = (int)(it % S);
+          if (it >= S && !mbar_wait(&empty_bar[s], (uint32_t)((it / S) + 1) & 1, &s_fail)) {
+            s_fail = 1;
+            ok = false;
+            break;
+          }
+          unsigned char* a = smem + s * stage_bytes;
+          mbar_expect_tx(&full_bar[s], stage_bytes);
+          tma_load_2d(a, &tmA, kt * BK, ya, &full_bar[s]);
+          tma_load_2d(a + A_BYTES, &tmB, kt * BK, yb, &full_bar[s]);
+          s_issued = it + 1;
+        }
+      }
+    }
+  } else if (warp == kEpiWarps + 1) {
+    if (lane == 0) {
+      // kind::f16: D f32, A/B bf16, both K-major, M = 128, N = BN
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
+                             ((uint32_t)(BM >> 4) << 24);
+      long long it = 0;
+      uint32_t n = 0;   // chunks issued
+      bool ok = true;
+      for (long long id = blockIdx.x; id < g.items && ok; id += gridDim.x) {
+        int kt = 0;
+        for (int c = 0; c < g.chunks && ok; ++c, ++n) {
+          const uint32_t a = n & 1;
+          if (n >= 2 && !mbar_wait(&drained_bar[a], ((n >> 1) - 1) & 1, &s_fail)) {
+            ok = false;
+            break;
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t dacc = tmem + a * 256;
+          const int kend = min(kt + g.per, g.KT);
+          for (int j = 0; kt < kend; ++j, ++kt, ++it) {
+            const int s = (int)(it % S);
+            if (!mbar_wait(&full_bar[s], (uint32_t)(it / S) & 1, &s_fail)) {
+              ok = false;
+              break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t sa = smem_u32(smem + s * stage_bytes), sb = sa + A_BYTES;
+#pragma unroll
+            for (int kk = 0; kk < BK / 16; ++kk)
+              mma_bf16(dacc, smem_desc(sa + kk * 32), smem_desc(sb + kk * 32), idesc,
+                       (j | kk) != 0);
+            mma_commit(&empty_bar[s]);
+          }
+          if (ok) mma_commit(&ready_bar[a]);
+        }
+      }
+      if (!ok) s_fail = 1;
+      // every MMA issued has finished before TMEM and the ring are given up
+      mma_commit(&quiet_bar);
+      mbar_wait(&quiet_bar, 0, nullptr);
+    }
+  } else {
+    const int q = warp & 3, half = warp >> 2;
+    const int groups = BN / 16, g0 = half ? (groups + 1) / 2 : 0, g1 = half ? groups : (groups + 1) / 2;
+    const uint32_t lanes = (uint32_t)(q * 32) << 16;
+    uint32_t n = 0;
+    bool ok = true;
+    for (long long id = blockIdx.x; id < g.items && ok; id += gridDim.x) {
+      const long long mb = id / tiles;
+      const int tile = (int)(id - mb * tiles), l = (int)(mb / g.batch);
+      const int row = (tile / g.tn) * BM + q * 32 + lane, n0 = (tile % g.tn) * BN;
+      const float p = c_tab.pf[l], ip = c_tab.inv[l];
+      int8_t* out = g.R + (mb * g.M + row) * g.pitch + n0;
+      for (int c = 0; c < g.chunks; ++c, ++n) {
+        const uint32_t a = n & 1;
+        ok = mbar_wait(&ready_bar[a], (n >> 1) & 1, &s_fail);
+        if (!__all_sync(0xffffffffu, ok)) {   // warp-uniform: the loads below are collective
+          ok = false;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        for (int j = g0; j < g1; ++j) {
+          uint32_t v[16];
+          tmem_ld16(tmem + lanes + a * 256 + 16 * j, v);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          if (row < g.M && n0 + 16 * j < g.pitch) {
+            uint4* dst = reinterpret_cast<uint4*>(out + 16 * j);
+            uint32_t old[4] = {0, 0, 0, 0};
+            if (c > 0) {
+              const uint4 o = *dst;
+              old[0] = o.x; old[1] = o.y; old[2] = o.z; old[3] = o.w;
+            }
+            uint32_t w[4];
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+              float x = __uint_as_float(v[e]);
+              if (c > 0) x += (float)(int8_t)(old[e >> 2] >> (8 * (e & 3)));
+              const float k = fmaf(x, ip, 12582912.f) - 12582912.f;
+              const uint32_t y = __float_as_uint(fmaf(-p, k, x) + 12582912.f) & 0xffu;
+              w[e >> 2] = (e & 3) ? w[e >> 2] | (y << (8 * (e & 3))) : y;
+            }
+            *dst = make_uint4(w[0], w[1], w[2], w[3]);
+          }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        mbar_arrive(&drained_bar[a]);
+      }
+    }
+    if (!ok) {
+      s_fail = 1;
+      if (lane == 0 && g.err) atomicOr(g.err, 1u);
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (threadIdx.x == 0 && s_fail) {
+    // the copies already issued land before the CTA exits
+    if (g.err) atomicOr(g.err, 1u);
+    const long long issued = s_issued;
+    for (long long j = issued > S ? issued - S : 0; j < issued; ++j)
+      mbar_wait(&full_bar[j % S], (uint32_t)(j / S) & 1, nullptr);
+  }
+  __syncthreads();
+  if (warp == kEpiWarps + 1)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+                 "r"(kTmemCols)
+                 : "memory");
+}
+
+// ---------------------------------------------------------------- reconstruction
+struct CrtCombine {
+  int M, N, K, batch0, batch;
+  const int8_t* R;
+  int pitch;
+  const int *ea, *eb;
+  int t;
+  double alpha, beta;
+  double* C;
+  int ldc;
+  long long sC0, sC1;
+  // operands, for rows and columns that are not finite
+  const double *A, *B;
+  long long ak, ai, sA0, sA1, bk, bj, sB0, sB1;   // strides along k, i, j
+};
+
+// 128-bit two's complement value c3:c2:c1:c0 times 2^e, rounded to nearest even
+__device__ __forceinline__ double to_double(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3,
+                                            int e) {
+  unsigned long long lo = (unsigned long long)c1 << 32 | c0, hi = (unsigned long long)c3 << 32 | c2;
+  const uint32_t neg = c3 >> 31;
+  if (neg) {
+    lo = ~lo + 1;
+    hi = ~hi + (lo == 0);
+  }
+  if (!(lo | hi)) return 0.0;
+  const int lz = hi ? __clzll(hi) : 64 + __clzll(lo);
+  if (lz >= 64) {
+    hi = lo << (lz - 64);
+    lo = 0;
+  } else if (lz > 0) {
+    hi = hi << lz | lo >> (64 - lz);
+    lo <<= lz;
+  }
+  // value = hi.lo 2^(64 - lz) with the top bit of hi set: 53 bits kept
+  unsigned long long m = hi >> 11;
+  const unsigned long long rest = (hi & 0x7ff) << 1 | (lo != 0);
+  m += rest > 0x800 || (rest == 0x800 && (m & 1));
+  // m in [2^52, 2^53]; value m 2^(75 - lz + e)
+  const int field = 75 - lz + e + 1075;
+  double v;
+  if (field >= 1 && field <= 2045) {
+    v = __longlong_as_double((long long)(((unsigned long long)field << 52) +
+                                         (m - (1ULL << 52))));
+  } else {
+    v = ldexp((double)m, 75 - lz + e);
+  }
+  return neg ? -v : v;
+}
+
+// One thread per four consecutive elements of a row of C: four bytes of every
+// residue plane, transposed in registers so a __dp4a sums four moduli.
+__global__ void __launch_bounds__(256)
+crt_combine_kernel(const __grid_constant__ CrtCombine g) {
+  const int nq = (g.N + 3) / 4;
+  const long long total = (long long)g.batch * g.M * nq;
+  const long long plane = (long long)g.batch * g.M * g.pitch;
+  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < total;
+       q += (long long)gridDim.x * blockDim.x) {
+    const long long br = q / nq;                   // batch * M + row
+    const int j0 = 4 * (int)(q - br * nq), bt = (int)(br / g.M), i = (int)(br - (long long)bt * g.M);
+    const int b0 = bt % g.batch0, b1 = bt / g.batch0;
+    const int8_t* src = g.R + br * g.pitch + j0;
+    uint32_t r[NM];
+#pragma unroll
+    for (int l = 0; l < NM; ++l) r[l] = *reinterpret_cast<const uint32_t*>(src + l * plane);
+    // r[4 a + e] <- byte e of planes 4 a .. 4 a + 3
+#pragma unroll
+    for (int a = 0; a < NM; a += 4) {
+      const uint32_t x0 = __byte_perm(r[a], r[a + 1], 0x5140), x1 = __byte_perm(r[a], r[a + 1], 0x7362);
+      const uint32_t y0 = __byte_perm(r[a + 2], r[a + 3], 0x5140), y1 = __byte_perm(r[a + 2], r[a + 3], 0x7362);
+      r[a] = __byte_perm(x0, y0, 0x5410);
+      r[a + 1] = __byte_perm(x0, y0, 0x7632);
+      r[a + 2] = __byte_perm(x1, y1, 0x5410);
+      r[a + 3] = __byte_perm(x1, y1, 0x7632);
+    }
+    const int fa = g.ea[br];
+    double* c = g.C + b0 * g.sC0 + b1 * g.sC1 + (long long)i * g.ldc + j0;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      if (j0 + e >= g.N) break;
+      const int fb = g.eb[(long long)bt * g.N + j0 + e];
+      double v;
+      if (fa == 0x7ff || fb == 0x7ff) {
+        const double* ap = g.A + b0 * g.sA0 + b1 * g.sA1 + i * g.ai;
+        const double* bp = g.B + b0 * g.sB0 + b1 * g.sB1 + (j0 + e) * g.bj;
+        v = 0.0;
+        for (int k = 0; k < g.K; ++k) v = fma(ap[k * g.ak], bp[k * g.bk], v);
+      } else {
+        int s[16];
+#pragma unroll
+        for (int b = 0; b < 15; ++b) {
+          s[b] = 0;
+#pragma unroll
+          for (int a = 0; a < NM / 4; ++a) s[b] = dp4a_su(r[4 * a + e], c_tab.w[b][a], s[b]);
+        }
+        s[15] = 0;
+        // k = nearest integer to (sum of y_l P / p_l) / P; the product is below P / 4
+        const float f = fmaf((float)s[12], 1.0f / 65536.0f,
+                             fmaf((float)s[13], 1.0f / 256.0f, (float)s[14]));
+        const int k = __float2int_rn(f * c_tab.top);
+        // 16-bit pieces, then 32-bit words with carries
+        long long w[4];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+          const int u0 = s[4 * a] + (s[4 * a + 1] << 8) - k * c_tab.p16[2 * a];
+          const int u1 = s[4 * a + 2] + (s[4 * a + 3] << 8) - k * c_tab.p16[2 * a + 1];
+          w[a] = (long long)u1 * 65536 + u0;
+        }
+        w[1] += w[0] >> 32;
+        w[2] += w[1] >> 32;
+        w[3] += w[2] >> 32;
+        v = to_double((uint32_t)w[0], (uint32_t)w[1], (uint32_t)w[2], (uint32_t)w[3],
+                      max(fa, 1) + max(fb, 1) - 2 * (1022 + g.t));
+      }
+      if (g.alpha == -1.0) v = -v;
+      else if (g.alpha != 1.0) v *= g.alpha;
+      if (g.beta != 0.0) v = fma(g.beta, c[e], v);
+      c[e] = v;
+    }
+  }
+}
+
+// ---------------------------------------------------------------- host
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
+                                  const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+EncodeTiledFn encode_fn() {
+  static EncodeTiledFn fn = nullptr;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault,
+                                         &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      fn = reinterpret_cast<EncodeTiledFn>(p);
+  });
+  if (!fn) throw Error(SLU_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
+  return fn;
+}
+
+CUtensorMap residue_map(const void* base, long long rows, int Kp, int box_rows) {
+  CUtensorMap m;
+  cuuint64_t dims[2] = {(cuuint64_t)Kp, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)Kp * 2};
+  cuuint32_t box[2] = {BK, (cuuint32_t)box_rows};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = encode_fn()(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims,
+                           strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) throw Error(SLU_ERR_CUDA, "cuTensorMapEncodeTiled failed");
+  return m;
+}
+
+size_t up(size_t v, size_t a) { return (v + a - 1) / a * a; }
+
+// Workspace of one launch set (residues of A and B, result residues, exponents).
+size_t crt_bytes(int M, int N, int K, long long nb) {
+  const size_t Kp = up(K, BK), pitch = up(N, 16);
+  return up((size_t)2 * NM * nb * M * Kp, 1024) + up((size_t)2 * NM * nb * N * Kp, 1024) +
+         up((size_t)NM * nb * M * pitch, 1024) + up((size_t)4 * nb * (M + N), 1024) + 4096;
+}
+
+// Bound on the workspace of one launch set: larger products run in pieces
+// (deeper ones in slices of kDepthMax, accumulated in C).
+constexpr size_t kWsMax = size_t(768) << 20;
+constexpr int kDepthMax = 8192;
+
+struct Operand {
+  const double* x;
+  int ld;
+  bool trans;
+  long long s0, s1;
+};
+
+void crt_piece(Handle& h, int M, int N, int K, double alpha, const Operand& A, const Operand& B,
+               double beta, double* C, int ldc, long long sC0, long long sC1, int batch0,
+               int batch) {
+  cudaStream_t st = h.stream;
+  const int Kp = (int)up(K, BK), pitch = (int)up(N, 16), t = bits_for(K);
+  h.gemm_ws.reserve(crt_bytes(M, N, K, batch), st);
+  auto* ra = h.gemm_ws.take<__nv_bfloat16>((size_t)NM * batch * M * Kp);
+  auto* rb = h.gemm_ws.take<__nv_bfloat16>((size_t)NM * batch * N * Kp);
+  auto* R = h.gemm_ws.take<int8_t>((size_t)NM * batch * M * pitch);
+  int* ea = h.gemm_ws.take<int>((size_t)batch * M);
+  int* eb = h.gemm_ws.take<int>((size_t)batch * N);
+  const CrtOperand oa{A.x, A.ld, A.s0, A.s1, M, !A.trans, ra, ea};
+  const CrtOperand ob{B.x, B.ld, B.s0, B.s1, N, B.trans, rb, eb};
+  const int sa = (M + kStrip - 1) / kStrip, sb = (N + kStrip - 1) / kStrip;
+  crt_convert_kernel<<<dim3(sa + sb, batch), 256, 0, st>>>(oa, ob, sa, K, Kp, t, batch0, batch);
+  check_launch("crt_convert_kernel");
+  CrtGemm g{};
+  g.M = M;
+  g.N = N;
+  g.batch = batch;
+  g.tm = (M + BM - 1) / BM;
+  // widest tiles that still give every SM an item, evenly over the columns
+  g.tn = (N + 255) / 256;
+  while ((long long)NM * batch * g.tm * g.tn < num_sms() && (N + g.tn - 1) / g.tn > 64) ++g.tn;
+  g.BN = (int)up((N + g.tn - 1) / g.tn, 16);
+  g.tn = (N + g.BN - 1) / g.BN;
+  g.KT = Kp / BK;
+  g.chunks = g.KT <= kChunkOne ? 1 : (g.KT + kChunkMany - 1) / kChunkMany;
+  g.per = (g.KT + g.chunks - 1) / g.chunks;
+  g.stages = std::min(kMaxStages, kRing / (A_BYTES + g.BN * BK * 2));
+  g.items = (long long)NM * batch * g.tm * g.tn;
+  g.R = R;
+  g.pitch = pitch;
+  g.err = reinterpret_cast<unsigned int*>(h.info.as<int>()) + 1;
+  const CUtensorMap ma = residue_map(ra, (long long)NM * batch * M, Kp, BM);
+  const CUtensorMap mb = residue_map(rb, (long long)NM * batch * N, Kp, g.BN);
+  const size_t sm = (size_t)g.stages * (A_BYTES + g.BN * BK * 2) + 1024;
+  ensure_smem(reinterpret_cast<const void*>(crt_gemm_kernel), sm);
+  crt_gemm_kernel<<<(unsigned)std::min<long long>(g.items, num_sms()), kThreads, sm, st>>>(ma, mb,
+                                                                                           g);
+  check_launch("crt_gemm_kernel");
+  CrtCombine c{};
+  c.M = M;
+  c.N = N;
+  c.K = K;
+  c.batch0 = batch0;
+  c.batch = batch;
+  c.R = R;
+  c.pitch = pitch;
+  c.ea = ea;
+  c.eb = eb;
+  c.t = t;
+  c.alpha = alpha;
+  c.beta = beta;
+  c.C = C;
+  c.ldc = ldc;
+  c.sC0 = sC0;
+  c.sC1 = sC1;
+  c.A = A.x;
+  c.ak = A.trans ? A.ld : 1;
+  c.ai = A.trans ? 1 : A.ld;
+  c.sA0 = A.s0;
+  c.sA1 = A.s1;
+  c.B = B.x;
+  c.bk = B.trans ? 1 : B.ld;
+  c.bj = B.trans ? B.ld : 1;
+  c.sB0 = B.s0;
+  c.sB1 = B.s1;
+  const long long total = (long long)batch * M * ((N + 3) / 4);
+  crt_combine_kernel<<<(unsigned)std::min<long long>((total + 255) / 256, 32LL * num_sms()), 256, 0,
+                       st>>>(c);
+  check_launch("crt_combine_kernel");
+}
+
+}  // namespace
+
+void gemm_f64_tensor(Handle& h, bool ta, bool tb, int M, int N, int K, double alpha,
+                     const double* A, int lda, long long sA0, long long sA1, const double* B,
+                     int ldb, long long sB0, long long sB1, double beta, double* C, int ldc,
+                     long long sC0, long long sC1, int batch0, int batch1) {
+  if (K > kDepthMax) {
+    for (int k0 = 0; k0 < K; k0 += kDepthMax)
+      gemm_f64_tensor(h, ta, tb, M, N, std::min(kDepthMax, K - k0), alpha,
+                      A + (ta ? (long long)k0 * lda : (long long)k0), lda, sA0, sA1,
+                      B + (tb ? (long long)k0 : (long long)k0 * ldb), ldb, sB0, sB1,
+                      k0 ? 1.0 : beta, C, ldc, sC0, sC1, batch0, batch1);
+    return;
+  }
+  // pieces of at most kWsMax workspace: rows and columns halved (each half a
+  // multiple of a tile) until one matrix fits, then as many matrices as fit
+  int Mp = M, Np = N;
+  while (crt_bytes(Mp, Np, K, 1) > kWsMax && (Mp > 1024 || Np > 1024)) {
+    if (Mp >= Np) Mp = (int)up((Mp + 1) / 2, 256);
+    else Np = (int)up((Np + 1) / 2, 256);
+  }
+  const long long nb = (long long)batch0 * batch1;
+  long long fit = std::max<long long>(1, kWsMax / crt_bytes(Mp, Np, K, 1));
+  fit = std::min<long long>(fit, 65535);
+  // residue rows are indexed by 32-bit TMA coordinates
+  fit = std::max<long long>(1, std::min(fit, (1LL << 30) / NM / std::max(Mp, Np)));
+  for (int i0 = 0; i0 < M; i0 += Mp)
+    for (int j0 = 0; j0 < N; j0 += Np) {
+      const int m = std::min(Mp, M - i0), n = std::min(Np, N - j0);
+      const double* a = A + (ta ? (long long)i0 : (long long)i0 * lda);
+      const double* b = B + (tb ? (long long)j0 * ldb : (long long)j0);
+      double* c = C + (long long)i0 * ldc + j0;
+      if (fit >= nb) {
+        crt_piece(h, m, n, K, alpha, {a, lda, ta, sA0, sA1}, {b, ldb, tb, sB0, sB1}, beta, c, ldc,
+                  sC0, sC1, batch0, (int)nb);
+        continue;
+      }
+      for (int q1 = 0; q1 < batch1; ++q1)
+        for (int q0 = 0; q0 < batch0; q0 += (int)fit) {
+          const int cnt = (int)std::min<long long>(fit, batch0 - q0);
+          crt_piece(h, m, n, K, alpha, {a + q0 * sA0 + q1 * sA1, lda, ta, sA0, 0},
+                    {b + q0 * sB0 + q1 * sB1, ldb, tb, sB0, 0}, beta, c + q0 * sC0 + q1 * sC1, ldc,
+                    sC0, 0, cnt, cnt);
+        }
+    }
+}
+
+// Residue products pay where the float64 pipe is the bound: enough flops to
+// cover three launches, and enough of them per element of C and of the
+// operands to cover the conversions.
+bool gemm_tensor_pays(int M, int N, int K, long long nb) {
+  return M >= 64 && N >= 32 && K >= 64 && 2.0 * M * N * K * nb >= 2.0e7;
+}
+
+void gemm_f64(Handle& h, bool ta, bool tb, int M, int N, int K, double alpha, const double* A,
+              int lda, long long sA0, long long sA1, const double* B, int ldb, long long sB0,
+              long long sB1, double beta, double* C, int ldc, long long sC0, long long sC1,
+              int batch0, int batch1) {
+  if (batch0 > 0 && batch1 > 0 && gemm_tensor_pays(M, N, K, (long long)batch0 * batch1))
+    gemm_f64_tensor(h, ta, tb, M, N, K, alpha, A, lda, sA0, sA1, B, ldb, sB0, sB1, beta, C, ldc,
+                    sC0, sC1, batch0, batch1);
+  else
+    gemm_batched<double>(h.stream, ta, tb, M, N, K, alpha, A, lda, sA0, sA1, B, ldb, sB0, sB1,
+                         beta, C, ldc, sC0, sC1, batch0, batch1);
+}
+
+}  // namespace slu

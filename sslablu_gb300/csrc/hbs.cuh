@@ -63,10 +63,24 @@ struct HostStage {
 struct Handle {
   cudaStream_t stream = nullptr;
   Workspace ws;
+  Workspace gemm_ws;   // residues of gemm_f64 (crt_gemm.cu), at most about 1 GB
   HostStage upload, readback;
   DevBuf info;  // int[64] device status words
   std::string last_error;
 };
+
+// gemm_batched<double> for dense products: on the tensor cores by residue
+// arithmetic where that is faster (crt_gemm.cu; float64-accurate), else the
+// float64 kernel.  C must not overlap A or B.
+void gemm_f64(Handle& h, bool ta, bool tb, int M, int N, int K, double alpha, const double* A,
+              int lda, long long sA0, long long sA1, const double* B, int ldb, long long sB0,
+              long long sB1, double beta, double* C, int ldc, long long sC0, long long sC1,
+              int batch0, int batch1 = 1);
+void gemm_f64_tensor(Handle& h, bool ta, bool tb, int M, int N, int K, double alpha,
+                     const double* A, int lda, long long sA0, long long sA1, const double* B,
+                     int ldb, long long sB0, long long sB1, double beta, double* C, int ldc,
+                     long long sC0, long long sC1, int batch0, int batch1 = 1);
+bool gemm_tensor_pays(int M, int N, int K, long long nb);
 
 // A step operator in the digit form of the tensor-core sweep (ozaki.cu):
 // each row of every block scaled by its own power of two 2^E (max |row| <

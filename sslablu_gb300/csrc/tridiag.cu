@@ -67,7 +67,8 @@ __global__ void ident_wide_kernel(int nb, int m, int w, double* __restrict__ F) 
 }
 
 // The fused solve operators of every reduction level (see RbLevel).
-void build_fused_ops(cudaStream_t st, RbSolver& S) {
+void build_fused_ops(Handle& h, RbSolver& S) {
+  cudaStream_t st = h.stream;
   const int m = S.m;
   const long long mm = (long long)m * m, w = 3LL * m;
   for (size_t l = 0; l + 1 < S.levels.size(); ++l) {
@@ -83,16 +84,16 @@ void build_fused_ops(cudaStream_t st, RbSolver& S) {
     check_launch("rb_fop_init_kernel");
     // -SiM_{2j} Inv_{2j-1} (j >= 1), -SiP_{2j} Inv_{2j+1}
     if (nR > 1)
-      gemm_batched<double>(st, false, false, m, m, m, -1.0, dp(P.SiM) + 2 * mm, m, 2 * mm, 0,
+      gemm_f64(h, false, false, m, m, m, -1.0, dp(P.SiM) + 2 * mm, m, 2 * mm, 0,
                            dp(P.Inv) + mm, m, 2 * mm, 0, 0.0, F + 3 * mm + m, (int)w, 3 * mm, 0,
                            nR - 1);
-    gemm_batched<double>(st, false, false, m, m, m, -1.0, dp(P.SiP), m, 2 * mm, 0, dp(P.Inv) + mm,
+    gemm_f64(h, false, false, m, m, m, -1.0, dp(P.SiP), m, 2 * mm, 0, dp(P.Inv) + mm,
                          m, 2 * mm, 0, 0.0, F + 2 * m, (int)w, 3 * mm, 0, nR);
     // [Inv_o | -Inv_o SiM_o | -Inv_o SiP_o]
     copy_batched<double>(st, m, m, dp(P.Inv) + mm, m, 2 * mm, 0, Bo, (int)w, 3 * mm, 0, nR);
-    gemm_batched<double>(st, false, false, m, m, m, -1.0, dp(P.Inv) + mm, m, 2 * mm, 0,
+    gemm_f64(h, false, false, m, m, m, -1.0, dp(P.Inv) + mm, m, 2 * mm, 0,
                          dp(P.SiM) + mm, m, 2 * mm, 0, 0.0, Bo + m, (int)w, 3 * mm, 0, nR);
-    gemm_batched<double>(st, false, false, m, m, m, -1.0, dp(P.Inv) + mm, m, 2 * mm, 0,
+    gemm_f64(h, false, false, m, m, m, -1.0, dp(P.Inv) + mm, m, 2 * mm, 0,
                          dp(P.SiP) + mm, m, 2 * mm, 0, 0.0, Bo + 2 * m, (int)w, 3 * mm, 0, nR);
   }
   S.fused = true;
@@ -232,17 +233,17 @@ void rb_factor(Handle& h, RbSolver& S, int nblk, int m, const double* SiM, const
     // X_o = T_o^{-1} [SiM_o | SiP_o] for odd o, as products with the
     // inverses formed when the level was factored (GEMMs over all SMs
     // instead of substitutions)
-    gemm_batched<double>(st, false, false, m, m, m, 1.0, dp(P.Inv) + mm, m, 2 * mm, 0,
+    gemm_f64(h, false, false, m, m, m, 1.0, dp(P.Inv) + mm, m, 2 * mm, 0,
                          dp(P.SiM) + mm, m, 2 * mm, 0, 0.0, X, (int)m2, 2 * mm, 0, nR);
-    gemm_batched<double>(st, false, false, m, m, m, 1.0, dp(P.Inv) + mm, m, 2 * mm, 0,
+    gemm_f64(h, false, false, m, m, m, 1.0, dp(P.Inv) + mm, m, 2 * mm, 0,
                          dp(P.SiP) + mm, m, 2 * mm, 0, 0.0, X + m, (int)m2, 2 * mm, 0, nR);
     // G1_j = SiM_{2j} X_{2j-1} (j >= 1; SiM_0 is zero), G2_j = SiP_{2j} X_{2j+1}
     if (!mixed) {
       if (nR > 1)
-        gemm_batched<double>(st, false, false, m, (int)m2, m, 1.0, dp(P.SiM) + 2 * mm, m, 2 * mm,
+        gemm_f64(h, false, false, m, (int)m2, m, 1.0, dp(P.SiM) + 2 * mm, m, 2 * mm,
                              0, X, (int)m2, 2 * mm, 0, 0.0, G1 + 2 * mm, (int)m2, 2 * mm, 0,
                              nR - 1);
-      gemm_batched<double>(st, false, false, m, (int)m2, m, 1.0, dp(P.SiP), m, 2 * mm, 0, X,
+      gemm_f64(h, false, false, m, (int)m2, m, 1.0, dp(P.SiP), m, 2 * mm, 0, X,
                            (int)m2, 2 * mm, 0, 0.0, G2, (int)m2, 2 * mm, 0, nR);
     } else {
       // Schur products on the tensor cores (split-BF16x3, float32 accumulation)
@@ -256,7 +257,7 @@ void rb_factor(Handle& h, RbSolver& S, int nblk, int m, const double* SiM, const
     }
     if (cyclic) {
       // block 0's left neighbour is the last odd block (index 2 nR - 1)
-      gemm_batched<double>(st, false, false, m, (int)m2, m, 1.0, dp(P.SiM), m, 0, 0,
+      gemm_f64(h, false, false, m, (int)m2, m, 1.0, dp(P.SiM), m, 0, 0,
                            X + 2 * (size_t)(nR - 1) * mm, (int)m2, 0, 0, 0.0, G1, (int)m2, 0, 0,
                            1);
     } else {
@@ -282,7 +283,7 @@ void rb_factor(Handle& h, RbSolver& S, int nblk, int m, const double* SiM, const
     l = nR;
   }
   S.fused = false;
-  if (m <= kRbFusedMax && !cyclic) build_fused_ops(st, S);
+  if (m <= kRbFusedMax && !cyclic) build_fused_ops(h, S);
 }
 
 void rb_solve(Handle& h, const RbSolver& S, double* B, int ldb, int c, bool tc) {
@@ -309,7 +310,7 @@ void rb_solve(Handle& h, const RbSolver& S, double* B, int ldb, int c, bool tc) 
   auto G = [&](double alpha, const double* A, long long sA, const double* V, long long sV,
                double beta, double* C, long long sC, int batch) {
     if (!tc) {
-      gemm_batched<double>(st, false, false, m, c, m, alpha, A, m, sA, 0, V, c, sV, 0, beta, C, c,
+      gemm_f64(h, false, false, m, c, m, alpha, A, m, sA, 0, V, c, sV, 0, beta, C, c,
                            sC, 0, batch);
       return;
     }
@@ -360,18 +361,18 @@ void rb_apply(Handle& h, const RbSolver& S, const double* X, int ldx, double* Y,
   const RbLevel& L0 = S.levels[0];
   const long long bx = (long long)m * ldx, by = (long long)m * ldy;
   // Y_i = T_i X_i + SiM_i X_{i-1} + SiP_i X_{i+1}  (SiM_0 = SiP_{n-1} = 0)
-  gemm_batched<double>(st, false, false, m, c, m, 1.0, dp(L0.T), m, mm, 0, X, ldx, bx, 0, 0.0, Y,
+  gemm_f64(h, false, false, m, c, m, 1.0, dp(L0.T), m, mm, 0, X, ldx, bx, 0, 0.0, Y,
                        ldy, by, 0, n);
   if (n > 1) {
-    gemm_batched<double>(st, false, false, m, c, m, 1.0, dp(L0.SiM) + mm, m, mm, 0, X, ldx, bx, 0,
+    gemm_f64(h, false, false, m, c, m, 1.0, dp(L0.SiM) + mm, m, mm, 0, X, ldx, bx, 0,
                          1.0, Y + by, ldy, by, 0, n - 1);
-    gemm_batched<double>(st, false, false, m, c, m, 1.0, dp(L0.SiP), m, mm, 0, X + bx, ldx, bx, 0,
+    gemm_f64(h, false, false, m, c, m, 1.0, dp(L0.SiP), m, mm, 0, X + bx, ldx, bx, 0,
                          1.0, Y, ldy, by, 0, n - 1);
   }
   if (S.cyclic) {   // wrap-around couplings of a periodic system
-    gemm_batched<double>(st, false, false, m, c, m, 1.0, dp(L0.SiM), m, 0, 0,
+    gemm_f64(h, false, false, m, c, m, 1.0, dp(L0.SiM), m, 0, 0,
                          X + (long long)(n - 1) * bx, ldx, 0, 0, 1.0, Y, ldy, 0, 0, 1);
-    gemm_batched<double>(st, false, false, m, c, m, 1.0, dp(L0.SiP) + (size_t)(n - 1) * mm, m, 0,
+    gemm_f64(h, false, false, m, c, m, 1.0, dp(L0.SiP) + (size_t)(n - 1) * mm, m, 0,
                          0, X, ldx, 0, 0, 1.0, Y + (long long)(n - 1) * by, ldy, 0, 0, 1);
   }
 }
@@ -467,7 +468,7 @@ void thomas_factor(Handle& h, RbSolver& S, int nblk, int m, const double* SiM, c
                      m, 0, m, 1);
     // B_i = T_i - A_i C_{i-1}  (omsdirectsolve.py:94), then LU
     double* Bi = dp(L.LU) + i * mm;
-    gemm_batched<double>(st, true, false, m, m, m, -1.0, At, m, 0, 0, dp(L.SiP) + (i - 1) * mm, m,
+    gemm_f64(h, true, false, m, m, m, -1.0, At, m, 0, 0, dp(L.SiP) + (i - 1) * mm, m,
                          0, 0, 1.0, Bi, m, 0, 0, 1);
     lu_factor(st, m, Bi, m, 0, ip(L.piv) + i * m, 0, 1, h.info.as<int>());
   }
@@ -496,7 +497,7 @@ void thomas_factor(Handle& h, RbSolver& S, int nblk, int m, const double* SiM, c
     copy_batched<double>(st, m, m, dp(L.Inv), m, (long long)mm, 0, dp(L.Bop), (int)w,
                          2 * (long long)mm, 0, nblk);
     if (nblk > 1)
-      gemm_batched<double>(st, false, false, m, m, m, -1.0, dp(L.Inv), m, (long long)mm, 0,
+      gemm_f64(h, false, false, m, m, m, -1.0, dp(L.Inv), m, (long long)mm, 0,
                            dp(L.SiP), m, (long long)mm, 0, 0.0, dp(L.Bop) + m, (int)w,
                            2 * (long long)mm, 0, nblk - 1);
     S.fused = true;
@@ -552,7 +553,7 @@ void thomas_solve(Handle& h, const RbSolver& S, double* B, int ldb, int c) {
   }
   // d_i -= A_i d_{i-1}  (omsdirectsolve.py:125-126)
   for (int i = 1; i < n; ++i)
-    gemm_batched<double>(st, false, false, m, c, m, -1.0, dp(L.T) + i * mm, m, 0, 0,
+    gemm_f64(h, false, false, m, c, m, -1.0, dp(L.T) + i * mm, m, 0, 0,
                          B + (size_t)(i - 1) * m * ldb, ldb, 0, 0, 1.0, B + (size_t)i * m * ldb,
                          ldb, 0, 0, 1);
   // x_n = B_n^{-1} d_n; x_i = B_i^{-1}(d_i - C_i x_{i+1})  (131-139)
@@ -560,13 +561,13 @@ void thomas_solve(Handle& h, const RbSolver& S, double* B, int ldb, int c) {
   double* z = h.ws.take<double>((size_t)m * c);
   auto block_solve = [&](int i) {
     double* Bi = B + (size_t)i * m * ldb;
-    gemm_batched<double>(st, false, false, m, c, m, 1.0, dp(L.Inv) + i * mm, m, 0, 0, Bi, ldb, 0,
+    gemm_f64(h, false, false, m, c, m, 1.0, dp(L.Inv) + i * mm, m, 0, 0, Bi, ldb, 0,
                          0, 0.0, z, c, 0, 0, 1);
     copy_batched<double>(st, m, c, z, c, 0, 0, Bi, ldb, 0, 0, 1);
   };
   block_solve(n - 1);
   for (int i = n - 2; i >= 0; --i) {
-    gemm_batched<double>(st, false, false, m, c, m, -1.0, dp(L.SiP) + i * mm, m, 0, 0,
+    gemm_f64(h, false, false, m, c, m, -1.0, dp(L.SiP) + i * mm, m, 0, 0,
                          B + (size_t)(i + 1) * m * ldb, ldb, 0, 0, 1.0, B + (size_t)i * m * ldb,
                          ldb, 0, 0, 1);
     block_solve(i);
