@@ -64,6 +64,7 @@ struct Handle {
   cudaStream_t stream = nullptr;
   Workspace ws;
   Workspace gemm_ws;   // residues of gemm_f64 (crt_gemm.cu), at most about 1 GB
+  Workspace lu_ws;     // permutations and triangles of lu_factor / lu_inverse
   HostStage upload, readback;
   DevBuf info;  // int[64] device status words
   std::string last_error;
@@ -80,6 +81,13 @@ void gemm_f64_tensor(Handle& h, bool ta, bool tb, int M, int N, int K, double al
                      const double* A, int lda, long long sA0, long long sA1, const double* B,
                      int ldb, long long sB0, long long sB1, double beta, double* C, int ldc,
                      long long sC0, long long sC1, int batch0, int batch1 = 1);
+// Batched LU with partial pivoting, in place (A_b n x n row-major), pivots
+// piv_b[i] = row swapped with row i (LAPACK getrf convention, 0-based).
+void lu_factor(Handle& h, int n, double* A, int lda, long long sA, int* piv, long long sP,
+               int batch, int* info);
+// Inv_b = A_b^{-1} from the LU factors.
+void lu_inverse(Handle& h, int n, const double* LU, int lda, long long sA, const int* piv,
+                long long sP, double* Inv, int ldi, long long sI, int batch);
 bool gemm_tensor_pays(int M, int N, int K, long long nb);
 
 // A step operator in the digit form of the tensor-core sweep (ozaki.cu):

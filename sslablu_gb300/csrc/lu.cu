@@ -1,0 +1,565 @@
+// LU with partial pivoting (LAPACK getrf's pivots and storage) and explicit
+// inverses, batched: the pivot blocks of the red-black and Thomas
+// eliminations (direct_solve/omsdirectsolve.py:89-94, 211, 333).
+//
+// Right-looking in two block sizes.  A panel of 32 columns is factored by one
+// thread-block cluster per matrix with the panel in registers; its row swaps
+// go to every other column at once; inside an outer block of 128 columns the
+// following panels are updated on the float64 units, and right of it the
+// trailing matrix takes one rank-128 update per outer block as a tensor-core
+// product (gemm_f64), which carries nearly all flops of a large block.
+#include <cooperative_groups.h>
+
+#include <algorithm>
+
+#include "hbs.cuh"
+
+namespace cg = cooperative_groups;
+
+namespace slu {
+namespace {
+
+constexpr int kPanel = 32;       // columns per panel
+constexpr int kOuter = 128;      // columns per outer block
+constexpr int kPanelRows = 512;  // rows (threads) per CTA of the panel kernel at most
+
+// Small matrices: one CTA each, in place.
+__device__ inline void argmax_abs_block(double v, int idx, double* sv, int* si, double& out_v,
+                                        int& out_i) {
+  // warp reduce
+  for (int o = 16; o > 0; o >>= 1) {
+    double ov = __shfl_down_sync(0xffffffffu, v, o);
+    int oi = __shfl_down_sync(0xffffffffu, idx, o);
+    if (ov > v || (ov == v && oi < idx)) { v = ov; idx = oi; }
+  }
+  int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (lane == 0) { sv[w] = v; si[w] = idx; }
+  __syncthreads();
+  if (w == 0) {
+    int nw = (blockDim.x + 31) >> 5;
+    v = lane < nw ? sv[lane] : -1.0;
+    idx = lane < nw ? si[lane] : 0x7fffffff;
+    for (int o = 16; o > 0; o >>= 1) {
+      double ov = __shfl_down_sync(0xffffffffu, v, o);
+      int oi = __shfl_down_sync(0xffffffffu, idx, o);
+      if (ov > v || (ov == v && oi < idx)) { v = ov; idx = oi; }
+    }
+    if (lane == 0) { sv[0] = v; si[0] = idx; }
+  }
+  __syncthreads();
+  out_v = sv[0];
+  out_i = si[0];
+  __syncthreads();
+}
+
+// Panels of more rows than a cluster holds: the panel in global memory, one
+// CTA per matrix.  src[i] = the row that ends at row i.
+__global__ void __launch_bounds__(1024)
+lu_panel_global_kernel(int n, int k0, int kb, double* __restrict__ A, int lda, long long sA,
+                       int* __restrict__ piv, long long sP, int* __restrict__ src, int* info) {
+  A += blockIdx.x * sA;
+  piv += blockIdx.x * sP;
+  src += (long long)blockIdx.x * n;
+  __shared__ double sv[32];
+  __shared__ int si[32];
+  int first_zero = 0;
+  const int k1 = k0 + kb;
+  for (int i = k0 + threadIdx.x; i < n; i += blockDim.x) src[i] = i;
+  __syncthreads();
+  for (int j = k0; j < k1; ++j) {
+    double best = -1.0;
+    int bi = j;
+    for (int i = j + threadIdx.x; i < n; i += blockDim.x) {
+      const double v = fabs(A[(long long)i * lda + j]);
+      if (v > best) { best = v; bi = i; }
+    }
+    double pv;
+    int p;
+    argmax_abs_block(best, bi, sv, si, pv, p);
+    if (threadIdx.x == 0) {
+      piv[j] = p;
+      const int t = src[j];
+      src[j] = src[p];
+      src[p] = t;
+    }
+    if (p != j) {
+      for (int c = k0 + threadIdx.x; c < k1; c += blockDim.x) {
+        const double t = A[(long long)j * lda + c];
+        A[(long long)j * lda + c] = A[(long long)p * lda + c];
+        A[(long long)p * lda + c] = t;
+      }
+    }
+    __syncthreads();
+    const double d = A[(long long)j * lda + j];
+    if (d == 0.0) {
+      if (!first_zero) first_zero = j + 1;
+      __syncthreads();
+      continue;
+    }
+    const double inv = 1.0 / d;
+    for (int i = j + 1 + threadIdx.x; i < n; i += blockDim.x) A[(long long)i * lda + j] *= inv;
+    __syncthreads();
+    const int w = k1 - j - 1;   // panel columns right of j
+    if (w > 0) {
+      const long long tot = (long long)(n - j - 1) * w;
+      for (long long e = threadIdx.x; e < tot; e += blockDim.x) {
+        const int i = j + 1 + (int)(e / w), c = j + 1 + (int)(e % w);
+        A[(long long)i * lda + c] -= A[(long long)i * lda + j] * A[(long long)j * lda + c];
+      }
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0 && first_zero && info) atomicCAS(info + blockIdx.x, 0, first_zero);
+}
+
+// Panel factorisation by one cluster per matrix.  Thread = row, the row's kb
+// panel entries in registers, so the rank-1 updates spread over the cluster's
+// SMs: one SM's float64 pipe (2 FMA per clock) would need ~4 us per column of
+// a 1024-row panel.  Rows are never moved: a thread carries the position its
+// row has after the swaps and stores it there at the end.
+// Per column: each CTA finds its largest entry (integer reductions of the
+// bit pattern), its owner puts 1/d and the row in shared memory, the
+// candidates' keys go to every CTA of the cluster, one cluster barrier, and
+// each warp reads the winner's row through distributed shared memory.  The
+// two buffers alternate, so one barrier per column suffices.
+// 1024 rows, 32 columns: 112 us; in one CTA, the panel in global memory, 422.
+struct PanelKey {
+  uint32_t hi, lo;   // |value| bits, hi + 1 (0: no candidate)
+  int pos;
+  int rank;
+};
+
+template <int KB>
+__global__ void __launch_bounds__(kPanelRows)
+lu_panel_kernel(int n, int k0, int kb, double* __restrict__ A, int lda, long long sA,
+                int* __restrict__ piv, long long sP, int* __restrict__ src, int* info) {
+  cg::cluster_group cl = cg::this_cluster();
+  const int cs = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const int b = blockIdx.x / cs;
+  A += b * sA;
+  piv += b * sP;
+  src += (long long)b * n;
+  __shared__ PanelKey s_key[2][8];        // per CTA of the cluster
+  __shared__ uint32_t s_hi[2][kPanelRows / 32], s_lo[2][kPanelRows / 32];
+  __shared__ int s_pos[2][kPanelRows / 32];
+  __shared__ double s_row[2][KB + 1];     // candidate row, 1/d last
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int R = n - k0, r = rank * blockDim.x + threadIdx.x;
+  const bool have = r < R;
+  double a[KB];
+  {
+    const double* row = A + (long long)(k0 + (have ? r : 0)) * lda + k0;
+#pragma unroll
+    for (int c = 0; c < KB; ++c) a[c] = (have && c < kb) ? row[c] : 0.0;
+  }
+  int pos = have ? r : -1;   // -1: no row
+  int first_zero = 0;
+#pragma unroll
+  for (int j = 0; j < KB; ++j) {
+    if (j < kb) {   // uniform
+      const int buf = j & 1;
+      const unsigned long long bits = (unsigned long long)__double_as_longlong(fabs(a[j]));
+      const bool cand = pos >= j && a[j] == a[j];
+      const uint32_t hi = cand ? (uint32_t)(bits >> 32) + 1 : 0, lo = (uint32_t)bits;
+      const uint32_t mh = __reduce_max_sync(0xffffffffu, hi);
+      const uint32_t ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0);
+      const int mp = __reduce_min_sync(0xffffffffu,
+                                       (cand && hi == mh && lo == ml) ? pos : 0x7fffffff);
+      if (lane == 0) {
+        s_hi[buf][warp] = mh;
+        s_lo[buf][warp] = ml;
+        s_pos[buf][warp] = mp;
+      }
+      __syncthreads();
+      const uint32_t wh = lane < nw ? s_hi[buf][lane] : 0;
+      const uint32_t bh = __reduce_max_sync(0xffffffffu, wh);
+      const uint32_t wl = lane < nw && wh == bh ? s_lo[buf][lane] : 0;
+      const uint32_t bl = __reduce_max_sync(0xffffffffu, wl);
+      const int bp = __reduce_min_sync(
+          0xffffffffu, (lane < nw && wh == bh && wl == bl) ? s_pos[buf][lane] : 0x7fffffff);
+      // no finite candidate in the column: row j itself (NaN column)
+      const int mine = bh ? bp : j;
+      if (pos == mine) {
+#pragma unroll
+        for (int c = j; c < KB; ++c) s_row[buf][c] = a[c];
+        s_row[buf][KB] = 1.0 / a[j];
+      }
+      if (threadIdx.x < cs) {
+        // a NaN column's row j is held by one CTA only
+        PanelKey* dst = cl.map_shared_rank(&s_key[buf][rank], threadIdx.x);
+        *dst = PanelKey{bh, bl, mine, rank};
+      }
+      cl.sync();
+      // the winner among the CTAs: largest entry, then the first position
+      PanelKey k = s_key[buf][0];
+      for (int q = 1; q < cs; ++q) {
+        const PanelKey o = s_key[buf][q];
+        if (o.hi > k.hi || (o.hi == k.hi && (o.lo > k.lo || (o.lo == k.lo && o.pos < k.pos))))
+          k = o;
+      }
+      const int p = k.pos;
+      // k.hi == 0: every remaining entry of the column is NaN; the row at
+      // position j is its own pivot, wherever it is held
+      const int owner = k.hi ? k.rank : -1;
+      double u = 0.0, inv = 0.0;
+      if (owner >= 0) {
+        const double* row = cl.map_shared_rank(&s_row[buf][0], owner);
+        u = row[lane < KB ? lane : 0];
+        inv = row[KB];
+      } else {
+        u = inv = __longlong_as_double(0x7ff8000000000000LL);
+      }
+      if (rank == 0 && threadIdx.x == 0) piv[k0 + j] = k0 + p;
+      const double d = __shfl_sync(0xffffffffu, u, j);
+      // position swap j <-> p
+      const bool retire = pos == p;
+      if (pos == j) pos = p;
+      if (retire) pos = j;
+      if (d == 0.0) {
+        if (!first_zero) first_zero = k0 + j + 1;
+      } else {
+        const bool live = pos > j;
+        const double l = live ? a[j] * inv : 0.0;
+        if (live) a[j] = l;
+#pragma unroll
+        for (int c = j + 1; c < KB; ++c) {
+          const double uc = __shfl_sync(0xffffffffu, u, c);
+          if (live) a[c] = fma(-l, uc, a[c]);
+        }
+      }
+    }
+  }
+  cl.sync();   // no CTA leaves while another may still read its shared memory
+  if (have) {
+    double* row = A + (long long)(k0 + pos) * lda + k0;
+#pragma unroll
+    for (int c = 0; c < KB; ++c)
+      if (c < kb) row[c] = a[c];
+    src[k0 + pos] = k0 + r;
+  }
+  if (rank == 0 && threadIdx.x == 0 && first_zero && info) atomicCAS(info + b, 0, first_zero);
+}
+
+// The panel's row swaps on every column outside it, from the net permutation
+// (src[i]: the row that ends at row i): the kb top rows and the up to kb
+// pivot rows below, one column per thread, all reads before the writes.  For
+// columns k1 .. ct the top rows are then solved with the panel's unit lower
+// triangle.  One warp per CTA: the solves of 32 columns keep one SM's
+// float64 pipe busy for 4 us.
+__global__ void __launch_bounds__(32)
+lu_swap_trsm_kernel(int n, int k0, int kb, int ct, double* __restrict__ A, int lda, long long sA,
+                    const int* __restrict__ piv, long long sP, const int* __restrict__ src) {
+  A += blockIdx.y * sA;
+  piv += blockIdx.y * sP;
+  src += (long long)blockIdx.y * n;
+  __shared__ double L11[kPanel][kPanel + 1];
+  const int lane = threadIdx.x, k1 = k0 + kb;
+  const int c = blockIdx.x * 32 + lane;
+  const bool solve = blockIdx.x * 32 < ct && blockIdx.x * 32 + 31 >= k1;   // uniform
+  if (solve)
+    for (int i = 0; i < kb; ++i) L11[i][lane] = lane < kb ? A[(long long)(k0 + i) * lda + k0 + lane] : 0.0;
+  __syncwarp();
+  // rows from (top, below) and to (below), one per lane
+  const int st = lane < kb ? src[k0 + lane] : -1;
+  const int pr = lane < kb ? piv[k0 + lane] : -1;
+  const int sb = pr >= k1 ? src[pr] : -1;
+  const bool on = c < n && (c < k0 || c >= k1);
+  double x[kPanel], y[kPanel];
+#pragma unroll
+  for (int i = 0; i < kPanel; ++i) {
+    const int rt = __shfl_sync(0xffffffffu, st, i), rb = __shfl_sync(0xffffffffu, sb, i);
+    x[i] = (on && rt >= 0) ? A[(long long)rt * lda + c] : 0.0;
+    y[i] = (on && rb >= 0) ? A[(long long)rb * lda + c] : 0.0;
+  }
+#pragma unroll
+  for (int i = 0; i < kPanel; ++i) {
+    const int to = __shfl_sync(0xffffffffu, pr, i);
+    if (on && to >= k1) A[(long long)to * lda + c] = y[i];
+  }
+  if (!on) return;
+  if (c >= k1 && c < ct) {
+#pragma unroll
+    for (int i = 1; i < kPanel; ++i) {
+      if (i < kb) {
+        double acc = x[i];
+#pragma unroll
+        for (int r = 0; r < i; ++r) acc = fma(-L11[i][r], x[r], acc);
+        x[i] = acc;
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < kPanel; ++i)
+    if (i < kb) A[(long long)(k0 + i) * lda + c] = x[i];
+}
+
+// U12 = L11^{-1} A12 for the nb rows of an outer block, columns c0 .. n-1:
+// eight columns per CTA (so a few hundred columns fill the GPU), the columns
+// in shared memory, 32 rows at a time: the diagonal tile by one warp per
+// column (lane = row, finished entries broadcast by shuffle), then the rows
+// below it as products.  Float64-pipe bound: nb^2 / 2 FMA per column.
+constexpr int kTrsmCols = 8;
+__global__ void __launch_bounds__(256)
+lu_block_trsm_kernel(int n, int k0, int nb, int c0, double* __restrict__ A, int lda,
+                     long long sA) {
+  A += blockIdx.y * sA;
+  __shared__ double X[kOuter][kTrsmCols + 1];
+  __shared__ double Lt[kPanel][kPanel + 1];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int cb = c0 + blockIdx.x * kTrsmCols, nc = min(kTrsmCols, n - cb);
+  for (int e = tid; e < nb * kTrsmCols; e += 256) {
+    const int i = e / kTrsmCols, c = e % kTrsmCols;
+    X[i][c] = c < nc ? A[(long long)(k0 + i) * lda + cb + c] : 0.0;
+  }
+  for (int t0 = 0; t0 < nb; t0 += kPanel) {
+    const int tn = min(kPanel, nb - t0);
+    __syncthreads();
+    for (int e = tid; e < tn * tn; e += 256) {
+      const int i = e / tn, j = e - i * tn;
+      Lt[i][j] = A[(long long)(k0 + t0 + i) * lda + k0 + t0 + j];
+    }
+    __syncthreads();
+    {
+      double x = lane < tn ? X[t0 + lane][warp] : 0.0;
+      for (int i = 0; i < tn; ++i) {
+        const double xi = __shfl_sync(0xffffffffu, x, i);
+        if (lane > i && lane < tn) x = fma(-Lt[lane][i], xi, x);
+      }
+      if (lane < tn) X[t0 + lane][warp] = x;
+    }
+    __syncthreads();
+    // rows below: thread = (row, column)
+    const int c = tid & 7;
+    for (int i = t0 + tn + (tid >> 3); i < nb; i += 32) {
+      const double* l = A + (long long)(k0 + i) * lda + k0 + t0;
+      double acc = X[i][c];
+      if (tn == kPanel) {
+#pragma unroll
+        for (int j = 0; j < kPanel; ++j) acc = fma(-__ldg(l + j), X[t0 + j][c], acc);
+      } else {
+        for (int j = 0; j < tn; ++j) acc = fma(-__ldg(l + j), X[t0 + j][c], acc);
+      }
+      X[i][c] = acc;
+    }
+  }
+  __syncthreads();
+  for (int e = tid; e < nb * kTrsmCols; e += 256) {
+    const int i = e / kTrsmCols, c = e % kTrsmCols;
+    if (c < nc) A[(long long)(k0 + i) * lda + cb + c] = X[i][c];
+  }
+}
+
+void launch_panel(cudaStream_t st, int n, int k0, int kb, double* A, int lda, long long sA,
+                  int* piv, long long sP, int* src, int batch, int* info) {
+  const int R = n - k0;
+  // about 64 rows per CTA, up to the portable cluster size of 8
+  int cs = 1;
+  while (cs < 8 && R > 64 * cs) cs *= 2;
+  const int threads = ((R + cs - 1) / cs + 31) / 32 * 32;
+  if (threads > kPanelRows) {
+    lu_panel_global_kernel<<<batch, 1024, 0, st>>>(n, k0, kb, A, lda, sA, piv, sP, src, info);
+    check_launch("lu_panel_global_kernel");
+    return;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(batch * cs));
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)cs;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  SLU_CHECK_CUDA(cudaLaunchKernelEx(&cfg, lu_panel_kernel<kPanel>, n, k0, kb, A, lda, sA, piv, sP,
+                                    src, info));
+  check_launch("lu_panel_kernel");
+}
+
+// ---------------------------------------------------------------- inverses
+// Lp (np x np) = L with identity padding, Ut = U^T likewise (both lower
+// triangular, zeros above); perm: the net row permutation of the pivots
+// (P A = L U, (P A)_i = A_perm[i]), by one extra CTA per matrix.
+__global__ void __launch_bounds__(256)
+tri_pack_kernel(int n, int np, const double* __restrict__ LU, int lda, long long sA,
+                const int* __restrict__ piv, long long sP, double* __restrict__ T,
+                int* __restrict__ perm) {
+  const int b = blockIdx.z, tid = threadIdx.x;
+  LU += b * sA;
+  extern __shared__ int s_perm[];
+  if (blockIdx.y == gridDim.y - 1) {
+    if (blockIdx.x != 0) return;
+    piv += b * sP;
+    int* pv = s_perm + n;
+    for (int i = tid; i < n; i += 256) {
+      s_perm[i] = i;
+      pv[i] = piv[i];
+    }
+    __syncthreads();
+    if (tid == 0)
+      for (int i = 0; i < n; ++i) {
+        const int p = pv[i], t = s_perm[i];
+        s_perm[i] = s_perm[p];
+        s_perm[p] = t;
+      }
+    __syncthreads();
+    for (int i = tid; i < n; i += 256) perm[(long long)b * n + i] = s_perm[i];
+    return;
+  }
+  const long long nn = (long long)np * np;
+  double* Lp = T + 2 * b * nn;
+  double* Ut = Lp + nn;
+  __shared__ double tile[32][33];
+  const int i0 = blockIdx.y * 32, j0 = blockIdx.x * 32, tx = tid & 31, ty = tid >> 5;
+  for (int r = ty; r < 32; r += 8) {
+    const int i = i0 + r, j = j0 + tx;
+    double v = 0.0;
+    if (i < n && j < n) v = LU[(long long)i * lda + j];
+    tile[r][tx] = v;
+    if (i < np && j < np)
+      Lp[(long long)i * np + j] = i == j ? 1.0 : (i > j && i < n ? v : 0.0);
+  }
+  __syncthreads();
+  for (int r = ty; r < 32; r += 8) {
+    const int i = j0 + r, j = i0 + tx;   // Ut[i][j] = U[j][i]
+    if (i < np && j < np)
+      Ut[(long long)i * np + j] =
+          i < n ? (j <= i ? tile[tx][r] : 0.0) : (i == j ? 1.0 : 0.0);
+  }
+}
+
+// In-place inverses of the w x w (w <= 32) diagonal blocks of lower triangular
+// matrices: one warp per block, lane = column, forward substitution with the
+// column in registers.
+__global__ void __launch_bounds__(32)
+tri_base_kernel(int np, int w, double* __restrict__ T) {
+  double* D = T + (long long)blockIdx.y * np * np + (long long)blockIdx.x * w * (np + 1);
+  __shared__ double L[32][33];
+  const int lane = threadIdx.x;
+  for (int i = 0; i < w; ++i)
+    if (lane < w) L[i][lane] = D[(long long)i * np + lane];
+  __syncwarp();
+  const double rd = lane < w ? 1.0 / L[lane][lane] : 0.0;
+  double x[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) {
+    const double ri = __shfl_sync(0xffffffffu, rd, i);
+    double acc = i == lane ? 1.0 : 0.0;
+    if (i < w) {
+#pragma unroll
+      for (int j = 0; j < i; ++j) acc = fma(-L[i][j], x[j], acc);
+    }
+    x[i] = acc * ri;
+  }
+  if (lane < w)
+    for (int i = 0; i < w; ++i) {
+      double v = 0.0;
+#pragma unroll
+      for (int q = 0; q < 32; ++q)
+        if (q == i) v = x[q];
+      D[(long long)i * np + lane] = v;
+    }
+}
+
+// Y (np x n) = columns of X permuted: Y[:, perm[i]] = X[:, i]
+__global__ void __launch_bounds__(256)
+permute_cols_kernel(int n, int np, const double* __restrict__ X, long long sX,
+                    const int* __restrict__ perm, double* __restrict__ Y, long long sY) {
+  X += blockIdx.z * sX;
+  Y += blockIdx.z * sY;
+  perm += (long long)blockIdx.z * n;
+  const int r = blockIdx.y;
+  for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += 256 * gridDim.x)
+    Y[(long long)r * n + perm[i]] = X[(long long)r * np + i];
+}
+
+}  // namespace
+
+void lu_factor(Handle& h, int n, double* A, int lda, long long sA, int* piv, long long sP,
+               int batch, int* info) {
+  if (n <= 0 || batch <= 0) return;
+  SLU_REQUIRE(batch <= 65535, "LU batch too large");
+  cudaStream_t st = h.stream;
+  h.lu_ws.reserve(sizeof(int) * (size_t)n * batch + 256, st);
+  int* src = h.lu_ws.take<int>((size_t)n * batch);
+  for (int K0 = 0; K0 < n; K0 += kOuter) {
+    const int K1 = std::min(K0 + kOuter, n);
+    for (int k0 = K0; k0 < K1; k0 += kPanel) {
+      const int kb = std::min(kPanel, K1 - k0), k1 = k0 + kb;
+      launch_panel(st, n, k0, kb, A, lda, sA, piv, sP, src, batch, info);
+      if (n > kb) {
+        lu_swap_trsm_kernel<<<dim3((n + 31) / 32, batch), 32, 0, st>>>(n, k0, kb, K1, A, lda, sA,
+                                                                       piv, sP, src);
+        check_launch("lu_swap_trsm_kernel");
+      }
+      if (k1 < K1)
+        gemm_batched<double>(st, false, false, n - k1, K1 - k1, kb, -1.0,
+                             A + (long long)k1 * lda + k0, lda, sA, 0,
+                             A + (long long)k0 * lda + k1, lda, sA, 0, 1.0,
+                             A + (long long)k1 * lda + k1, lda, sA, 0, batch);
+    }
+    if (K1 < n) {
+      lu_block_trsm_kernel<<<dim3((n - K1 + kTrsmCols - 1) / kTrsmCols, batch), 256, 0, st>>>(
+          n, K0, K1 - K0, K1, A, lda, sA);
+      check_launch("lu_block_trsm_kernel");
+      gemm_f64(h, false, false, n - K1, n - K1, K1 - K0, -1.0, A + (long long)K1 * lda + K0, lda,
+               sA, 0, A + (long long)K0 * lda + K1, lda, sA, 0, 1.0, A + (long long)K1 * lda + K1,
+               lda, sA, 0, batch);
+    }
+  }
+}
+
+// Inv = U^{-1} L^{-1} P.  L and U^T are inverted together by doubling: blocks
+// of at most 32 rows by substitution, then for pairs of inverted neighbours
+// the off-diagonal block becomes -C^{-1} (B A^{-1}), two batched products per
+// level over every pair of both triangles of all matrices; the last product
+// joins them.  ~log2(n / 32) levels of wide products instead of n / 32
+// dependent substitution steps (against the identity, by 32-row tiles, eight
+// 1024 blocks took 18 ms; the inverses of a whole 8 x 1024 red-black
+// factorisation, 15 blocks, now take about 3 ms).
+void lu_inverse(Handle& h, int n, const double* LU, int lda, long long sA, const int* piv,
+                long long sP, double* Inv, int ldi, long long sI, int batch) {
+  if (n <= 0 || batch <= 0) return;
+  cudaStream_t st = h.stream;
+  int q = 0;
+  while (((n + (1 << q) - 1) >> q) > 32) ++q;
+  const int w = (n + (1 << q) - 1) >> q, np = w << q;
+  const size_t nn = (size_t)np * np;
+  const size_t per = 8 * (3 * nn + (size_t)np * n) + sizeof(int) * (size_t)n + 4 * 256;
+  const int fit = (int)std::max<size_t>(1, std::min<size_t>((size_t(1) << 30) / per, 65535 >> (q + 1)));
+  for (int b0 = 0; b0 < batch; b0 += fit) {
+    const int nb = std::min(fit, batch - b0);
+    h.lu_ws.reserve(per * nb + 4096, st);
+    double* T = h.lu_ws.take<double>(2 * nn * nb);
+    double* W = h.lu_ws.take<double>(nn * nb);
+    double* LP = h.lu_ws.take<double>((size_t)np * n * nb);
+    int* perm = h.lu_ws.take<int>((size_t)n * nb);
+    const size_t sm = 2 * sizeof(int) * (size_t)n;
+    SLU_REQUIRE(sm <= 200 * 1024, "LU inverse: block too large");
+    ensure_smem(reinterpret_cast<const void*>(tri_pack_kernel), sm);
+    const int tl = (np + 31) / 32;
+    tri_pack_kernel<<<dim3(tl, tl + 1, nb), 256, sm, st>>>(n, np, LU + b0 * sA, lda, sA,
+                                                           piv + b0 * sP, sP, T, perm);
+    check_launch("tri_pack_kernel");
+    tri_base_kernel<<<dim3(1 << q, 2 * nb), 32, 0, st>>>(np, w, T);
+    check_launch("tri_base_kernel");
+    for (int s = w; s < np; s *= 2) {
+      const int pairs = np / (2 * s);
+      const long long sd = 2LL * s * (np + 1), ss = (long long)s * s;
+      double* B = T + (long long)s * np;           // below the first block of a pair
+      double* C = T + (long long)s * (np + 1);     // the second block
+      gemm_f64(h, false, false, s, s, s, 1.0, B, np, sd, (long long)nn, T, np, sd, (long long)nn,
+               0.0, W, s, ss, ss * pairs, pairs, 2 * nb);
+      gemm_f64(h, false, false, s, s, s, -1.0, C, np, sd, (long long)nn, W, s, ss, ss * pairs, 0.0,
+               B, np, sd, (long long)nn, pairs, 2 * nb);
+    }
+    permute_cols_kernel<<<dim3(std::min((n + 255) / 256, 8), np, nb), 256, 0, st>>>(
+        n, np, T, 2 * (long long)nn, perm, LP, (long long)np * n);
+    check_launch("permute_cols_kernel");
+    gemm_f64(h, true, false, n, n, np, 1.0, T + nn, np, 2 * (long long)nn, 0, LP, n,
+             (long long)np * n, 0, 0.0, Inv + b0 * sI, ldi, sI, 0, nb);
+  }
+}
+
+}  // namespace slu

@@ -158,10 +158,6 @@ void trsm_upper(cudaStream_t st, bool trans, int n, const T* R, long long rRs, l
                 long long sR, T* X, long long xRs, long long xCs, long long sX, int nrhs,
                 int batch);
 
-// Batched LU with partial pivoting, in place (A_b n x n row-major), pivots
-// piv_b[i] = row swapped with row i (LAPACK getrf convention, 0-based).
-void lu_factor(cudaStream_t st, int n, double* A, int lda, long long sA, int* piv,
-               long long sP, int batch, int* info);
 // X <- A^{-1} X (trans=false) or A^{-T} X using the LU factors; X_b n x nrhs row-major.
 template <typename T>
 void lu_solve(cudaStream_t st, bool trans, int n, const T* LU, int lda, long long sA,

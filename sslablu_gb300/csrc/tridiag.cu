@@ -34,16 +34,25 @@ namespace {
 inline double* dp(const DevBuf& b) { return b.as<double>(); }
 inline int* ip(const DevBuf& b) { return b.as<int>(); }
 
-// Inv_b = T_b^{-1} from the LU factors of nS blocks (m x m each): a batched
-// LU solve against the identity.
-void make_inverses(cudaStream_t st, int m, const DevBuf& LU, const DevBuf& piv, int nS,
-                   DevBuf& Inv) {
-  const size_t mm = (size_t)m * m;
-  Inv.alloc(8 * nS * mm, st);
-  identity_cols(st, m, 0, m, dp(Inv), (long long)mm, nS);
-  lu_solve<double>(st, false, m, dp(LU), m, (long long)mm, ip(piv), m, dp(Inv), m,
-                   (long long)mm, m, nS);
+// Products of the factorisations (depth m).  From m = 64 on they run as
+// residue products whatever their size: their error is a tenth of the float64
+// kernel's, and the explicit inverses and composed solve operators inherit it
+// (on 12 copies of a near-resonant 4 x 64 system perturbed by 1e-15, median
+// solution residual 8.7e-9 with float64 products and LU-solved inverses, at
+// most 3e-9 in the same test with exact products); at m = 64 both take about
+// 25 us.
+constexpr int kExactMin = 64;
+void gemm_factor(Handle& h, int M, int N, int m, double alpha, const double* A, int lda,
+                 long long sA, const double* B, int ldb, long long sB, double beta, double* C,
+                 int ldc, long long sC, int batch) {
+  if (m >= kExactMin)
+    gemm_f64_tensor(h, false, false, M, N, m, alpha, A, lda, sA, 0, B, ldb, sB, 0, beta, C, ldc, sC,
+                    0, batch);
+  else
+    gemm_batched<double>(h.stream, false, false, M, N, m, alpha, A, lda, sA, 0, B, ldb, sB, 0, beta,
+                         C, ldc, sC, 0, batch);
 }
+
 // Fop_j <- [I | 0 | 0] (nR blocks of m x 3m)
 __global__ void rb_fop_init_kernel(int nR, int m, double* __restrict__ F) {
   const long long w = 3LL * m, total = (long long)nR * m * w;
@@ -84,17 +93,16 @@ void build_fused_ops(Handle& h, RbSolver& S) {
     check_launch("rb_fop_init_kernel");
     // -SiM_{2j} Inv_{2j-1} (j >= 1), -SiP_{2j} Inv_{2j+1}
     if (nR > 1)
-      gemm_f64(h, false, false, m, m, m, -1.0, dp(P.SiM) + 2 * mm, m, 2 * mm, 0,
-                           dp(P.Inv) + mm, m, 2 * mm, 0, 0.0, F + 3 * mm + m, (int)w, 3 * mm, 0,
-                           nR - 1);
-    gemm_f64(h, false, false, m, m, m, -1.0, dp(P.SiP), m, 2 * mm, 0, dp(P.Inv) + mm,
-                         m, 2 * mm, 0, 0.0, F + 2 * m, (int)w, 3 * mm, 0, nR);
+      gemm_factor(h, m, m, m, -1.0, dp(P.SiM) + 2 * mm, m, 2 * mm, dp(P.Inv) + mm, m, 2 * mm, 0.0,
+                  F + 3 * mm + m, (int)w, 3 * mm, nR - 1);
+    gemm_factor(h, m, m, m, -1.0, dp(P.SiP), m, 2 * mm, dp(P.Inv) + mm, m, 2 * mm, 0.0, F + 2 * m,
+                (int)w, 3 * mm, nR);
     // [Inv_o | -Inv_o SiM_o | -Inv_o SiP_o]
     copy_batched<double>(st, m, m, dp(P.Inv) + mm, m, 2 * mm, 0, Bo, (int)w, 3 * mm, 0, nR);
-    gemm_f64(h, false, false, m, m, m, -1.0, dp(P.Inv) + mm, m, 2 * mm, 0,
-                         dp(P.SiM) + mm, m, 2 * mm, 0, 0.0, Bo + m, (int)w, 3 * mm, 0, nR);
-    gemm_f64(h, false, false, m, m, m, -1.0, dp(P.Inv) + mm, m, 2 * mm, 0,
-                         dp(P.SiP) + mm, m, 2 * mm, 0, 0.0, Bo + 2 * m, (int)w, 3 * mm, 0, nR);
+    gemm_factor(h, m, m, m, -1.0, dp(P.Inv) + mm, m, 2 * mm, dp(P.SiM) + mm, m, 2 * mm, 0.0,
+                Bo + m, (int)w, 3 * mm, nR);
+    gemm_factor(h, m, m, m, -1.0, dp(P.Inv) + mm, m, 2 * mm, dp(P.SiP) + mm, m, 2 * mm, 0.0,
+                Bo + 2 * m, (int)w, 3 * mm, nR);
   }
   S.fused = true;
 }
@@ -211,8 +219,9 @@ void rb_factor(Handle& h, RbSolver& S, int nblk, int m, const double* SiM, const
     }
     SLU_CHECK_CUDA(cudaMemcpyAsync(dp(L0.T), T, 8 * nblk * mm, cudaMemcpyDeviceToDevice, st));
     SLU_CHECK_CUDA(cudaMemcpyAsync(dp(L0.LU), T, 8 * nblk * mm, cudaMemcpyDeviceToDevice, st));
-    lu_factor(st, m, dp(L0.LU), m, mm, ip(L0.piv), m, nblk, h.info.as<int>());
-    make_inverses(st, m, L0.LU, L0.piv, nblk, L0.Inv);
+    lu_factor(h, m, dp(L0.LU), m, mm, ip(L0.piv), m, nblk, h.info.as<int>());
+    L0.Inv.alloc(8 * nblk * mm, st);
+    lu_inverse(h, m, dp(L0.LU), m, mm, ip(L0.piv), m, dp(L0.Inv), m, mm, nblk);
   }
   h.ws.reserve(8 * ((size_t)nblk / 2 * 2 * mm * 3) + 8 * 256, st);
   double* X = h.ws.take<double>(std::max<size_t>(1, (size_t)nblk / 2) * 2 * mm);  // per odd block: m x 2m
@@ -233,18 +242,17 @@ void rb_factor(Handle& h, RbSolver& S, int nblk, int m, const double* SiM, const
     // X_o = T_o^{-1} [SiM_o | SiP_o] for odd o, as products with the
     // inverses formed when the level was factored (GEMMs over all SMs
     // instead of substitutions)
-    gemm_f64(h, false, false, m, m, m, 1.0, dp(P.Inv) + mm, m, 2 * mm, 0,
-                         dp(P.SiM) + mm, m, 2 * mm, 0, 0.0, X, (int)m2, 2 * mm, 0, nR);
-    gemm_f64(h, false, false, m, m, m, 1.0, dp(P.Inv) + mm, m, 2 * mm, 0,
-                         dp(P.SiP) + mm, m, 2 * mm, 0, 0.0, X + m, (int)m2, 2 * mm, 0, nR);
+    gemm_factor(h, m, m, m, 1.0, dp(P.Inv) + mm, m, 2 * mm, dp(P.SiM) + mm, m, 2 * mm, 0.0, X,
+                (int)m2, 2 * mm, nR);
+    gemm_factor(h, m, m, m, 1.0, dp(P.Inv) + mm, m, 2 * mm, dp(P.SiP) + mm, m, 2 * mm, 0.0, X + m,
+                (int)m2, 2 * mm, nR);
     // G1_j = SiM_{2j} X_{2j-1} (j >= 1; SiM_0 is zero), G2_j = SiP_{2j} X_{2j+1}
     if (!mixed) {
       if (nR > 1)
-        gemm_f64(h, false, false, m, (int)m2, m, 1.0, dp(P.SiM) + 2 * mm, m, 2 * mm,
-                             0, X, (int)m2, 2 * mm, 0, 0.0, G1 + 2 * mm, (int)m2, 2 * mm, 0,
-                             nR - 1);
-      gemm_f64(h, false, false, m, (int)m2, m, 1.0, dp(P.SiP), m, 2 * mm, 0, X,
-                           (int)m2, 2 * mm, 0, 0.0, G2, (int)m2, 2 * mm, 0, nR);
+        gemm_factor(h, m, (int)m2, m, 1.0, dp(P.SiM) + 2 * mm, m, 2 * mm, X, (int)m2, 2 * mm, 0.0,
+                    G1 + 2 * mm, (int)m2, 2 * mm, nR - 1);
+      gemm_factor(h, m, (int)m2, m, 1.0, dp(P.SiP), m, 2 * mm, X, (int)m2, 2 * mm, 0.0, G2,
+                  (int)m2, 2 * mm, nR);
     } else {
       // Schur products on the tensor cores (split-BF16x3, float32 accumulation)
       unsigned int* err = reinterpret_cast<unsigned int*>(h.info.as<int>()) + 1;
@@ -257,9 +265,8 @@ void rb_factor(Handle& h, RbSolver& S, int nblk, int m, const double* SiM, const
     }
     if (cyclic) {
       // block 0's left neighbour is the last odd block (index 2 nR - 1)
-      gemm_f64(h, false, false, m, (int)m2, m, 1.0, dp(P.SiM), m, 0, 0,
-                           X + 2 * (size_t)(nR - 1) * mm, (int)m2, 0, 0, 0.0, G1, (int)m2, 0, 0,
-                           1);
+      gemm_factor(h, m, (int)m2, m, 1.0, dp(P.SiM), m, 0, X + 2 * (size_t)(nR - 1) * mm, (int)m2,
+                  0, 0.0, G1, (int)m2, 0, 1);
     } else {
       SLU_CHECK_CUDA(cudaMemsetAsync(G1, 0, 8 * 2 * mm, st));
     }
@@ -277,8 +284,9 @@ void rb_factor(Handle& h, RbSolver& S, int nblk, int m, const double* SiM, const
       add_batched<double>(st, m, m, 1.0, dp(N.SiP), m, 0, 0, dp(N.T), m, 0, 0, 1);
     }
     SLU_CHECK_CUDA(cudaMemcpyAsync(dp(N.LU), dp(N.T), 8 * nR * mm, cudaMemcpyDeviceToDevice, st));
-    lu_factor(st, m, dp(N.LU), m, mm, ip(N.piv), m, nR, h.info.as<int>());
-    make_inverses(st, m, N.LU, N.piv, nR, N.Inv);
+    lu_factor(h, m, dp(N.LU), m, mm, ip(N.piv), m, nR, h.info.as<int>());
+    N.Inv.alloc(8 * nR * mm, st);
+    lu_inverse(h, m, dp(N.LU), m, mm, ip(N.piv), m, dp(N.Inv), m, mm, nR);
     S.levels.push_back(std::move(N));
     l = nR;
   }
@@ -453,32 +461,30 @@ void thomas_factor(Handle& h, RbSolver& S, int nblk, int m, const double* SiM, c
   RbLevel& L = S.levels.back();
   const size_t mm = (size_t)m * m;
   L.nS = nblk;
-  L.SiM.alloc(8 * nblk * mm, st);  // holds A_i^T = (SiM_i B_{i-1}^{-1})^T (T: A_i)
-  L.SiP.alloc(8 * nblk * mm, st);  // C_i
+  L.SiP.alloc(8 * nblk * mm, st);  // C_i (T: A_i)
   L.LU.alloc(8 * nblk * mm, st);   // LU(B_i)
   L.piv.alloc(4 * (size_t)nblk * m, st);
+  L.T.alloc(8 * nblk * mm, st);
+  L.Inv.alloc(8 * nblk * mm, st);
   SLU_CHECK_CUDA(cudaMemcpyAsync(dp(L.SiP), SiP, 8 * nblk * mm, cudaMemcpyDeviceToDevice, st));
   SLU_CHECK_CUDA(cudaMemcpyAsync(dp(L.LU), T, 8 * nblk * mm, cudaMemcpyDeviceToDevice, st));
-  lu_factor(st, m, dp(L.LU), m, mm, ip(L.piv), m, 1, h.info.as<int>());
-  for (int i = 1; i < nblk; ++i) {
-    double* At = dp(L.SiM) + i * mm;
-    // A_i = SiM_i B_{i-1}^{-1}  ->  A_i^T = B_{i-1}^{-T} SiM_i^T  (omsdirectsolve.py:89-91)
-    transpose_batched(st, m, m, SiM + i * mm, m, 0, 0, At, m, 0, 0, 1);
-    lu_solve<double>(st, true, m, dp(L.LU) + (i - 1) * mm, m, 0, ip(L.piv) + (i - 1) * m, 0, At,
-                     m, 0, m, 1);
-    // B_i = T_i - A_i C_{i-1}  (omsdirectsolve.py:94), then LU
-    double* Bi = dp(L.LU) + i * mm;
-    gemm_f64(h, true, false, m, m, m, -1.0, At, m, 0, 0, dp(L.SiP) + (i - 1) * mm, m,
-                         0, 0, 1.0, Bi, m, 0, 0, 1);
-    lu_factor(st, m, Bi, m, 0, ip(L.piv) + i * m, 0, 1, h.info.as<int>());
-  }
-  make_inverses(st, m, L.LU, L.piv, nblk, L.Inv);
-  // A_i itself (the solve multiplies by it; block 0 is unused)
-  L.T.alloc(8 * nblk * mm, st);
+  // block 0 of the multipliers is unused
   SLU_CHECK_CUDA(cudaMemsetAsync(dp(L.T), 0, 8 * mm, st));
-  if (nblk > 1)
-    transpose_batched(st, m, m, dp(L.SiM) + mm, m, (long long)mm, 0, dp(L.T) + mm, m,
-                      (long long)mm, 0, nblk - 1);
+  for (int i = 0; i < nblk; ++i) {
+    double* Bi = dp(L.LU) + i * mm;
+    if (i > 0) {
+      // A_i = SiM_i B_{i-1}^{-1}, B_i = T_i - A_i C_{i-1}  (omsdirectsolve.py:89-94),
+      // with the inverse the solve phase applies anyway: one product instead
+      // of a transposed LU solve with m right-hand sides (0.8 ms of the
+      // 2.7 ms per 256-point block)
+      gemm_factor(h, m, m, m, 1.0, SiM + i * mm, m, 0, dp(L.Inv) + (i - 1) * mm, m, 0, 0.0,
+                  dp(L.T) + i * mm, m, 0, 1);
+      gemm_factor(h, m, m, m, -1.0, dp(L.T) + i * mm, m, 0, dp(L.SiP) + (i - 1) * mm, m, 0, 1.0,
+                  Bi, m, 0, 1);
+    }
+    lu_factor(h, m, Bi, m, 0, ip(L.piv) + i * m, 0, 1, h.info.as<int>());
+    lu_inverse(h, m, Bi, m, 0, ip(L.piv) + i * m, 0, dp(L.Inv) + i * mm, m, 0, 1);
+  }
   S.fused = false;
   if (m <= kRbFusedMax) {
     // fused solve operators (m x 2m per block): Fop_i = [I | -A_i] (i >= 1),
@@ -497,9 +503,8 @@ void thomas_factor(Handle& h, RbSolver& S, int nblk, int m, const double* SiM, c
     copy_batched<double>(st, m, m, dp(L.Inv), m, (long long)mm, 0, dp(L.Bop), (int)w,
                          2 * (long long)mm, 0, nblk);
     if (nblk > 1)
-      gemm_f64(h, false, false, m, m, m, -1.0, dp(L.Inv), m, (long long)mm, 0,
-                           dp(L.SiP), m, (long long)mm, 0, 0.0, dp(L.Bop) + m, (int)w,
-                           2 * (long long)mm, 0, nblk - 1);
+      gemm_factor(h, m, m, m, -1.0, dp(L.Inv), m, (long long)mm, dp(L.SiP), m, (long long)mm, 0.0,
+                  dp(L.Bop) + m, (int)w, 2 * (long long)mm, nblk - 1);
     S.fused = true;
   }
 }
