@@ -133,26 +133,92 @@ apply_q_kernel(bool transpose, int m, int k, const double* __restrict__ V, int l
 
 // ---------------------------------------------------------------- Jacobi SVD
 // One-sided (Hestenes) Jacobi on the columns of A (m x n), round-robin pair
-// ordering.  Each column pair belongs to JAC_LANES consecutive lanes of a
-// warp; a lane owns rows part, part + JAC_LANES, ...  The lanes form the
-// three inner products of the pair over their rows (two partial sums each,
-// then a shuffle butterfly -- the pair's sums are combined the same way on
-// every lane), compute the rotation redundantly and rotate their own rows,
-// so no shared-memory traffic beyond the columns themselves and one block
-// barrier per round.  The rotation is orthogonal in float64 whatever its
-// angle, so the angle is computed in float32 from the float64 quotient
-// zeta = (beta - alpha) / (2 gamma) and the float64 (c, s) are renormalised
-// to c^2 + s^2 = 1 to float64 rounding; an angle good to ~1e-7 still cuts
-// gamma by that factor per rotation, and the sweep test (|gamma| <= m eps
-// sqrt(alpha beta) for every pair) is unchanged.  Small angles
-// (|zeta| > 1e7, where zeta^2 would leave float32 range) take t = 1/(2 zeta)
-// in float64 instead.  Columns live in shared
-// memory with an odd leading dimension.  At convergence the columns are
-// sigma_j u_j; the r largest are normalised and written as U (m x r).
+// ordering.  A column pair belongs to LANES consecutive lanes of a warp; a
+// lane owns rows part, part + LANES, ... of both columns, in registers from
+// the inner product to the rotation (RPL rows; RPL = 0: more rows than
+// registers, read twice).
+//
+// Bound by the float64 pipe: one warp instruction per 64 clocks and SM
+// sub-partition, so what counts is float64 instructions per round, and
+// everything that need not be float64 runs on the integer and float32 units:
+//   * the squared column norms are kept in shared memory and updated by the
+//     rotation (exact for whatever angle is taken; recomputed each sweep, and
+//     at once where a norm falls by cancellation), so a round forms one inner
+//     product instead of three;
+//   * the convergence test and the rotation angle come from the bit patterns
+//     of the norms and the inner product (exponents as integers, mantissas as
+//     float32).  An angle good to 1e-6 still cuts the inner product by that
+//     factor per rotation, and the test (|gamma| <= m eps sqrt(alpha beta)
+//     for every pair) needs no more;
+//   * the rotation is applied as three shears (x -= tau y, y += s x,
+//     x -= tau y; tau = tan(theta / 2), s = 2 tau / (1 + tau^2) to float64
+//     rounding), three FMAs per row instead of two and two products; it is
+//     orthogonal to float64 rounding whatever the angle.
+// 64 x 64: 82 float64 instructions per round and warp; with float64 angles
+// and three inner products 160 (128 problems: 10.99 -> 5.76 ms).
+// Columns live in shared memory with an odd leading dimension.  At
+// convergence the columns are sigma_j u_j; the r largest are normalised and
+// written as U (m x r).
 constexpr int JAC_MAX_SWEEPS = 40;
-constexpr int JAC_LANES = 4;
 
-__global__ void __launch_bounds__(1024)
+__device__ __forceinline__ uint32_t hi32(double v) { return (uint32_t)__double2hiint(v); }
+// mantissa in [1, 2) as a float32 (the leading 23 bits)
+__device__ __forceinline__ float mantissa(double v) {
+  return __uint_as_float(0x3f800000u | (hi32(v) & 0xfffffu) << 3 |
+                         (uint32_t)__double2loint(v) >> 29);
+}
+__device__ __forceinline__ int expo(double v) { return (int)(hi32(v) >> 20 & 0x7ff); }
+__device__ __forceinline__ float pow2f(int e) { return __int_as_float((e + 127) << 23); }
+// float32 -> float64 on the integer units (normal numbers and zero)
+__device__ __forceinline__ double widen(float f) {
+  const uint32_t u = __float_as_uint(f), mag = u & 0x7fffffffu;
+  const uint32_t h = mag < 0x00800000u ? 0u : (mag >> 3) + 0x38000000u;
+  return __hiloint2double((int)((u & 0x80000000u) | h),
+                          mag < 0x00800000u ? 0 : (int)(u << 29));
+}
+
+// Rotation of a pair with squared norms al, be and inner product ga: false
+// where the pair is orthogonal to |ga| <= tol sqrt(al be) (tol2 = tol^2).
+__device__ __forceinline__ bool jac_angle(double al, double be, double ga, float tol2, double& tau,
+                                          double& s) {
+  const int eg = expo(ga), ea = expo(al), eb = expo(be);
+  const uint32_t gbits = (hi32(ga) & 0x7fffffffu) | (uint32_t)__double2loint(ga);
+  if (gbits == 0 || eg == 0x7ff || ea == 0x7ff || eb == 0x7ff) return false;
+  const float mg = mantissa(ga);
+  const float q = mg * mg / (mantissa(al) * mantissa(be));
+  if (q * pow2f(min(max(2 * eg - ea - eb, -120), 60)) <= tol2) return false;
+  const double d = be - al;
+  const int ez = expo(d) - eg - 1;   // exponent of zeta = d / (2 ga)
+  if (ez > 100) {   // t below 2^-100: t = s = ga / d, c = 1
+    s = ga / d;
+    tau = 0.5 * s;
+    return s != 0.0;
+  }
+  const float az = expo(d) == 0 ? 0.f : __fdividef(mantissa(d), mg) * pow2f(max(ez, -100));
+  const float t = az > 1e9f ? __fdividef(0.5f, az)
+                            : __fdividef(1.0f, az + sqrtf(fmaf(az, az, 1.0f)));
+  const float h = __fdividef(t, 1.0f + sqrtf(fmaf(t, t, 1.0f)));   // tan(theta / 2) <= 0.42
+  const uint32_t neg = (hi32(d) ^ hi32(ga)) & 0x80000000u;
+  const float hs = __uint_as_float(__float_as_uint(h) | (az == 0.f ? 0u : neg));
+  tau = widen(hs);
+  // s = 2 tau / (1 + tau^2): float32 reciprocal and one cubic Newton step
+  const double u = fma(tau, tau, 1.0);
+  const double r0 = widen(__frcp_rn(fmaf(hs, hs, 1.0f)));
+  const double e = fma(-u, r0, 1.0);
+  s = (tau + tau) * fma(r0, fma(e, e, e), r0);
+  return true;
+}
+
+template <int LANES>
+__device__ __forceinline__ double lanes_sum(double v, uint32_t mask) {
+#pragma unroll
+  for (int o = 1; o < LANES; o <<= 1) v += __shfl_xor_sync(mask, v, o);
+  return v;
+}
+
+constexpr int JAC_THREADS = 512;
+template <int LANES, int RPL>
+__global__ void __launch_bounds__(JAC_THREADS)
 jacobi_kernel(int m, int n, const double* __restrict__ A, int lda, long long sA, int r,
               double* __restrict__ U, int ldu, long long sU, double* __restrict__ sv,
               long long sS, int* info, int lower, const double* __restrict__ A2,
@@ -161,7 +227,7 @@ jacobi_kernel(int m, int n, const double* __restrict__ A, int lda, long long sA,
   const int np = n + (n & 1);            // even number of columns (a zero pad column)
   const int lda_s = m | 1;               // odd column stride
   double* a = sm;                        // column-major, column c at a + c * lda_s
-  double* nrm = a + (long long)lda_s * np;   // np
+  double* nrm = a + (long long)lda_s * np;   // np: squared norms, then norms
   int* order = reinterpret_cast<int*>(nrm + np);   // np
   __shared__ int s_rot;
   // blocks nsplit.. work on the second batch (A2 -> U2), same shapes
@@ -176,83 +242,110 @@ jacobi_kernel(int m, int n, const double* __restrict__ A, int lda, long long sA,
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  const double tol = 2.220446049250313e-16 * (double)m;
-  const int npairs = np / 2;
-  const int part = threadIdx.x & (JAC_LANES - 1);
-  // every lane of a warp runs the pair loop the same number of times, so the
-  // shuffles below always see the whole warp
-  const int slots = (npairs * JAC_LANES + blockDim.x - 1) / blockDim.x * blockDim.x;
+  const float tolf = 2.220446049250313e-16f * (float)m, tol2 = tolf * tolf;
+  const int npairs = np / 2, ring = np - 1;
+  const int part = threadIdx.x & (LANES - 1), group = threadIdx.x / LANES;
+  const int ngroups = blockDim.x / LANES;
+  const uint32_t gmask = LANES == 32 ? 0xffffffffu
+                                     : ((1u << LANES) - 1) << (lane & ~(LANES - 1));
   int sweep = 0;
   for (; sweep < JAC_MAX_SWEEPS; ++sweep) {
+    // (loops of the same length on every lane: the whole warp joins the sums)
+    for (int c0 = 0; c0 < np; c0 += ngroups) {
+      const int c = c0 + group;
+      double v = 0.0;
+      if (c < np) {
+        const double* ac = a + (long long)c * lda_s;
+        for (int i = part; i < m; i += LANES) v = fma(ac[i], ac[i], v);
+      }
+      v = lanes_sum<LANES>(v, 0xffffffffu);
+      if (part == 0 && c < np) nrm[c] = v;
+    }
     if (threadIdx.x == 0) s_rot = 0;
     __syncthreads();
-    for (int rnd = 0; rnd < np - 1; ++rnd) {
-      for (int t = threadIdx.x; t < slots; t += blockDim.x) {
-        const int pi = t / JAC_LANES;
-        const bool on = pi < npairs;
+    for (int rnd = 0; rnd < ring; ++rnd) {
+      for (int p0 = 0; p0 < npairs; p0 += ngroups) {
         // circle method: slot 0 fixed, others rotate
-        const int s1 = pi, s2 = np - 1 - pi;
-        const int p = (s1 == 0) ? 0 : 1 + (s1 - 1 + rnd) % (np - 1);
-        const int q = 1 + (s2 - 1 + rnd) % (np - 1);
-        double* ap = a + (long long)(on ? p : 0) * lda_s;
-        double* aq = a + (long long)(on ? q : 0) * lda_s;
-        double a0 = 0.0, b0 = 0.0, g0 = 0.0, a1 = 0.0, b1 = 0.0, g1 = 0.0;
-        if (on) {
-          int i = part;
-          for (; i + JAC_LANES < m; i += 2 * JAC_LANES) {
-            const double x0 = ap[i], y0 = aq[i];
-            const double x1 = ap[i + JAC_LANES], y1 = aq[i + JAC_LANES];
-            a0 = fma(x0, x0, a0);
-            b0 = fma(y0, y0, b0);
-            g0 = fma(x0, y0, g0);
-            a1 = fma(x1, x1, a1);
-            b1 = fma(y1, y1, b1);
-            g1 = fma(x1, y1, g1);
-          }
-          if (i < m) {
-            const double x0 = ap[i], y0 = aq[i];
-            a0 = fma(x0, x0, a0);
-            b0 = fma(y0, y0, b0);
-            g0 = fma(x0, y0, g0);
-          }
-        }
-        double al = a0 + a1, be = b0 + b1, ga = g0 + g1;
+        const bool on = p0 + group < npairs;
+        const int pi = on ? p0 + group : 0;
+        int p = pi - 1 + rnd, q = np - 2 - pi + rnd;
+        p = pi == 0 ? 0 : 1 + (p >= ring ? p - ring : p);
+        q = 1 + (q >= ring ? q - ring : q);
+        double* ap = a + (long long)p * lda_s;
+        double* aq = a + (long long)q * lda_s;
+        double x[RPL > 0 ? RPL : 1], y[RPL > 0 ? RPL : 1];
+        double g[4] = {0.0, 0.0, 0.0, 0.0};
+        if constexpr (RPL > 0) {
 #pragma unroll
-        for (int o = 1; o < JAC_LANES; o <<= 1) {
-          al += __shfl_xor_sync(0xffffffffu, al, o);
-          be += __shfl_xor_sync(0xffffffffu, be, o);
-          ga += __shfl_xor_sync(0xffffffffu, ga, o);
+          for (int i = 0; i < RPL; ++i) {
+            const int row = part + LANES * i;
+            x[i] = row < m ? ap[row] : 0.0;
+            y[i] = row < m ? aq[row] : 0.0;
+          }
+#pragma unroll
+          for (int i = 0; i < RPL; ++i) g[i & 3] = fma(x[i], y[i], g[i & 3]);
+        } else {
+          for (int row = part; row < m; row += LANES) g[0] = fma(ap[row], aq[row], g[0]);
         }
-        if (on && ga != 0.0 && fabs(ga) > tol * sqrt(al * be)) {
-          const double zeta = (be - al) / (2.0 * ga);
-          double c, s;
-          float tf;
-          if (fabs(zeta) > 1e7) {
-            // small angle: t = 1 / (2 zeta) to relative 1e-14, c^2 + s^2 = 1 + O(t^4)
-            const double t = 0.5 / zeta;
-            c = fma(-0.5 * t, t, 1.0);
-            s = t * c;
-            tf = (float)t;
-          } else {
-            const float zf = (float)zeta;
-            tf = copysignf(1.0f, zf) / (fabsf(zf) + sqrtf(fmaf(zf, zf, 1.0f)));
-            const float cf = rsqrtf(fmaf(tf, tf, 1.0f));
-            c = (double)cf;
-            s = (double)cf * (double)tf;
-            // renormalise: (c, s) /= sqrt(1 + d), d = c^2 + s^2 - 1 ~ 1e-7
-            const double d = fma(c, c, fma(s, s, -1.0));
-            const double f = fma(d, fma(0.375, d, -0.5), 1.0);
-            c *= f;
-            s *= f;
-          }
-          if (s != 0.0) {
-            for (int i = part; i < m; i += JAC_LANES) {
-              const double x = ap[i], y = aq[i];
-              ap[i] = c * x - s * y;
-              aq[i] = s * x + c * y;
+        double ga = RPL > 2 ? (g[0] + g[2]) + (g[1] + g[3]) : g[0] + g[1];
+        ga = lanes_sum<LANES>(ga, 0xffffffffu);
+        const double al = nrm[p], be = nrm[q];
+        double tau, s;
+        if (!on || !jac_angle(al, be, ga, tol2, tau, s)) continue;
+        double na = 0.0, nb = 0.0;
+        if constexpr (RPL > 0) {
+#pragma unroll
+          for (int i = 0; i < RPL; ++i) {
+            const int row = part + LANES * i;
+            x[i] = fma(-tau, y[i], x[i]);
+            y[i] = fma(s, x[i], y[i]);
+            x[i] = fma(-tau, y[i], x[i]);
+            if (row < m) {
+              ap[row] = x[i];
+              aq[row] = y[i];
             }
-            s_rot = 1;
           }
+        } else {
+          for (int row = part; row < m; row += LANES) {
+            double xv = ap[row], yv = aq[row];
+            xv = fma(-tau, yv, xv);
+            yv = fma(s, xv, yv);
+            xv = fma(-tau, yv, xv);
+            ap[row] = xv;
+            aq[row] = yv;
+          }
+        }
+        // |x'|^2 = al + s (s (be - al) - 2 c ga), c = 1 - tau s
+        const double c = fma(-tau, s, 1.0);
+        const double w = s * fma(s, be - al, -(c + c) * ga);
+        na = al + w;
+        nb = be - w;
+        // a norm that fell by cancellation has lost its digits: form it anew
+        // (the whole group sees the same values)
+        if ((int)hi32(na) < 0 || expo(na) < expo(al) - 3) {
+          na = 0.0;
+          if constexpr (RPL > 0) {
+#pragma unroll
+            for (int i = 0; i < RPL; ++i) na = fma(x[i], x[i], na);
+          } else {
+            for (int row = part; row < m; row += LANES) na = fma(ap[row], ap[row], na);
+          }
+          na = lanes_sum<LANES>(na, gmask);
+        }
+        if ((int)hi32(nb) < 0 || expo(nb) < expo(be) - 3) {
+          nb = 0.0;
+          if constexpr (RPL > 0) {
+#pragma unroll
+            for (int i = 0; i < RPL; ++i) nb = fma(y[i], y[i], nb);
+          } else {
+            for (int row = part; row < m; row += LANES) nb = fma(aq[row], aq[row], nb);
+          }
+          nb = lanes_sum<LANES>(nb, gmask);
+        }
+        if (part == 0) {
+          nrm[p] = na;
+          nrm[q] = nb;
+          s_rot = 1;
         }
       }
       __syncthreads();
@@ -456,34 +549,75 @@ void apply_q(cudaStream_t st, bool transpose, int m, int k, const double* V, int
   check_launch("apply_q_kernel");
 }
 
+namespace {
+template <int LANES, int RPL>
+void launch_jacobi(cudaStream_t st, int grid, int threads, size_t sm, int m, int n,
+                   const double* A, int lda, long long sA, int r, double* U, int ldu,
+                   long long sU, double* sv, long long sS, int* info, bool lower,
+                   const double* A2, double* U2, int nsplit) {
+  auto kern = jacobi_kernel<LANES, RPL>;
+  ensure_smem(reinterpret_cast<const void*>(kern), sm);
+  kern<<<grid, threads, sm, st>>>(m, n, A, lda, sA, r, U, ldu, sU, sv, sS, info, lower ? 1 : 0, A2,
+                                  U2, nsplit);
+  check_launch("jacobi_kernel");
+}
+
+// Lanes per pair and rows per lane: the float64 instructions of the busiest
+// SM sub-partition, (warps on it) x (4 per row + ~19), are least.  Four lanes
+// put the 32 pairs of 64 columns on exactly one warp per sub-partition; other
+// column counts fill it more evenly with eight.
+void jacobi_dispatch(cudaStream_t st, int grid, int m, int n, const double* A, int lda,
+                     long long sA, int r, double* U, int ldu, long long sU, double* sv,
+                     long long sS, int* info, bool lower, const double* A2, double* U2,
+                     int nsplit) {
+  SLU_REQUIRE(r <= m, "jacobi: rank larger than rows");
+  const int np = n + (n & 1);
+  const size_t sm = (size_t)(m | 1) * np * sizeof(double) + np * sizeof(double) + np * sizeof(int);
+  SLU_REQUIRE(sm <= 220 * 1024, "jacobi: block too large for shared memory");
+  const int pairs = np / 2;
+  auto rows = [&](int lanes) { return (m + lanes - 1) / lanes; };
+  auto cost = [&](int lanes) {
+    const int warps = (pairs * lanes + 31) / 32;
+    return (warps + 3) / 4 * (4 * rows(lanes) + 19);
+  };
+  int lanes = 4;
+  if (rows(4) > 16 || cost(8) < cost(4)) lanes = 8;
+  const int threads = std::min(JAC_THREADS, std::max(64, (pairs * lanes + 31) / 32 * 32));
+#define SLU_JACOBI(L, R)                                                                        \
+  return launch_jacobi<L, R>(st, grid, threads, sm, m, n, A, lda, sA, r, U, ldu, sU, sv, sS, info, \
+                             lower, A2, U2, nsplit)
+  const int rp = rows(lanes);
+  if (lanes == 4) {
+    if (rp <= 4) SLU_JACOBI(4, 4);
+    if (rp <= 8) SLU_JACOBI(4, 8);
+    if (rp <= 10) SLU_JACOBI(4, 10);
+    if (rp <= 12) SLU_JACOBI(4, 12);
+    if (rp <= 14) SLU_JACOBI(4, 14);
+    SLU_JACOBI(4, 16);
+  }
+  if (rp <= 4) SLU_JACOBI(8, 4);
+  if (rp <= 8) SLU_JACOBI(8, 8);
+  if (rp <= 10) SLU_JACOBI(8, 10);
+  if (rp <= 12) SLU_JACOBI(8, 12);
+  if (rp <= 16) SLU_JACOBI(8, 16);
+  SLU_JACOBI(8, 0);
+#undef SLU_JACOBI
+}
+}  // namespace
+
 void jacobi_left_sv(cudaStream_t st, int m, int n, const double* A, int lda, long long sA, int r,
                     double* U, int ldu, long long sU, double* sv, long long sS, int batch,
                     int* info, bool lower) {
   if (batch <= 0 || r <= 0) return;
-  SLU_REQUIRE(r <= m, "jacobi: rank larger than rows");
-  int np = n + (n & 1);
-  size_t sm = (size_t)(m | 1) * np * sizeof(double) + np * sizeof(double) + np * sizeof(int);
-  SLU_REQUIRE(sm <= 220 * 1024, "jacobi: block too large for shared memory");
-  ensure_smem(reinterpret_cast<const void*>(jacobi_kernel), sm);
-  int threads = 32 * std::min(32, std::max(2, (np / 2 * JAC_LANES + 31) / 32));
-  jacobi_kernel<<<batch, threads, sm, st>>>(m, n, A, lda, sA, r, U, ldu, sU, sv, sS, info,
-                                            lower ? 1 : 0, A, U, batch);
-  check_launch("jacobi_kernel");
+  jacobi_dispatch(st, batch, m, n, A, lda, sA, r, U, ldu, sU, sv, sS, info, lower, A, U, batch);
 }
 
 void jacobi_left_sv2(cudaStream_t st, int m, int n, const double* A, const double* A2, int lda,
                      long long sA, int r, double* U, double* U2, int ldu, long long sU, int batch,
                      int* info, bool lower) {
   if (batch <= 0 || r <= 0) return;
-  SLU_REQUIRE(r <= m, "jacobi: rank larger than rows");
-  int np = n + (n & 1);
-  size_t sm = (size_t)(m | 1) * np * sizeof(double) + np * sizeof(double) + np * sizeof(int);
-  SLU_REQUIRE(sm <= 220 * 1024, "jacobi: block too large for shared memory");
-  ensure_smem(reinterpret_cast<const void*>(jacobi_kernel), sm);
-  int threads = 32 * std::min(32, std::max(2, (np / 2 * JAC_LANES + 31) / 32));
-  jacobi_kernel<<<2 * batch, threads, sm, st>>>(m, n, A, lda, sA, r, U, ldu, sU, nullptr, 0, info,
-                                                lower ? 1 : 0, A2, U2, batch);
-  check_launch("jacobi_kernel");
+  jacobi_dispatch(st, 2 * batch, m, n, A, lda, sA, r, U, ldu, sU, nullptr, 0, info, lower, A2, U2,
+                  batch);
 }
 
 }  // namespace slu
