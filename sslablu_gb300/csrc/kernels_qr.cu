@@ -528,7 +528,7 @@ jacobi_kernel(int m, int n_in, const double* __restrict__ A, int lda, long long 
   const double smax = nrm[order[0]];
   const double tiny = (smax > 0.0) ? smax * 1e-150 : 1e-300;
   // normalised leading columns; columns that carry no direction are
-  // completed below by Gram-Schmidt on the unit vectors
+  // completed below
   for (int j = warp; j < r; j += nwarps) {
     const int c = min(max(order[j < np ? j : np - 1], 0), np - 1);
     double s = nrm[c];
@@ -538,34 +538,57 @@ jacobi_kernel(int m, int n_in, const double* __restrict__ A, int lda, long long 
       Ub[(long long)(pre ? rows[i] : i) * ldu + j] = ok ? a[(long long)c * lda_s + i] / s : 0.0;
   }
   __syncthreads();
-  // completion (rare: zero or rank-deficient input); serial over columns
-  if (warp == 0) {
-    for (int j = 0; j < r; ++j) {
-      const int c = min(max(order[j < np ? j : np - 1], 0), np - 1);
-      bool ok = (j < n) && nrm[c] > tiny;
-      if (ok) continue;
-      for (int e = 0; e < m; ++e) {
-        // candidate e_e, orthogonalise against columns 0..j-1 (twice)
-        for (int i = lane; i < m; i += 32) Ub[(long long)i * ldu + j] = (i == e) ? 1.0 : 0.0;
-        __syncwarp();
-        for (int pass = 0; pass < 2; ++pass)
-          for (int q = 0; q < j; ++q) {
-            double d = 0.0;
-            for (int i = lane; i < m; i += 32) d += Ub[(long long)i * ldu + q] * Ub[(long long)i * ldu + j];
-            d = warp_sum(d);
-            for (int i = lane; i < m; i += 32) Ub[(long long)i * ldu + j] -= d * Ub[(long long)i * ldu + q];
-            __syncwarp();
-          }
-        double s = 0.0;
-        for (int i = lane; i < m; i += 32) s += Ub[(long long)i * ldu + j] * Ub[(long long)i * ldu + j];
-        s = sqrt(warp_sum(s));
-        if (s > 0.5) {
-          for (int i = lane; i < m; i += 32) Ub[(long long)i * ldu + j] /= s;
-          __syncwarp();
-          break;
-        }
+  // completion by unit vectors, orthogonalised against the columns before
+  // (classical Gram-Schmidt twice, over the whole block).  Every boundary
+  // coupling of a red-black level is a zero block, so this is no rare case.
+  // A unit vector once rejected stays rejected (its residual only shrinks as
+  // columns join), so each is tried once: the compression of a zero 512-point
+  // block (rank 24) takes 9 ms where retrying all of them for every column
+  // took 30.
+  int j0 = 0;
+  while (j0 < r && j0 < n && nrm[min(max(order[j0 < np ? j0 : np - 1], 0), np - 1)] > tiny) ++j0;
+  __syncthreads();
+  double* v = a;        // candidate (the columns are no longer needed)
+  double* d = a + m;    // its products with the columns before
+  double thr = 0.5;
+  int cand = 0;
+  for (int j = j0; j < r; ++j) {
+    for (;;) {
+      if (cand >= m) {
+        // fewer than r unit vectors leave half their length outside: some
+        // vector still has 1 / sqrt(m) of it
+        if (thr < 0.5) break;
+        thr = 0.5 / sqrt((double)m);
+        cand = 0;
       }
+      for (int i = threadIdx.x; i < m; i += blockDim.x) v[i] = (i == cand) ? 1.0 : 0.0;
+      __syncthreads();
+      for (int pass = 0; pass < 2; ++pass) {
+        for (int q = warp; q < j; q += nwarps) {
+          double s = 0.0;
+          for (int i = lane; i < m; i += 32) s = fma(Ub[(long long)i * ldu + q], v[i], s);
+          s = warp_sum(s);
+          if (lane == 0) d[q] = s;
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < m; i += blockDim.x) {
+          double x = v[i];
+          for (int q = 0; q < j; ++q) x = fma(-d[q], Ub[(long long)i * ldu + q], x);
+          v[i] = x;
+        }
+        __syncthreads();
+      }
+      double s = 0.0;
+      for (int i = lane; i < m; i += 32) s = fma(v[i], v[i], s);
+      s = sqrt(warp_sum(s));
+      ++cand;
+      if (s > thr) {
+        for (int i = threadIdx.x; i < m; i += blockDim.x) Ub[(long long)i * ldu + j] = v[i] / s;
+        break;
+      }
+      __syncthreads();
     }
+    __syncthreads();
   }
 }
 // Compact WY form of a factored panel of jb reflectors (LAPACK larft,
