@@ -78,34 +78,19 @@ __device__ void panel_qr_dev(int m, int nfac, int ncol, double* a, int lda, doub
   }
 }
 
+// Panels too large for one CTA's shared memory, in global memory.
 __global__ void __launch_bounds__(512)
 panel_qr_kernel(int m, int nfac, int ncol, double* __restrict__ W, int ldw, long long sW,
-                double* __restrict__ tau, long long sTau, int use_smem, double* __restrict__ W2,
+                double* __restrict__ tau, long long sTau, double* __restrict__ W2,
                 double* __restrict__ tau2, int nsplit) {
-  extern __shared__ double sm[];
   // blocks nsplit.. work on the second batch (W2, tau2), same shapes
   const bool second = (int)blockIdx.x >= nsplit;
   const long long b = second ? blockIdx.x - nsplit : blockIdx.x;
-  double* w = (second ? W2 : W) + b * sW;
-  double* t = (second ? tau2 : tau) + b * sTau;
-  if (use_smem) {
-    for (long long e = threadIdx.x; e < (long long)m * ncol; e += blockDim.x) {
-      int c = (int)(e / m), i = (int)(e % m);
-      sm[e] = w[(long long)c * ldw + i];
-    }
-    __syncthreads();
-    panel_qr_dev(m, nfac, ncol, sm, m, t);
-    __syncthreads();
-    for (long long e = threadIdx.x; e < (long long)m * ncol; e += blockDim.x) {
-      int c = (int)(e / m), i = (int)(e % m);
-      w[(long long)c * ldw + i] = sm[e];
-    }
-  } else {
-    panel_qr_dev(m, nfac, ncol, w, ldw, t);
-  }
+  panel_qr_dev(m, nfac, ncol, (second ? W2 : W) + b * sW, ldw, (second ? tau2 : tau) + b * sTau);
 }
 
-// C <- Q C (transpose = false) or Q^T C; each warp owns whole columns of C.
+// C <- Q C (transpose = false) or Q^T C for tall columns; each warp owns whole
+// columns of C.
 __global__ void __launch_bounds__(256)
 apply_q_kernel(bool transpose, int m, int k, const double* __restrict__ V, int ldv, long long sV,
                const double* __restrict__ tau, long long sTau, double* __restrict__ C, int ldc,
@@ -128,6 +113,250 @@ apply_q_kernel(bool transpose, int m, int k, const double* __restrict__ V, int l
     if (lane == 0) cc[j] -= d;
     for (int i = j + 1 + lane; i < m; i += 32) cc[i] -= d * v[i];
     __syncwarp();
+  }
+}
+
+// ---------------------------------------------------------------- float64 economy
+// One warp instruction on the float64 pipe takes 64 clocks of its SM
+// sub-partition, so scalars are formed from bit patterns and float32 seeds.
+__device__ __forceinline__ uint32_t hi32(double v) { return (uint32_t)__double2hiint(v); }
+// mantissa in [1, 2) as a float32 (the leading 23 bits)
+__device__ __forceinline__ float mantissa(double v) {
+  return __uint_as_float(0x3f800000u | (hi32(v) & 0xfffffu) << 3 |
+                         (uint32_t)__double2loint(v) >> 29);
+}
+__device__ __forceinline__ int expo(double v) { return (int)(hi32(v) >> 20 & 0x7ff); }
+__device__ __forceinline__ float pow2f(int e) { return __int_as_float((e + 127) << 23); }
+// float32 -> float64 on the integer units (normal numbers and zero)
+__device__ __forceinline__ double widen(float f) {
+  const uint32_t u = __float_as_uint(f), mag = u & 0x7fffffffu;
+  const uint32_t h = mag < 0x00800000u ? 0u : (mag >> 3) + 0x38000000u;
+  return __hiloint2double((int)((u & 0x80000000u) | h),
+                          mag < 0x00800000u ? 0 : (int)(u << 29));
+}
+
+template <int LANES>
+__device__ __forceinline__ double lanes_sum(double v, uint32_t mask) {
+#pragma unroll
+  for (int o = 1; o < LANES; o <<= 1) v += __shfl_xor_sync(mask, v, o);
+  return v;
+}
+
+// 1 / sqrt(t): float32 seed, one cubic Newton step (relative error ~1e-20
+// before rounding); t positive, finite and normal
+__device__ __forceinline__ double inv_sqrt(double t) {
+  const int e = expo(t) - 1023, e2 = e & ~1;
+  const double q = __hiloint2double((int)hi32(t) - (e2 << 20), __double2loint(t));   // in [1, 4)
+  const double y = widen(rsqrtf(mantissa(t) * (float)(1 + (e & 1))));
+  const double r = fma(-q * y, y, 1.0);
+  const double z = fma(y * r, fma(0.375, r, 0.5), y);
+  return __hiloint2double((int)hi32(z) - (e2 / 2 << 20), __double2loint(z));
+}
+// 1 / q likewise; q positive, finite and normal, 1 / q normal
+__device__ __forceinline__ double inv_pos(double q) {
+  const int e = expo(q) - 1023;
+  const double m = __hiloint2double((int)hi32(q) - (e << 20), __double2loint(q));   // in [1, 2)
+  const double z = widen(__frcp_rn(mantissa(q)));
+  const double r = fma(-m, z, 1.0);
+  const double w = fma(z, fma(r, r, r), z);
+  return __hiloint2double((int)hi32(w) - (e << 20), __double2loint(w));
+}
+
+// Householder reflector of a column with diagonal entry alpha and ss the sum
+// of squares below it: v = (v0, rest), H = I - f v v^T, new diagonal beta.
+struct Reflector {
+  double v0, f, beta, tau, sc;   // tau, sc = 1 / v0: the LAPACK form (v[0] = 1)
+};
+__device__ __forceinline__ Reflector make_reflector(double alpha, double ss) {
+  Reflector h{0.0, 0.0, alpha, 0.0, 0.0};
+  if (ss == 0.0) return h;
+  const double t = fma(alpha, alpha, ss);
+  const int e = expo(t);
+  if (e > 1023 - 900 && e < 1023 + 900) {
+    const double y = inv_sqrt(t), nrm = t * y;
+    h.beta = -copysign(nrm, alpha);
+    h.v0 = alpha - h.beta;
+    const double a = fabs(h.v0);
+    h.f = inv_pos(nrm * a);
+    h.tau = a * y;
+    h.sc = copysign(nrm * h.f, h.v0);
+  } else {   // near the ends of the range, or not finite
+    h.beta = -copysign(sqrt(t), alpha);
+    h.v0 = alpha - h.beta;
+    h.tau = -h.v0 / h.beta;
+    h.sc = 1.0 / h.v0;
+    h.f = h.tau * h.sc * h.sc;
+  }
+  return h;
+}
+
+// ---------------------------------------------------------------- panels in shared memory
+// QR of an m x n column-major panel, one CTA, the panel in shared memory
+// (column stride ld, 8 mod 16: the 2 x 8 entries of a wavefront hit distinct
+// banks).  Warp 0 carries the chain: it applies reflector j to column j + 1
+// with all its lanes and forms reflector j + 1 at once; meanwhile the other
+// warps apply reflector j to the columns after it, eight lanes per column
+// (three butterfly additions per product instead of five).  One barrier per
+// column.  Bound by the float64 pipe for wide panels, by warp 0's chain of
+// ~50 float64 instructions per column for the last ones.
+// 128 panels of 261 x 64 with 64 carried columns: 0.40 ms, and 0.64 for the
+// carried ones (apply_q_reg_kernel); 1.71 by panel_qr_kernel in global memory.
+__global__ void __launch_bounds__(512)
+panel_qr_smem_kernel(int m, int n, double* __restrict__ W, int ldw, long long sW,
+                     double* __restrict__ tau, long long sTau, int ld, double* __restrict__ W2,
+                     double* __restrict__ tau2, int nsplit) {
+  extern __shared__ double sm[];
+  double* s_sc = sm + (size_t)ld * n;   // n: 1 / v0
+  __shared__ double s_v0[2], s_f[2];
+  const bool second = (int)blockIdx.x >= nsplit;
+  const long long b = second ? blockIdx.x - nsplit : blockIdx.x;
+  double* w = (second ? W2 : W) + b * sW;
+  double* tg = (second ? tau2 : tau) + b * sTau;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+  for (int c = warp; c < n; c += nwarps)
+    for (int i = lane; i < m; i += 32) sm[(size_t)c * ld + i] = w[(long long)c * ldw + i];
+  __syncthreads();
+  const int steps = min(n, m);
+  // reflector of column j from its entries below the diagonal (warp 0)
+  auto reflect = [&](int j) {
+    double* col = sm + (size_t)j * ld;
+    double ss = 0.0, s1 = 0.0;
+    int i = j + 1 + lane;
+    for (; i + 32 < m; i += 64) {
+      ss = fma(col[i], col[i], ss);
+      s1 = fma(col[i + 32], col[i + 32], s1);
+    }
+    if (i < m) ss = fma(col[i], col[i], ss);
+    ss = warp_sum(ss + s1);
+    const Reflector h = make_reflector(col[j], ss);
+    __syncwarp();
+    if (lane == 0) {
+      s_v0[j & 1] = h.v0;
+      s_f[j & 1] = h.f;
+      s_sc[j] = h.sc;
+      col[j] = h.beta;
+      tg[j] = h.tau;
+    }
+  };
+  if (warp == 0) reflect(0);
+  __syncthreads();
+  for (int j = 0; j < steps; ++j) {
+    const double* v = sm + (size_t)j * ld;
+    const double v0 = s_v0[j & 1], f = s_f[j & 1];
+    if (warp == 0) {
+      if (j + 1 < n) {
+        double* cc = sm + (size_t)(j + 1) * ld;
+        if (f != 0.0) {
+          double d = lane == 0 ? v0 * cc[j] : 0.0, d1 = 0.0;
+          int i = j + 1 + lane;
+          for (; i + 32 < m; i += 64) {
+            d = fma(v[i], cc[i], d);
+            d1 = fma(v[i + 32], cc[i + 32], d1);
+          }
+          if (i < m) d = fma(v[i], cc[i], d);
+          d = f * warp_sum(d + d1);
+          for (i = j + 1 + lane; i < m; i += 32) cc[i] = fma(-d, v[i], cc[i]);
+          if (lane == 0) cc[j] = fma(-d, v0, cc[j]);
+          __syncwarp();
+        }
+        if (j + 1 < steps) reflect(j + 1);
+      }
+    } else if (f != 0.0) {
+      const int part = lane & 7, per = 4 * (nwarps - 1);
+      for (int c0 = j + 2; c0 < n; c0 += per) {
+        const int c = c0 + 4 * (warp - 1) + (lane >> 3);
+        if (c0 + 4 * (warp - 1) >= n) break;   // uniform
+        const bool on = c < n;
+        double* cc = sm + (size_t)(on ? c : j) * ld;
+        const int i0 = ((j + 1) & ~7) + part;
+        double d = part == 0 ? v0 * cc[j] : 0.0, d1 = 0.0;
+        int i = i0 > j ? i0 : i0 + 8;
+        const int first = i;
+        for (; i + 8 < m; i += 16) {
+          d = fma(v[i], cc[i], d);
+          d1 = fma(v[i + 8], cc[i + 8], d1);
+        }
+        if (i < m) d = fma(v[i], cc[i], d);
+        d = f * lanes_sum<8>(d + d1, 0xffffffffu);
+        if (on) {
+#pragma unroll 4
+          for (i = first; i < m; i += 8) cc[i] = fma(-d, v[i], cc[i]);
+          if (part == 0) cc[j] = fma(-d, v0, cc[j]);
+        }
+      }
+    }
+    __syncthreads();
+  }
+  for (int c = warp; c < n; c += nwarps) {
+    const double sc = c < steps ? s_sc[c] : 0.0;
+    for (int i = lane; i < m; i += 32) {
+      const double x = sm[(size_t)c * ld + i];
+      w[(long long)c * ldw + i] = (i > c && sc != 0.0) ? x * sc : x;
+    }
+  }
+}
+
+// C <- Q^T C (transpose) or Q C for the m x k reflectors of a factored panel,
+// columns of C in registers (eight lanes per column, RPL rows each), the
+// reflectors through shared memory kRefl at a time with their unit diagonal
+// and the zeros above it.  Few problems spread their columns over more CTAs.
+// Bound by the float64 pipe (2 FMA per row, reflector and column).
+constexpr int kRefl = 16;
+template <int RPL>
+__global__ void __launch_bounds__(512)
+apply_q_reg_kernel(bool transpose, int m, int k, const double* __restrict__ V, int ldv,
+                   long long sV, const double* __restrict__ tau, long long sTau,
+                   double* __restrict__ C, int ldc, long long sC, int nc,
+                   const double* __restrict__ V2, const double* __restrict__ tau2,
+                   double* __restrict__ C2, int nsplit) {
+  extern __shared__ double sv[];   // kRefl x 8 RPL
+  __shared__ double st[kRefl];
+  const bool second = (int)blockIdx.y >= nsplit;
+  const long long b = second ? blockIdx.y - nsplit : blockIdx.y;
+  V = (second ? V2 : V) + b * sV;
+  tau = (second ? tau2 : tau) + b * sTau;
+  C = (second ? C2 : C) + b * sC;
+  constexpr int P = 8 * RPL;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+  const int part = lane & 7, c = (blockIdx.x * nwarps + warp) * 4 + (lane >> 3);
+  const bool on = c < nc;
+  double* cc = C + (long long)(on ? c : 0) * ldc;
+  double x[RPL];
+#pragma unroll
+  for (int i = 0; i < RPL; ++i) {
+    const int r = part + 8 * i;
+    x[i] = (on && r < m) ? cc[r] : 0.0;
+  }
+  const int chunks = (k + kRefl - 1) / kRefl;
+  for (int q = 0; q < chunks; ++q) {
+    const int j0 = (transpose ? q : chunks - 1 - q) * kRefl, nj = min(kRefl, k - j0);
+    __syncthreads();
+    for (int e = tid; e < nj * P; e += blockDim.x) {
+      const int jj = e / P, r = e - jj * P, j = j0 + jj;
+      sv[e] = r < j ? 0.0 : (r == j ? 1.0 : (r < m ? V[(long long)j * ldv + r] : 0.0));
+    }
+    if (tid < nj) st[tid] = tau[j0 + tid];
+    __syncthreads();
+    for (int s = 0; s < nj; ++s) {
+      const int jj = transpose ? s : nj - 1 - s;
+      const double t = st[jj];
+      if (t == 0.0) continue;   // uniform
+      const double* v = sv + jj * P + part;
+      double d[2] = {0.0, 0.0};
+#pragma unroll
+      for (int i = 0; i < RPL; ++i)
+        if (8 * i + 7 >= j0) d[i & 1] = fma(v[8 * i], x[i], d[i & 1]);
+      const double g = t * lanes_sum<8>(d[0] + d[1], 0xffffffffu);
+#pragma unroll
+      for (int i = 0; i < RPL; ++i)
+        if (8 * i + 7 >= j0) x[i] = fma(-g, v[8 * i], x[i]);
+    }
+  }
+  if (!on) return;
+#pragma unroll
+  for (int i = 0; i < RPL; ++i) {
+    const int r = part + 8 * i;
+    if (r < m) cc[r] = x[i];
   }
 }
 
@@ -167,22 +396,6 @@ apply_q_kernel(bool transpose, int m, int k, const double* __restrict__ V, int l
 // written as U (m x r).
 constexpr int JAC_MAX_SWEEPS = 40;
 
-__device__ __forceinline__ uint32_t hi32(double v) { return (uint32_t)__double2hiint(v); }
-// mantissa in [1, 2) as a float32 (the leading 23 bits)
-__device__ __forceinline__ float mantissa(double v) {
-  return __uint_as_float(0x3f800000u | (hi32(v) & 0xfffffu) << 3 |
-                         (uint32_t)__double2loint(v) >> 29);
-}
-__device__ __forceinline__ int expo(double v) { return (int)(hi32(v) >> 20 & 0x7ff); }
-__device__ __forceinline__ float pow2f(int e) { return __int_as_float((e + 127) << 23); }
-// float32 -> float64 on the integer units (normal numbers and zero)
-__device__ __forceinline__ double widen(float f) {
-  const uint32_t u = __float_as_uint(f), mag = u & 0x7fffffffu;
-  const uint32_t h = mag < 0x00800000u ? 0u : (mag >> 3) + 0x38000000u;
-  return __hiloint2double((int)((u & 0x80000000u) | h),
-                          mag < 0x00800000u ? 0 : (int)(u << 29));
-}
-
 // Rotation of a pair with squared norms al, be and inner product ga: false
 // where the pair is orthogonal to |ga| <= tol sqrt(al be) (tol2 = tol^2).
 __device__ __forceinline__ bool jac_angle(double al, double be, double ga, float tol2, double& tau,
@@ -213,13 +426,6 @@ __device__ __forceinline__ bool jac_angle(double al, double be, double ga, float
   const double e = fma(-u, r0, 1.0);
   s = (tau + tau) * fma(r0, fma(e, e, e), r0);
   return true;
-}
-
-template <int LANES>
-__device__ __forceinline__ double lanes_sum(double v, uint32_t mask) {
-#pragma unroll
-  for (int o = 1; o < LANES; o <<= 1) v += __shfl_xor_sync(mask, v, o);
-  return v;
 }
 
 // |v| as a float32 relative to 2^(E0 - 1023), E0 the largest exponent field
@@ -687,34 +893,91 @@ void qr_blocked(cudaStream_t st, int m, int nfac, int ncol, double* W, int ldw, 
   }
 }
 
+namespace {
+
+template <int RPL>
+void launch_apply(cudaStream_t st, bool transpose, int m, int k, const double* V, int ldv,
+                  long long sV, const double* tau, long long sTau, double* C, int ldc,
+                  long long sC, int nc, const double* V2, const double* tau2, double* C2,
+                  int nsplit, int batch) {
+  // up to 16 warps (64 columns) per CTA, fewer while SMs would stay empty
+  int warps = std::min(16, (nc + 3) / 4);
+  while (warps > 2 && (long long)batch * ((nc + 4 * warps - 1) / (4 * warps)) < num_sms())
+    warps = (warps + 1) / 2;
+  const size_t sm = sizeof(double) * kRefl * 8 * RPL;
+  auto kern = apply_q_reg_kernel<RPL>;
+  ensure_smem(reinterpret_cast<const void*>(kern), sm);
+  kern<<<dim3((nc + 4 * warps - 1) / (4 * warps), batch), 32 * warps, sm, st>>>(
+      transpose, m, k, V, ldv, sV, tau, sTau, C, ldc, sC, nc, V2, tau2, C2, nsplit);
+  check_launch("apply_q_reg_kernel");
+}
+
+// Rows that eight lanes hold in registers; taller columns stay in memory.
+constexpr int kApplyRows = 320;
+
+void apply_q_dispatch(cudaStream_t st, bool transpose, int m, int k, const double* V, int ldv,
+                      long long sV, const double* tau, long long sTau, double* C, int ldc,
+                      long long sC, int nc, const double* V2, const double* tau2, double* C2,
+                      int nsplit, int batch) {
+#define SLU_APPLY(R)                                                                           \
+  return launch_apply<R>(st, transpose, m, k, V, ldv, sV, tau, sTau, C, ldc, sC, nc, V2, tau2, \
+                         C2, nsplit, batch)
+  if (m <= 32) SLU_APPLY(4);
+  if (m <= 64) SLU_APPLY(8);
+  if (m <= 96) SLU_APPLY(12);
+  if (m <= 128) SLU_APPLY(16);
+  if (m <= 192) SLU_APPLY(24);
+  if (m <= 264) SLU_APPLY(33);
+  SLU_APPLY(40);
+#undef SLU_APPLY
+}
+
+// One or two (W2 != W) batches of panels.  The factored columns in shared
+// memory where they fit, the carried columns afterwards from registers; else
+// everything by the one-CTA kernel in global memory.
+void panel_qr_any(cudaStream_t st, int m, int nfac, int ncol, double* W, double* W2, int ldw,
+                  long long sW, double* tau, double* tau2, long long sTau, int batch, int total) {
+  const int ld = (m + 7) / 16 * 16 + 8;   // >= m, 8 mod 16
+  const size_t sm = sizeof(double) * ((size_t)ld * nfac + nfac);
+  if (sm <= 220 * 1024 && (ncol == nfac || m <= kApplyRows)) {
+    ensure_smem(reinterpret_cast<const void*>(panel_qr_smem_kernel), sm);
+    const int warps = std::min(16, std::max(2, 1 + (nfac + 3) / 4));
+    panel_qr_smem_kernel<<<total, 32 * warps, sm, st>>>(m, nfac, W, ldw, sW, tau, sTau, ld, W2,
+                                                        tau2, batch);
+    check_launch("panel_qr_smem_kernel");
+    if (ncol > nfac)
+      apply_q_dispatch(st, true, m, std::min(nfac, m), W, ldw, sW, tau, sTau,
+                       W + (long long)nfac * ldw, ldw, sW, ncol - nfac, W2, tau2,
+                       W2 + (long long)nfac * ldw, batch, total);
+    return;
+  }
+  panel_qr_kernel<<<total, 512, 0, st>>>(m, nfac, ncol, W, ldw, sW, tau, sTau, W2, tau2, batch);
+  check_launch("panel_qr_kernel");
+}
+
+}  // namespace
+
 void panel_qr(cudaStream_t st, int m, int nfac, int ncol, double* W, int ldw, long long sW,
               double* tau, long long sTau, int batch) {
   if (batch <= 0 || m <= 0 || nfac <= 0) return;
-  size_t sm = (size_t)m * ncol * sizeof(double);
-  int use_smem = sm <= 200 * 1024;
-  if (!use_smem) sm = 0;
-  ensure_smem(reinterpret_cast<const void*>(panel_qr_kernel), sm);
-  panel_qr_kernel<<<batch, 512, sm, st>>>(m, nfac, ncol, W, ldw, sW, tau, sTau, use_smem, W,
-                                          tau, batch);
-  check_launch("panel_qr_kernel");
+  panel_qr_any(st, m, nfac, ncol, W, W, ldw, sW, tau, tau, sTau, batch, batch);
 }
 
 void panel_qr2(cudaStream_t st, int m, int nfac, int ncol, double* W, double* W2, int ldw,
                long long sW, double* tau, double* tau2, long long sTau, int batch) {
   if (batch <= 0 || m <= 0 || nfac <= 0) return;
-  size_t sm = (size_t)m * ncol * sizeof(double);
-  int use_smem = sm <= 200 * 1024;
-  if (!use_smem) sm = 0;
-  ensure_smem(reinterpret_cast<const void*>(panel_qr_kernel), sm);
-  panel_qr_kernel<<<2 * batch, 512, sm, st>>>(m, nfac, ncol, W, ldw, sW, tau, sTau, use_smem,
-                                              W2, tau2, batch);
-  check_launch("panel_qr_kernel");
+  panel_qr_any(st, m, nfac, ncol, W, W2, ldw, sW, tau, tau2, sTau, batch, 2 * batch);
 }
 
 void apply_q(cudaStream_t st, bool transpose, int m, int k, const double* V, int ldv,
              long long sV, const double* tau, long long sTau, double* C, int ldc, long long sC,
              int nc, int batch) {
   if (batch <= 0 || nc <= 0 || m <= 0) return;
+  if (m <= kApplyRows) {
+    apply_q_dispatch(st, transpose, m, k, V, ldv, sV, tau, sTau, C, ldc, sC, nc, V, tau, C, batch,
+                     batch);
+    return;
+  }
   dim3 grid((nc + 7) / 8, batch);
   apply_q_kernel<<<grid, 256, 0, st>>>(transpose, m, k, V, ldv, sV, tau, sTau, C, ldc, sC, nc);
   check_launch("apply_q_kernel");
