@@ -1,0 +1,195 @@
+// Residue arithmetic of the exact tensor-core products (crt_gemm.cu,
+// crt_step.cu): the moduli and their tables, balanced residues of scaled
+// float64 values, and the reconstruction of a float64 from the residues of an
+// integer product.
+#pragma once
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+namespace slu {
+namespace crt {
+namespace {
+
+constexpr int NM = 16;   // moduli
+struct Tables {
+  int p[NM];
+  float pf[NM], inv[NM];
+  uint32_t ca[2][NM], cb[2][NM];   // balanced 2^(8 i) mod p (A), times (P/p)^-1 (B), packed bytes
+  int ba[NM], bb[NM];              // -(2^59) mod p (A), times (P/p)^-1 (B)
+  uint32_t w[15][NM / 4];          // byte i of P/p_l, four moduli packed
+  int p16[8];                      // P in 16-bit pieces
+  float top;                       // 2^112 / P
+};
+
+constexpr unsigned long long mod_pow2(int e, int p) {
+  unsigned long long r = 1;
+  for (int i = 0; i < e; ++i) r = r * 2 % p;
+  return r;
+}
+constexpr int balanced(int v, int p) { return 2 * v > p ? v - p : v; }
+
+constexpr Tables make_tables() {
+  Tables T{};
+  const int p[NM] = {256, 253, 251, 249, 247, 245, 241, 239, 233, 229, 227, 223, 211, 199, 197, 193};
+  unsigned __int128 P = 1;
+  for (int l = 0; l < NM; ++l) P *= (unsigned)p[l];
+  for (int l = 0; l < NM; ++l) {
+    T.p[l] = p[l];
+    T.pf[l] = (float)p[l];
+    T.inv[l] = 1.0f / (float)p[l];
+    const unsigned __int128 W = P / (unsigned)p[l];
+    const int wm = (int)(W % (unsigned)p[l]);
+    int m = 1;   // inverse of P/p modulo p
+    while (m * wm % p[l] != 1) ++m;
+    for (int i = 0; i < 8; ++i) {
+      const int c = (int)mod_pow2(8 * i, p[l]);
+      // p = 256: 128 is its own balanced form's limit; store -128
+      int a = balanced(c, p[l]), b = balanced(c * m % p[l], p[l]);
+      if (a == 128) a = -128;
+      if (b == 128) b = -128;
+      T.ca[i / 4][l] |= (uint32_t)(uint8_t)a << (8 * (i % 4));
+      T.cb[i / 4][l] |= (uint32_t)(uint8_t)b << (8 * (i % 4));
+    }
+    const int h = (int)mod_pow2(59, p[l]);
+    T.ba[l] = -h;
+    T.bb[l] = -(h * m % p[l]);
+    for (int i = 0; i < 15; ++i)
+      T.w[i][l / 4] |= (uint32_t)(uint8_t)(W >> (8 * i)) << (8 * (l % 4));
+  }
+  for (int i = 0; i < 8; ++i) T.p16[i] = (int)(uint16_t)(P >> (16 * i));
+  T.top = (float)(5192296858534827628530496329220096.0 / (double)P);   // 2^112 / P
+  return T;
+}
+__constant__ Tables c_tab = make_tables();
+
+// Largest |a'| exponent for products of depth K: |X| <= K 2^(2t) <= 2^123 < P / 4.
+inline int bits_for(int K) {
+  int lg = 0;
+  while ((1LL << lg) < K) ++lg;
+  return (123 - lg) / 2;
+}
+
+// dp4a of unsigned bytes of a with signed bytes of b, and the reverse
+__device__ __forceinline__ int dp4a_us(uint32_t a, uint32_t b, int c) {
+  int d;
+  asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  return d;
+}
+__device__ __forceinline__ int dp4a_su(uint32_t a, uint32_t b, int c) {
+  int d;
+  asm("dp4a.s32.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  return d;
+}
+
+
+__device__ __forceinline__ uint32_t hi32(double v) { return (uint32_t)__double2hiint(v); }
+
+// A float64 (its bits) whose exponent field is at most F (>= 1) as a t-bit
+// integer, rounded to nearest and shifted by 2^59 to be non-negative (the
+// tables take the shift off again); ok = false gives zero.
+__device__ __forceinline__ void scaled(uint32_t hi, uint32_t lo, int F, int t, bool ok,
+                                       uint32_t& zlo, uint32_t& zhi) {
+  const int fe = (int)((hi >> 20) & 0x7ff);
+  unsigned long long m = (unsigned long long)(hi & 0xfffffu) << 32 | lo;
+  if (fe) m |= 1ULL << 52;
+  // a' = m 2^(t - 53 - (F - max(fe, 1)))
+  const int sh = t - 53 - (F - max(fe, 1));
+  unsigned long long q;
+  if (sh >= 0) q = m << sh;
+  else if (sh > -55) q = (m + (1ULL << (-sh - 1))) >> -sh;
+  else q = 0;
+  if (!ok) q = 0;
+  const unsigned long long z = (hi >> 31) ? (1ULL << 59) - q : (1ULL << 59) + q;
+  zlo = (uint32_t)z;
+  zhi = (uint32_t)(z >> 32);
+}
+
+// Balanced residue modulo p (ip = 1 / p) of the shifted integer, from the byte
+// weights c0, c1 and the bias (table entry + 0x4B400000): |s| < 2^19 is exact
+// as the low bits of a float of magnitude 1.5 2^23.
+__device__ __forceinline__ float residue(uint32_t zlo, uint32_t zhi, uint32_t c0, uint32_t c1,
+                                         int bias, float p, float ip) {
+  const int s = dp4a_us(zlo, c0, dp4a_us(zhi, c1, bias));
+  const float g = __int_as_float(s) - 12582912.f;
+  const float q = fmaf(g, ip, 12582912.f) - 12582912.f;
+  return fmaf(-p, q, g);
+}
+__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+// An exact product sum (|x| < 2^24 + 2^8) reduced modulo p: the residue in the
+// low byte.
+__device__ __forceinline__ uint32_t reduced(float x, float p, float ip) {
+  const float k = fmaf(x, ip, 12582912.f) - 12582912.f;
+  return __float_as_uint(fmaf(-p, k, x) + 12582912.f);
+}
+
+// 128-bit two's complement value c3:c2:c1:c0 times 2^e, rounded to nearest even
+__device__ __forceinline__ double to_double(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3,
+                                            int e) {
+  unsigned long long lo = (unsigned long long)c1 << 32 | c0, hi = (unsigned long long)c3 << 32 | c2;
+  const uint32_t neg = c3 >> 31;
+  if (neg) {
+    lo = ~lo + 1;
+    hi = ~hi + (lo == 0);
+  }
+  if (!(lo | hi)) return 0.0;
+  const int lz = hi ? __clzll(hi) : 64 + __clzll(lo);
+  if (lz >= 64) {
+    hi = lo << (lz - 64);
+    lo = 0;
+  } else if (lz > 0) {
+    hi = hi << lz | lo >> (64 - lz);
+    lo <<= lz;
+  }
+  // value = hi.lo 2^(64 - lz) with the top bit of hi set: 53 bits kept
+  unsigned long long m = hi >> 11;
+  const unsigned long long rest = (hi & 0x7ff) << 1 | (lo != 0);
+  m += rest > 0x800 || (rest == 0x800 && (m & 1));
+  // m in [2^52, 2^53]; value m 2^(75 - lz + e)
+  const int field = 75 - lz + e + 1075;
+  double v;
+  if (field >= 1 && field <= 2045) {
+    v = __longlong_as_double((long long)(((unsigned long long)field << 52) +
+                                         (m - (1ULL << 52))));
+  } else {
+    v = ldexp((double)m, 75 - lz + e);
+  }
+  return __hiloint2double(__double2hiint(v) | (int)(neg << 31), __double2loint(v));
+}
+
+// X 2^e for the integer product X with residues r (one byte per modulus, four
+// moduli per word): X = sum_l y_l P/p_l - k P, byte position by byte position
+// (__dp4a sums four moduli), then 16-bit pieces and 32-bit words with carries.
+__device__ __forceinline__ double combine(uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3,
+                                          int e) {
+  int s[16];
+#pragma unroll
+  for (int b = 0; b < 15; ++b)
+    s[b] = dp4a_su(r3, c_tab.w[b][3],
+                   dp4a_su(r2, c_tab.w[b][2],
+                           dp4a_su(r1, c_tab.w[b][1], dp4a_su(r0, c_tab.w[b][0], 0))));
+  s[15] = 0;
+  // k = nearest integer to (sum of y_l P / p_l) / P; the product is below P / 4
+  const float f = fmaf((float)s[12], 1.0f / 65536.0f,
+                       fmaf((float)s[13], 1.0f / 256.0f, (float)s[14]));
+  const int k = __float2int_rn(f * c_tab.top);
+  long long w[4];
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    const int u0 = s[4 * a] + (s[4 * a + 1] << 8) - k * c_tab.p16[2 * a];
+    const int u1 = s[4 * a + 2] + (s[4 * a + 3] << 8) - k * c_tab.p16[2 * a + 1];
+    w[a] = (long long)u1 * 65536 + u0;
+  }
+  w[1] += w[0] >> 32;
+  w[2] += w[1] >> 32;
+  w[3] += w[2] >> 32;
+  return to_double((uint32_t)w[0], (uint32_t)w[1], (uint32_t)w[2], (uint32_t)w[3], e);
+}
+
+}  // namespace
+}  // namespace crt
+}  // namespace slu

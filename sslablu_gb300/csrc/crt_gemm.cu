@@ -34,89 +34,21 @@
 //
 // Work per element of A and B: 16 residues at ~9 integer / float32 slots;
 // per element of C: 16 x 2K bfloat16 flops, 16 bytes and ~220 slots of step
-// 3.  At 1024^3 that is 34 tensor GFLOP (~25 us) beside ~8 us of conversion
-// and ~6 us of reconstruction, against 2.1 ms on the float64 pipe.
+// 3.  Two 1024^3 products: 42 us of conversion, 61 of products (1.1 PFLOP/s on
+// the tensor cores) and 24 of reconstruction, against 4.1 ms on the float64
+// pipe.
 #include <cuda.h>
-#include <cuda_bf16.h>
 
 #include <algorithm>
 #include <mutex>
 
+#include "crt.cuh"
 #include "hbs.cuh"
 
 namespace slu {
 namespace {
 
-constexpr int NM = 16;   // moduli
-struct Tables {
-  int p[NM];
-  float pf[NM], inv[NM];
-  uint32_t ca[2][NM], cb[2][NM];   // balanced 2^(8 i) mod p (A), times (P/p)^-1 (B), packed bytes
-  int ba[NM], bb[NM];              // -(2^59) mod p (A), times (P/p)^-1 (B)
-  uint32_t w[15][NM / 4];          // byte i of P/p_l, four moduli packed
-  int p16[8];                      // P in 16-bit pieces
-  float top;                       // 2^112 / P
-};
-
-constexpr unsigned long long mod_pow2(int e, int p) {
-  unsigned long long r = 1;
-  for (int i = 0; i < e; ++i) r = r * 2 % p;
-  return r;
-}
-constexpr int balanced(int v, int p) { return 2 * v > p ? v - p : v; }
-
-constexpr Tables make_tables() {
-  Tables T{};
-  const int p[NM] = {256, 253, 251, 249, 247, 245, 241, 239, 233, 229, 227, 223, 211, 199, 197, 193};
-  unsigned __int128 P = 1;
-  for (int l = 0; l < NM; ++l) P *= (unsigned)p[l];
-  for (int l = 0; l < NM; ++l) {
-    T.p[l] = p[l];
-    T.pf[l] = (float)p[l];
-    T.inv[l] = 1.0f / (float)p[l];
-    const unsigned __int128 W = P / (unsigned)p[l];
-    const int wm = (int)(W % (unsigned)p[l]);
-    int m = 1;   // inverse of P/p modulo p
-    while (m * wm % p[l] != 1) ++m;
-    for (int i = 0; i < 8; ++i) {
-      const int c = (int)mod_pow2(8 * i, p[l]);
-      // p = 256: 128 is its own balanced form's limit; store -128
-      int a = balanced(c, p[l]), b = balanced(c * m % p[l], p[l]);
-      if (a == 128) a = -128;
-      if (b == 128) b = -128;
-      T.ca[i / 4][l] |= (uint32_t)(uint8_t)a << (8 * (i % 4));
-      T.cb[i / 4][l] |= (uint32_t)(uint8_t)b << (8 * (i % 4));
-    }
-    const int h = (int)mod_pow2(59, p[l]);
-    T.ba[l] = -h;
-    T.bb[l] = -(h * m % p[l]);
-    for (int i = 0; i < 15; ++i)
-      T.w[i][l / 4] |= (uint32_t)(uint8_t)(W >> (8 * i)) << (8 * (l % 4));
-  }
-  for (int i = 0; i < 8; ++i) T.p16[i] = (int)(uint16_t)(P >> (16 * i));
-  T.top = (float)(5192296858534827628530496329220096.0 / (double)P);   // 2^112 / P
-  return T;
-}
-__constant__ Tables c_tab = make_tables();
-
-// Largest |a'| exponent for products of depth K: |X| <= K 2^(2t) <= 2^123 < P / 4.
-int bits_for(int K) {
-  int lg = 0;
-  while ((1LL << lg) < K) ++lg;
-  return (123 - lg) / 2;
-}
-
-// dp4a of unsigned bytes of a with signed bytes of b, and the reverse
-__device__ __forceinline__ int dp4a_us(uint32_t a, uint32_t b, int c) {
-  int d;
-  asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-  return d;
-}
-__device__ __forceinline__ int dp4a_su(uint32_t a, uint32_t b, int c) {
-  int d;
-  asm("dp4a.s32.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-  return d;
-}
+using namespace crt;
 
 // ---------------------------------------------------------------- conversion
 struct CrtOperand {
@@ -129,96 +61,102 @@ struct CrtOperand {
   int* ex;               // exponent field per [batch][row]; 2047 = not finite
 };
 
-constexpr int kStrip = 8;                     // rows per CTA
-constexpr int kChunkK = 256;                  // k per staged chunk
-constexpr int kPitch = kChunkK + kChunkK / 8; // one pad every 8 values: conflict-free
-
-// a CTA converts kStrip rows over the whole depth: exponents first (one
-// pass), then residues chunk by chunk through shared memory, which also
-// turns k-strided operands around.  Eight k per thread and modulus: 16-byte
-// stores.  Bound by the ~150 integer / float32 slots per element.
-__global__ void __launch_bounds__(256)
+// A CTA converts ROWS rows, 2048 / ROWS consecutive k at a time (32, 16 or 8
+// rows, so that operands 64 or 128 deep keep every thread busy), through
+// shared memory, which also turns k-strided operands around.  Eight k per
+// thread and modulus: 16-byte stores.  One chunk: the exponents come from the
+// staged values; more: one pass over the rows before.  ~190 instructions per
+// element; 4 M elements (two 1024 x 1024 pairs): 42 us; 128 x (64 + 261) rows
+// of 64: 29 us (88 with 8 rows per CTA, which leaves most threads idle).
+template <int ROWS>
+__global__ void __launch_bounds__(256, 2)
 crt_convert_kernel(CrtOperand a, CrtOperand b, int strips_a, int K, int Kp, int t, int batch0,
                    int batch) {
-  __shared__ long long tile[kStrip * kPitch];
-  __shared__ int s_ex[kStrip];
-  __shared__ int s_red[8][kStrip];
+  constexpr int KC = 2048 / ROWS, G = KC / 8;   // k per chunk; threads per row
+  constexpr int P = KC + KC / 8 + 1;            // a pad every 8 values, rows one bank apart
+  __shared__ uint2 tile[ROWS * P];
+  __shared__ int s_ex[ROWS];
   const bool second = (int)blockIdx.x >= strips_a;
   const CrtOperand& o = second ? b : a;
-  const int r0 = (second ? blockIdx.x - strips_a : blockIdx.x) * kStrip;
+  const int r0 = (second ? blockIdx.x - strips_a : blockIdx.x) * ROWS;
   const int bt = blockIdx.y, b0 = bt % batch0, b1 = bt / batch0;
-  const long long* x = reinterpret_cast<const long long*>(o.x + b0 * o.s0 + b1 * o.s1);
+  const uint2* x = reinterpret_cast<const uint2*>(o.x + b0 * o.s0 + b1 * o.s1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int nr = min(kStrip, o.rows - r0);
-  // ---- exponent field of every row
-  int f = 0;
-  if (o.kcontig) {
-    if (warp < nr) {
-      const long long* row = x + (long long)(r0 + warp) * o.ld;
-      for (int k = lane; k < K; k += 32) f = max(f, (int)((row[k] >> 52) & 0x7ff));
-    }
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) f = max(f, __shfl_xor_sync(0xffffffffu, f, s));
-    if (lane == 0) s_ex[warp] = f;
-  } else {
-    const int r = tid & 7;
-    if (r < nr) {
-      const long long* col = x + r0 + r;
-      for (int k = tid >> 3; k < K; k += 32)
-        f = max(f, (int)((col[(long long)k * o.ld] >> 52) & 0x7ff));
-    }
-    f = max(f, __shfl_xor_sync(0xffffffffu, f, 8));
-    f = max(f, __shfl_xor_sync(0xffffffffu, f, 16));
-    if (lane < 8) s_red[warp][lane] = f;
-    __syncthreads();
-    if (tid < 8) {
-      int g = 0;
-      for (int w = 0; w < 8; ++w) g = max(g, s_red[w][tid]);
-      s_ex[tid] = g;
-    }
-  }
-  __syncthreads();
-  if (tid < nr) o.ex[(long long)bt * o.rows + r0 + tid] = s_ex[tid];
-  // ---- residues
-  const int row = warp, k8 = 8 * lane;
-  const int F = max(s_ex[row], 1);
-  const bool live = row < nr, finite = s_ex[row] != 0x7ff;
-  const long long plane = (long long)batch * o.rows * Kp;
-  __nv_bfloat16* dst = o.out + ((long long)bt * o.rows + r0 + row) * Kp + k8;
-  for (int kc = 0; kc < Kp; kc += kChunkK) {
-    const int kn = min(kChunkK, K - kc);   // may be <= 0 in the padding
+  const int nr = min(ROWS, o.rows - r0);
+  const bool single = Kp <= KC;
+  if (!single) {
+    // exponent field of every row (ROWS = 8 here: one warp per row)
+    if (tid < ROWS) s_ex[tid] = 0;
     __syncthreads();
     if (o.kcontig) {
-      for (int k = lane; k < kChunkK; k += 32)
-        tile[warp * kPitch + k + (k >> 3)] =
-            (live && k < kn) ? x[(long long)(r0 + warp) * o.ld + kc + k] : 0;
+      for (int r = warp; r < nr; r += 8) {
+        const uint2* row = x + (long long)(r0 + r) * o.ld;
+        int f = 0;
+        for (int k = lane; k < K; k += 32) f = max(f, (int)(row[k].y & 0x7fffffffu));
+        f = __reduce_max_sync(0xffffffffu, f);
+        if (lane == 0) s_ex[r] = f >> 20;
+      }
     } else {
-      const int r = tid & 7;
-      for (int k = tid >> 3; k < kChunkK; k += 32)
-        tile[r * kPitch + k + (k >> 3)] =
-            (r < nr && k < kn) ? x[(long long)(kc + k) * o.ld + r0 + r] : 0;
+      const int r = tid % ROWS;
+      if (r < nr) {
+        const uint2* col = x + r0 + r;
+        int f = 0;
+        for (int k = tid / ROWS; k < K; k += 256 / ROWS)
+          f = max(f, (int)(col[(long long)k * o.ld].y & 0x7fffffffu));
+        atomicMax(&s_ex[r], f >> 20);
+      }
+    }
+  }
+  const int row = tid / G, kq = tid % G;
+  const bool live = row < nr;
+  const long long plane = (long long)batch * o.rows * Kp;
+  __nv_bfloat16* dst = o.out + ((long long)bt * o.rows + r0 + row) * Kp + 8 * kq;
+  for (int kc = 0; kc < Kp; kc += KC) {
+    const int kn = min(KC, K - kc);   // may be <= 0 in the padding
+    __syncthreads();
+    // eight values per thread, all loads before the first store
+    uint2 v[8];
+    if (o.kcontig) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int r = (tid + 256 * i) / KC, k = (tid + 256 * i) % KC;
+        v[i] = (r < nr && k < kn) ? x[(long long)(r0 + r) * o.ld + kc + k] : make_uint2(0, 0);
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int r = (tid + 256 * i) / KC, k = (tid + 256 * i) % KC;
+        tile[r * P + k + (k >> 3)] = v[i];
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int r = tid % ROWS, k = (tid + 256 * i) / ROWS;
+        v[i] = (r < nr && k < kn) ? x[(long long)(kc + k) * o.ld + r0 + r] : make_uint2(0, 0);
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int r = tid % ROWS, k = (tid + 256 * i) / ROWS;
+        tile[r * P + k + (k >> 3)] = v[i];
+      }
     }
     __syncthreads();
-    if (!live || kc + k8 >= Kp) continue;
+    const uint2* src = tile + row * P + 9 * kq;
+    int ex;
+    if (single) {
+      ex = 0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) ex = max(ex, (int)((src[u].y >> 20) & 0x7ff));
+#pragma unroll
+      for (int s = G / 2; s > 0; s >>= 1) ex = max(ex, __shfl_xor_sync(0xffffffffu, ex, s));
+    } else {
+      ex = s_ex[row];
+    }
+    if (kc == 0 && kq == 0 && live) o.ex[(long long)bt * o.rows + r0 + row] = ex;
+    if (!live || kc + 8 * kq >= Kp) continue;
     uint32_t lo[8], hi[8];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const long long v = tile[row * kPitch + 9 * lane + u];
-      const int fe = (int)((v >> 52) & 0x7ff);
-      unsigned long long m = (unsigned long long)v & 0xfffffffffffffULL;
-      if (fe) m |= 1ULL << 52;
-      // a' = m 2^(t - 53 - (F - max(fe, 1))), rounded to nearest
-      const int sh = t - 53 - (F - max(fe, 1));
-      unsigned long long q;
-      if (sh >= 0) q = m << sh;
-      else if (sh > -55) q = (m + (1ULL << (-sh - 1))) >> -sh;
-      else q = 0;
-      if (!finite) q = 0;
-      // shifted by 2^59 to be non-negative (the tables take it off again)
-      const unsigned long long z = v < 0 ? (1ULL << 59) - q : (1ULL << 59) + q;
-      lo[u] = (uint32_t)z;
-      hi[u] = (uint32_t)(z >> 32);
-    }
+    for (int u = 0; u < 8; ++u)
+      scaled(src[u].y, src[u].x, max(ex, 1), t, ex != 0x7ff, lo[u], hi[u]);
 #pragma unroll
     for (int l = 0; l < NM; ++l) {
       const uint32_t c0 = second ? c_tab.cb[0][l] : c_tab.ca[0][l];
@@ -227,19 +165,9 @@ crt_convert_kernel(CrtOperand a, CrtOperand b, int strips_a, int K, int Kp, int 
       const float p = c_tab.pf[l], ip = c_tab.inv[l];
       uint32_t w[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        float r[2];
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          // |s| < 2^19: exact as the low bits of a float of magnitude 1.5 2^23
-          const int s = dp4a_us(lo[2 * u + e], c0, dp4a_us(hi[2 * u + e], c1, bias));
-          const float g = __int_as_float(s) - 12582912.f;
-          const float q = fmaf(g, ip, 12582912.f) - 12582912.f;
-          r[e] = fmaf(-p, q, g);
-        }
-        const __nv_bfloat162 h = __floats2bfloat162_rn(r[0], r[1]);
-        w[u] = *reinterpret_cast<const uint32_t*>(&h);
-      }
+      for (int u = 0; u < 4; ++u)
+        w[u] = pack_bf16(residue(lo[2 * u], hi[2 * u], c0, c1, bias, p, ip),
+                         residue(lo[2 * u + 1], hi[2 * u + 1], c0, c1, bias, p, ip));
       *reinterpret_cast<uint4*>(dst + l * plane + kc) = make_uint4(w[0], w[1], w[2], w[3]);
     }
   }
@@ -491,8 +419,7 @@ crt_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             for (int e = 0; e < 16; ++e) {
               float x = __uint_as_float(v[e]);
               if (c > 0) x += (float)(int8_t)(old[e >> 2] >> (8 * (e & 3)));
-              const float k = fmaf(x, ip, 12582912.f) - 12582912.f;
-              const uint32_t y = __float_as_uint(fmaf(-p, k, x) + 12582912.f) & 0xffu;
+              const uint32_t y = reduced(x, p, ip) & 0xffu;
               w[e >> 2] = (e & 3) ? w[e >> 2] | (y << (8 * (e & 3))) : y;
             }
             *dst = make_uint4(w[0], w[1], w[2], w[3]);
@@ -531,6 +458,8 @@ struct CrtCombine {
   const int *ea, *eb;
   int t;
   double alpha, beta;
+  int kind;   // alpha, beta: 0 = 1, 0; 1 = -1, 0; 2 = 1, 1; 3 = -1, 1; 4 = any (a float64 compare
+              // costs as much as 30 integer instructions)
   double* C;
   int ldc;
   long long sC0, sC1;
@@ -538,40 +467,6 @@ struct CrtCombine {
   const double *A, *B;
   long long ak, ai, sA0, sA1, bk, bj, sB0, sB1;   // strides along k, i, j
 };
-
-// 128-bit two's complement value c3:c2:c1:c0 times 2^e, rounded to nearest even
-__device__ __forceinline__ double to_double(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3,
-                                            int e) {
-  unsigned long long lo = (unsigned long long)c1 << 32 | c0, hi = (unsigned long long)c3 << 32 | c2;
-  const uint32_t neg = c3 >> 31;
-  if (neg) {
-    lo = ~lo + 1;
-    hi = ~hi + (lo == 0);
-  }
-  if (!(lo | hi)) return 0.0;
-  const int lz = hi ? __clzll(hi) : 64 + __clzll(lo);
-  if (lz >= 64) {
-    hi = lo << (lz - 64);
-    lo = 0;
-  } else if (lz > 0) {
-    hi = hi << lz | lo >> (64 - lz);
-    lo <<= lz;
-  }
-  // value = hi.lo 2^(64 - lz) with the top bit of hi set: 53 bits kept
-  unsigned long long m = hi >> 11;
-  const unsigned long long rest = (hi & 0x7ff) << 1 | (lo != 0);
-  m += rest > 0x800 || (rest == 0x800 && (m & 1));
-  // m in [2^52, 2^53]; value m 2^(75 - lz + e)
-  const int field = 75 - lz + e + 1075;
-  double v;
-  if (field >= 1 && field <= 2045) {
-    v = __longlong_as_double((long long)(((unsigned long long)field << 52) +
-                                         (m - (1ULL << 52))));
-  } else {
-    v = ldexp((double)m, 75 - lz + e);
-  }
-  return neg ? -v : v;
-}
 
 // One thread per four consecutive elements of a row of C: four bytes of every
 // residue plane, transposed in registers so a __dp4a sums four moduli.
@@ -612,35 +507,16 @@ crt_combine_kernel(const __grid_constant__ CrtCombine g) {
         v = 0.0;
         for (int k = 0; k < g.K; ++k) v = fma(ap[k * g.ak], bp[k * g.bk], v);
       } else {
-        int s[16];
-#pragma unroll
-        for (int b = 0; b < 15; ++b) {
-          s[b] = 0;
-#pragma unroll
-          for (int a = 0; a < NM / 4; ++a) s[b] = dp4a_su(r[4 * a + e], c_tab.w[b][a], s[b]);
-        }
-        s[15] = 0;
-        // k = nearest integer to (sum of y_l P / p_l) / P; the product is below P / 4
-        const float f = fmaf((float)s[12], 1.0f / 65536.0f,
-                             fmaf((float)s[13], 1.0f / 256.0f, (float)s[14]));
-        const int k = __float2int_rn(f * c_tab.top);
-        // 16-bit pieces, then 32-bit words with carries
-        long long w[4];
-#pragma unroll
-        for (int a = 0; a < 4; ++a) {
-          const int u0 = s[4 * a] + (s[4 * a + 1] << 8) - k * c_tab.p16[2 * a];
-          const int u1 = s[4 * a + 2] + (s[4 * a + 3] << 8) - k * c_tab.p16[2 * a + 1];
-          w[a] = (long long)u1 * 65536 + u0;
-        }
-        w[1] += w[0] >> 32;
-        w[2] += w[1] >> 32;
-        w[3] += w[2] >> 32;
-        v = to_double((uint32_t)w[0], (uint32_t)w[1], (uint32_t)w[2], (uint32_t)w[3],
-                      max(fa, 1) + max(fb, 1) - 2 * (1022 + g.t));
+        v = combine(r[e], r[4 + e], r[8 + e], r[12 + e],
+                    max(fa, 1) + max(fb, 1) - 2 * (1022 + g.t));
       }
-      if (g.alpha == -1.0) v = -v;
-      else if (g.alpha != 1.0) v *= g.alpha;
-      if (g.beta != 0.0) v = fma(g.beta, c[e], v);
+      if (g.kind == 4) {
+        v *= g.alpha;
+        if (g.beta != 0.0) v = fma(g.beta, c[e], v);
+      } else {
+        if (g.kind & 1) v = __hiloint2double((int)(hi32(v) ^ 0x80000000u), __double2loint(v));
+        if (g.kind & 2) v = c[e] + v;
+      }
       c[e] = v;
     }
   }
@@ -715,9 +591,14 @@ void crt_piece(Handle& h, int M, int N, int K, double alpha, const Operand& A, c
   int* eb = h.gemm_ws.take<int>((size_t)batch * N);
   const CrtOperand oa{A.x, A.ld, A.s0, A.s1, M, !A.trans, ra, ea};
   const CrtOperand ob{B.x, B.ld, B.s0, B.s1, N, B.trans, rb, eb};
-  const int sa = (M + kStrip - 1) / kStrip, sb = (N + kStrip - 1) / kStrip;
-  crt_convert_kernel<<<dim3(sa + sb, batch), 256, 0, st>>>(oa, ob, sa, K, Kp, t, batch0, batch);
-  check_launch("crt_convert_kernel");
+  auto convert = [&](auto kern, int rows) {
+    const int sa = (M + rows - 1) / rows, sb = (N + rows - 1) / rows;
+    kern<<<dim3(sa + sb, batch), 256, 0, st>>>(oa, ob, sa, K, Kp, t, batch0, batch);
+    check_launch("crt_convert_kernel");
+  };
+  if (Kp <= 64) convert(crt_convert_kernel<32>, 32);
+  else if (Kp <= 128) convert(crt_convert_kernel<16>, 16);
+  else convert(crt_convert_kernel<8>, 8);
   CrtGemm g{};
   g.M = M;
   g.N = N;
@@ -756,6 +637,9 @@ void crt_piece(Handle& h, int M, int N, int K, double alpha, const Operand& A, c
   c.t = t;
   c.alpha = alpha;
   c.beta = beta;
+  c.kind = (alpha != 1.0 && alpha != -1.0) || (beta != 0.0 && beta != 1.0)
+               ? 4
+               : (alpha == -1.0 ? 1 : 0) + (beta == 1.0 ? 2 : 0);
   c.C = C;
   c.ldc = ldc;
   c.sC0 = sC0;

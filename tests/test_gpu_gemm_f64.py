@@ -29,7 +29,8 @@ def _gemm(A, B, C, ta, tb, alpha, beta):
 # several chunks of depth, both orientations of both operands
 SHAPES = [(1, 64, 2600, 64, 0, 0), (2, 128, 256, 256, 0, 1), (1, 129, 257, 320, 1, 0),
           (3, 333, 97, 385, 1, 1), (1, 200, 65, 1024, 0, 0), (1, 130, 72, 1153, 1, 0),
-          (1, 257, 33, 4097, 0, 1), (5, 191, 47, 512, 0, 0), (1, 127, 49, 9000, 1, 1)]
+          (1, 257, 33, 4097, 0, 1), (5, 191, 47, 512, 0, 0), (1, 127, 49, 9000, 1, 1),
+          (2, 300, 200, 100, 0, 0), (2, 210, 301, 113, 1, 1), (9, 177, 261, 64, 1, 1)]
 
 
 @pytest.mark.parametrize("nb,M,N,K,ta,tb", SHAPES)
@@ -58,7 +59,7 @@ def test_integer_products_are_exact(nb, M, N, K, ta, tb):
         np.testing.assert_allclose(got, want, rtol=0, atol=2e-16 * float(np.abs(want).max()) * 3)
 
 
-@pytest.mark.parametrize("nb,M,N,K,ta,tb", SHAPES[1:6])
+@pytest.mark.parametrize("nb,M,N,K,ta,tb", SHAPES[1:6] + SHAPES[9:])
 def test_gaussian_products(nb, M, N, K, ta, tb):
     need_gpu()
     import torch
