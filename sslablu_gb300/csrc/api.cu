@@ -77,7 +77,13 @@ int slu_sync(slu_handle_t h) {
     SLU_CHECK_CUDA(cudaMemcpy(info, h->h.info.p, sizeof(info), cudaMemcpyDeviceToHost));
   });
   if (st != SLU_OK) return st;
-  if (info[1] != 0) {
+  bool plan_err = false;
+  for (const auto& w : h->h.plan_err)
+    if (const auto p = w.lock()) {
+      plan_err = plan_err || *p;
+      *p = 0;
+    }
+  if (info[1] != 0 || plan_err) {
     cudaMemset(h->h.info.p, 0, sizeof(info));
     g_err = "a tensor-core GEMM gave up waiting on its TMA / MMA pipeline";
     h->h.last_error = g_err;
@@ -192,6 +198,7 @@ int slu_hbs_set_level(slu_handle_t h, slu_hbs_t op, int level, int Nb, int n, in
       H.has_ulv = false;
       H.has_sweep = false;
       H.has_oz = H.has_ozT = false;
+      H.drop_crt();
       H.has_f32 = false;
       H.has_dfs = false;
       H.has_df = false;
@@ -239,6 +246,7 @@ int slu_hbs_set_ulv_level(slu_handle_t h, slu_hbs_t op, int level, const double*
     H.has_dfs = false;
     H.has_sweep = false;
     H.has_oz = H.has_ozT = false;
+    H.drop_crt();
     H.invalidate_plans();
     if (all) slu::hbs_make_sweep(h->h, H);
   });
@@ -273,14 +281,17 @@ int slu_ulv_solve_into(slu_handle_t h, slu_hbs_t op, const double* X, int ldx, d
   return guard(h, [&] {
     SLU_REQUIRE(h && op && X && Y, "null argument");
     SLU_REQUIRE(nrhs >= 1 && ldx >= nrhs && ldy >= nrhs, "bad right-hand side shape");
-    const slu::Hbs& H = op->H;
+    slu::Hbs& H = op->H;
     SLU_REQUIRE(H.has_ulv, "HBS operator has no ULV factorisation");
     cudaStream_t st = h->h.stream;
+    const bool crt = slu::crt_prepare(h->h, H, true, trans != 0, nrhs);
     const size_t bytes = slu::hbs_solve_scratch_bytes(H, nrhs, sizeof(double));
     h->h.ws.reserve(bytes + 256, st);
     double* scratch = h->h.ws.take<double>(bytes / sizeof(double));
     const size_t stride = ((sizeof(double) * (size_t)H.N * nrhs + 255) & ~size_t(255)) / 8;
-    if (trans) slu::ulv_solve_T<double>(st, H, Y, ldy, nrhs, scratch, stride, X, ldx);
+    if (crt)
+      slu::crt_solve(st, H, trans != 0, X, ldx, Y, ldy, nrhs, scratch, stride, h->h.err_word());
+    else if (trans) slu::ulv_solve_T<double>(st, H, Y, ldy, nrhs, scratch, stride, X, ldx);
     else slu::ulv_solve_fused<double>(st, H, Y, ldy, nrhs, scratch, stride, nullptr, X, ldx);
   });
 }

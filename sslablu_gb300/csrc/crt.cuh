@@ -87,21 +87,20 @@ __device__ __forceinline__ int dp4a_su(uint32_t a, uint32_t b, int c) {
 __device__ __forceinline__ uint32_t hi32(double v) { return (uint32_t)__double2hiint(v); }
 
 // A float64 (its bits) whose exponent field is at most F (>= 1) as a t-bit
-// integer, rounded to nearest and shifted by 2^59 to be non-negative (the
-// tables take the shift off again); ok = false gives zero.
+// integer (t <= 59), rounded to nearest and shifted by 2^59 to be non-negative
+// (the tables take the shift off again); ok = false gives zero.
 __device__ __forceinline__ void scaled(uint32_t hi, uint32_t lo, int F, int t, bool ok,
                                        uint32_t& zlo, uint32_t& zhi) {
   const int fe = (int)((hi >> 20) & 0x7ff);
-  unsigned long long m = (unsigned long long)(hi & 0xfffffu) << 32 | lo;
-  if (fe) m |= 1ULL << 52;
-  // a' = m 2^(t - 53 - (F - max(fe, 1)))
-  const int sh = t - 53 - (F - max(fe, 1));
-  unsigned long long q;
-  if (sh >= 0) q = m << sh;
-  else if (sh > -55) q = (m + (1ULL << (-sh - 1))) >> -sh;
-  else q = 0;
-  if (!ok) q = 0;
-  const unsigned long long z = (hi >> 31) ? (1ULL << 59) - q : (1ULL << 59) + q;
+  // the mantissa from bit 63 down: |a'| = m 2^-(s + 1), rounded half away
+  const uint32_t mh = (__funnelshift_l(lo, hi, 11) & 0x7fffffffu) | (fe ? 0x80000000u : 0u);
+  const uint32_t ml = lo << 11;
+  const int s = ok ? 63 - t + F - max(fe, 1) : 64;
+  const uint32_t ql = s < 32 ? __funnelshift_r(ml, mh, s) : (s < 64 ? mh >> (s - 32) : 0u);
+  const uint32_t qh = s < 32 ? mh >> s : 0u;
+  const unsigned long long q = (((unsigned long long)qh << 32 | ql) + 1) >> 1;
+  const unsigned long long sg = (long long)(int)hi >> 63;
+  const unsigned long long z = (q ^ sg) + ((1ULL << 59) - sg);
   zlo = (uint32_t)z;
   zhi = (uint32_t)(z >> 32);
 }
@@ -127,15 +126,10 @@ __device__ __forceinline__ uint32_t reduced(float x, float p, float ip) {
   return __float_as_uint(fmaf(-p, k, x) + 12582912.f);
 }
 
-// 128-bit two's complement value c3:c2:c1:c0 times 2^e, rounded to nearest even
+// The magnitude c3:c2:c1:c0 times 2^e, rounded to nearest even, with a sign
 __device__ __forceinline__ double to_double(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3,
-                                            int e) {
+                                            int e, uint32_t neg) {
   unsigned long long lo = (unsigned long long)c1 << 32 | c0, hi = (unsigned long long)c3 << 32 | c2;
-  const uint32_t neg = c3 >> 31;
-  if (neg) {
-    lo = ~lo + 1;
-    hi = ~hi + (lo == 0);
-  }
   if (!(lo | hi)) return 0.0;
   const int lz = hi ? __clzll(hi) : 64 + __clzll(lo);
   if (lz >= 64) {
@@ -187,7 +181,27 @@ __device__ __forceinline__ double combine(uint32_t r0, uint32_t r1, uint32_t r2,
   w[1] += w[0] >> 32;
   w[2] += w[1] >> 32;
   w[3] += w[2] >> 32;
-  return to_double((uint32_t)w[0], (uint32_t)w[1], (uint32_t)w[2], (uint32_t)w[3], e);
+  uint32_t x0 = (uint32_t)w[0], x1 = (uint32_t)w[1], x2 = (uint32_t)w[2], x3 = (uint32_t)w[3];
+  // nearly always the magnitude is 2^96 or more and the result a normal number
+  const uint32_t neg = x3 >> 31;
+  if (neg) {
+    x0 = ~x0 + 1;
+    x1 = ~x1 + (x0 == 0);
+    x2 = ~x2 + ((x0 | x1) == 0);
+    x3 = ~x3 + ((x0 | x1 | x2) == 0);
+  }
+  const int lz = __clz(x3), field = 1023 + 127 + e - lz;
+  if (x3 == 0 || field < 1 || field > 2045)
+    return to_double(x0, x1, x2, x3, e, neg);
+  // the top bit to bit 31 of a; what is below b as its lowest bit
+  const uint32_t a = __funnelshift_l(x2, x3, lz);
+  const uint32_t b = __funnelshift_l(x1, x2, lz) | ((x1 << lz | x0) != 0);
+  const uint32_t lo = __funnelshift_r(b, a, 11);
+  const uint32_t up = (b & 0x7ff) + (lo & 1) > 0x400;
+  // m in [2^52, 2^53]; value m 2^(field - 1075)
+  const unsigned long long m = ((unsigned long long)(a >> 11) << 32 | lo) + up;
+  return __longlong_as_double(
+      (long long)((((unsigned long long)(field - 1) << 52) + m) | (unsigned long long)neg << 63));
 }
 
 }  // namespace

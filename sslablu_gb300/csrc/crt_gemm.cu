@@ -616,7 +616,7 @@ void crt_piece(Handle& h, int M, int N, int K, double alpha, const Operand& A, c
   g.items = (long long)NM * batch * g.tm * g.tn;
   g.R = R;
   g.pitch = pitch;
-  g.err = reinterpret_cast<unsigned int*>(h.info.as<int>()) + 1;
+  g.err = h.err_word();
   const CUtensorMap ma = residue_map(ra, (long long)NM * batch * M, Kp, BM);
   const CUtensorMap mb = residue_map(rb, (long long)NM * batch * N, Kp, g.BN);
   const size_t sm = (size_t)g.stages * (A_BYTES + g.BN * BK * 2) + 1024;

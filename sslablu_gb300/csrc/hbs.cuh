@@ -4,6 +4,8 @@
 #include "dfloat.cuh"
 #include "slablu_internal.cuh"
 
+#include <cuda_bf16.h>
+
 #include <mutex>
 
 namespace slu {
@@ -67,6 +69,10 @@ struct Handle {
   Workspace lu_ws;     // permutations and triangles of lu_factor / lu_inverse
   HostStage upload, readback;
   DevBuf info;  // int[64] device status words
+  // set by a tensor-core kernel whose waits ran out (slu_sync reports it)
+  unsigned int* err_word() const { return info.as<unsigned int>() + 1; }
+  // the same words of the solve plans launched on this handle
+  std::vector<std::weak_ptr<volatile unsigned>> plan_err;
   std::string last_error;
 };
 
@@ -104,6 +110,16 @@ struct OzOp {
   int NT = 0, wP = 0, ntile = 0;
 };
 
+// A step operator as residue images for the exact tensor-core steps
+// (crt_step.cu): per (block, row tile of RT rows, modulus) one RT x wP bfloat16
+// image in core-matrix order; ex holds every row's largest exponent field.
+struct CrtOp {
+  const __nv_bfloat16* img = nullptr;   // into Hbs::crt_buf
+  const int* ex = nullptr;
+  int Nb = 0, rows = 0, w = 0;
+  int RT = 0, wP = 0, ntile = 0;
+};
+
 struct Level {
   int Nb = 0;   // blocks on this level
   int n = 0;    // rows (and columns of D) per block
@@ -135,6 +151,8 @@ struct Level {
   // and of the transposed solve and apply: Q, SwT (the root: SwT), AupT,
   // AdnT (the root: AdnT)
   OzOp ozQ, ozSwT, ozUpT, ozDnT;
+  // residue images of the solve and apply steps (crt_step.cu)
+  CrtOp crQt, crSw, crQ, crSwT, crUp, crDn, crUpT, crDnT;
 };
 
 struct RefinePlan;  // refine.cu: buffers + CUDA graphs of one refinement iteration
@@ -171,6 +189,16 @@ struct Hbs {
   // set only after the composing stream has finished (other threads may read
   // them from their own streams right after)
   std::atomic<bool> has_apply[2] = {false, false};
+  // residue images (crt_step.cu) of the solve N, T and the apply N, T; made on
+  // first use, likewise
+  std::atomic<bool> has_crt[4] = {false, false, false, false};
+  DevBuf crt_buf[4];
+  void drop_crt() {
+    for (int i = 0; i < 4; ++i) {
+      has_crt[i] = false;
+      crt_buf[i].release();
+    }
+  }
   std::mutex lazy_mu;   // serialises first-use composition across threads
   // inner sweep of the mixed-precision refinement: 0 float32, 1 double-float,
   // 2 tensor-core digit sweep with a tensor-core digit residual (ozaki.cu)
@@ -204,6 +232,9 @@ struct SolvePlan {
   std::vector<std::weak_ptr<char>> alive;
   std::vector<unsigned long long> gen;
   DevBuf scratch;
+  // mapped host word of the captured tensor-core kernels (the plan may outlive
+  // the handle it was made on)
+  std::shared_ptr<volatile unsigned> err;
   cudaGraphExec_t exec = nullptr;
   long long kernels = 0;
   SolvePlan() = default;
@@ -213,7 +244,7 @@ struct SolvePlan {
     if (exec) cudaGraphExecDestroy(exec);
   }
 };
-void solve_plan_create(Handle& h, const Hbs& H, const double* X, int ldx, double* Y, int ldy,
+void solve_plan_create(Handle& h, Hbs& H, const double* X, int ldx, double* Y, int ldy,
                        int c, bool trans, SolvePlan& P);
 void solve_plan_launch(Handle& h, SolvePlan& P, bool wait);
 // The grouped mode-N solve of hbs_solve_grouped (B[i] <- A_i^{-1} B[i]) for
@@ -256,7 +287,7 @@ void hbs_apply(Handle& h, Hbs& H, bool trans, const double* X, int ldx, double* 
                int ldy, int nrhs);
 // ULV solve, reference semantics of HBSMAT.solve (with the permutation)
 template <typename T>
-void hbs_solve(Handle& h, const Hbs& H, bool trans, T* B, int ldb, int nrhs);
+void hbs_solve(Handle& h, Hbs& H, bool trans, T* B, int ldb, int nrhs);
 // The same solve with caller-provided scratch of hbs_solve_scratch_bytes()
 // bytes (256-byte aligned); it makes no allocation of its own.
 template <typename T>
@@ -344,6 +375,18 @@ void hbs_apply_df(cudaStream_t st, const Hbs& H, const double* X, int ldx, doubl
 size_t hbs_nbytes(const Hbs& H, int which);
 
 // ---------------------------------------------------------------- tensor-core sweep
+// (crt_step.cu) Solves and applies of many right-hand sides as exact residue
+// products, float64 in and out.  crt_steps_pay: by the operator's shape and c
+// alone, so every entry point takes the same path for them.  crt_prepare also
+// makes the residue images on first use (false inside a stream capture that
+// would need it: take the float64 steps).
+bool crt_steps_pay(const Hbs& H, bool solve, bool trans, int c);
+bool crt_prepare(Handle& h, Hbs& H, bool solve, bool trans, int c);
+void crt_solve(cudaStream_t st, const Hbs& H, bool trans, const double* X, int ldx, double* B,
+               int ldb, int c, double* scratch, size_t stride, volatile unsigned* err);
+void crt_apply(cudaStream_t st, const Hbs& H, bool trans, const double* X, int ldx, double* Y,
+               int ldy, int c, double* scratch, volatile unsigned* err);
+
 // (ozaki.cu) Digit forms of the mode-N solve and apply step operators, and the
 // solve / apply run as tcgen05 block products of bfloat16 digits with exact
 // float32 accumulation.  Vectors between steps are double-float pairs.

@@ -157,7 +157,7 @@ void ulv_solve_fused(cudaStream_t st, const Hbs& H, T* B, int ldb, int c, T* scr
                 kn ? (*kn)[i] : PlanKnobs());
 }
 
-void solve_plan_create(Handle& h, const Hbs& H, const double* X, int ldx, double* Y, int ldy,
+void solve_plan_create(Handle& h, Hbs& H, const double* X, int ldx, double* Y, int ldy,
                        int c, bool trans, SolvePlan& P) {
   SLU_REQUIRE(H.has_sweep, "step operators not composed");
   cudaStream_t st = h.stream;
@@ -174,6 +174,16 @@ void solve_plan_create(Handle& h, const Hbs& H, const double* X, int ldx, double
     auto it = H.tuned.find({type_code<double>(), c});
     if (it != H.tuned.end() && it->second.size() == steps.size()) kn = &it->second;
   }
+  // the path of a solve call of this shape (residue steps for many columns)
+  const bool crt = crt_prepare(h, H, true, trans, c);
+  if (crt) {
+    void* w = nullptr;
+    SLU_CHECK_CUDA(cudaHostAlloc(&w, 64, cudaHostAllocPortable | cudaHostAllocMapped));
+    P.err = std::shared_ptr<volatile unsigned>(
+        static_cast<volatile unsigned*>(w),
+        [](volatile unsigned* p) { cudaFreeHost(const_cast<unsigned*>(p)); });
+    *P.err = 0;
+  }
   for (size_t i = 0; i < steps.size(); ++i)
     sweep::prepare_step(steps[i].s, kn ? (*kn)[i] : PlanKnobs());
   stream_wait(st);   // the scratch exists before the capture
@@ -186,8 +196,11 @@ void solve_plan_create(Handle& h, const Hbs& H, const double* X, int ldx, double
   try {
     SLU_CHECK_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
     try {
-      for (size_t i = 0; i < steps.size(); ++i)
-        launch_step(cs, steps[i].s, steps[i].what, nullptr, 0, 0, kn ? (*kn)[i] : PlanKnobs());
+      if (crt)
+        crt_solve(cs, H, trans, X, ldx, Y, ldy, c, scratch, stride, P.err.get());
+      else
+        for (size_t i = 0; i < steps.size(); ++i)
+          launch_step(cs, steps[i].s, steps[i].what, nullptr, 0, 0, kn ? (*kn)[i] : PlanKnobs());
     } catch (...) {
       cudaStreamEndCapture(cs, &g);
       if (g) cudaGraphDestroy(g);
@@ -220,9 +233,31 @@ void solve_plan_launch(Handle& h, SolvePlan& P, bool wait) {
       throw Error(SLU_ERR_STATE, "an operator was refactored after the solve plan was made");
   }
   if (!P.exec) return;   // a grouped plan without members
+  auto check = [&] {
+    if (P.err && *P.err) {
+      *P.err = 0;
+      throw Error(SLU_ERR_TIMEOUT, "a tensor-core step of the solve plan gave up waiting");
+    }
+  };
+  check();   // an earlier launch that was not waited for
+  if (P.err) {
+    bool known = false;
+    for (size_t i = 0; i < h.plan_err.size();) {
+      if (h.plan_err[i].expired()) {
+        h.plan_err.erase(h.plan_err.begin() + i);
+        continue;
+      }
+      known = known || h.plan_err[i].lock() == P.err;
+      ++i;
+    }
+    if (!known) h.plan_err.push_back(P.err);
+  }
   SLU_CHECK_CUDA(cudaGraphLaunch(P.exec, h.stream));
   count_launches(P.kernels);
-  if (wait) stream_wait(h.stream);
+  if (wait) {
+    stream_wait(h.stream);
+    check();
+  }
 }
 
 namespace {
