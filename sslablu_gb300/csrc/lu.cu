@@ -113,37 +113,107 @@ lu_panel_global_kernel(int n, int k0, int kb, double* __restrict__ A, int lda, l
 }
 
 // Panel factorisation by one cluster per matrix.  Thread = row, the row's kb
-// panel entries in registers, so the rank-1 updates spread over the cluster's
-// SMs: one SM's float64 pipe (2 FMA per clock) would need ~4 us per column of
-// a 1024-row panel.  Rows are never moved: a thread carries the position its
-// row has after the swaps and stores it there at the end.
-// Per column: each CTA finds its largest entry (integer reductions of the
-// bit pattern), its owner puts 1/d and the row in shared memory, the
-// candidates' keys go to every CTA of the cluster, one cluster barrier, and
-// each warp reads the winner's row through distributed shared memory.  The
-// two buffers alternate, so one barrier per column suffices.
-// 1024 rows, 32 columns: 112 us; in one CTA, the panel in global memory, 422.
-struct PanelKey {
-  uint32_t hi, lo;   // |value| bits, hi + 1 (0: no candidate)
-  int pos;
-  int rank;
+// panel entries in registers, so the rank-1 updates spread over the float64
+// pipes of the cluster's SMs (2 FMA per clock each).  Rows are never moved: a
+// thread carries the position its row has after the swaps and stores it there
+// at the end.
+// A column is a chain of latencies: largest entry, its row to all, multiplier,
+// update of the next column.  It is kept short by
+//  * no barrier: every warp sends its candidate (key, row, 1/d) straight to
+//    every CTA of the cluster with asynchronous stores that complete on the
+//    receiver's mbarrier, and every warp picks the winner of all candidates
+//    itself; two buffers alternate (a warp sends for column j after all have
+//    sent for j - 1, that is after all have read j - 2);
+//  * only the next column's entry is updated at once; the other columns lag by
+//    one update, applied while the messages travel.  A candidate's row is sent
+//    as it stands with its multiplier, and the receiver applies the update.
+//  * one loop body for all columns: the registers move down by one column, a
+//    finished entry goes to shared memory.  Unrolled over the columns the code
+//    runs once per launch and waits for its own instructions.
+// Per column at 1024 rows, in clocks: candidate 200, reciprocal and row 490,
+// sending 620 (the messages' bytes), lagging updates 90 per column still to go
+// (1500 on average), winner 360, update of the next column 430.  1024 rows, 32
+// columns, eight matrices, cold: 67 us; with a cluster barrier per column, the
+// winner's row read through distributed shared memory and the loop unrolled
+// 122 us; in one CTA, the panel in global memory, 422.
+struct PanelMsg {
+  double row[kPanel];
+  unsigned long long key;   // bits of |entry| + 1; 0: no candidate
+  long long pos;
+  double lprev, inv;        // its multiplier of the column before; 1 / entry
 };
+constexpr uint32_t kMsgBytes = sizeof(PanelMsg);
 
-template <int KB>
-__global__ void __launch_bounds__(kPanelRows)
+__device__ __forceinline__ uint32_t smem_u32(const void* p) {
+  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+__device__ __forceinline__ uint32_t remote_u32(uint32_t addr, int rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void send_2b64(uint32_t addr, ulonglong2 v, uint32_t bar) {
+  asm volatile(
+      "st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(
+          addr),
+      "l"(v.x), "l"(v.y), "r"(bar)
+      : "memory");
+}
+// 1 / d: the hardware's approximation (relative error 2^-23) and one step of
+// third order, x (1 + e + e^2) with e = 1 - d x, so that only the last
+// rounding counts; three dependent operations, half the division's time.
+// Outside its range (subnormal, near overflow, zero, infinite) the division.
+__device__ __forceinline__ double reciprocal(double d) {
+  const int f = (__double2hiint(d) >> 20) & 0x7ff;
+  if (f < 64 || f > 1980) return 1.0 / d;
+  double x;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(d));
+  const double e = fma(-d, x, 1.0);
+  return fma(x, fma(e, e, e), x);
+}
+__device__ __forceinline__ bool panel_wait(uint32_t bar, uint32_t parity) {
+  for (int i = 0; i < (1 << 22); ++i) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (done) return true;
+  }
+  return false;
+}
+
+// MAXT: threads per CTA at most (registers)
+template <int MAXT>
+__global__ void __launch_bounds__(MAXT)
 lu_panel_kernel(int n, int k0, int kb, double* __restrict__ A, int lda, long long sA,
-                int* __restrict__ piv, long long sP, int* __restrict__ src, int* info) {
+                int* __restrict__ piv, long long sP, int* __restrict__ src, int* info,
+                unsigned* err) {
+  constexpr int KB = kPanel;
+  extern __shared__ __align__(16) unsigned char s_raw[];
   cg::cluster_group cl = cg::this_cluster();
   const int cs = (int)cl.num_blocks(), rank = (int)cl.block_rank();
   const int b = blockIdx.x / cs;
   A += b * sA;
   piv += b * sP;
   src += (long long)b * n;
-  __shared__ PanelKey s_key[2][8];        // per CTA of the cluster
-  __shared__ uint32_t s_hi[2][kPanelRows / 32], s_lo[2][kPanelRows / 32];
-  __shared__ int s_pos[2][kPanelRows / 32];
-  __shared__ double s_row[2][KB + 1];     // candidate row, 1/d last
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int nmsg = cs * nw;
+  PanelMsg* msg = reinterpret_cast<PanelMsg*>(s_raw);                     // [2][nmsg]
+  PanelMsg& out = msg[2 * nmsg + warp];                                   // this warp's candidate
+  double* us = reinterpret_cast<double*>(msg + 2 * nmsg + nw) + KB * warp;   // its pivot row
+  // finished entries, [column][thread]
+  double* fin = reinterpret_cast<double*>(msg + 2 * nmsg + nw) + KB * nw + threadIdx.x;
+  __shared__ __align__(8) unsigned long long bars[2];
+  const uint32_t bar0 = smem_u32(bars);
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 2; ++i)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + 8 * i) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
   const int R = n - k0, r = rank * blockDim.x + threadIdx.x;
   const bool have = r < R;
   double a[KB];
@@ -154,87 +224,131 @@ lu_panel_kernel(int n, int k0, int kb, double* __restrict__ A, int lda, long lon
   }
   int pos = have ? r : -1;   // -1: no row
   int first_zero = 0;
+  double lp = 0.0, up = 0.0;        // pending: multiplier, pivot row (lane = column)
+  bool pend = false, lag = false;   // any; for this row
+  bool ok = true;
+  uint32_t slot[8], rbar[8];   // this warp's message and the barriers in every CTA
 #pragma unroll
-  for (int j = 0; j < KB; ++j) {
-    if (j < kb) {   // uniform
-      const int buf = j & 1;
-      const unsigned long long bits = (unsigned long long)__double_as_longlong(fabs(a[j]));
-      const bool cand = pos >= j && a[j] == a[j];
-      const uint32_t hi = cand ? (uint32_t)(bits >> 32) + 1 : 0, lo = (uint32_t)bits;
-      const uint32_t mh = __reduce_max_sync(0xffffffffu, hi);
-      const uint32_t ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0);
-      const int mp = __reduce_min_sync(0xffffffffu,
-                                       (cand && hi == mh && lo == ml) ? pos : 0x7fffffff);
-      if (lane == 0) {
-        s_hi[buf][warp] = mh;
-        s_lo[buf][warp] = ml;
-        s_pos[buf][warp] = mp;
-      }
-      __syncthreads();
-      const uint32_t wh = lane < nw ? s_hi[buf][lane] : 0;
-      const uint32_t bh = __reduce_max_sync(0xffffffffu, wh);
-      const uint32_t wl = lane < nw && wh == bh ? s_lo[buf][lane] : 0;
-      const uint32_t bl = __reduce_max_sync(0xffffffffu, wl);
-      const int bp = __reduce_min_sync(
-          0xffffffffu, (lane < nw && wh == bh && wl == bl) ? s_pos[buf][lane] : 0x7fffffff);
-      // no finite candidate in the column: row j itself (NaN column)
-      const int mine = bh ? bp : j;
-      if (pos == mine) {
+  for (int q = 0; q < 8; ++q) {
+    slot[q] = remote_u32(smem_u32(&msg[rank * nw + warp]), q < cs ? q : 0) + 16 * lane;
+    rbar[q] = remote_u32(bar0, q < cs ? q : 0);
+  }
+  cl.sync();   // the barriers are there
+  // a[i]: column j + i
+#pragma unroll 1
+  for (int j = 0; j < kb && ok; ++j) {
+    const int buf = j & 1;
+    const uint32_t bar = bar0 + 8 * buf;
+    if (threadIdx.x == 0)
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
+                   "r"(nmsg * kMsgBytes)
+                   : "memory");
+    // the warp's candidate (NaNs are none)
+    const unsigned long long bits =
+        (unsigned long long)__double_as_longlong(a[0]) & 0x7fffffffffffffffULL;
+    const bool cand = pos >= j && bits <= 0x7ff0000000000000ULL;
+    const uint32_t hi = cand ? (uint32_t)(bits >> 32) + 1 : 0, lo = (uint32_t)bits;
+    const uint32_t mh = __reduce_max_sync(0xffffffffu, hi);
+    const uint32_t ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0);
+    const int mp =
+        __reduce_min_sync(0xffffffffu, (cand && hi == mh && lo == ml) ? pos : 0x7fffffff);
+    if (cand && pos == mp) {
 #pragma unroll
-        for (int c = j; c < KB; ++c) s_row[buf][c] = a[c];
-        s_row[buf][KB] = 1.0 / a[j];
-      }
-      if (threadIdx.x < cs) {
-        // a NaN column's row j is held by one CTA only
-        PanelKey* dst = cl.map_shared_rank(&s_key[buf][rank], threadIdx.x);
-        *dst = PanelKey{bh, bl, mine, rank};
-      }
-      cl.sync();
-      // the winner among the CTAs: largest entry, then the first position
-      PanelKey k = s_key[buf][0];
-      for (int q = 1; q < cs; ++q) {
-        const PanelKey o = s_key[buf][q];
-        if (o.hi > k.hi || (o.hi == k.hi && (o.lo > k.lo || (o.lo == k.lo && o.pos < k.pos))))
-          k = o;
-      }
-      const int p = k.pos;
-      // k.hi == 0: every remaining entry of the column is NaN; the row at
-      // position j is its own pivot, wherever it is held
-      const int owner = k.hi ? k.rank : -1;
-      double u = 0.0, inv = 0.0;
-      if (owner >= 0) {
-        const double* row = cl.map_shared_rank(&s_row[buf][0], owner);
-        u = row[lane < KB ? lane : 0];
-        inv = row[KB];
-      } else {
-        u = inv = __longlong_as_double(0x7ff8000000000000LL);
-      }
-      if (rank == 0 && threadIdx.x == 0) piv[k0 + j] = k0 + p;
-      const double d = __shfl_sync(0xffffffffu, u, j);
-      // position swap j <-> p
-      const bool retire = pos == p;
-      if (pos == j) pos = p;
-      if (retire) pos = j;
-      if (d == 0.0) {
-        if (!first_zero) first_zero = k0 + j + 1;
-      } else {
-        const bool live = pos > j;
-        const double l = live ? a[j] * inv : 0.0;
-        if (live) a[j] = l;
+      for (int c = 0; c < KB; c += 2)
+        *reinterpret_cast<double2*>(&out.row[c]) = make_double2(a[c], a[c + 1]);
+      out.lprev = lp;
+      out.inv = reciprocal(a[0]);
+    }
+    __syncwarp();
+    {
+      // 16 bytes per lane
+      ulonglong2 v = reinterpret_cast<const ulonglong2*>(&out)[lane < 18 ? lane : 0];
+      if (lane == 16) v = make_ulonglong2(mh ? (unsigned long long)mh << 32 | ml : 0, mp);
+      const uint32_t off = buf * nmsg * kMsgBytes;
 #pragma unroll
-        for (int c = j + 1; c < KB; ++c) {
-          const double uc = __shfl_sync(0xffffffffu, u, c);
-          if (live) a[c] = fma(-l, uc, a[c]);
-        }
+      for (int q = 0; q < 8; ++q)
+        if (q < cs && lane < 18) send_2b64(slot[q] + off, v, rbar[q] + 8 * buf);
+    }
+    // the update that columns j + 1 .. lag by
+    if (pend) {
+      const double ln = lag ? -lp : 0.0;
+#pragma unroll
+      for (int c4 = 0; c4 < KB; c4 += 4) {
+        if (c4 >= KB - j) break;   // a branch: predicated off, the pipe is taken all the same
+#pragma unroll
+        for (int c = c4 ? c4 : 1; c < c4 + 4; ++c)
+          if (lag) a[c] = fma(ln, us[c], a[c]);
       }
     }
+    ok = panel_wait(bar, (uint32_t)(j >> 1) & 1);
+    if (!__all_sync(0xffffffffu, ok)) {
+      ok = false;
+      if (lane == 0 && err) *(volatile unsigned*)err = 1;
+      break;
+    }
+    // the winner: largest entry, then the first position
+    const PanelMsg* m = msg + buf * nmsg;
+    unsigned long long key = lane < nmsg ? m[lane].key : 0;
+    int kp = lane < nmsg ? (int)m[lane].pos : 0x7fffffff, ki = lane;
+    for (int q = lane + 32; q < nmsg; q += 32) {
+      const unsigned long long qk = m[q].key;
+      const int qp = (int)m[q].pos;
+      if (qk > key || (qk == key && qp < kp)) {
+        key = qk;
+        kp = qp;
+        ki = q;
+      }
+    }
+    const uint32_t kh = (uint32_t)(key >> 32), kl = (uint32_t)key;
+    const uint32_t wh = __reduce_max_sync(0xffffffffu, kh);
+    const uint32_t wl = __reduce_max_sync(0xffffffffu, kh == wh ? kl : 0);
+    const int wp = __reduce_min_sync(0xffffffffu, (kh == wh && kl == wl) ? kp : 0x7fffffff);
+    const unsigned own = __ballot_sync(0xffffffffu, kh == wh && kl == wl && kp == wp);
+    const int wi = __shfl_sync(0xffffffffu, ki, __ffs(own) - 1);
+    // no key: every remaining entry of the column is NaN; the row at position j
+    // is its own pivot, wherever it is held
+    const int p = wh ? wp : j;
+    const double ul = __shfl_down_sync(0xffffffffu, up, 1);   // of the column before
+    double u, inv;
+    if (wh) {
+      u = m[wi].row[lane];
+      inv = m[wi].inv;
+      if (pend && lane > 0) u = fma(-m[wi].lprev, ul, u);
+    } else {
+      u = inv = __longlong_as_double(0x7ff8000000000000LL);
+    }
+    if (rank == 0 && threadIdx.x == 0) piv[k0 + j] = k0 + p;
+    // position swap j <-> p
+    const bool retire = pos == p;
+    if (pos == j) pos = p;
+    if (retire) pos = j;
+    // the pivot is zero when its key says so
+    if (wh == 1 && wl == 0) {
+      if (!first_zero) first_zero = k0 + j + 1;
+      pend = lag = false;
+    } else {
+      up = u;
+      pend = true;
+      lag = pos > j;
+      const double u1 = __shfl_sync(0xffffffffu, u, 1);
+      __syncwarp();
+      if (lane > 0) us[lane - 1] = u;   // for the next column's a[]
+      __syncwarp();
+      if (lag) {
+        lp = a[0] * inv;
+        a[0] = lp;
+        a[1] = fma(-lp, u1, a[1]);
+      }
+    }
+    fin[j * blockDim.x] = a[0];
+#pragma unroll
+    for (int c = 0; c + 1 < KB; ++c) a[c] = a[c + 1];
+    a[KB - 1] = 0.0;
   }
-  cl.sync();   // no CTA leaves while another may still read its shared memory
+  cl.sync();   // no CTA leaves while another may still write to its shared memory
   if (have) {
     double* row = A + (long long)(k0 + pos) * lda + k0;
-#pragma unroll
-    for (int c = 0; c < KB; ++c)
-      if (c < kb) row[c] = a[c];
+    for (int c = 0; c < kb; ++c) row[c] = fin[c * blockDim.x];
     src[k0 + pos] = k0 + r;
   }
   if (rank == 0 && threadIdx.x == 0 && first_zero && info) atomicCAS(info + b, 0, first_zero);
@@ -350,20 +464,27 @@ lu_block_trsm_kernel(int n, int k0, int nb, int c0, double* __restrict__ A, int 
 }
 
 void launch_panel(cudaStream_t st, int n, int k0, int kb, double* A, int lda, long long sA,
-                  int* piv, long long sP, int* src, int batch, int* info) {
+                  int* piv, long long sP, int* src, int batch, int* info, unsigned* err) {
   const int R = n - k0;
-  // about 64 rows per CTA, up to the portable cluster size of 8
+  // a warp per scheduler of an SM (128 rows per CTA), up to the portable
+  // cluster size of 8
   int cs = 1;
-  while (cs < 8 && R > 64 * cs) cs *= 2;
+  while (cs < 8 && R > 128 * cs) cs *= 2;
   const int threads = ((R + cs - 1) / cs + 31) / 32 * 32;
   if (threads > kPanelRows) {
     lu_panel_global_kernel<<<batch, 1024, 0, st>>>(n, k0, kb, A, lda, sA, piv, sP, src, info);
     check_launch("lu_panel_global_kernel");
     return;
   }
+  const int nw = threads / 32;
+  const size_t sm = (size_t)(2 * cs * nw + nw) * sizeof(PanelMsg) +
+                    8 * (size_t)kPanel * (nw + threads);
+  auto kern = threads <= 128 ? lu_panel_kernel<128> : lu_panel_kernel<kPanelRows>;
+  ensure_smem(reinterpret_cast<const void*>(kern), sm);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(batch * cs));
   cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = sm;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -372,8 +493,8 @@ void launch_panel(cudaStream_t st, int n, int k0, int kb, double* A, int lda, lo
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  SLU_CHECK_CUDA(cudaLaunchKernelEx(&cfg, lu_panel_kernel<kPanel>, n, k0, kb, A, lda, sA, piv, sP,
-                                    src, info));
+  SLU_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, n, k0, kb, A, lda, sA, piv, sP, src,
+                                    info, err));
   check_launch("lu_panel_kernel");
 }
 
@@ -487,7 +608,7 @@ void lu_factor(Handle& h, int n, double* A, int lda, long long sA, int* piv, lon
     const int K1 = std::min(K0 + kOuter, n);
     for (int k0 = K0; k0 < K1; k0 += kPanel) {
       const int kb = std::min(kPanel, K1 - k0), k1 = k0 + kb;
-      launch_panel(st, n, k0, kb, A, lda, sA, piv, sP, src, batch, info);
+      launch_panel(st, n, k0, kb, A, lda, sA, piv, sP, src, batch, info, h.err_word());
       if (n > kb) {
         lu_swap_trsm_kernel<<<dim3((n + 31) / 32, batch), 32, 0, st>>>(n, k0, kb, K1, A, lda, sA,
                                                                        piv, sP, src);
