@@ -163,6 +163,75 @@ gemm_kernel(int M, int N, int K, T alpha, const T* __restrict__ A, int lda, long
     }
   }
 }
+// Few outputs: TM x 16 tiles (TM = 16 or 8), one output per thread, K in steps
+// of 32 with the next step's operands in flight.  A warp's multiplication
+// holds a quarter of an SM's float64 pipe for 72 clocks, so a 32 x 32 tile 32
+// deep takes 9 us on its SM and a 64 x 64 one 35, whatever the others do;
+// spread over the idle SMs it is 2.  Same order of summation as the others.
+template <typename T, int TM>
+__global__ void __launch_bounds__(16 * TM)
+gemm_small_kernel(int M, int N, int K, T alpha, const T* __restrict__ A, int lda, long long sA0,
+                  long long sA1, bool ta, const T* __restrict__ B, int ldb, long long sB0,
+                  long long sB1, bool tb, T beta, T* __restrict__ C, int ldc, long long sC0,
+                  long long sC1, int batch0) {
+  constexpr int KS = 32, NT = 16 * TM, EA = TM * KS / NT, EB = 16 * KS / NT;
+  __shared__ T As[KS][TM + 1];
+  __shared__ T Bs[KS][17];
+  const int b = blockIdx.z;
+  const int b0 = b % batch0, b1 = b / batch0;
+  A += b0 * sA0 + b1 * sA1;
+  B += b0 * sB0 + b1 * sB1;
+  C += b0 * sC0 + b1 * sC1;
+  const int row0 = blockIdx.y * TM, col0 = blockIdx.x * 16, tid = threadIdx.x;
+  T va[EA], vb[EB];
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int u = 0; u < EA; ++u) {
+      const int e = tid + u * NT;
+      const int i = ta ? e % TM : e / KS, kk = ta ? e / TM : e % KS;
+      const int gi = row0 + i, gk = k0 + kk;
+      va[u] = T(0);
+      if (gi < M && gk < K)
+        va[u] = ta ? A[(long long)gk * lda + gi] : A[(long long)gi * lda + gk];
+    }
+#pragma unroll
+    for (int u = 0; u < EB; ++u) {
+      const int e = tid + u * NT;
+      const int j = tb ? e / KS : e % 16, kk = tb ? e % KS : e / 16;
+      const int gj = col0 + j, gk = k0 + kk;
+      vb[u] = T(0);
+      if (gj < N && gk < K)
+        vb[u] = tb ? B[(long long)gj * ldb + gk] : B[(long long)gk * ldb + gj];
+    }
+  };
+  const int tx = tid & 15, ty = tid >> 4;
+  const int gi = row0 + ty, gj = col0 + tx;
+  T acc = T(0);
+  fetch(0);
+  for (int k0 = 0; k0 < K; k0 += KS) {
+#pragma unroll
+    for (int u = 0; u < EA; ++u) {
+      const int e = tid + u * NT;
+      As[ta ? e / TM : e % KS][ta ? e % TM : e / KS] = va[u];
+    }
+#pragma unroll
+    for (int u = 0; u < EB; ++u) {
+      const int e = tid + u * NT;
+      Bs[tb ? e % KS : e / 16][tb ? e / KS : e % 16] = vb[u];
+    }
+    __syncthreads();
+    if (k0 + KS < K) fetch(k0 + KS);
+#pragma unroll
+    for (int kk = 0; kk < KS; ++kk) acc = fma(As[kk][ty], Bs[kk][tx], acc);
+    __syncthreads();
+  }
+  if (gi >= M || gj >= N) return;
+  T* c = C + (long long)gi * ldc + gj;
+  T v = alpha * acc;
+  if (beta != T(0)) v = fma(beta, *c, v);
+  *c = v;
+}
+
 // Skinny products (N <= kSkinny columns, B not transposed): the 64 x 64 tile
 // kernel would compute 64 output columns per tile regardless of N.  Here each
 // output row is one warp (A row-major: lanes stride over K, coalesced, then a
@@ -251,7 +320,20 @@ void gemm_batched(cudaStream_t st, bool ta, bool tb, int M, int N, int K, T alph
     return;
   }
   const long long tiles64 = (long long)((N + 63) / 64) * ((M + 63) / 64) * nb;
-  if (tiles64 < num_sms()) {
+  const long long tiles32 = (long long)((N + 31) / 32) * ((M + 31) / 32) * nb;
+  const long long tiles16 = (long long)((N + 15) / 16) * ((M + 15) / 16) * nb;
+  // the largest tile that gives every SM one
+  if (tiles32 < num_sms()) {
+    if (2 * tiles16 <= num_sms()) {
+      dim3 grid((N + 15) / 16, (M + 7) / 8, (unsigned)nb);
+      gemm_small_kernel<T, 8><<<grid, 128, 0, st>>>(M, N, K, alpha, A, lda, sA0, sA1, ta, B, ldb,
+                                                    sB0, sB1, tb, beta, C, ldc, sC0, sC1, batch0);
+    } else {
+      dim3 grid((N + 15) / 16, (M + 15) / 16, (unsigned)nb);
+      gemm_small_kernel<T, 16><<<grid, 256, 0, st>>>(M, N, K, alpha, A, lda, sA0, sA1, ta, B, ldb,
+                                                     sB0, sB1, tb, beta, C, ldc, sC0, sC1, batch0);
+    }
+  } else if (tiles64 < num_sms()) {
     dim3 grid((N + 31) / 32, (M + 31) / 32, (unsigned)nb);
     gemm_kernel<T, 32><<<grid, 256, 0, st>>>(M, N, K, alpha, A, lda, sA0, sA1, ta, B, ldb, sB0,
                                              sB1, tb, beta, C, ldc, sC0, sC1, batch0);

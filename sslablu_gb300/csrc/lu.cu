@@ -356,55 +356,54 @@ lu_panel_kernel(int n, int k0, int kb, double* __restrict__ A, int lda, long lon
 
 // The panel's row swaps on every column outside it, from the net permutation
 // (src[i]: the row that ends at row i): the kb top rows and the up to kb
-// pivot rows below, one column per thread, all reads before the writes.  For
-// columns k1 .. ct the top rows are then solved with the panel's unit lower
-// triangle.  One warp per CTA: the solves of 32 columns keep one SM's
-// float64 pipe busy for 4 us.
-__global__ void __launch_bounds__(32)
+// pivot rows below, all reads before the writes.  For columns k1 .. ct the top
+// rows are then solved with the panel's unit lower triangle: a warp per
+// column, lane = row, a finished entry broadcast by shuffle.  Eight columns
+// per CTA: a step of a solve holds a quarter of the SM's float64 pipe for 72
+// clocks (a column per lane instead, 32 per warp: 17 us for the 496 steps).
+constexpr int kSwapCols = 8;
+__global__ void __launch_bounds__(32 * kSwapCols)
 lu_swap_trsm_kernel(int n, int k0, int kb, int ct, double* __restrict__ A, int lda, long long sA,
                     const int* __restrict__ piv, long long sP, const int* __restrict__ src) {
   A += blockIdx.y * sA;
   piv += blockIdx.y * sP;
   src += (long long)blockIdx.y * n;
-  __shared__ double L11[kPanel][kPanel + 1];
-  const int lane = threadIdx.x, k1 = k0 + kb;
-  const int c = blockIdx.x * 32 + lane;
-  const bool solve = blockIdx.x * 32 < ct && blockIdx.x * 32 + 31 >= k1;   // uniform
-  if (solve)
-    for (int i = 0; i < kb; ++i) L11[i][lane] = lane < kb ? A[(long long)(k0 + i) * lda + k0 + lane] : 0.0;
-  __syncwarp();
-  // rows from (top, below) and to (below), one per lane
-  const int st = lane < kb ? src[k0 + lane] : -1;
-  const int pr = lane < kb ? piv[k0 + lane] : -1;
-  const int sb = pr >= k1 ? src[pr] : -1;
-  const bool on = c < n && (c < k0 || c >= k1);
-  double x[kPanel], y[kPanel];
+  __shared__ double X[kPanel][kSwapCols + 1];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, k1 = k0 + kb;
+  const int cb = blockIdx.x * kSwapCols;
+  const bool solve = cb < ct && cb + kSwapCols > k1;   // uniform
+  // L11: lane = row
+  double l[kPanel];
+  if (solve) {
 #pragma unroll
-  for (int i = 0; i < kPanel; ++i) {
-    const int rt = __shfl_sync(0xffffffffu, st, i), rb = __shfl_sync(0xffffffffu, sb, i);
-    x[i] = (on && rt >= 0) ? A[(long long)rt * lda + c] : 0.0;
-    y[i] = (on && rb >= 0) ? A[(long long)rb * lda + c] : 0.0;
+    for (int r = 0; r < kPanel; ++r)
+      l[r] = r < lane && lane < kb ? A[(long long)(k0 + lane) * lda + k0 + r] : 0.0;
   }
-#pragma unroll
-  for (int i = 0; i < kPanel; ++i) {
-    const int to = __shfl_sync(0xffffffffu, pr, i);
-    if (on && to >= k1) A[(long long)to * lda + c] = y[i];
+  const int i = threadIdx.x / kSwapCols, w = threadIdx.x % kSwapCols, c = cb + w;
+  const bool on = i < kb && c < n && (c < k0 || c >= k1);
+  double x = 0.0, y = 0.0;
+  int to = -1;
+  if (on) {
+    const int rt = src[k0 + i];
+    to = piv[k0 + i];
+    x = A[(long long)rt * lda + c];
+    if (to >= k1) y = A[(long long)src[to] * lda + c];
   }
-  if (!on) return;
-  if (c >= k1 && c < ct) {
+  X[i][w] = x;
+  __syncthreads();   // all reads before the writes
+  if (on && to >= k1) A[(long long)to * lda + c] = y;
+  const int cs = cb + warp;
+  if (solve && cs >= k1 && cs < ct) {
+    double v = X[lane][warp];
 #pragma unroll
-    for (int i = 1; i < kPanel; ++i) {
-      if (i < kb) {
-        double acc = x[i];
-#pragma unroll
-        for (int r = 0; r < i; ++r) acc = fma(-L11[i][r], x[r], acc);
-        x[i] = acc;
-      }
+    for (int r = 0; r + 1 < kPanel; ++r) {
+      const double xr = __shfl_sync(0xffffffffu, v, r);
+      if (lane > r) v = fma(-l[r], xr, v);
     }
+    X[lane][warp] = v;
   }
-#pragma unroll
-  for (int i = 0; i < kPanel; ++i)
-    if (i < kb) A[(long long)(k0 + i) * lda + c] = x[i];
+  __syncthreads();
+  if (on) A[(long long)(k0 + i) * lda + c] = X[i][w];
 }
 
 // U12 = L11^{-1} A12 for the nb rows of an outer block, columns c0 .. n-1:
@@ -610,8 +609,8 @@ void lu_factor(Handle& h, int n, double* A, int lda, long long sA, int* piv, lon
       const int kb = std::min(kPanel, K1 - k0), k1 = k0 + kb;
       launch_panel(st, n, k0, kb, A, lda, sA, piv, sP, src, batch, info, h.err_word());
       if (n > kb) {
-        lu_swap_trsm_kernel<<<dim3((n + 31) / 32, batch), 32, 0, st>>>(n, k0, kb, K1, A, lda, sA,
-                                                                       piv, sP, src);
+        lu_swap_trsm_kernel<<<dim3((n + kSwapCols - 1) / kSwapCols, batch), 32 * kSwapCols, 0, st>>>(
+            n, k0, kb, K1, A, lda, sA, piv, sP, src);
         check_launch("lu_swap_trsm_kernel");
       }
       if (k1 < K1)
