@@ -354,9 +354,93 @@ template void gemm_batched<float>(cudaStream_t, bool, bool, int, int, int, float
                                   long long, float, float*, int, long long, long long, int, int);
 
 // ============================================================== triangular solve
-// One CTA per (matrix, chunk of right-hand sides).  Column-oriented
-// substitution: after x_i is final, every remaining row subtracts R_ri x_i.
+// Substitution with R or R^T for a chunk of right-hand sides per CTA.
 namespace {
+// y / d with r = 1 / d: the product, corrected once by its exact residual (the
+// last rounding decides, as in a division) where neither leaves the range of
+// normal numbers.  Three dependent operations instead of a division.
+__device__ __forceinline__ float quotient(float y, float d, float) { return y / d; }
+__device__ __forceinline__ double quotient(double y, double d, double r) {
+  const double q = y * r;
+  const int fq = (__double2hiint(q) >> 20) & 0x7ff, fr = (__double2hiint(r) >> 20) & 0x7ff;
+  if ((fq < 64 || fq > 1980 || fr < 64 || fr > 1980) && !(y == 0.0 && fr > 0 && fr < 0x7ff))
+    return y / d;
+  return fma(fma(-d, q, y), r, q);
+}
+
+// n up to kTrsmSmall rows.  G lanes per right-hand side, row s in lane s mod G;
+// R and the right-hand sides in shared memory, no barrier but the warp's.
+// Pivot t of either direction is row t here, L[t][s] its factor for row s > t.
+// Float64-pipe bound: a warp's step is three operations for its 32 / G
+// quotients and one per G rows, 72 clocks each; the previous kernel divided by
+// every thread's own quotient and met two block barriers and R in global
+// memory per step (64 x 64, 64 columns, 64 matrices: 120 -> 63 us;
+// one 48 x 48: 150 -> 68).
+constexpr int kTrsmSmall = 128;
+template <typename T, int G>
+__global__ void __launch_bounds__(128)
+trsm_small_kernel(bool trans, int n, const T* __restrict__ R, long long rRs, long long rCs,
+                  long long sR, T* __restrict__ X, long long xRs, long long xCs, long long sX,
+                  int nrhs) {
+  constexpr int NC = 128 / G;   // columns per CTA
+  R += blockIdx.y * sR;
+  X += blockIdx.y * sX;
+  extern __shared__ unsigned char smraw[];
+  const int ld = n | 1;
+  T* L = reinterpret_cast<T*>(smraw);   // [t][s]
+  T* xs = L + n * ld;                   // [column][s]
+  T* rd = xs + NC * ld;                 // 1 / L[t][t]
+  const int tid = threadIdx.x, c0 = blockIdx.x * NC, nc = min(NC, nrhs - c0);
+  const bool rows = rCs == 1;   // consecutive threads along the contiguous index
+  for (int e = tid; e < n * n; e += 128) {
+    const int hi = e / n, lo = e - hi * n, i = rows ? hi : lo, j = rows ? lo : hi;
+    const int t = trans ? i : n - 1 - j, u = trans ? j : n - 1 - i;
+    if (u >= t) L[t * ld + u] = R[i * rRs + j * rCs];
+  }
+  const bool cols = xRs == 1;
+  for (int e = tid; e < n * NC; e += 128) {
+    const int i = cols ? e % n : e / NC, c = cols ? e / n : e % NC;
+    if (c < nc) xs[c * ld + (trans ? i : n - 1 - i)] = X[i * xRs + (c0 + c) * xCs];
+  }
+  __syncthreads();
+  for (int t = tid; t < n; t += 128) rd[t] = T(1) / L[t * ld + t];
+  __syncthreads();
+  const int c = tid / G, g = tid % G;
+  T* x = xs + c * ld;
+  // (columns beyond the last compute on what is there)
+  for (int t = 0; t < n; ++t) {
+    const T q = quotient(x[t], L[t * ld + t], rd[t]);
+    __syncwarp();
+    if (g == t % G) x[t] = q;
+    // loads of eight rows before their stores
+    for (int u0 = t - t % G + g; u0 < n; u0 += 8 * G) {
+      T l[8], y[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int u = u0 + i * G;
+        const bool on = u > t && u < n;
+        l[i] = on ? L[t * ld + u] : T(0);
+        y[i] = on ? x[u] : T(0);
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int u = u0 + i * G;
+        if (u0 - g + i * G >= n) break;   // uniform; the pipe is taken by idle lanes too
+        y[i] = fma(-l[i], q, y[i]);
+        if (u > t && u < n) x[u] = y[i];
+      }
+    }
+    __syncwarp();
+  }
+  __syncthreads();
+  for (int e = tid; e < n * NC; e += 128) {
+    const int i = cols ? e % n : e / NC, cc = cols ? e / n : e % NC;
+    if (cc < nc) X[i * xRs + (c0 + cc) * xCs] = xs[cc * ld + (trans ? i : n - 1 - i)];
+  }
+}
+
+// Any n: column-oriented substitution; after x_i is final, every remaining row
+// subtracts R_ri x_i.
 template <typename T>
 __global__ void trsm_upper_kernel(bool trans, int n, const T* __restrict__ R, long long rRs,
                                   long long rCs, long long sR, T* __restrict__ X, long long xRs,
@@ -412,6 +496,18 @@ void trsm_upper(cudaStream_t st, bool trans, int n, const T* R, long long rRs, l
                 long long sR, T* X, long long xRs, long long xCs, long long sX, int nrhs,
                 int batch) {
   if (n <= 0 || nrhs <= 0 || batch <= 0) return;
+  if (n <= kTrsmSmall) {
+    // eight lanes per column where four of them would leave schedulers idle
+    const bool wide = (long long)nrhs * batch * 4 / 32 > 4LL * num_sms();
+    const int nc = wide ? 32 : 16;
+    auto kern = wide ? trsm_small_kernel<T, 4> : trsm_small_kernel<T, 8>;
+    const size_t sm = sizeof(T) * ((size_t)(n | 1) * (n + nc) + n);
+    ensure_smem(reinterpret_cast<const void*>(kern), sm);
+    kern<<<dim3((nrhs + nc - 1) / nc, batch), 128, sm, st>>>(trans, n, R, rRs, rCs, sR, X, xRs, xCs,
+                                                             sX, nrhs);
+    check_launch("trsm_small_kernel");
+    return;
+  }
   int chunk = nrhs;
   while ((size_t)n * chunk * sizeof(T) > 96 * 1024 && chunk > 1) chunk = (chunk + 1) / 2;
   while (chunk > 16 && (long long)batch * ((nrhs + chunk - 1) / chunk) < num_sms()) chunk /= 2;

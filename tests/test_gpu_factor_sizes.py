@@ -1,0 +1,44 @@
+"""HBS construction and ULV solves at block sizes around the edges of the small
+triangular solves and panel kernels, against the dense matrix."""
+import numpy as np
+import pytest
+
+from tests._gpu import need_gpu
+
+pytestmark = pytest.mark.gpu
+
+
+def _dense(U, D, V, Nbvec):
+    A = D[-1]
+    for t in range(len(D) - 2, -1, -1):
+        nb, k = Nbvec[t], U[t].shape[1]
+        n = D[t].shape[0] // nb
+        B = np.zeros((nb * n, nb * n))
+        for i in range(nb):
+            for j in range(nb):
+                b = U[t][i * n:(i + 1) * n] @ A[i * k:(i + 1) * k, j * k:(j + 1) * k] \
+                    @ V[t][j * n:(j + 1) * n].T
+                B[i * n:(i + 1) * n, j * n:(j + 1) * n] = b
+            B[i * n:(i + 1) * n, i * n:(i + 1) * n] += D[t][i * n:(i + 1) * n]
+        A = B
+    return A
+
+
+@pytest.mark.parametrize("leaf,k,L,c", [(9, 3, 3, 1), (33, 5, 3, 3), (40, 8, 3, 17), (64, 31, 2, 64),
+                                        (65, 16, 3, 5), (128, 20, 2, 33), (131, 64, 2, 4),
+                                        (140, 66, 3, 2)])
+def test_ulv_solves(leaf, k, L, c):
+    need_gpu()
+    from sslablu_gb300.matAssembly.HBS.HBSnew import HBSMAT
+    from sslablu_gb300.synthetic import random_hbs_factors
+    rng = np.random.default_rng(leaf + k)
+    U, D, V, Nbvec = random_hbs_factors(k, leaf, L, rng=rng, shift=4.0 * np.sqrt(leaf))
+    A = _dense(U, D, V, Nbvec)
+    H = HBSMAT()
+    H.set_mats(U, D, V, list(Nbvec), fac=2)
+    H.compute_ULV()
+    b = rng.standard_normal((A.shape[0], c))
+    for M, x in ((A, H.solve(b)), (A.T, H.solve(b, mode="T"))):
+        # backward error of a backward stable solve: a modest multiple of n u
+        r = np.linalg.norm(M @ x - b) / (np.linalg.norm(M, 2) * np.linalg.norm(x))
+        assert r < 10 * A.shape[0] * 1.2e-16
