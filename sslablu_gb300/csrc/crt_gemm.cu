@@ -709,9 +709,11 @@ void gemm_f64_tensor(Handle& h, bool ta, bool tb, int M, int N, int K, double al
 
 // Residue products pay where the float64 pipe is the bound: enough flops to
 // cover three launches, and enough of them per element of C and of the
-// operands to cover the conversions.
+// operands to cover the conversions.  Products of 32 rows, 261 columns and
+// depth 64: 8 of them 14 us in float64, 16 (1.7e7 flops) 22, 32 135 -> 33, 64
+// 200 -> 49; 48 x 200 x 64, 32 of them 55 -> 29.
 bool gemm_tensor_pays(int M, int N, int K, long long nb) {
-  return M >= 64 && N >= 32 && K >= 64 && 2.0 * M * N * K * nb >= 2.0e7;
+  return M >= 32 && N >= 32 && K >= 64 && 2.0 * M * N * K * nb >= 2.0e7;
 }
 
 void gemm_f64(Handle& h, bool ta, bool tb, int M, int N, int K, double alpha, const double* A,

@@ -274,18 +274,18 @@ void hbs_compress(Handle& h, Hbs& H, int Nb0, int rk, int s, const double* Om, c
       double* Psi_n = set[nxt][1];
       double* Y_n = set[nxt][2];
       double* Z_n = set[nxt][3];
-      gemm<double>(st, false, false, nc, s, nc, -1.0, dp(c.D), nc, ncc, 0, Om_t, s, ncs, 0, 1.0,
-                   Y_t, s, ncs, 0, Nbc);
-      gemm<double>(st, true, false, kc, s, nc, 1.0, dp(c.U), kc, (long long)nc * kc, 0, Y_t, s,
-                   ncs, 0, 0.0, Y_n, s, kcs, 0, Nbc);
-      gemm<double>(st, true, false, nc, s, nc, -1.0, dp(c.D), nc, ncc, 0, Psi_t, s, ncs, 0, 1.0,
-                   Z_t, s, ncs, 0, Nbc);
-      gemm<double>(st, true, false, kc, s, nc, 1.0, dp(c.V), kc, (long long)nc * kc, 0, Z_t, s,
-                   ncs, 0, 0.0, Z_n, s, kcs, 0, Nbc);
-      gemm<double>(st, true, false, kc, s, nc, 1.0, dp(c.V), kc, (long long)nc * kc, 0, Om_t, s,
-                   ncs, 0, 0.0, Om_n, s, kcs, 0, Nbc);
-      gemm<double>(st, true, false, kc, s, nc, 1.0, dp(c.U), kc, (long long)nc * kc, 0, Psi_t, s,
-                   ncs, 0, 0.0, Psi_n, s, kcs, 0, Nbc);
+      gemm_f64(h, false, false, nc, s, nc, -1.0, dp(c.D), nc, ncc, 0, Om_t, s, ncs, 0, 1.0, Y_t, s,
+               ncs, 0, Nbc, 1);
+      gemm_f64(h, true, false, kc, s, nc, 1.0, dp(c.U), kc, (long long)nc * kc, 0, Y_t, s, ncs, 0,
+               0.0, Y_n, s, kcs, 0, Nbc, 1);
+      gemm_f64(h, true, false, nc, s, nc, -1.0, dp(c.D), nc, ncc, 0, Psi_t, s, ncs, 0, 1.0, Z_t, s,
+               ncs, 0, Nbc, 1);
+      gemm_f64(h, true, false, kc, s, nc, 1.0, dp(c.V), kc, (long long)nc * kc, 0, Z_t, s, ncs, 0,
+               0.0, Z_n, s, kcs, 0, Nbc, 1);
+      gemm_f64(h, true, false, kc, s, nc, 1.0, dp(c.V), kc, (long long)nc * kc, 0, Om_t, s, ncs, 0,
+               0.0, Om_n, s, kcs, 0, Nbc, 1);
+      gemm_f64(h, true, false, kc, s, nc, 1.0, dp(c.U), kc, (long long)nc * kc, 0, Psi_t, s, ncs, 0,
+               0.0, Psi_n, s, kcs, 0, Nbc, 1);
       Om_t = Om_n;
       Psi_t = Psi_n;
       Y_t = Y_n;

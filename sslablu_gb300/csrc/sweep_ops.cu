@@ -106,8 +106,8 @@ void hbs_make_sweep(Handle& h, Hbs& H) {
     add_batched<double>(st, n, k, 1.0, l.W.as<double>() + nu, n, nn, 0, S + nu + k, w, sS, 0, Nb);
     if (!leaf) {
       // H = D G + [0 | U | 0]
-      gemm_batched<double>(st, false, false, n, w, n, 1.0, l.D.as<double>(), n, nn, 0, S, w, sS,
-                           0, 0.0, S + (long long)n * w, w, sS, 0, Nb);
+      gemm_f64(h, false, false, n, w, n, 1.0, l.D.as<double>(), n, nn, 0, S, w, sS, 0, 0.0,
+               S + (long long)n * w, w, sS, 0, Nb, 1);
       add_batched<double>(st, n, k, 1.0, l.U.as<double>(), k, (long long)n * k, 0,
                           S + (long long)n * w + nu, w, sS, 0, Nb);
     }

@@ -107,3 +107,9 @@ def test_residue_sums_at_their_limit(s):
         C = torch.empty((1, 128, 96), dtype=torch.float64, device="cuda")
         _gemm(A, B, C, 0, 0, 1.0, 0.0)
         assert bool((C == s * 2.0 ** e * (2.0 ** e - 128 * (e == 55)) * 1024).all())
+
+
+@pytest.mark.parametrize("nb,M,N,K,ta,tb", [(64, 32, 261, 64, 1, 0), (9, 33, 300, 129, 0, 0),
+                                            (40, 63, 65, 70, 0, 1), (70, 47, 33, 100, 1, 1)])
+def test_few_rows_are_exact(nb, M, N, K, ta, tb):
+    test_integer_products_are_exact(nb, M, N, K, ta, tb)
