@@ -297,12 +297,18 @@ void hbs_compress(Handle& h, Hbs& H, int Nb0, int rk, int s, const double* Om, c
     // same shapes, so a level with few blocks fills twice as many SMs)
     copy_blocks(st, Nb, 8 * ns, Om_t, 8 * ns, WSA, 16 * ns);
     copy_blocks(st, Nb, 8 * ns, Y_t, 8 * ns, WSA + ns, 16 * ns);
-    if (root) panel_qr(st, s, n, 2 * n, WSA, s, 2 * ns, tauA, n, Nb);
+    const bool wy = wy_pays(s, n, n);
+    const int carried = wy ? n : 2 * n;   // columns of the panel kernels
+    if (root) {
+      panel_qr(st, s, n, carried, WSA, s, 2 * ns, tauA, n, Nb);
+      if (wy) apply_wy(h, s, n, WSA, nullptr, s, 2 * ns, tauA, nullptr, n, n, Nb);
+    }
     const double* YQ1A = WSA + ns;   // row-major n x n (ld s): Y_blk * Q_1
     if (!root) {
       copy_blocks(st, Nb, 8 * ns, Psi_t, 8 * ns, WSB, 16 * ns);
       copy_blocks(st, Nb, 8 * ns, Z_t, 8 * ns, WSB + ns, 16 * ns);
-      panel_qr2(st, s, n, 2 * n, WSA, WSB, s, 2 * ns, tauA, tauB, n, Nb);
+      panel_qr2(st, s, n, carried, WSA, WSB, s, 2 * ns, tauA, tauB, n, Nb);
+      if (wy) apply_wy(h, s, n, WSA, WSB, s, 2 * ns, tauA, tauB, n, n, Nb);
       int* info = h.info.as<int>();
       // U, V: leading left singular vectors of Y_blk Q[:, s-n:s] (HBSnew.py:26-27)
       // or of Y_blk Q[:, n:s] (HBStorch.py:73-82)

@@ -374,6 +374,13 @@ void hbs_apply_df(cudaStream_t st, const Hbs& H, const double* X, int ldx, doubl
                   int c, void* scratch);
 size_t hbs_nbytes(const Hbs& H, int which);
 
+// (wy.cu) Q^T applied to the nc columns behind the k factored ones of one or two
+// (W2) batches of panels of m rows, in the compact WY form; wy_pays: where that
+// is faster than panel_qr's reflectors one by one.
+bool wy_pays(int m, int k, int nc);
+void apply_wy(Handle& h, int m, int k, double* W, double* W2, int ldw, long long sW, double* tau,
+              double* tau2, long long sTau, int nc, int batch);
+
 // ---------------------------------------------------------------- tensor-core sweep
 // (crt_step.cu) Solves and applies of many right-hand sides as exact residue
 // products, float64 in and out.  crt_steps_pay: by the operator's shape and c

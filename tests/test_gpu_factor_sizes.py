@@ -42,3 +42,10 @@ def test_ulv_solves(leaf, k, L, c):
         # backward error of a backward stable solve: a modest multiple of n u
         r = np.linalg.norm(M @ x - b) / (np.linalg.norm(M, 2) * np.linalg.norm(x))
         assert r < 10 * A.shape[0] * 1.2e-16
+
+
+@pytest.mark.parametrize("n,k", [(15, 5), (16, 5), (31, 9), (127, 30), (129, 30)])
+def test_carried_columns(n, k):
+    """Sketch panels either side of the sizes that take the compact WY form."""
+    from tests.test_gpu_svd_edges import test_two_level_compression as check
+    check(n, k, "full")
