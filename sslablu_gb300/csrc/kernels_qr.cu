@@ -11,9 +11,13 @@
 //     (ULVsparse.py:51-61).
 // Reflectors follow the LAPACK geqrf convention (beta = -sign(alpha)*norm,
 // v[0] = 1), so the trailing columns of Q match LAPACK's to rounding.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 
 #include "slablu_internal.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace slu {
 namespace {
@@ -537,11 +541,74 @@ __device__ void pivoted_qr_dev(int nr, int nc, double* b, int ld, int* perm, flo
   __syncthreads();
 }
 
+// Sums over the CTAs of a cluster: every CTA sends its terms to the others with
+// asynchronous stores that complete on the receiver's mbarrier, and adds all
+// of them in the order of the ranks, so all CTAs hold the same values.  Two
+// buffers alternate; a warp sends for one exchange after it has read the one
+// before, so nobody overwrites what is still to be read.
+template <int C>
+struct Exchange {
+  double* buf;         // [2][C][terms]
+  int terms, rank;
+  uint32_t bar;        // two mbarriers
+  int n = 0;           // exchanges so far
+  __device__ double* slot(int r, int i) const { return buf + ((n & 1) * C + r) * terms + i; }
+  // one thread per CTA: `count` terms from each other CTA are to come
+  __device__ void expect(int count) const {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar + 8 * (n & 1)),
+                 "r"((C - 1) * count * 8)
+                 : "memory");
+  }
+  __device__ void send(int i, double v) const {
+    *slot(rank, i) = v;
+    const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(slot(rank, i)));
+#pragma unroll
+    for (int q = 1; q < C; ++q) {
+      const int to = (rank + q) % C;
+      uint32_t d, b;
+      asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(to));
+      asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(b) : "r"(bar + 8 * (n & 1)), "r"(to));
+      asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(
+                       d),
+                   "l"(__double_as_longlong(v)), "r"(b)
+                   : "memory");
+    }
+  }
+  __device__ bool wait() const {
+    for (int i = 0; i < (1 << 22); ++i) {
+      uint32_t done;
+      asm volatile(
+          "{\n\t.reg .pred p;\n\t"
+          "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+          "selp.u32 %0, 1, 0, p;\n\t}"
+          : "=r"(done)
+          : "r"(bar + 8 * (n & 1)), "r"((uint32_t)(n >> 1) & 1)
+          : "memory");
+      if (done) return true;
+    }
+    return false;
+  }
+  __device__ double sum(int i) const {
+    double v = *slot(0, i);
+#pragma unroll
+    for (int r = 1; r < C; ++r) v += *slot(r, i);
+    return v;
+  }
+};
+
 constexpr int JAC_THREADS = 512;
+constexpr int JAC_CLUSTER_THREADS = 320;   // of a CTA where several share a problem
 // ld: column stride of the shared array, cols its columns (see jacobi_smem);
-// pre: QR preconditioning first
-template <int LANES, int RPL>
-__global__ void __launch_bounds__(JAC_THREADS)
+// pre: QR preconditioning first.
+// C > 1 (with pre): a cluster of C CTAs per problem.  Each does the whole QR
+// and then keeps its own rows of every column: a round is the partial inner
+// products, one exchange of them, the angles (in every CTA) and the rotation
+// of the own rows.  The float64 pipe of one SM bounds a round of 64 columns
+// of 64 rows (83 instructions of 72 clocks per warp); with four CTAs it is 37
+// and the exchange.  64 x 64, up to 38 problems: 2140 -> 1390 us, up to 76 with
+// two CTAs 1580; 80 x 80: 3640 -> 2210.
+template <int LANES, int RPL, int C>
+__global__ void __launch_bounds__(C > 1 ? JAC_CLUSTER_THREADS : JAC_THREADS)
 jacobi_kernel(int m, int n_in, const double* __restrict__ A, int lda, long long sA, int r,
               double* __restrict__ U, int ldu, long long sU, double* __restrict__ sv,
               long long sS, int* info, int lower, const double* __restrict__ A2,
@@ -555,9 +622,25 @@ jacobi_kernel(int m, int n_in, const double* __restrict__ A, int lda, long long 
   int* order = reinterpret_cast<int*>(nrm + cols);   // np
   int* rows = order + cols;                          // m: row i of the sweeps = row rows[i] of A
   __shared__ int s_rot, s_e0;
-  // blocks nsplit.. work on the second batch (A2 -> U2), same shapes
-  const bool second = (int)blockIdx.x >= nsplit;
-  const long long bi = second ? blockIdx.x - nsplit : blockIdx.x;
+  __shared__ __align__(8) unsigned long long s_bar[2];
+  // problems nsplit.. are the second batch (A2 -> U2), same shapes
+  const int prob = blockIdx.x / C, rank = C > 1 ? (int)blockIdx.x % C : 0;
+  const bool second = prob >= nsplit;
+  const long long bi = second ? prob - nsplit : prob;
+  Exchange<C> ex;
+  if constexpr (C > 1) {
+    ex.buf = reinterpret_cast<double*>(
+        (reinterpret_cast<uintptr_t>(rows + m) + 15) & ~uintptr_t(15));
+    ex.terms = np;
+    ex.rank = rank;
+    ex.bar = static_cast<uint32_t>(__cvta_generic_to_shared(s_bar));
+    if (threadIdx.x == 0) {
+      for (int i = 0; i < 2; ++i)
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(ex.bar + 8 * i) : "memory");
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    cg::this_cluster().sync();
+  }
   A = (second ? A2 : A) + bi * sA;
   if (pre) {
     // columns of A^T = rows of A; with `lower`, only A's lower triangle is read
@@ -602,22 +685,44 @@ jacobi_kernel(int m, int n_in, const double* __restrict__ A, int lda, long long 
   const int ngroups = blockDim.x / LANES;
   const uint32_t gmask = LANES == 32 ? 0xffffffffu
                                      : ((1u << LANES) - 1) << (lane & ~(LANES - 1));
-  int sweep = 0;
-  for (; sweep < JAC_MAX_SWEEPS; ++sweep) {
+  // own rows of every column
+  const int mr = (m + C - 1) / C, own0 = rank * mr, ml = C > 1 ? max(0, min(m - own0, mr)) : m;
+  double* al0 = a + own0;
+  bool failed = false;   // a wait ran out (the same on all threads)
+  // squared norms of all columns
+  auto norms = [&]() {
+    if (C > 1 && threadIdx.x == 0) ex.expect(np);
     // (loops of the same length on every lane: the whole warp joins the sums)
     for (int c0 = 0; c0 < np; c0 += ngroups) {
       const int c = c0 + group;
       double v = 0.0;
       if (c < np) {
-        const double* ac = a + (long long)c * lda_s;
-        for (int i = part; i < m; i += LANES) v = fma(ac[i], ac[i], v);
+        const double* ac = al0 + (long long)c * lda_s;
+        for (int i = part; i < ml; i += LANES) v = fma(ac[i], ac[i], v);
       }
       v = lanes_sum<LANES>(v, 0xffffffffu);
-      if (part == 0 && c < np) nrm[c] = v;
+      if (part == 0 && c < np) {
+        if constexpr (C > 1) ex.send(c, v);
+        else nrm[c] = v;
+      }
     }
+    if constexpr (C > 1) {
+      // (the barrier: the own terms are there too)
+      failed = __syncthreads_or(!ex.wait()) != 0;
+      for (int c = threadIdx.x; c < np; c += blockDim.x) nrm[c] = ex.sum(c);
+      __syncthreads();
+      ++ex.n;
+    }
+  };
+  int sweep = 0;
+  for (; sweep < JAC_MAX_SWEEPS; ++sweep) {
+    norms();
     if (threadIdx.x == 0) s_rot = 0;
     __syncthreads();
+    if (C > 1 && failed) break;
     for (int rnd = 0; rnd < ring; ++rnd) {
+      bool fresh = false, late = false;
+      if (C > 1 && threadIdx.x == 0) ex.expect(npairs);
       for (int p0 = 0; p0 < npairs; p0 += ngroups) {
         // circle method: slot 0 fixed, others rotate
         const bool on = p0 + group < npairs;
@@ -625,24 +730,31 @@ jacobi_kernel(int m, int n_in, const double* __restrict__ A, int lda, long long 
         int p = pi - 1 + rnd, q = np - 2 - pi + rnd;
         p = pi == 0 ? 0 : 1 + (p >= ring ? p - ring : p);
         q = 1 + (q >= ring ? q - ring : q);
-        double* ap = a + (long long)p * lda_s;
-        double* aq = a + (long long)q * lda_s;
+        double* ap = al0 + (long long)p * lda_s;
+        double* aq = al0 + (long long)q * lda_s;
         double x[RPL > 0 ? RPL : 1], y[RPL > 0 ? RPL : 1];
         double g[4] = {0.0, 0.0, 0.0, 0.0};
         if constexpr (RPL > 0) {
 #pragma unroll
           for (int i = 0; i < RPL; ++i) {
             const int row = part + LANES * i;
-            x[i] = row < m ? ap[row] : 0.0;
-            y[i] = row < m ? aq[row] : 0.0;
+            x[i] = row < ml ? ap[row] : 0.0;
+            y[i] = row < ml ? aq[row] : 0.0;
           }
 #pragma unroll
           for (int i = 0; i < RPL; ++i) g[i & 3] = fma(x[i], y[i], g[i & 3]);
         } else {
-          for (int row = part; row < m; row += LANES) g[0] = fma(ap[row], aq[row], g[0]);
+          for (int row = part; row < ml; row += LANES) g[0] = fma(ap[row], aq[row], g[0]);
         }
         double ga = RPL > 2 ? (g[0] + g[2]) + (g[1] + g[3]) : g[0] + g[1];
         ga = lanes_sum<LANES>(ga, 0xffffffffu);
+        if constexpr (C > 1) {
+          // (ngroups >= npairs: one pass)
+          if (on && part == 0) ex.send(pi, ga);
+          late = !ex.wait();
+          __syncwarp();
+          ga = ex.sum(pi);
+        }
         const double al = nrm[p], be = nrm[q];
         double tau, s;
         if (!on || !jac_angle(al, be, ga, tol2, tau, s)) continue;
@@ -654,13 +766,13 @@ jacobi_kernel(int m, int n_in, const double* __restrict__ A, int lda, long long 
             x[i] = fma(-tau, y[i], x[i]);
             y[i] = fma(s, x[i], y[i]);
             x[i] = fma(-tau, y[i], x[i]);
-            if (row < m) {
+            if (row < ml) {
               ap[row] = x[i];
               aq[row] = y[i];
             }
           }
         } else {
-          for (int row = part; row < m; row += LANES) {
+          for (int row = part; row < ml; row += LANES) {
             double xv = ap[row], yv = aq[row];
             xv = fma(-tau, yv, xv);
             yv = fma(s, xv, yv);
@@ -676,7 +788,11 @@ jacobi_kernel(int m, int n_in, const double* __restrict__ A, int lda, long long 
         nb = be - w;
         // a norm that fell by cancellation has lost its digits: form it anew
         // (the whole group sees the same values)
-        if ((int)hi32(na) < 0 || expo(na) < expo(al) - 3) {
+        if constexpr (C > 1) {
+          if ((int)hi32(na) < 0 || expo(na) < expo(al) - 3 || (int)hi32(nb) < 0 ||
+              expo(nb) < expo(be) - 3)
+            fresh = true;   // after the round, for all columns
+        } else if ((int)hi32(na) < 0 || expo(na) < expo(al) - 3) {
           na = 0.0;
           if constexpr (RPL > 0) {
 #pragma unroll
@@ -686,7 +802,7 @@ jacobi_kernel(int m, int n_in, const double* __restrict__ A, int lda, long long 
           }
           na = lanes_sum<LANES>(na, gmask);
         }
-        if ((int)hi32(nb) < 0 || expo(nb) < expo(be) - 3) {
+        if (C == 1 && ((int)hi32(nb) < 0 || expo(nb) < expo(be) - 3)) {
           nb = 0.0;
           if constexpr (RPL > 0) {
 #pragma unroll
@@ -702,18 +818,39 @@ jacobi_kernel(int m, int n_in, const double* __restrict__ A, int lda, long long 
           s_rot = 1;
         }
       }
-      __syncthreads();
+      if constexpr (C > 1) {
+        // decisions by the barrier itself, the same on all threads
+        const bool act = __syncthreads_or(fresh || late) != 0;
+        ++ex.n;
+        if (act) {
+          failed = __syncthreads_or(late) != 0;
+          if (failed) break;
+          norms();
+          if (failed) break;
+        }
+      } else {
+        __syncthreads();
+      }
     }
-    if (!s_rot) break;
+    if (!s_rot || (C > 1 && failed)) break;
     __syncthreads();
   }
-  if (threadIdx.x == 0 && sweep >= JAC_MAX_SWEEPS && info) atomicCAS(info, 0, 1);
+  if (threadIdx.x == 0 && (sweep >= JAC_MAX_SWEEPS || failed) && info)
+    atomicCAS(info, 0, 1);
   // column norms
-  for (int c = warp; c < np; c += nwarps) {
-    double s = 0.0;
-    for (int i = lane; i < m; i += 32) s += a[(long long)c * lda_s + i] * a[(long long)c * lda_s + i];
-    s = warp_sum(s);
-    if (lane == 0) nrm[c] = sqrt(s);
+  if constexpr (C > 1) {
+    __syncthreads();
+    if (!failed) norms();
+    __syncthreads();
+    for (int c = threadIdx.x; c < np; c += blockDim.x) nrm[c] = sqrt(nrm[c]);
+  } else {
+    for (int c = warp; c < np; c += nwarps) {
+      double s = 0.0;
+      for (int i = lane; i < m; i += 32)
+        s += a[(long long)c * lda_s + i] * a[(long long)c * lda_s + i];
+      s = warp_sum(s);
+      if (lane == 0) nrm[c] = sqrt(s);
+    }
   }
   __syncthreads();
   // rank of each column by decreasing norm (ties by index).  A NaN norm
@@ -738,9 +875,9 @@ jacobi_kernel(int m, int n_in, const double* __restrict__ A, int lda, long long 
   for (int j = warp; j < r; j += nwarps) {
     const int c = min(max(order[j < np ? j : np - 1], 0), np - 1);
     double s = nrm[c];
-    if (svb && lane == 0) svb[j] = (j < n) ? s : 0.0;
+    if (svb && lane == 0 && rank == 0) svb[j] = (j < n) ? s : 0.0;
     bool ok = (j < n) && s > tiny;
-    for (int i = lane; i < m; i += 32)
+    for (int i = own0 + lane; i < own0 + ml; i += 32)
       Ub[(long long)(pre ? rows[i] : i) * ldu + j] = ok ? a[(long long)c * lda_s + i] / s : 0.0;
   }
   __syncthreads();
@@ -751,6 +888,11 @@ jacobi_kernel(int m, int n_in, const double* __restrict__ A, int lda, long long 
   // columns join), so each is tried once: the compression of a zero 512-point
   // block (rank 24) takes 9 ms where retrying all of them for every column
   // took 30.
+  if constexpr (C > 1) {
+    // all rows are written; nothing is sent any more
+    cg::this_cluster().sync();
+    if (rank != 0) return;
+  }
   int j0 = 0;
   while (j0 < r && j0 < n && nrm[min(max(order[j0 < np ? j0 : np - 1], 0), np - 1)] > tiny) ++j0;
   __syncthreads();
@@ -984,15 +1126,27 @@ void apply_q(cudaStream_t st, bool transpose, int m, int k, const double* V, int
 }
 
 namespace {
-template <int LANES, int RPL>
+template <int LANES, int RPL, int C>
 void launch_jacobi(cudaStream_t st, int grid, int threads, size_t sm, int m, int n,
                    const double* A, int lda, long long sA, int r, double* U, int ldu,
                    long long sU, double* sv, long long sS, int* info, bool lower,
                    const double* A2, double* U2, int nsplit, int ld, int cols, int pre) {
-  auto kern = jacobi_kernel<LANES, RPL>;
+  auto kern = jacobi_kernel<LANES, RPL, C>;
   ensure_smem(reinterpret_cast<const void*>(kern), sm);
-  kern<<<grid, threads, sm, st>>>(m, n, A, lda, sA, r, U, ldu, sU, sv, sS, info, lower ? 1 : 0, A2,
-                                  U2, nsplit, ld, cols, pre);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(grid * C));
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = sm;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = C;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = C > 1 ? 1 : 0;
+  SLU_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, m, n, A, lda, sA, r, U, ldu, sU, sv, sS, info,
+                                    lower ? 1 : 0, A2, U2, nsplit, ld, cols, pre));
   check_launch("jacobi_kernel");
 }
 
@@ -1019,7 +1173,7 @@ void jacobi_dispatch(cudaStream_t st, int grid, int m, int n, const double* A, i
     ld = m | 1;
     cols = n + (n & 1);
   }
-  const size_t sm = bytes(ld, cols, pre);
+  size_t sm = bytes(ld, cols, pre);
   SLU_REQUIRE(sm <= 220 * 1024, "jacobi: block too large for shared memory");
   const int swept = pre ? k : n, pairs = (swept + (swept & 1)) / 2;
   auto rows = [&](int lanes) { return (m + lanes - 1) / lanes; };
@@ -1030,9 +1184,27 @@ void jacobi_dispatch(cudaStream_t st, int grid, int m, int n, const double* A, i
   int lanes = 4;
   if (rows(4) > 16 || cost(8) < cost(4)) lanes = 8;
   const int threads = std::min(JAC_THREADS, std::max(64, (pairs * lanes + 31) / 32 * 32));
-#define SLU_JACOBI(L, R)                                                                        \
-  return launch_jacobi<L, R>(st, grid, threads, sm, m, n, A, lda, sA, r, U, ldu, sU, sv, sS, info, \
-                             lower, A2, U2, nsplit, ld, cols, pre)
+#define SLU_JACOBI_C(L, R, C)                                                                  \
+  return launch_jacobi<L, R, C>(st, grid, threads, sm, m, n, A, lda, sA, r, U, ldu, sU, sv, sS, \
+                                info, lower, A2, U2, nsplit, ld, cols, pre)
+#define SLU_JACOBI(L, R) SLU_JACOBI_C(L, R, 1)
+  // few problems: four or two CTAs each, while every CTA gets an SM
+  if (pre && k >= 32 && pairs * 4 <= JAC_CLUSTER_THREADS && 2LL * grid <= num_sms()) {
+    const int C = 4LL * grid <= num_sms() ? 4 : 2, np = k + (k & 1);
+    const int rc = ((m + C - 1) / C + 3) / 4;   // rows per lane, four lanes per pair
+    const size_t more = 2 * sizeof(double) * C * np + 16;
+    if (rc <= 10 && sm + more <= 220 * 1024) {
+      sm += more;
+      const int threads = std::max(64, (pairs * 4 + 31) / 32 * 32);
+      if (C == 4) {
+        if (rc <= 4) SLU_JACOBI_C(4, 4, 4);
+        if (rc <= 6) SLU_JACOBI_C(4, 6, 4);
+        SLU_JACOBI_C(4, 10, 4);
+      }
+      if (rc <= 8) SLU_JACOBI_C(4, 8, 2);
+      SLU_JACOBI_C(4, 10, 2);
+    }
+  }
   const int rp = rows(lanes);
   if (lanes == 4) {
     if (rp <= 4) SLU_JACOBI(4, 4);
@@ -1049,6 +1221,7 @@ void jacobi_dispatch(cudaStream_t st, int grid, int m, int n, const double* A, i
   if (rp <= 16) SLU_JACOBI(8, 16);
   SLU_JACOBI(8, 0);
 #undef SLU_JACOBI
+#undef SLU_JACOBI_C
 }
 }  // namespace
 
