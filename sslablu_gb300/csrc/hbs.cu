@@ -55,6 +55,7 @@ void setup_geometry_common(Hbs& H) {
 //   Ud_out    : Nb*kslice x kU, R22_out: Nb*k x k (non-root)
 struct UlvScratch {
   double *WSV, *tauV, *Qk, *DWt, *tauQ, *Qc, *QtU;
+  int* info;
 };
 
 void ulv_level(cudaStream_t st, Level& l, bool root, const double* Rhat, const double* Uhat,
@@ -65,7 +66,7 @@ void ulv_level(cudaStream_t st, Level& l, bool root, const double* Rhat, const d
   if (!root) {
     // W1: trailing n-k columns of the complete QR of each V block (ULVsparse.py:18-25)
     transpose_batched(st, n, k, dp(l.V), k, (long long)n * k, 0, s.WSV, n, (long long)n * k, 0, Nb);
-    panel_qr(st, n, k, k, s.WSV, n, (long long)n * k, s.tauV, k, Nb);
+    panel_qr(st, n, k, k, s.WSV, n, (long long)n * k, s.tauV, k, Nb, s.info);
     if (n > k) {
       identity_cols(st, n, k, n - k, s.Qk, (long long)n * (n - k), Nb);
       apply_q(st, false, n, k, s.WSV, n, (long long)n * k, s.tauV, k, s.Qk, n,
@@ -82,7 +83,7 @@ void ulv_level(cudaStream_t st, Level& l, bool root, const double* Rhat, const d
     transpose_batched(st, n, n, Rhat, n, nn, 0, s.DWt, n, nn, 0, Nb);
   }
   // square QR of Rhat W (ULVsparse.py:51-61)
-  panel_qr(st, n, n, n, s.DWt, n, nn, s.tauQ, n, Nb);
+  panel_qr(st, n, n, n, s.DWt, n, nn, s.tauQ, n, Nb, s.info);
   extract_upper(st, 0, nu, 0, n, s.DWt, n, nn, dp(l.R), n, (long long)nu * n, Nb);
   if (!root && k > 0) extract_upper(st, nu, k, nu, k, s.DWt, n, nn, R22_out, k, (long long)k * k, Nb);
   identity_cols(st, n, 0, n, s.Qc, nn, Nb);
@@ -121,7 +122,7 @@ UlvScratch carve_ulv(Workspace& ws, const Hbs& H) {
     d = std::max(d, nb * n);
     e = std::max(e, nb * n * std::max<size_t>(std::max<size_t>(k, n), 1));
   }
-  UlvScratch s;
+  UlvScratch s{};
   s.WSV = ws.take<double>(a);
   s.tauV = ws.take<double>(b);
   s.Qk = ws.take<double>(c);
@@ -244,6 +245,7 @@ void hbs_compress(Handle& h, Hbs& H, int Nb0, int rk, int s, const double* Om, c
   double *Rhat = nullptr, *Uhat = nullptr, *Ud[2] = {nullptr, nullptr}, *R22[2] = {nullptr, nullptr};
   if (ulv) {
     us = carve_ulv(h.ws, H);
+    us.info = h.info.as<int>();
     Rhat = h.ws.take<double>((size_t)N * nmax);
     Uhat = h.ws.take<double>((size_t)N * nmax);
     for (int a = 0; a < 2; ++a) {
@@ -300,14 +302,14 @@ void hbs_compress(Handle& h, Hbs& H, int Nb0, int rk, int s, const double* Om, c
     const bool wy = wy_pays(s, n, n);
     const int carried = wy ? n : 2 * n;   // columns of the panel kernels
     if (root) {
-      panel_qr(st, s, n, carried, WSA, s, 2 * ns, tauA, n, Nb);
+      panel_qr(st, s, n, carried, WSA, s, 2 * ns, tauA, n, Nb, h.info.as<int>());
       if (wy) apply_wy(h, s, n, WSA, nullptr, s, 2 * ns, tauA, nullptr, n, n, Nb);
     }
     const double* YQ1A = WSA + ns;   // row-major n x n (ld s): Y_blk * Q_1
     if (!root) {
       copy_blocks(st, Nb, 8 * ns, Psi_t, 8 * ns, WSB, 16 * ns);
       copy_blocks(st, Nb, 8 * ns, Z_t, 8 * ns, WSB + ns, 16 * ns);
-      panel_qr2(st, s, n, carried, WSA, WSB, s, 2 * ns, tauA, tauB, n, Nb);
+      panel_qr2(st, s, n, carried, WSA, WSB, s, 2 * ns, tauA, tauB, n, Nb, h.info.as<int>());
       if (wy) apply_wy(h, s, n, WSA, WSB, s, 2 * ns, tauA, tauB, n, n, Nb);
       int* info = h.info.as<int>();
       // U, V: leading left singular vectors of Y_blk Q[:, s-n:s] (HBSnew.py:26-27)
@@ -319,7 +321,7 @@ void hbs_compress(Handle& h, Hbs& H, int Nb0, int rk, int s, const double* Om, c
         // wide n x jc block: its left singular vectors are those of R^T from
         // the QR of its transpose, which the panels already hold column-major
         // (column i = row i of the block); R^T is n x n lower triangular
-        panel_qr2(st, jc, n, n, WSA + ns + j0, WSB + ns + j0, s, 2 * ns, tauA, tauB, n, Nb);
+        panel_qr2(st, jc, n, n, WSA + ns + j0, WSB + ns + j0, s, 2 * ns, tauA, tauB, n, Nb, info);
         jacobi_left_sv2(st, n, n, WSA + ns + j0, WSB + ns + j0, s, 2 * ns, k, dp(l.U), dp(l.V),
                         k, (long long)n * k, Nb, info, true);
       } else {
@@ -403,6 +405,7 @@ void hbs_factor(Handle& h, Hbs& H) {
   }
   h.ws.reserve(ulv_scratch_bytes(H) + 8 * (2 * N * nmax + 4 * N * kmax) + 8 * 256, st);
   UlvScratch us = carve_ulv(h.ws, H);
+  us.info = h.info.as<int>();
   double* Rhat = h.ws.take<double>(N * nmax);
   double* Uhat = h.ws.take<double>(N * nmax);
   double *Ud[2], *R22[2];

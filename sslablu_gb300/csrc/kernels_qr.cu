@@ -194,6 +194,78 @@ __device__ __forceinline__ Reflector make_reflector(double alpha, double ss) {
   return h;
 }
 
+// ---------------------------------------------------------------- clusters
+// Sums over the CTAs of a cluster: every CTA sends its terms to the others with
+// asynchronous stores that complete on the receiver's mbarrier, and adds all
+// of them in the same order, so all CTAs hold the same values.  Two
+// buffers alternate; a warp sends for one exchange after it has read the one
+// before, so nobody overwrites what is still to be read.
+template <int C>
+struct Exchange {
+  double* buf;         // [2][C][terms]
+  int terms, rank;
+  uint32_t bar;        // two mbarriers
+  int n = 0;           // exchanges so far
+  __device__ void init(double* b, int t, int r, unsigned long long* bars) {
+    buf = b;
+    terms = t;
+    rank = r;
+    bar = static_cast<uint32_t>(__cvta_generic_to_shared(bars));
+    if (threadIdx.x == 0) {
+      for (int i = 0; i < 2; ++i)
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar + 8 * i) : "memory");
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    cg::this_cluster().sync();
+  }
+  __device__ double* slot(int r, int i) const { return buf + ((n & 1) * C + r) * terms + i; }
+  // one thread per CTA: `count` terms from the other CTAs are to come
+  __device__ void expect(int count) const {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar + 8 * (n & 1)),
+                 "r"(count * 8)
+                 : "memory");
+  }
+  __device__ void send(int i, double v) const {
+    *slot(rank, i) = v;
+    const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(slot(rank, i)));
+#pragma unroll
+    for (int q = 1; q < C; ++q) {
+      const int to = (rank + q) % C;
+      uint32_t d, b;
+      asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(to));
+      asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(b) : "r"(bar + 8 * (n & 1)), "r"(to));
+      asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(
+                       d),
+                   "l"(__double_as_longlong(v)), "r"(b)
+                   : "memory");
+    }
+  }
+  __device__ bool wait() const {
+    for (int i = 0; i < (1 << 22); ++i) {
+      uint32_t done;
+      asm volatile(
+          "{\n\t.reg .pred p;\n\t"
+          "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+          "selp.u32 %0, 1, 0, p;\n\t}"
+          : "=r"(done)
+          : "r"(bar + 8 * (n & 1)), "r"((uint32_t)(n >> 1) & 1)
+          : "memory");
+      if (done) return true;
+    }
+    return false;
+  }
+  __device__ double sum(int i) const {
+    double v[C];
+#pragma unroll
+    for (int r = 0; r < C; ++r) v[r] = *slot(r, i);
+#pragma unroll
+    for (int h = 1; h < C; h *= 2)
+#pragma unroll
+      for (int r = 0; r + h < C; r += 2 * h) v[r] += v[r + h];
+    return v[0];
+  }
+};
+
 // ---------------------------------------------------------------- panels in shared memory
 // QR of an m x n column-major panel, one CTA, the panel in shared memory
 // (column stride ld, 8 mod 16: the 2 x 8 entries of a wavefront hit distinct
@@ -298,6 +370,142 @@ panel_qr_smem_kernel(int m, int n, double* __restrict__ W, int ldw, long long sW
       w[(long long)c * ldw + i] = (i > c && sc != 0.0) ? x * sc : x;
     }
   }
+}
+
+// The same by a cluster of C CTAs per panel where there are few of them: each
+// CTA holds its rows of every column, four lanes per column.  Per column one
+// exchange: the partial products of the column with itself and all later ones,
+// and from the owner of the diagonal that row; every thread forms the
+// reflector's v0 and f, and the updates are local.  The float64 pipe of one SM
+// bounds panel_qr_smem_kernel (a 261 x 64 panel 360 us, alone or one of 128);
+// here up to 38 panels take 268 us (four CTAs each): 2K clocks of a column the
+// reflector, 1.2K the exchange.
+// A thread's entries (at most R of its column) stay in registers between the
+// product and the update; a multiplication of a warp takes 72 clocks however
+// few of its lanes it serves, so rows that are done are branched over.
+template <int C, int R>
+__global__ void __launch_bounds__(256)
+panel_qr_cluster_kernel(int m, int n, double* __restrict__ W, int ldw, long long sW,
+                        double* __restrict__ tau, long long sTau, int ld, double* __restrict__ W2,
+                        double* __restrict__ tau2, int nsplit, int* info) {
+  extern __shared__ double sm[];
+  double* s_sc = sm + (size_t)ld * n;   // n: 1 / v0
+  __shared__ __align__(8) unsigned long long s_bar[2];
+  __shared__ double s_v0, s_f;
+  const int prob = blockIdx.x / C, rank = (int)blockIdx.x % C;
+  const bool second = prob >= nsplit;
+  const long long b = second ? prob - nsplit : prob;
+  double* w = (second ? W2 : W) + b * sW;
+  double* tg = (second ? tau2 : tau) + b * sTau;
+  Exchange<C> ex;
+  ex.init(s_sc + n, 2 * n, rank, s_bar);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+  const int part = tid & 3, group = tid >> 2, ngroups = blockDim.x >> 2;
+  const int mr = (m + C - 1) / C, own0 = rank * mr, ml = max(0, min(m - own0, mr));
+  for (int c = warp; c < n; c += nwarps)
+    for (int i = lane; i < ml; i += 32) sm[(size_t)c * ld + i] = w[(long long)c * ldw + own0 + i];
+  __syncthreads();
+  const int steps = min(n, m);
+  bool failed = false;
+  for (int j = 0; j < steps && !failed; ++j) {
+    const int owner = j / mr, lj = j - own0;   // lj: local row of the diagonal, in its owner
+    const double* v = sm + (size_t)j * ld;
+    if (tid == 0) ex.expect((C - 1) * (n - j) + (rank != owner ? n - j : 0));
+    // rows lo .. ml - 1 are below the diagonal: entries u0 .. u1 - 1
+    const int lo = max(0, lj + 1), u0 = lo >> 2, u1 = (ml + 3) >> 2;
+    double y[R], x[R];   // the column's entries and the first product's
+#pragma unroll
+    for (int u = 0; u < R; ++u) {
+      const int i = 4 * u + part;
+      y[u] = i >= lo && i < ml ? v[i] : 0.0;
+    }
+    for (int c0 = j; c0 < n; c0 += ngroups) {
+      const int c = c0 + group;
+      const bool on = c < n;
+      if (c0 + (group & ~7) >= n) break;   // the whole warp
+      const double* cc = sm + (size_t)(on ? c : j) * ld;
+      double z[R], d[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+      for (int u = 0; u < R; ++u) {
+        const int i = 4 * u + part;
+        z[u] = i >= lo && i < ml ? cc[i] : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < R; ++u) {
+        if (u < u0) continue;
+        if (u >= u1) break;
+        d[u & 3] = fma(y[u], z[u], d[u & 3]);
+      }
+      const double s = lanes_sum<4>((d[0] + d[1]) + (d[2] + d[3]), 0xffffffffu);
+      if (on && part == 0) {
+        ex.send(c, s);
+        if (rank == owner) ex.send(n + c, cc[lj]);
+      }
+      if (c0 == j) {
+#pragma unroll
+        for (int u = 0; u < R; ++u) x[u] = z[u];
+      }
+    }
+    failed = __syncthreads_or(!ex.wait()) != 0;   // (and the own terms are there)
+    if (failed) break;
+    // warp 0 forms the reflector, the others add up their products meanwhile
+    const int c1 = j + group;   // the column whose entries are in x
+    const bool on1 = group > 0 && c1 < n;
+    const double r1 = on1 ? *ex.slot(owner, n + c1) : 0.0, d1 = on1 ? ex.sum(c1) : 0.0;
+    if (warp == 0) {
+      const Reflector h = make_reflector(*ex.slot(owner, n + j), ex.sum(j));
+      if (lane == 0) {
+        s_v0 = h.v0;
+        s_f = h.f;
+        s_sc[j] = h.sc;
+        if (rank == owner) {
+          tg[j] = h.tau;
+          sm[(size_t)j * ld + lj] = h.beta;
+        }
+      }
+    }
+    __syncthreads();
+    const double v0 = s_v0, f = s_f;
+    if (f != 0.0) {
+      for (int c0 = j; c0 < n; c0 += ngroups) {
+        const int c = c0 + group;
+        if (c0 + (group & ~7) >= n) break;
+        const bool on = c > j && c < n;
+        double* cc = sm + (size_t)(on ? c : j) * ld;
+        double rc = r1, t = d1;
+        if (c0 > j && on) {
+          rc = *ex.slot(owner, n + c);
+          t = ex.sum(c);
+#pragma unroll
+          for (int u = 0; u < R; ++u) {
+            const int i = 4 * u + part;
+            x[u] = i >= lo && i < ml ? cc[i] : 0.0;
+          }
+        }
+        t = f * fma(v0, rc, t);
+#pragma unroll
+        for (int u = 0; u < R; ++u) {
+          if (u < u0) continue;
+          if (u >= u1) break;
+          const int i = 4 * u + part;
+          const double q = fma(-t, y[u], x[u]);
+          if (on && i >= lo && i < ml) cc[i] = q;
+        }
+        if (rank == owner && part == 0 && on) cc[lj] = fma(-t, v0, rc);
+      }
+    }
+    ++ex.n;
+    __syncthreads();
+  }
+  if (tid == 0 && failed && info) atomicCAS(info, 0, 1);
+  for (int c = warp; c < n; c += nwarps) {
+    const double sc = c < steps ? s_sc[c] : 0.0;
+    for (int i = lane; i < ml; i += 32) {
+      const double x = sm[(size_t)c * ld + i];
+      w[(long long)c * ldw + own0 + i] = (own0 + i > c && sc != 0.0) ? x * sc : x;
+    }
+  }
+  cg::this_cluster().sync();   // nobody sends to a CTA that has left
 }
 
 // C <- Q^T C (transpose) or Q C for the m x k reflectors of a factored panel,
@@ -541,61 +749,6 @@ __device__ void pivoted_qr_dev(int nr, int nc, double* b, int ld, int* perm, flo
   __syncthreads();
 }
 
-// Sums over the CTAs of a cluster: every CTA sends its terms to the others with
-// asynchronous stores that complete on the receiver's mbarrier, and adds all
-// of them in the order of the ranks, so all CTAs hold the same values.  Two
-// buffers alternate; a warp sends for one exchange after it has read the one
-// before, so nobody overwrites what is still to be read.
-template <int C>
-struct Exchange {
-  double* buf;         // [2][C][terms]
-  int terms, rank;
-  uint32_t bar;        // two mbarriers
-  int n = 0;           // exchanges so far
-  __device__ double* slot(int r, int i) const { return buf + ((n & 1) * C + r) * terms + i; }
-  // one thread per CTA: `count` terms from each other CTA are to come
-  __device__ void expect(int count) const {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar + 8 * (n & 1)),
-                 "r"((C - 1) * count * 8)
-                 : "memory");
-  }
-  __device__ void send(int i, double v) const {
-    *slot(rank, i) = v;
-    const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(slot(rank, i)));
-#pragma unroll
-    for (int q = 1; q < C; ++q) {
-      const int to = (rank + q) % C;
-      uint32_t d, b;
-      asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(to));
-      asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(b) : "r"(bar + 8 * (n & 1)), "r"(to));
-      asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(
-                       d),
-                   "l"(__double_as_longlong(v)), "r"(b)
-                   : "memory");
-    }
-  }
-  __device__ bool wait() const {
-    for (int i = 0; i < (1 << 22); ++i) {
-      uint32_t done;
-      asm volatile(
-          "{\n\t.reg .pred p;\n\t"
-          "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-          "selp.u32 %0, 1, 0, p;\n\t}"
-          : "=r"(done)
-          : "r"(bar + 8 * (n & 1)), "r"((uint32_t)(n >> 1) & 1)
-          : "memory");
-      if (done) return true;
-    }
-    return false;
-  }
-  __device__ double sum(int i) const {
-    double v = *slot(0, i);
-#pragma unroll
-    for (int r = 1; r < C; ++r) v += *slot(r, i);
-    return v;
-  }
-};
-
 constexpr int JAC_THREADS = 512;
 constexpr int JAC_CLUSTER_THREADS = 320;   // of a CTA where several share a problem
 // ld: column stride of the shared array, cols its columns (see jacobi_smem);
@@ -629,17 +782,9 @@ jacobi_kernel(int m, int n_in, const double* __restrict__ A, int lda, long long 
   const long long bi = second ? prob - nsplit : prob;
   Exchange<C> ex;
   if constexpr (C > 1) {
-    ex.buf = reinterpret_cast<double*>(
-        (reinterpret_cast<uintptr_t>(rows + m) + 15) & ~uintptr_t(15));
-    ex.terms = np;
-    ex.rank = rank;
-    ex.bar = static_cast<uint32_t>(__cvta_generic_to_shared(s_bar));
-    if (threadIdx.x == 0) {
-      for (int i = 0; i < 2; ++i)
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(ex.bar + 8 * i) : "memory");
-      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    cg::this_cluster().sync();
+    ex.init(reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(rows + m) + 15) &
+                                      ~uintptr_t(15)),
+            np, rank, s_bar);
   }
   A = (second ? A2 : A) + bi * sA;
   if (pre) {
@@ -691,7 +836,7 @@ jacobi_kernel(int m, int n_in, const double* __restrict__ A, int lda, long long 
   bool failed = false;   // a wait ran out (the same on all threads)
   // squared norms of all columns
   auto norms = [&]() {
-    if (C > 1 && threadIdx.x == 0) ex.expect(np);
+    if (C > 1 && threadIdx.x == 0) ex.expect((C - 1) * np);
     // (loops of the same length on every lane: the whole warp joins the sums)
     for (int c0 = 0; c0 < np; c0 += ngroups) {
       const int c = c0 + group;
@@ -722,7 +867,7 @@ jacobi_kernel(int m, int n_in, const double* __restrict__ A, int lda, long long 
     if (C > 1 && failed) break;
     for (int rnd = 0; rnd < ring; ++rnd) {
       bool fresh = false, late = false;
-      if (C > 1 && threadIdx.x == 0) ex.expect(npairs);
+      if (C > 1 && threadIdx.x == 0) ex.expect((C - 1) * npairs);
       for (int p0 = 0; p0 < npairs; p0 += ngroups) {
         // circle method: slot 0 fixed, others rotate
         const bool on = p0 + group < npairs;
@@ -1056,6 +1201,10 @@ void launch_apply(cudaStream_t st, bool transpose, int m, int k, const double* V
 
 // Rows that eight lanes hold in registers; taller columns stay in memory.
 constexpr int kApplyRows = 320;
+// Rows from which few panels are shared by clusters of eight or four CTAs.  At
+// 64 rows the exchange and the reflector of a column take as long as one CTA's
+// column; with two CTAs per panel of 261 x 64 nothing is gained (398 -> 385 us).
+constexpr int kClusterRows = 128;
 
 void apply_q_dispatch(cudaStream_t st, bool transpose, int m, int k, const double* V, int ldv,
                       long long sV, const double* tau, long long sTau, double* C, int ldc,
@@ -1078,7 +1227,39 @@ void apply_q_dispatch(cudaStream_t st, bool transpose, int m, int k, const doubl
 // memory where they fit, the carried columns afterwards from registers; else
 // everything by the one-CTA kernel in global memory.
 void panel_qr_any(cudaStream_t st, int m, int nfac, int ncol, double* W, double* W2, int ldw,
-                  long long sW, double* tau, double* tau2, long long sTau, int batch, int total) {
+                  long long sW, double* tau, double* tau2, long long sTau, int batch, int total,
+                  int* info) {
+  if (info && m >= kClusterRows && 4LL * total <= num_sms()) {
+    const int C = 8LL * total <= num_sms() ? 8 : 4;
+    const int mr = (m + C - 1) / C, ldc = (mr + 11) / 16 * 16 + 4;   // >= mr, 4 mod 16
+    const size_t smc = sizeof(double) * ((size_t)ldc * nfac + nfac + 4 * (size_t)C * nfac);
+    const int rl = (mr + 3) / 4;   // rows per lane
+    if (rl <= 17 && smc <= 220 * 1024 && (ncol == nfac || m <= kApplyRows)) {
+      auto kern = C == 8 ? (rl <= 9 ? panel_qr_cluster_kernel<8, 9> : panel_qr_cluster_kernel<8, 17>)
+                         : (rl <= 9 ? panel_qr_cluster_kernel<4, 9> : panel_qr_cluster_kernel<4, 17>);
+      ensure_smem(reinterpret_cast<const void*>(kern), smc);
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3((unsigned)(total * C));
+      cfg.blockDim = dim3(256);
+      cfg.dynamicSmemBytes = smc;
+      cfg.stream = st;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = (unsigned)C;
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      SLU_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, m, nfac, W, ldw, sW, tau, sTau, ldc, W2, tau2,
+                                        batch, info));
+      check_launch("panel_qr_cluster_kernel");
+      if (ncol > nfac)
+        apply_q_dispatch(st, true, m, std::min(nfac, m), W, ldw, sW, tau, sTau,
+                         W + (long long)nfac * ldw, ldw, sW, ncol - nfac, W2, tau2,
+                         W2 + (long long)nfac * ldw, batch, total);
+      return;
+    }
+  }
   const int ld = (m + 7) / 16 * 16 + 8;   // >= m, 8 mod 16
   const size_t sm = sizeof(double) * ((size_t)ld * nfac + nfac);
   if (sm <= 220 * 1024 && (ncol == nfac || m <= kApplyRows)) {
@@ -1100,15 +1281,15 @@ void panel_qr_any(cudaStream_t st, int m, int nfac, int ncol, double* W, double*
 }  // namespace
 
 void panel_qr(cudaStream_t st, int m, int nfac, int ncol, double* W, int ldw, long long sW,
-              double* tau, long long sTau, int batch) {
+              double* tau, long long sTau, int batch, int* info) {
   if (batch <= 0 || m <= 0 || nfac <= 0) return;
-  panel_qr_any(st, m, nfac, ncol, W, W, ldw, sW, tau, tau, sTau, batch, batch);
+  panel_qr_any(st, m, nfac, ncol, W, W, ldw, sW, tau, tau, sTau, batch, batch, info);
 }
 
 void panel_qr2(cudaStream_t st, int m, int nfac, int ncol, double* W, double* W2, int ldw,
-               long long sW, double* tau, double* tau2, long long sTau, int batch) {
+               long long sW, double* tau, double* tau2, long long sTau, int batch, int* info) {
   if (batch <= 0 || m <= 0 || nfac <= 0) return;
-  panel_qr_any(st, m, nfac, ncol, W, W2, ldw, sW, tau, tau2, sTau, batch, 2 * batch);
+  panel_qr_any(st, m, nfac, ncol, W, W2, ldw, sW, tau, tau2, sTau, batch, 2 * batch, info);
 }
 
 void apply_q(cudaStream_t st, bool transpose, int m, int k, const double* V, int ldv,

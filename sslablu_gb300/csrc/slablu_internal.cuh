@@ -111,8 +111,9 @@ void gemm_batched(cudaStream_t st, bool ta, bool tb, int M, int N, int K, T alph
 // its first nfac columns are factored in place (R on/above the diagonal,
 // reflectors below), tau_b[j] the scalar factors; the Householder reflectors
 // are applied to all remaining columns nfac..ncol-1 (which then hold Q^T c).
+// info (device, for waits that run out) lets few panels go over clusters.
 void panel_qr(cudaStream_t st, int m, int nfac, int ncol, double* W, int ldw,
-              long long sW, double* tau, long long sTau, int batch);
+              long long sW, double* tau, long long sTau, int batch, int* info = nullptr);
 
 // The same factorisation for wide panels (nfac > 64): 32-column panels by
 // panel_qr, the trailing columns updated in the compact WY form
@@ -126,7 +127,8 @@ void qr_blocked(cudaStream_t st, int m, int nfac, int ncol, double* W, int ldw, 
 // Two panel factorisations of the same shapes in one launch (W, tau and
 // W2, tau2, batch blocks each).
 void panel_qr2(cudaStream_t st, int m, int nfac, int ncol, double* W, double* W2, int ldw,
-               long long sW, double* tau, double* tau2, long long sTau, int batch);
+               long long sW, double* tau, double* tau2, long long sTau, int batch,
+               int* info = nullptr);
 
 // Apply the reflectors of a factored panel (m x k, column-major, ldv) to the
 // columns of C (m x nc, column-major, ldc): C <- Q C (left = false means

@@ -49,3 +49,28 @@ def test_carried_columns(n, k):
     """Sketch panels either side of the sizes that take the compact WY form."""
     from tests.test_gpu_svd_edges import test_two_level_compression as check
     check(n, k, "full")
+
+
+@pytest.mark.parametrize("leaf,k,L", [(48, 12, 5), (64, 32, 5), (100, 24, 2), (40, 20, 6)])
+def test_compression_levels(leaf, k, L):
+    """Compression from sketches at block counts that share panels and sweeps
+    between eight, four, two or one CTAs."""
+    need_gpu()
+    import torch
+    from sslablu_gb300.matAssembly.HBS.HBSnew import HBSMAT, samples_for
+    from sslablu_gb300.synthetic import random_hbs_factors
+    rng = np.random.default_rng(leaf * L + k)
+    U, D, V, Nbvec = random_hbs_factors(k, leaf, L, rng=rng, shift=4.0 * np.sqrt(leaf))
+    A = _dense(U, D, V, Nbvec)
+    N, s = A.shape[0], samples_for(k, leaf, 2)
+    H = HBSMAT(A, None, False)
+    H.set_Nbvec(list(Nbvec))
+    H.Nbvec = []
+    Om, Psi = rng.standard_normal((N, s)), rng.standard_normal((N, s))
+    H.compress_from_sketches(k, Om, Psi, A @ Om, A.T @ Psi, compute_ULV=True)
+    X = rng.standard_normal((N, 3))
+    got, ref = H.matmat(torch.from_numpy(X).cuda()).cpu().numpy(), A @ X
+    # as the two-level compressions: condition numbers below 20, n roundings a level
+    assert np.linalg.norm(got - ref) <= 1e-13 * leaf * L * np.linalg.norm(ref)
+    x = H.solve(X)
+    assert np.linalg.norm(A @ x - X) <= 1e-12 * leaf * L * np.linalg.norm(A, 2) * np.linalg.norm(x)
