@@ -504,13 +504,25 @@ void launch_panel(cudaStream_t st, int n, int k0, int kb, double* A, int lda, lo
 __global__ void __launch_bounds__(256)
 tri_pack_kernel(int n, int np, const double* __restrict__ LU, int lda, long long sA,
                 const int* __restrict__ piv, long long sP, double* __restrict__ T,
-                int* __restrict__ perm) {
+                int* perm, int in_place) {
   const int b = blockIdx.z, tid = threadIdx.x;
   LU += b * sA;
   extern __shared__ int s_perm[];
   if (blockIdx.y == gridDim.y - 1) {
     if (blockIdx.x != 0) return;
     piv += b * sP;
+    if (in_place) {   // too large for shared memory
+      int* pm = perm + (long long)b * n;
+      for (int i = tid; i < n; i += 256) pm[i] = i;
+      __syncthreads();
+      if (tid == 0)
+        for (int i = 0; i < n; ++i) {
+          const int p = piv[i], t = pm[i];
+          pm[i] = pm[p];
+          pm[p] = t;
+        }
+      return;
+    }
     int* pv = s_perm + n;
     for (int i = tid; i < n; i += 256) {
       s_perm[i] = i;
@@ -655,12 +667,13 @@ void lu_inverse(Handle& h, int n, const double* LU, int lda, long long sA, const
     double* W = h.lu_ws.take<double>(nn * nb);
     double* LP = h.lu_ws.take<double>((size_t)np * n * nb);
     int* perm = h.lu_ws.take<int>((size_t)n * nb);
-    const size_t sm = 2 * sizeof(int) * (size_t)n;
-    SLU_REQUIRE(sm <= 200 * 1024, "LU inverse: block too large");
+    const int in_place = 2 * sizeof(int) * (size_t)n > 200 * 1024;
+    const size_t sm = in_place ? 0 : 2 * sizeof(int) * (size_t)n;
     ensure_smem(reinterpret_cast<const void*>(tri_pack_kernel), sm);
     const int tl = (np + 31) / 32;
     tri_pack_kernel<<<dim3(tl, tl + 1, nb), 256, sm, st>>>(n, np, LU + b0 * sA, lda, sA,
-                                                           piv + b0 * sP, sP, T, perm);
+                                                           piv + b0 * sP, sP, T, perm,
+                                                           in_place);
     check_launch("tri_pack_kernel");
     tri_base_kernel<<<dim3(1 << q, 2 * nb), 32, 0, st>>>(np, w, T);
     check_launch("tri_base_kernel");

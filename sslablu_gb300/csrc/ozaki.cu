@@ -35,8 +35,8 @@
 //     2^-48 of the largest one.
 // The dropped digit pairs and the truncated digits leave a relative error of
 // about 2^-55 of |S| |z| per product: float64-level.  Vectors between steps
-// are double-float pairs (8 bytes, ~48 bits), so no step uses the float64
-// pipe; only a float64 input is split and a float64 output assembled.
+// are double-float pairs (8 bytes, ~48 bits), so no step is
+// bound by the float64 pipe: it adds the pairs of the float64 outputs only.
 //
 // Kernel (one CTA per block, row tile of NT <= 64 operator rows and 128
 // right-hand-side columns; 16 digitiser warps + 1 MMA warp, one CTA per SM):
@@ -53,9 +53,12 @@
 //      accumulators of NT columns as soon as the chunk is written, and hands
 //      the buffer back with tcgen05.commit: chunk c + 1 is digitised while
 //      the tensor cores work on chunk c;
-//   4. the digitiser warps read the accumulators (tcgen05.ld), combine,
-//      scale and store (one thread per column: coalesced rows); float64
-//      outputs are assembled from the float32 pair with integer operations.
+//   4. the epilogue warps read the accumulators (tcgen05.ld), combine, scale
+//      and store (one thread per column: coalesced rows), eight rows at a time
+//      without a branch: row by row each waited for its own loads, addition
+//      and store (a tile with a float64 residual took 53K clocks, now 25K).
+// 1024 columns of a 4096-row operator, solve and residual (26 steps): 826 -> 727
+// us with those epilogues and the digitisers' loads issued together.
 // Every mbarrier wait is bounded (2^22 polls); on a timeout the kernel sets
 // the handle's device error word, waits (bounded) for its own copies, frees
 // its TMEM and returns.
@@ -305,6 +308,34 @@ __device__ __forceinline__ double pair_to_f64(float H, float Lo, int sh) {
       (long long)(sgn | ((unsigned long long)e << 52) | ((unsigned long long)M & 0xFFFFFFFFFFFFFull)));
 }
 
+// f 2^sh from the bits (a normal number or zero and a result in float64's
+// normal range: the caller has looked)
+__device__ __forceinline__ double scaled_f64(float f, int sh) {
+  const uint32_t u = __float_as_uint(f), m = u & 0x7fffffffu;
+  const uint32_t hi = m ? (u & 0x80000000u) | ((m >> 3) + ((uint32_t)(896 + sh) << 20)) : 0u;
+  return __hiloint2double((int)hi, (int)(u << 29));
+}
+// Whether scaled_f64(H) + scaled_f64(Lo), one addition on the float64 pipe that
+// the rest of the epilogue leaves idle, gives (H + Lo) 2^sh: both zero or with
+// float64 exponents in range.  (pair_to_f64 takes about 100 clocks of integer
+// operations, the addition 72 of its own pipe.)
+__device__ __forceinline__ bool pair_sum_plain(float H, float Lo, int sh) {
+  const int eh = (int)((__float_as_uint(H) >> 23) & 255);
+  const int el = (int)((__float_as_uint(Lo) >> 23) & 255);
+  const int xh = eh + 896 + sh, xl = el + 896 + sh;
+  return (eh != 0 || H == 0.f) && (el != 0 || Lo == 0.f) && eh != 255 &&
+         (eh == 0 || (xh >= 1 && xh <= 2045)) && (el == 0 || (eh != 0 && xl >= 1));
+}
+// r 2^-sh as a float32, rounded (0 below, infinite above its range)
+__device__ __forceinline__ float scaled_f32(double r, int sh) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(r) + (1ULL << 28);
+  const uint32_t hi = (uint32_t)(b >> 32);
+  const int e = (int)((hi >> 20) & 0x7ff) - 896 - sh;
+  if (e < 1) return 0.f;
+  const uint32_t m = (hi & 0xfffffu) << 3 | (uint32_t)b >> 29;
+  return __uint_as_float((hi & 0x80000000u) | (e > 254 ? 0x7f800000u : (uint32_t)e << 23 | m));
+}
+
 // ---------------------------------------------------------------- the kernel
 // Tile t of a step: block b, row tile rt, column tile ct (ct fastest, so the
 // consecutive tiles of a CTA share their operator digits).
@@ -544,57 +575,78 @@ __global__ void __launch_bounds__(kThreads, 1) oz_step_kernel(const OzStep o) {
       float rsq = 0.f;   // squared residual norm of this column (residual form)
       for (int r8 = rh * 8; r8 < NT; r8 += 16) {
         uint32_t v[kDig][8];
-        float hp[2], lp[2];
 #pragma unroll
         for (int di = 0; di < kDig; ++di)
           tmem_ld8(tmem + lanes + (uint32_t)(di * NT + r8), v[di]);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        // rows i8, i8 + 1 combined together (packed float32x2)
+        float H[8], Lo[8];
+#pragma unroll
+        for (int i8 = 0; i8 < 8; i8 += 2) {
+          float2 a[kDig], H2, L2;
+#pragma unroll
+          for (int di = 0; di < kDig; ++di)
+            a[di] = make_float2(__uint_as_float(v[di][i8]), __uint_as_float(v[di][i8 + 1]));
+          diag_pair2(a, H2, L2);
+          H[i8] = H2.x;
+          H[i8 + 1] = H2.y;
+          Lo[i8] = L2.x;
+          Lo[i8 + 1] = L2.y;
+        }
+        if (o.out_f64 && r0 + r8 < s.split) {
+          // float64 rows (output 0; the split is at a multiple of eight rows
+          // or the tile's end).  All eight without a branch where the sums
+          // stay in range, so that their latencies overlap
+          bool plain = r0 + min(r8 + 8, nr) <= s.split;
+          int sh[8];
+          double bv[8];
+#pragma unroll
+          for (int i8 = 0; i8 < 8; ++i8) {
+            const int row = r8 + i8, ge =
+                (int)((__float_as_uint(__fmul_rn(rs[row], csc)) >> 23) & 255);
+            sh[i8] = ge - 127 + osh;
+            if (!ge) H[i8] = Lo[i8] = 0.f;   // a zero row or column
+            plain = plain && pair_sum_plain(H[i8], Lo[i8], sh[i8]);
+            bv[i8] = (resp[row] && row < nr && cok)
+                         ? *reinterpret_cast<const double*>(resp[row] + 8 * col)
+                         : 0.0;
+          }
+          if (__all_sync(0xffffffffu, plain)) {
+            double y[8];
+#pragma unroll
+            for (int i8 = 0; i8 < 8; ++i8)
+              y[i8] = scaled_f64(H[i8], sh[i8]) + scaled_f64(Lo[i8], sh[i8]);
+            if (o.resb) {
+#pragma unroll
+              for (int i8 = 0; i8 < 8; ++i8) {
+                y[i8] = bv[i8] - y[i8];
+                const float rr = r8 + i8 < nr ? scaled_f32(y[i8], osh) : 0.f;
+                rsq = __fmaf_rn(rr, rr, rsq);
+              }
+            }
+#pragma unroll
+            for (int i8 = 0; i8 < 8; ++i8)
+              if (r8 + i8 < nr && cok) *reinterpret_cast<double*>(outp[r8 + i8] + 8 * col) = y[i8];
+            continue;
+          }
+        }
 #pragma unroll
         for (int i8 = 0; i8 < 8; ++i8) {
           const int row = r8 + i8;
-          // rows i8, i8 + 1 combined together (packed float32x2)
-          float2 H2, L2;
-          if ((i8 & 1) == 0) {
-            float2 a[kDig];
-#pragma unroll
-            for (int di = 0; di < kDig; ++di)
-              a[di] = make_float2(__uint_as_float(v[di][i8]), __uint_as_float(v[di][i8 + 1]));
-            diag_pair2(a, H2, L2);
-            hp[0] = H2.x;
-            hp[1] = H2.y;
-            lp[0] = L2.x;
-            lp[1] = L2.y;
-          }
           if (row >= nr || !cok) continue;
-          float H = hp[i8 & 1], Lo = lp[i8 & 1];
           const float gs = __fmul_rn(rs[row], csc);   // a power of two, or 0
           char* p = outp[row] + 8 * col;
           if (outf64[row]) {
             const int ge = (int)((__float_as_uint(gs) >> 23) & 255);
+            double y = ge ? pair_to_f64(H[i8], Lo[i8], ge - 127 + osh) : 0.0;
             if (resp[row]) {
-              // r = b - S z in the row's scale 2^sh: b split into a float
-              // pair there (integer operations), one double-float
-              // subtraction, then back to float64 like the plain output
-              const int sh = ge ? ge - 127 + osh : osh;
-              const double bv = *reinterpret_cast<const double*>(resp[row] + 8 * col);
-              float bh, bl;
-              f64_split(bv, sh, bh, bl);
-              if (!ge) {
-                H = 0.f;
-                Lo = 0.f;
-              }
-              float rh, rl;
-              two_sum(bh, -H, rh, rl);
-              rl = __fadd_rn(rl, __fsub_rn(bl, Lo));
-              two_sum(rh, rl, rh, rl);
-              *reinterpret_cast<double*>(p) = pair_to_f64(rh, rl, sh);
-              const float rr = ge ? __fmul_rn(rh, gs) : rh;
+              y = *reinterpret_cast<const double*>(resp[row] + 8 * col) - y;
+              const float rr = scaled_f32(y, osh);
               rsq = __fmaf_rn(rr, rr, rsq);
-            } else {
-              *reinterpret_cast<double*>(p) = ge ? pair_to_f64(H, Lo, ge - 127 + osh) : 0.0;
             }
+            *reinterpret_cast<double*>(p) = y;
           } else {
-            *reinterpret_cast<float2*>(p) = make_float2(__fmul_rn(H, gs), __fmul_rn(Lo, gs));
+            *reinterpret_cast<float2*>(p) = make_float2(__fmul_rn(H[i8], gs), __fmul_rn(Lo[i8], gs));
           }
         }
       }
@@ -635,18 +687,22 @@ __global__ void __launch_bounds__(kThreads, 1) oz_step_kernel(const OzStep o) {
       asm volatile("bar.sync 1, %0;" ::"r"(kDigWarps * 32) : "memory");
       const bool col_ok = c0 + j < s.c;
       const int csh = (o.colbits && col_ok) ? col_shift(__ldg(o.colbits + c0 + j)) : 0;
-      auto load = [&](int k, float& h, float& l) {
-        h = 0.f;
-        l = 0.f;
-        if (col_ok && k < w) {
-          const char* p = rowp[k] + 8 * j;
-          if (rowf64[k]) {
-            f64_split(*reinterpret_cast<const double*>(p), csh, h, l);
-          } else {
-            const float2 v = *reinterpret_cast<const float2*>(p);
-            h = v.x;
-            l = v.y;
-          }
+      // eight values of a chunk: the loads first (what they hold, float64 or
+      // float pairs, is looked at afterwards; a branch per load would wait for
+      // each before the next)
+      auto fetch = [&](int k, uint2 (&r)[8]) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          r[u] = (col_ok && k + u < w) ? *reinterpret_cast<const uint2*>(rowp[k + u] + 8 * j)
+                                       : make_uint2(0, 0);
+      };
+      auto convert = [&](int k, const uint2 (&r)[8], float (&h)[8], float (&l)[8]) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          h[u] = __uint_as_float(r[u].x);
+          l[u] = __uint_as_float(r[u].y);
+          if (k + u < w && rowf64[k + u])
+            f64_split(__hiloint2double((int)r[u].y, (int)r[u].x), csh, h[u], l[u]);
         }
       };
       // column scale: largest |h| over the column's k (8 loads in flight),
@@ -655,29 +711,18 @@ __global__ void __launch_bounds__(kThreads, 1) oz_step_kernel(const OzStep o) {
       // (the next chunk's loads are in flight while this chunk is scanned)
       float mx = 0.f;
       float hv[8], lv[8];
+      uint2 nx[8];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) hv[u] = lv[u] = 0.f;
-      if ((nch - 1) * kKC + qk * 8 < wP) {
-#pragma unroll
-        for (int u = 0; u < 8; ++u) load((nch - 1) * kKC + qk * 8 + u, hv[u], lv[u]);
-      }
+      for (int u = 0; u < 8; ++u) nx[u] = make_uint2(0, 0);
+      if ((nch - 1) * kKC + qk * 8 < wP) fetch((nch - 1) * kKC + qk * 8, nx);
       for (int c = nch - 1; c >= 0; --c) {
-        float ph[8], pl[8];
+        uint2 cu[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) ph[u] = pl[u] = 0.f;
-        if (c > 0 && (c - 1) * kKC + qk * 8 < wP) {
-#pragma unroll
-          for (int u = 0; u < 8; ++u) load((c - 1) * kKC + qk * 8 + u, ph[u], pl[u]);
-        }
+        for (int u = 0; u < 8; ++u) cu[u] = nx[u];
+        if (c > 0) fetch((c - 1) * kKC + qk * 8, nx);
+        convert(c * kKC + qk * 8, cu, hv, lv);
 #pragma unroll
         for (int u = 0; u < 8; ++u) mx = fmaxf(mx, fabsf(hv[u]));
-        if (c > 0) {
-#pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            hv[u] = ph[u];
-            lv[u] = pl[u];
-          }
-        }
       }
       colmax[qk][j] = mx;
       asm volatile("bar.sync 1, %0;" ::"r"(kDigWarps * 32) : "memory");
@@ -703,17 +748,8 @@ __global__ void __launch_bounds__(kThreads, 1) oz_step_kernel(const OzStep o) {
         const int b2 = g & 1;
         const int k0 = c * kKC + qk * 8;
         // the next chunk's loads go out before this chunk is digitised
-        float nh[8], nl[8];
         const bool more = c + 1 < nch && k0 + kKC < wP;
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          nh[u] = 0.f;
-          nl[u] = 0.f;
-        }
-        if (more) {
-#pragma unroll
-          for (int u = 0; u < 8; ++u) load(k0 + kKC + u, nh[u], nl[u]);
-        }
+        if (more) fetch(k0 + kKC, nx);
         if (g >= 2 && !mbar_wait(&zempty[b2], (uint32_t)((g >> 1) - 1) & 1u)) fail = true;
         if (k0 < wP) {
           uint32_t wd[kDig][4];
@@ -762,11 +798,7 @@ __global__ void __launch_bounds__(kThreads, 1) oz_step_kernel(const OzStep o) {
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(&zfull[b2]);
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          hv[u] = nh[u];
-          lv[u] = nl[u];
-        }
+        if (more) convert(k0 + kKC, nx, hv, lv);
       }
     }
     sweep::launch_dependents();
