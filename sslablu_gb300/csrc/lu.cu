@@ -133,7 +133,8 @@ lu_panel_global_kernel(int n, int k0, int kb, double* __restrict__ A, int lda, l
 // Per column at 1024 rows, in clocks: candidate 200, reciprocal and row 490,
 // sending 620 (the messages' bytes), lagging updates 90 per column still to go
 // (1500 on average), winner 360, update of the next column 430.  1024 rows, 32
-// columns, eight matrices, cold: 67 us; with a cluster barrier per column, the
+// columns, eight matrices, cold: 67 us (lu_panel_split_kernel takes those now);
+// with a cluster barrier per column, the
 // winner's row read through distributed shared memory and the loop unrolled
 // 122 us; in one CTA, the panel in global memory, 422.
 struct PanelMsg {
@@ -186,9 +187,7 @@ __device__ __forceinline__ bool panel_wait(uint32_t bar, uint32_t parity) {
   return false;
 }
 
-// MAXT: threads per CTA at most (registers)
-template <int MAXT>
-__global__ void __launch_bounds__(MAXT)
+__global__ void __launch_bounds__(kPanelRows)
 lu_panel_kernel(int n, int k0, int kb, double* __restrict__ A, int lda, long long sA,
                 int* __restrict__ piv, long long sP, int* __restrict__ src, int* info,
                 unsigned* err) {
@@ -354,6 +353,205 @@ lu_panel_kernel(int n, int k0, int kb, double* __restrict__ A, int lda, long lon
   if (rank == 0 && threadIdx.x == 0 && first_zero && info) atomicCAS(info + b, 0, first_zero);
 }
 
+// The same for up to 1024 rows, four warps per 32 rows: warp g of them holds
+// columns g, g + 4, .. of its rows, so that a column's lagging updates (72
+// clocks of a scheduler's float64 pipe each) spread over the four schedulers.
+// The warp of the pivot's column finds the candidate and shows the others its
+// entries; each sends its eight columns of the candidate's row (one
+// asynchronous store per lane serves all CTAs) and forms the multipliers
+// itself once the winner is known.
+// 256 rows, 32 columns: 63 -> 42 us (cold); over the panels of a 1024-row
+// factorisation 61 -> 47 us on average, at 1024 rows the same (four warps per
+// scheduler there).  More rows take the kernel above.
+constexpr int kSplitRows = 1024;
+__global__ void __launch_bounds__(512)
+lu_panel_split_kernel(int n, int k0, int kb, double* __restrict__ A, int lda, long long sA,
+                      int* __restrict__ piv, long long sP, int* __restrict__ src, int* info,
+                      unsigned* err) {
+  constexpr int KB = kPanel, NC = KB / 4;   // columns per warp
+  extern __shared__ __align__(16) unsigned char s_raw[];
+  cg::cluster_group cl = cg::this_cluster();
+  const int cs = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const int b = blockIdx.x / cs;
+  A += b * sA;
+  piv += b * sP;
+  src += (long long)b * n;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nrg = blockDim.x >> 7, rg = warp >> 2, g = warp & 3;   // row and column groups
+  const int nmsg = cs * nrg, rows = 32 * nrg;
+  PanelMsg* msg = reinterpret_cast<PanelMsg*>(s_raw);   // [2][nmsg]
+  PanelMsg& out = msg[2 * nmsg + rg];                   // this row group's candidate
+  double* colv = reinterpret_cast<double*>(msg + 2 * nmsg + nrg);   // [2][rows]: pivot column
+  double* us = colv + 2 * rows + NC * warp;             // pivot row, own columns
+  double* fin = colv + 2 * rows + NC * 4 * nrg + 32 * rg + lane;    // finished: [column][row]
+  __shared__ int4 s_cand[2][4];                         // key, position, lane
+  __shared__ __align__(8) unsigned long long bars[2];
+  const uint32_t bar0 = smem_u32(bars);
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 2; ++i)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + 8 * i) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  const int R = n - k0, r = rank * rows + 32 * rg + lane;
+  const bool have = r < R;
+  double a[NC];   // a[i]: column 4 (j4 + i) + g
+  {
+    const double* row = A + (long long)(k0 + (have ? r : 0)) * lda + k0;
+#pragma unroll
+    for (int i = 0; i < NC; ++i) a[i] = (have && 4 * i + g < kb) ? row[4 * i + g] : 0.0;
+  }
+  int pos = have ? r : -1;
+  int first_zero = 0;
+  double lp = 0.0, up = 0.0;        // pending: multiplier, pivot row (lane = own column)
+  bool pend = false, lag = false;
+  bool ok = true;
+  // four lanes per CTA send 64 bytes of the row, two the rest of the message
+  const uint32_t own = smem_u32(&msg[rank * nrg + rg]);
+  const int to4 = lane >> 2, to2 = lane >> 1;
+  const uint32_t row_to = remote_u32(own, to4 < cs ? to4 : 0) + 64 * g + 16 * (lane & 3);
+  const uint32_t row_bar = remote_u32(bar0, to4 < cs ? to4 : 0);
+  const uint32_t key_to = remote_u32(own, to2 < cs ? to2 : 0) + 8 * KB + 16 * (lane & 1);
+  const uint32_t key_bar = remote_u32(bar0, to2 < cs ? to2 : 0);
+  cl.sync();   // the barriers are there
+#pragma unroll 1
+  for (int j4 = 0; 4 * j4 < kb; ++j4) {
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      const int j = 4 * j4 + s;
+      if (j >= kb) break;   // uniform
+      if (!ok) {
+        // given up: only the barriers, which know no limit, for the warps that
+        // have not found out yet
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + rg) : "memory");
+        continue;
+      }
+      const int buf = s & 1;
+      const uint32_t bar = bar0 + 8 * buf;
+      if (threadIdx.x == 0)
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
+                     "r"(nmsg * kMsgBytes)
+                     : "memory");
+      double pv = a[0];   // this row's entry of column j
+      if (g == s) {
+        // the row group's candidate (NaNs are none)
+        const unsigned long long bits =
+            (unsigned long long)__double_as_longlong(pv) & 0x7fffffffffffffffULL;
+        const bool cand = pos >= j && bits <= 0x7ff0000000000000ULL;
+        const uint32_t hi = cand ? (uint32_t)(bits >> 32) + 1 : 0, lo = (uint32_t)bits;
+        const uint32_t mh = __reduce_max_sync(0xffffffffu, hi);
+        const uint32_t ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0);
+        const int mp =
+            __reduce_min_sync(0xffffffffu, (cand && hi == mh && lo == ml) ? pos : 0x7fffffff);
+        const unsigned at = __ballot_sync(0xffffffffu, cand && pos == mp);
+        colv[buf * rows + 32 * rg + lane] = pv;
+        if (lane == 0) s_cand[buf][rg] = make_int4((int)mh, (int)ml, mp, at ? __ffs(at) - 1 : -1);
+      }
+      asm volatile("bar.sync %0, 128;" ::"r"(1 + rg) : "memory");
+      const int4 cd = s_cand[buf][rg];
+      if (g != s) pv = colv[buf * rows + 32 * rg + lane];
+      if (lane == cd.w) {
+#pragma unroll
+        for (int i = 0; i < NC; i += 2)
+          *reinterpret_cast<double2*>(&out.row[NC * g + i]) = make_double2(a[i], a[i + 1]);
+        if (g == s) {
+          out.lprev = lp;
+          out.inv = reciprocal(pv);
+        }
+      }
+      __syncwarp();
+      const uint32_t off = buf * nmsg * kMsgBytes;
+      if (to4 < cs)
+        send_2b64(row_to + off,
+                  reinterpret_cast<const ulonglong2*>(&out.row[NC * g])[lane & 3],
+                  row_bar + 8 * buf);
+      if (g == s && to2 < cs) {
+        ulonglong2 v = reinterpret_cast<const ulonglong2*>(&out.lprev)[0];
+        if ((lane & 1) == 0)
+          v = make_ulonglong2(cd.x ? (unsigned long long)(uint32_t)cd.x << 32 | (uint32_t)cd.y : 0,
+                              (unsigned long long)(long long)cd.z);
+        send_2b64(key_to + off, v, key_bar + 8 * buf);
+      }
+      // the update that columns j + 1 .. lag by
+      if (pend) {
+        const double ln = lag ? -lp : 0.0;
+#pragma unroll
+        for (int i = 0; i < NC; ++i) {
+          if (i >= NC - j4) break;
+          if (i == 0 && g <= s) continue;
+          if (lag) a[i] = fma(ln, us[i], a[i]);
+        }
+      }
+      ok = panel_wait(bar, (uint32_t)(j >> 1) & 1);
+      if (!__all_sync(0xffffffffu, ok)) {
+        ok = false;
+        if (lane == 0 && err) *(volatile unsigned*)err = 1;
+        continue;
+      }
+      // the winner: largest entry, then the first position
+      const PanelMsg* m = msg + buf * nmsg;
+      const unsigned long long key = lane < nmsg ? m[lane].key : 0;
+      const int kp = lane < nmsg ? (int)m[lane].pos : 0x7fffffff;
+      const uint32_t kh = (uint32_t)(key >> 32), kl = (uint32_t)key;
+      const uint32_t wh = __reduce_max_sync(0xffffffffu, kh);
+      const uint32_t wl = __reduce_max_sync(0xffffffffu, kh == wh ? kl : 0);
+      const int wp = __reduce_min_sync(0xffffffffu, (kh == wh && kl == wl) ? kp : 0x7fffffff);
+      const unsigned win = __ballot_sync(0xffffffffu, kh == wh && kl == wl && kp == wp);
+      const int wi = __ffs(win) - 1;
+      // no key: every remaining entry of the column is NaN; the row at position
+      // j is its own pivot, wherever it is held
+      const int p = wh ? wp : j;
+      double u, inv;
+      if (wh) {
+        u = m[wi].row[NC * g + (lane & (NC - 1))];
+        inv = m[wi].inv;
+        if (pend && ((lane & (NC - 1)) > 0 || g > s)) u = fma(-m[wi].lprev, up, u);
+      } else {
+        u = inv = __longlong_as_double(0x7ff8000000000000LL);
+      }
+      if (rank == 0 && threadIdx.x == 0) piv[k0 + j] = k0 + p;
+      // position swap j <-> p
+      const bool retire = pos == p;
+      if (pos == j) pos = p;
+      if (retire) pos = j;
+      // the pivot is zero when its key says so
+      if (wh == 1 && wl == 0) {
+        if (!first_zero) first_zero = k0 + j + 1;
+        pend = lag = false;
+      } else {
+        up = u;
+        pend = true;
+        lag = pos > j;
+        // the next column: s + 1's first, or group 0's second
+        const int nx = s < 3 ? 0 : 1;
+        const double u1 = __shfl_sync(0xffffffffu, u, nx);
+        __syncwarp();
+        // (the registers move down after s = 3)
+        if (s < 3 ? lane < NC : (lane > 0 && lane < NC)) us[s < 3 ? lane : lane - 1] = u;
+        __syncwarp();
+        if (lag) {
+          lp = pv * inv;
+          if (g == s) a[0] = lp;
+          if (g == ((s + 1) & 3)) a[nx] = fma(-lp, u1, a[nx]);
+        }
+      }
+      if (g == s) fin[j * rows] = a[0];
+    }
+#pragma unroll
+    for (int i = 0; i + 1 < NC; ++i) a[i] = a[i + 1];
+    a[NC - 1] = 0.0;
+    up = __shfl_down_sync(0xffffffffu, up, 1);
+  }
+  cl.sync();   // no CTA leaves while another may still write to its shared memory
+  if (have) {
+    double* row = A + (long long)(k0 + pos) * lda + k0;
+#pragma unroll
+    for (int i = 0; i < NC; ++i)
+      if (4 * i + g < kb) row[4 * i + g] = fin[(4 * i + g) * rows];
+    if (g == 0) src[k0 + pos] = k0 + r;
+  }
+  if (rank == 0 && threadIdx.x == 0 && first_zero && info) atomicCAS(info + b, 0, first_zero);
+}
+
 // The panel's row swaps on every column outside it, from the net permutation
 // (src[i]: the row that ends at row i): the kb top rows and the up to kb
 // pivot rows below, all reads before the writes.  For columns k1 .. ct the top
@@ -465,20 +663,22 @@ lu_block_trsm_kernel(int n, int k0, int nb, int c0, double* __restrict__ A, int 
 void launch_panel(cudaStream_t st, int n, int k0, int kb, double* A, int lda, long long sA,
                   int* piv, long long sP, int* src, int batch, int* info, unsigned* err) {
   const int R = n - k0;
-  // a warp per scheduler of an SM (128 rows per CTA), up to the portable
-  // cluster size of 8
+  // 32 rows per CTA (four warps), then up to 128, in clusters of up to eight
+  // (the portable size); above 1024 rows a thread per row
+  const bool split = R <= kSplitRows;
   int cs = 1;
-  while (cs < 8 && R > 128 * cs) cs *= 2;
-  const int threads = ((R + cs - 1) / cs + 31) / 32 * 32;
+  while (cs < 8 && R > (split ? 32 : 128) * cs) cs *= 2;
+  const int warps = ((R + cs - 1) / cs + 31) / 32;   // row groups of 32
+  const int threads = 32 * warps * (split ? 4 : 1);
   if (threads > kPanelRows) {
     lu_panel_global_kernel<<<batch, 1024, 0, st>>>(n, k0, kb, A, lda, sA, piv, sP, src, info);
     check_launch("lu_panel_global_kernel");
     return;
   }
-  const int nw = threads / 32;
-  const size_t sm = (size_t)(2 * cs * nw + nw) * sizeof(PanelMsg) +
-                    8 * (size_t)kPanel * (nw + threads);
-  auto kern = threads <= 128 ? lu_panel_kernel<128> : lu_panel_kernel<kPanelRows>;
+  // messages, (pivot column), pivot rows, finished entries
+  const size_t sm = (size_t)(2 * cs * warps + warps) * sizeof(PanelMsg) +
+                    8 * (size_t)warps * (kPanel + (split ? 64 : 0) + 32 * kPanel);
+  auto kern = split ? lu_panel_split_kernel : lu_panel_kernel;
   ensure_smem(reinterpret_cast<const void*>(kern), sm);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(batch * cs));
