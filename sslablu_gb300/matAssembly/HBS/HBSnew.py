@@ -306,8 +306,11 @@ class HBSMAT:
         # out of place: no copy of the right-hand sides
         X = dv.as_2d(X).contiguous()
         Y = torch.empty_like(X)
-        L.check(L.lib().slu_ulv_solve_into(L.handle(), self._op, L.ptr(X), X.shape[1],
-                                           L.ptr(Y), Y.shape[1], X.shape[1], int(trans)))
+        c = X.shape[1]
+        st = L.lib().slu_ulv_solve_into(L.handle(), self._op, X.data_ptr(), c, Y.data_ptr(), c, c,
+                                        1 if trans else 0)
+        if st:
+            L.check(st)
         return Y
 
     def matvec(self, v):
@@ -352,6 +355,9 @@ class HBSMAT:
                                                c, int(mode == "T")))
             torch.cuda.current_stream().synchronize()
             return out
+        if (isinstance(b, torch.Tensor) and b.is_cuda and b.dtype == torch.float64
+                and b.dim() == 2 and b.get_device() == L.device()):
+            return self._dev_solve(b, mode == "T")   # as it is
         X, one = dv.prepare_rhs(b)
         return dv.finish(self._dev_solve(X, mode == "T"), b, one)
 
