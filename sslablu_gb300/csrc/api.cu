@@ -198,7 +198,7 @@ int slu_hbs_set_level(slu_handle_t h, slu_hbs_t op, int level, int Nb, int n, in
       H.has_ulv = false;
       H.has_sweep = false;
       H.has_oz = H.has_ozT = false;
-      H.drop_crt();
+      H.drop_crt(true);
       H.has_f32 = false;
       H.has_dfs = false;
       H.has_df = false;
@@ -246,7 +246,7 @@ int slu_hbs_set_ulv_level(slu_handle_t h, slu_hbs_t op, int level, const double*
     H.has_dfs = false;
     H.has_sweep = false;
     H.has_oz = H.has_ozT = false;
-    H.drop_crt();
+    H.drop_crt(false);
     H.invalidate_plans();
     if (all) slu::hbs_make_sweep(h->h, H);
   });

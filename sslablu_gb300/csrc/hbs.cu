@@ -377,7 +377,7 @@ void hbs_compress(Handle& h, Hbs& H, int Nb0, int rk, int s, const double* Om, c
   H.has_df = false;
   H.has_sweep = false;
   H.has_oz = H.has_ozT = false;
-  H.drop_crt();
+  H.drop_crt(true);
   H.has_apply[0] = H.has_apply[1] = false;
   H.invalidate_plans();
   if (ulv) hbs_make_sweep(h, H);
@@ -430,7 +430,7 @@ void hbs_factor(Handle& h, Hbs& H) {
   H.has_f32 = false;
   H.has_dfs = false;
   H.has_oz = H.has_ozT = false;   // digit forms of the step operators are stale
-  H.drop_crt();
+  H.drop_crt(false);
   H.invalidate_plans();
   hbs_make_sweep(h, H);
 }

@@ -193,8 +193,9 @@ struct Hbs {
   // first use, likewise
   std::atomic<bool> has_crt[4] = {false, false, false, false};
   DevBuf crt_buf[4];
-  void drop_crt() {
-    for (int i = 0; i < 4; ++i) {
+  // (a new ULV factorisation leaves the applies' operators as they are)
+  void drop_crt(bool applies) {
+    for (int i = 0; i < (applies ? 4 : 2); ++i) {
       has_crt[i] = false;
       crt_buf[i].release();
     }
