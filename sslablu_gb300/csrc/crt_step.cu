@@ -34,8 +34,8 @@
 // tile of 64 x 64 x 32 takes 17K clocks where that work is 8K (the phases of a
 // tile follow one another), the float64 pipe 66K.
 // Measured (us, float64 steps -> these): 8192 rows with leaves of 64 and rank
-// 32, 261 columns: solve 2100 -> 425, transposed 2017 -> 444, apply 1317 ->
-// 388; 4096 rows, 64 columns: 252 -> 119, 275 -> 124, 180 -> 112.  The relative
+// 32, 261 columns: solve 2100 -> 413, transposed 2017 -> 432, apply 1317 ->
+// 377; 4096 rows, 64 columns: 252 -> 118, 275 -> 123, 180 -> 111.  The relative
 // error against 64 bits over those shapes: solves 1.2e-15 (float64 steps
 // 1.2e-15), applies 1.1e-15 (1.1e-15): that of the operators, not of the steps.
 // Columns or operator rows that are not finite take float64 dot products.
@@ -180,15 +180,19 @@ __device__ __forceinline__ Tile tile_of(int t, int nrt, int nct) {
 }
 
 // Moduli per hand-over of z residues from the conversion to the MMAs: eight
-// where two z buffers and eight images of any width fit in shared memory.
-__host__ __device__ constexpr int handover(int nc, bool half) { return nc < 32 && half ? 8 : 4; }
+// where two z buffers and eight images fit in shared memory (up to 64 rows and
+// fewer than 32 columns or 64 of the operator's: 444 -> 432 us against four).
+__host__ __device__ constexpr int handover(int nc, bool half, bool narrow) {
+  return half && (nc < 32 || narrow) ? 8 : 4;
+}
 
 // NC: columns per tile (MMA N).  KPT: consecutive k per thread (512 threads,
 // NC columns).  HALF: at most 64 rows, as MMAs of M = 64 (16 rows in each
 // quarter of TMEM).
 template <int NC, int KPT, bool HALF>
 __global__ void __launch_bounds__(kThreads, 1) crt_step_kernel(const CrtStep o) {
-  constexpr int MH = handover(NC, HALF);   // moduli per hand-over of z residues
+  // moduli per hand-over of z residues (KPT NC: 128 up to 64 columns of the operator)
+  constexpr int MH = handover(NC, HALF, KPT * NC == 128);
   constexpr int NHO = NM / MH;
   constexpr int PH = MH / kMma;          // of one MMA warp
   extern __shared__ unsigned char smraw[];
@@ -690,7 +694,8 @@ void launch(cudaStream_t st, const sweep::Step<double>& s, const CrtOp& op, vola
   const size_t tail = (size_t)((half ? 64 : kRows) - o.RS) * op.wP * 2;
   // z group buffers: all where the images then still fit as a whole, else half
   // (at least two); the rest of shared memory holds operator images
-  const int mh = handover(nc, half), all = NM / mh;
+  const bool narrow = op.wP <= 64;
+  const int mh = handover(nc, half, narrow), all = NM / mh;
   o.groups = z + NM * a + tail + 1024 <= kSmemMax ? all : 2;
   const size_t zb = z / all * o.groups;
   o.slots = (int)std::min<size_t>(NM, (kSmemMax - 1024 - zb - tail) / a) / mh * mh;
@@ -699,7 +704,6 @@ void launch(cudaStream_t st, const sweep::Step<double>& s, const CrtOp& op, vola
   p.ctas = std::min<long long>(g.tiles, num_sms());
   p.threads = kThreads;
   p.smem = 1024 + zb + tail + o.slots * a;
-  const bool narrow = op.wP <= 64;
   auto kern = nc == 32 ? (half ? (narrow ? crt_step_kernel<32, 4, true> : crt_step_kernel<32, 8, true>)
                                : (narrow ? crt_step_kernel<32, 4, false>
                                          : crt_step_kernel<32, 8, false>))
@@ -740,7 +744,8 @@ bool ready(Handle& h, Hbs& H, bool solve, bool trans) {
   if (cap != cudaStreamCaptureStatusNone) return false;
   std::lock_guard<std::mutex> lock(H.lazy_mu);
   if (have) return true;
-  if (!solve && !H.has_apply[trans ? 1 : 0]) hbs_make_apply(h, H, trans);
+  const bool compose = !solve && !H.has_apply[trans ? 1 : 0];
+  if (compose) hbs_make_apply(h, H, trans, false);
   std::vector<Part> parts;
   auto add = [&](CrtOp& o, const DevBuf& S, int nb, int rows, int w) {
     o.Nb = nb;
@@ -762,10 +767,12 @@ bool ready(Handle& h, Hbs& H, bool solve, bool trans) {
       add(trans ? l.crDnT : l.crDn, trans ? l.AdnT : l.Adn, nb, l.n, root ? l.n : l.n + l.k);
     }
   }
-  if (!make_images(st, parts, H.crt_buf[(solve ? 0 : 2) + (trans ? 1 : 0)])) return false;
+  const bool made = make_images(st, parts, H.crt_buf[(solve ? 0 : 2) + (trans ? 1 : 0)]);
+  if (!made && !compose) return false;
   stream_wait(st);   // other streams may use the images from here on
-  have = true;
-  return true;
+  if (compose) H.has_apply[trans ? 1 : 0] = true;
+  have = made;
+  return made;
 }
 
 }  // namespace

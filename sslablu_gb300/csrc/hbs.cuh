@@ -351,7 +351,8 @@ void enqueue_device_lead(cudaStream_t st, int us);
 // elements of T; the operators of the direction must have been composed
 // (hbs_make_apply; for T = dfloat, hbs_make_df).
 size_t hbs_apply_scratch_elems(const Hbs& H, int c);
-void hbs_make_apply(Handle& h, Hbs& H, bool trans);
+// wait = false: the caller waits for the stream and sets has_apply.
+void hbs_make_apply(Handle& h, Hbs& H, bool trans, bool wait = true);
 template <typename T>
 void hbs_apply_fused(cudaStream_t st, const Hbs& H, bool trans, const T* X, int ldx, T* Y,
                      int ldy, int c, T* scratch);

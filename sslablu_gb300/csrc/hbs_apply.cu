@@ -99,7 +99,7 @@ struct ApplyOps<dfloat> {
 
 }  // namespace
 
-void hbs_make_apply(Handle& h, Hbs& H, bool trans) {
+void hbs_make_apply(Handle& h, Hbs& H, bool trans, bool wait) {
   SLU_REQUIRE(H.has_mats, "HBS factors not loaded");
   cudaStream_t st = h.stream;
   const int L = H.L;
@@ -126,6 +126,7 @@ void hbs_make_apply(Handle& h, Hbs& H, bool trans) {
   compose_down_kernel<<<grid_for((long long)r.n * r.n), 256, 0, st>>>(
       1, r.n, 0, trans, r.D.as<double>(), nullptr, dn.as<double>());
   check_launch("compose_down_kernel");
+  if (!wait) return;
   stream_wait(st);
   H.has_apply[trans ? 1 : 0] = true;
 }
