@@ -64,12 +64,23 @@ constexpr Tables make_tables() {
 }
 __constant__ Tables c_tab = make_tables();
 
-// Largest |a'| exponent for products of depth K: |X| <= K 2^(2t) <= 2^123 < P / 4.
-inline int bits_for(int K) {
+// Largest |a'| exponent for products of depth K: |X| <= K 2^(2t) <= 2^123 < P / 4,
+// and at most the 59 bits that `scaled` shifts by (depths of 8 and less).
+constexpr int kMaxBits = 59;
+constexpr int bits_for(int K) {
   int lg = 0;
   while ((1LL << lg) < K) ++lg;
-  return (123 - lg) / 2;
+  return (123 - lg) / 2 < kMaxBits ? (123 - lg) / 2 : kMaxBits;
 }
+constexpr bool bits_fit() {
+  for (int K = 1; K <= 8192; ++K) {
+    int lg = 0;
+    while ((1 << lg) < K) ++lg;
+    if (bits_for(K) > kMaxBits || lg + 2 * bits_for(K) > 123) return false;
+  }
+  return true;
+}
+static_assert(bits_fit(), "scaled operands must fit the shift and the moduli");
 
 // dp4a of unsigned bytes of a with signed bytes of b, and the reverse
 __device__ __forceinline__ int dp4a_us(uint32_t a, uint32_t b, int c) {
@@ -87,7 +98,7 @@ __device__ __forceinline__ int dp4a_su(uint32_t a, uint32_t b, int c) {
 __device__ __forceinline__ uint32_t hi32(double v) { return (uint32_t)__double2hiint(v); }
 
 // A float64 (its bits) whose exponent field is at most F (>= 1) as a t-bit
-// integer (t <= 59), rounded to nearest and shifted by 2^59 to be non-negative
+// integer (t <= kMaxBits), rounded to nearest and shifted by 2^59 to be non-negative
 // (the tables take the shift off again); ok = false gives zero.
 __device__ __forceinline__ void scaled(uint32_t hi, uint32_t lo, int F, int t, bool ok,
                                        uint32_t& zlo, uint32_t& zhi) {
