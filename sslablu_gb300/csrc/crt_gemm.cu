@@ -1,4 +1,4 @@
-// Float64-accurate GEMM on the tensor cores (tcgen05) by residue arithmetic.
+// Float64 GEMM on the tensor cores (tcgen05) by residue arithmetic.
 //
 // The dense products of the float64 path -- sampling a dense interface block
 // (matAssembly/HBS/HBSnew.py:211-227), the Schur complements, pivot-block
@@ -16,6 +16,7 @@
 //      |a'| <= 2^t, and their balanced residues modulo p_0 .. p_15, |r| <=
 //      128: exact in bfloat16.  B's residues carry the factor (P/p)^-1 mod p
 //      of the reconstruction.
+//      A seventeenth plane holds the magnitudes |a| / a in bfloat16.
 //   2. crt_gemm_kernel: per modulus a bfloat16 GEMM with float32 accumulation
 //      in TMEM.  The sum of 1024 products of two residues is at most 2^24,
 //      so every accumulator holds the exact integer; deeper products are
@@ -27,20 +28,38 @@
 //
 // With t = (123 - log2 K) / 2 (56 at K = 1024) the only errors are the
 // rounding of the inputs at 2^-(t+1) of their row's (column's) largest entry
-// and the final rounding; a float64 FMA chain rounds once per term.  Measured
-// against exact products the result is no further off than the float64
-// kernel's at every tested shape.  Rows or columns that hold an infinity or a
-// NaN take float64 dot products in step 3, with the float64 kernel's result.
+// and the final rounding; a float64 FMA chain rounds once per term.  So the
+// error of an output is at most K 2^-t a b, a the largest entry of its row of
+// op(A), b of its column of op(B), where that of an FMA chain is K 2^-53 times
+// its own sum s of |a_ik| |b_kj|.  Where the scales of op(A) and op(B) oppose
+// along k, s is far below a b (rows diag(d) R against diag(1/d) C).  One more
+// bfloat16 product, of the magnitudes |a_ik| / a and |b_kj| / b, gives s / (a b)
+// (the terms rounded down by at most 2^-6), and step 3 forms an output by a
+// float64 dot product instead
+//   * where it is below 2^(51-t) everywhere in the output's row or everywhere
+//     in its column: no output there would be as accurate as an FMA chain's to
+//     within a factor of four, and
+//   * where it is below 2^-44 for the output itself.
+// Elsewhere the error is below 4 K 2^-53 times the largest s of the row and of
+// the column, both scaled by the columns' b and the rows' a: a normwise bound
+// that no scaling of rows, columns or k can spoil.  (An output whose own s is
+// small beside the others of both its row and its column has fewer right digits
+// than an FMA chain's, down to a few at 2^-44.)
+// Rows or columns that hold an infinity or a NaN take the dot products too,
+// with the float64 kernel's result.
 //
-// Work per element of A and B: 16 residues at ~9 integer / float32 slots;
-// per element of C: 16 x 2K bfloat16 flops, 16 bytes and ~220 slots of step
-// 3.  Two 1024^3 products: 42 us of conversion, 61 of products (1.1 PFLOP/s on
-// the tensor cores) and 24 of reconstruction, against 4.1 ms on the float64
-// pipe.
+// Work per element of A and B: 16 residues at ~9 integer / float32 slots and
+// the magnitude; per element of C: 17 x 2K bfloat16 flops, 17 bytes and ~220
+// slots of step 3.  Four 1024^3 products: 78 us of conversion, 123 of products
+// (1.2 PFLOP/s on the tensor cores) and 43 of reconstruction (80, 116 and 40
+// without the magnitudes), against 7.2 ms on the float64 pipe; with operands of
+// which every output is a dot product 8.0 ms.
 #include <cuda.h>
 
 #include <algorithm>
+#include <cmath>
 #include <mutex>
+#include <numeric>
 
 #include "crt.cuh"
 #include "hbs.cuh"
@@ -57,9 +76,20 @@ struct CrtOperand {
   long long s0, s1;
   int rows;              // rows of op(A), columns of op(B)
   int kcontig;           // consecutive k adjacent in memory
-  __nv_bfloat16* out;    // residues [modulus][batch][row][Kp]
+  __nv_bfloat16* out;    // residues [modulus][batch][row][Kp], magnitudes behind them
   int* ex;               // exponent field per [batch][row]; 2047 = not finite
+  int* wide;             // zeroed here: see CrtGemm
 };
+
+// |v| / 2^(F - 1022) as a bfloat16, rounded down, in the upper half of a word
+// (F: the row's largest exponent field); what is below 2^-60 as 2^-60, zero as
+// zero.  sub = (max(F, 187) - 126) << 20: in rows all below 2^-836 (their
+// subnormals have no exponent to subtract from) everything counts as small, and
+// the row takes float64 dot products.
+__device__ __forceinline__ uint32_t magnitude(uint2 v, int sub) {
+  const uint32_t h = v.y & 0x7fffffffu;
+  return (h | v.x) ? (uint32_t)max((int)h - sub, 67 << 20) << 3 : 0u;
+}
 
 // A CTA converts ROWS rows, 2048 / ROWS consecutive k at a time (32, 16 or 8
 // rows, so that operands 64 or 128 deep keep every thread busy), through
@@ -151,8 +181,19 @@ crt_convert_kernel(CrtOperand a, CrtOperand b, int strips_a, int K, int Kp, int 
     } else {
       ex = s_ex[row];
     }
-    if (kc == 0 && kq == 0 && live) o.ex[(long long)bt * o.rows + r0 + row] = ex;
+    if (kc == 0 && kq == 0 && live) {
+      o.ex[(long long)bt * o.rows + r0 + row] = ex;
+      o.wide[(long long)bt * o.rows + r0 + row] = 0;
+    }
     if (!live || kc + 8 * kq >= Kp) continue;
+    {
+      const int sub = (max(ex, 187) - 126) << 20;
+      uint32_t w[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        w[u] = __byte_perm(magnitude(src[2 * u], sub), magnitude(src[2 * u + 1], sub), 0x7632);
+      *reinterpret_cast<uint4*>(dst + NM * plane + kc) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
     uint32_t lo[8], hi[8];
 #pragma unroll
     for (int u = 0; u < 8; ++u)
@@ -255,14 +296,22 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
       : "r"(taddr));
 }
 
+// Exponent field of the smallest magnitude sum (beside the operands' largest
+// entries) that an output may have.
+constexpr uint32_t kSumFloor = 127 - 44;
+
 struct CrtGemm {
   int M, N, batch;
   int tm, tn;            // tiles
   int BN;                // tile columns, a multiple of 16, at most 256
   int KT, chunks, per;   // k-tiles; chunks of `per` k-tiles
   int stages;
-  long long items;       // NM * batch * tm * tn
-  int8_t* R;             // residues [modulus][batch][M][pitch]
+  long long items;       // (NM + 1) * batch * tm * tn
+  int8_t* R;             // residues [modulus][batch][M][pitch], then the
+                         // exponent field of every magnitude sum (0: zero,
+                         // every product has a zero factor)
+  float theta;           // 2^(51 - t)
+  int *wa, *wb;          // rows and columns with a sum of theta or more
   int pitch;
   unsigned int* err;
 };
@@ -393,7 +442,9 @@ crt_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       const long long mb = id / tiles;
       const int tile = (int)(id - mb * tiles), l = (int)(mb / g.batch);
       const int row = (tile / g.tn) * BM + q * 32 + lane, n0 = (tile % g.tn) * BN;
-      const float p = c_tab.pf[l], ip = c_tab.inv[l];
+      const bool mags = l == NM;
+      const float p = mags ? 0.f : c_tab.pf[l], ip = mags ? 0.f : c_tab.inv[l];
+      const long long bt = mb - (long long)l * g.batch;
       int8_t* out = g.R + (mb * g.M + row) * g.pitch + n0;
       for (int c = 0; c < g.chunks; ++c, ++n) {
         const uint32_t a = n & 1;
@@ -407,7 +458,33 @@ crt_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           uint32_t v[16];
           tmem_ld16(tmem + lanes + a * 256 + 16 * j, v);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          if (row < g.M && n0 + 16 * j < g.pitch) {
+          if (mags) {
+            if (n0 + 16 * j >= g.pitch) continue;   // uniform
+            uint32_t w[4], wide = 0;
+#pragma unroll
+            for (int e = 0; e < 16; ++e)
+              wide |= (__uint_as_float(v[e]) >= g.theta ? 1u : 0u) << e;
+#pragma unroll
+            for (int e = 0; e < 16; e += 4)
+              w[e >> 2] = __byte_perm(__byte_perm(v[e] << 1, v[e + 1] << 1, 0x73),
+                                      __byte_perm(v[e + 2] << 1, v[e + 3] << 1, 0x73), 0x5410);
+            const int nc = min(16, g.N - n0 - 16 * j);
+            wide &= row < g.M && nc > 0 ? 0xffffu >> (16 - nc) : 0u;
+            const uint32_t cols = __reduce_or_sync(0xffffffffu, wide);
+            if (cols >> lane & 1) g.wb[bt * g.N + n0 + 16 * j + lane] = 1;
+            if (row < g.M) {
+              if (wide) g.wa[bt * g.M + row] = 1;
+              uint4* dst = reinterpret_cast<uint4*>(out + 16 * j);
+              if (c > 0) {   // the largest of the chunks
+                const uint4 o = *dst;
+                w[0] = __vmaxu4(w[0], o.x);
+                w[1] = __vmaxu4(w[1], o.y);
+                w[2] = __vmaxu4(w[2], o.z);
+                w[3] = __vmaxu4(w[3], o.w);
+              }
+              *dst = make_uint4(w[0], w[1], w[2], w[3]);
+            }
+          } else if (row < g.M && n0 + 16 * j < g.pitch) {
             uint4* dst = reinterpret_cast<uint4*>(out + 16 * j);
             uint32_t old[4] = {0, 0, 0, 0};
             if (c > 0) {
@@ -456,6 +533,7 @@ struct CrtCombine {
   const int8_t* R;
   int pitch;
   const int *ea, *eb;
+  const int *wa, *wb;     // see CrtGemm
   int t;
   double alpha, beta;
   int kind;   // alpha, beta: 0 = 1, 0; 1 = -1, 0; 2 = 1, 1; 3 = -1, 1; 4 = any (a float64 compare
@@ -468,57 +546,97 @@ struct CrtCombine {
   long long ak, ai, sA0, sA1, bk, bj, sB0, sB1;   // strides along k, i, j
 };
 
+__device__ __forceinline__ void put(const CrtCombine& g, double* c, double v) {
+  if (g.kind == 4) {
+    v *= g.alpha;
+    if (g.beta != 0.0) v = fma(g.beta, *c, v);
+  } else {
+    if (g.kind & 1) v = __hiloint2double((int)(hi32(v) ^ 0x80000000u), __double2loint(v));
+    if (g.kind & 2) v = *c + v;
+  }
+  *c = v;
+}
+
 // One thread per four consecutive elements of a row of C: four bytes of every
-// residue plane, transposed in registers so a __dp4a sums four moduli.
+// residue plane, transposed in registers so a __dp4a sums four moduli.  Eight
+// threads take a segment of 32 outputs (a sector of every plane), a CTA every
+// gridDim-th segment.  The outputs that take a dot product go to a list and are
+// spread over the CTA, eight lanes each.  They come as whole rows, columns or
+// corners, and a CTA forms 1024 of them in 300 us (depth 1024, float64 pipe): so
+// the grid has no factor in common with the segments of a row, and they fall
+// to all CTAs alike.
 __global__ void __launch_bounds__(256)
 crt_combine_kernel(const __grid_constant__ CrtCombine g) {
-  const int nq = (g.N + 3) / 4;
-  const long long total = (long long)g.batch * g.M * nq;
+  __shared__ unsigned short list[1024];   // 32 segment + column
+  __shared__ int listed;
+  const int tid = threadIdx.x, tn = (g.N + 31) / 32;
+  const long long segs = (long long)g.batch * g.M * tn, T = gridDim.x;
   const long long plane = (long long)g.batch * g.M * g.pitch;
-  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < total;
-       q += (long long)gridDim.x * blockDim.x) {
-    const long long br = q / nq;                   // batch * M + row
-    const int j0 = 4 * (int)(q - br * nq), bt = (int)(br / g.M), i = (int)(br - (long long)bt * g.M);
-    const int b0 = bt % g.batch0, b1 = bt / g.batch0;
-    const int8_t* src = g.R + br * g.pitch + j0;
-    uint32_t r[NM];
+  if (tid == 0) listed = 0;
+  for (long long s0 = blockIdx.x; s0 < segs; s0 += 32 * T) {
+    const long long sg = s0 + (tid >> 3) * T;
+    const long long br = sg / tn;   // batch * M + row
+    const int j0 = 32 * (int)(sg - br * tn) + 4 * (tid & 7);
+    uint32_t bad = 0;
+    if (sg < segs && j0 < g.N) {
+      const int bt = (int)(br / g.M), i = (int)(br - (long long)bt * g.M);
+      const int b0 = bt % g.batch0, b1 = bt / g.batch0;
+      const int8_t* src = g.R + br * g.pitch + j0;
+      uint32_t r[NM];
 #pragma unroll
-    for (int l = 0; l < NM; ++l) r[l] = *reinterpret_cast<const uint32_t*>(src + l * plane);
-    // r[4 a + e] <- byte e of planes 4 a .. 4 a + 3
+      for (int l = 0; l < NM; ++l) r[l] = *reinterpret_cast<const uint32_t*>(src + l * plane);
+      const uint32_t sums = *reinterpret_cast<const uint32_t*>(src + NM * plane);
+      // r[4 a + e] <- byte e of planes 4 a .. 4 a + 3
 #pragma unroll
-    for (int a = 0; a < NM; a += 4) {
-      const uint32_t x0 = __byte_perm(r[a], r[a + 1], 0x5140), x1 = __byte_perm(r[a], r[a + 1], 0x7362);
-      const uint32_t y0 = __byte_perm(r[a + 2], r[a + 3], 0x5140), y1 = __byte_perm(r[a + 2], r[a + 3], 0x7362);
-      r[a] = __byte_perm(x0, y0, 0x5410);
-      r[a + 1] = __byte_perm(x0, y0, 0x7632);
-      r[a + 2] = __byte_perm(x1, y1, 0x5410);
-      r[a + 3] = __byte_perm(x1, y1, 0x7632);
-    }
-    const int fa = g.ea[br];
-    double* c = g.C + b0 * g.sC0 + b1 * g.sC1 + (long long)i * g.ldc + j0;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      if (j0 + e >= g.N) break;
-      const int fb = g.eb[(long long)bt * g.N + j0 + e];
-      double v;
-      if (fa == 0x7ff || fb == 0x7ff) {
-        const double* ap = g.A + b0 * g.sA0 + b1 * g.sA1 + i * g.ai;
-        const double* bp = g.B + b0 * g.sB0 + b1 * g.sB1 + (j0 + e) * g.bj;
-        v = 0.0;
-        for (int k = 0; k < g.K; ++k) v = fma(ap[k * g.ak], bp[k * g.bk], v);
-      } else {
-        v = combine(r[e], r[4 + e], r[8 + e], r[12 + e],
-                    max(fa, 1) + max(fb, 1) - 2 * (1022 + g.t));
+      for (int a = 0; a < NM; a += 4) {
+        const uint32_t x0 = __byte_perm(r[a], r[a + 1], 0x5140), x1 = __byte_perm(r[a], r[a + 1], 0x7362);
+        const uint32_t y0 = __byte_perm(r[a + 2], r[a + 3], 0x5140), y1 = __byte_perm(r[a + 2], r[a + 3], 0x7362);
+        r[a] = __byte_perm(x0, y0, 0x5410);
+        r[a + 1] = __byte_perm(x0, y0, 0x7632);
+        r[a + 2] = __byte_perm(x1, y1, 0x5410);
+        r[a + 3] = __byte_perm(x1, y1, 0x7632);
       }
-      if (g.kind == 4) {
-        v *= g.alpha;
-        if (g.beta != 0.0) v = fma(g.beta, c[e], v);
-      } else {
-        if (g.kind & 1) v = __hiloint2double((int)(hi32(v) ^ 0x80000000u), __double2loint(v));
-        if (g.kind & 2) v = c[e] + v;
+      const int fa = g.ea[br];
+      const bool wide = g.wa[br] != 0;
+      double* c = g.C + b0 * g.sC0 + b1 * g.sC1 + (long long)i * g.ldc + j0;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        if (j0 + e >= g.N) break;
+        const long long jb = (long long)bt * g.N + j0 + e;
+        const int fb = g.eb[jb];
+        const uint32_t s = sums >> (8 * e) & 0xff;
+        if (fa == 0x7ff || fb == 0x7ff || (s && (s < kSumFloor || !(wide && g.wb[jb])))) {
+          bad |= 1u << e;
+        } else {
+          put(g, c + e, combine(r[e], r[4 + e], r[8 + e], r[12 + e],
+                                max(fa, 1) + max(fb, 1) - 2 * (1022 + g.t)));
+        }
       }
-      c[e] = v;
     }
+    if (!__syncthreads_or(bad)) continue;
+    if (bad) {
+      int at = atomicAdd(&listed, __popc(bad));
+      for (; bad; bad &= bad - 1) list[at++] = (unsigned short)(4 * tid + __ffs(bad) - 1);
+    }
+    __syncthreads();
+    const int n = listed;
+    for (int x0 = 0; x0 < n; x0 += 32) {
+      const int x = x0 + (tid >> 3), el = list[min(x, n - 1)];
+      const long long sl = s0 + (el >> 5) * T, br = sl / tn;
+      const int j = 32 * (int)(sl - br * tn) + (el & 31), bt = (int)(br / g.M);
+      const int i = (int)(br - (long long)bt * g.M), b0 = bt % g.batch0, b1 = bt / g.batch0;
+      const double* ap = g.A + b0 * g.sA0 + b1 * g.sA1 + i * g.ai;
+      const double* bp = g.B + b0 * g.sB0 + b1 * g.sB1 + j * g.bj;
+      double v = 0.0;
+#pragma unroll 8
+      for (int k = tid & 7; k < g.K; k += 8) v = fma(ap[k * g.ak], bp[k * g.bk], v);
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (x < n && (tid & 7) == 0)
+        put(g, g.C + b0 * g.sC0 + b1 * g.sC1 + (long long)i * g.ldc + j, v);
+    }
+    __syncthreads();
+    if (tid == 0) listed = 0;
   }
 }
 
@@ -559,11 +677,12 @@ CUtensorMap residue_map(const void* base, long long rows, int Kp, int box_rows) 
 
 size_t up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
-// Workspace of one launch set (residues of A and B, result residues, exponents).
+// Workspace of one launch set (residues and magnitudes of A and B, result
+// residues and sums, exponents and largest sums).
 size_t crt_bytes(int M, int N, int K, long long nb) {
   const size_t Kp = up(K, BK), pitch = up(N, 16);
-  return up((size_t)2 * NM * nb * M * Kp, 1024) + up((size_t)2 * NM * nb * N * Kp, 1024) +
-         up((size_t)NM * nb * M * pitch, 1024) + up((size_t)4 * nb * (M + N), 1024) + 4096;
+  return up((size_t)2 * (NM + 1) * nb * M * Kp, 1024) + up((size_t)2 * (NM + 1) * nb * N * Kp, 1024) +
+         up((size_t)(NM + 1) * nb * M * pitch, 1024) + up((size_t)8 * nb * (M + N), 1024) + 4096;
 }
 
 // Bound on the workspace of one launch set: larger products run in pieces
@@ -584,13 +703,16 @@ void crt_piece(Handle& h, int M, int N, int K, double alpha, const Operand& A, c
   cudaStream_t st = h.stream;
   const int Kp = (int)up(K, BK), pitch = (int)up(N, 16), t = bits_for(K);
   h.gemm_ws.reserve(crt_bytes(M, N, K, batch), st);
-  auto* ra = h.gemm_ws.take<__nv_bfloat16>((size_t)NM * batch * M * Kp);
-  auto* rb = h.gemm_ws.take<__nv_bfloat16>((size_t)NM * batch * N * Kp);
-  auto* R = h.gemm_ws.take<int8_t>((size_t)NM * batch * M * pitch);
+  constexpr size_t NP = NM + 1;   // planes: residues and magnitudes
+  auto* ra = h.gemm_ws.take<__nv_bfloat16>(NP * batch * M * Kp);
+  auto* rb = h.gemm_ws.take<__nv_bfloat16>(NP * batch * N * Kp);
+  auto* R = h.gemm_ws.take<int8_t>(NP * batch * M * pitch);
   int* ea = h.gemm_ws.take<int>((size_t)batch * M);
   int* eb = h.gemm_ws.take<int>((size_t)batch * N);
-  const CrtOperand oa{A.x, A.ld, A.s0, A.s1, M, !A.trans, ra, ea};
-  const CrtOperand ob{B.x, B.ld, B.s0, B.s1, N, B.trans, rb, eb};
+  int* wa = h.gemm_ws.take<int>((size_t)batch * M);
+  int* wb = h.gemm_ws.take<int>((size_t)batch * N);
+  const CrtOperand oa{A.x, A.ld, A.s0, A.s1, M, !A.trans, ra, ea, wa};
+  const CrtOperand ob{B.x, B.ld, B.s0, B.s1, N, B.trans, rb, eb, wb};
   auto convert = [&](auto kern, int rows) {
     const int sa = (M + rows - 1) / rows, sb = (N + rows - 1) / rows;
     kern<<<dim3(sa + sb, batch), 256, 0, st>>>(oa, ob, sa, K, Kp, t, batch0, batch);
@@ -606,19 +728,22 @@ void crt_piece(Handle& h, int M, int N, int K, double alpha, const Operand& A, c
   g.tm = (M + BM - 1) / BM;
   // widest tiles that still give every SM an item, evenly over the columns
   g.tn = (N + 255) / 256;
-  while ((long long)NM * batch * g.tm * g.tn < num_sms() && (N + g.tn - 1) / g.tn > 64) ++g.tn;
+  while ((long long)NP * batch * g.tm * g.tn < num_sms() && (N + g.tn - 1) / g.tn > 64) ++g.tn;
   g.BN = (int)up((N + g.tn - 1) / g.tn, 16);
   g.tn = (N + g.BN - 1) / g.BN;
   g.KT = Kp / BK;
   g.chunks = g.KT <= kChunkOne ? 1 : (g.KT + kChunkMany - 1) / kChunkMany;
   g.per = (g.KT + g.chunks - 1) / g.chunks;
   g.stages = std::min(kMaxStages, kRing / (A_BYTES + g.BN * BK * 2));
-  g.items = (long long)NM * batch * g.tm * g.tn;
+  g.items = (long long)NP * batch * g.tm * g.tn;
   g.R = R;
+  g.theta = std::ldexp(1.0f, 51 - t);
+  g.wa = wa;
+  g.wb = wb;
   g.pitch = pitch;
   g.err = h.err_word();
-  const CUtensorMap ma = residue_map(ra, (long long)NM * batch * M, Kp, BM);
-  const CUtensorMap mb = residue_map(rb, (long long)NM * batch * N, Kp, g.BN);
+  const CUtensorMap ma = residue_map(ra, (long long)NP * batch * M, Kp, BM);
+  const CUtensorMap mb = residue_map(rb, (long long)NP * batch * N, Kp, g.BN);
   const size_t sm = (size_t)g.stages * (A_BYTES + g.BN * BK * 2) + 1024;
   ensure_smem(reinterpret_cast<const void*>(crt_gemm_kernel), sm);
   crt_gemm_kernel<<<(unsigned)std::min<long long>(g.items, num_sms()), kThreads, sm, st>>>(ma, mb,
@@ -634,6 +759,8 @@ void crt_piece(Handle& h, int M, int N, int K, double alpha, const Operand& A, c
   c.pitch = pitch;
   c.ea = ea;
   c.eb = eb;
+  c.wa = wa;
+  c.wb = wb;
   c.t = t;
   c.alpha = alpha;
   c.beta = beta;
@@ -654,9 +781,10 @@ void crt_piece(Handle& h, int M, int N, int K, double alpha, const Operand& A, c
   c.bj = B.trans ? B.ld : 1;
   c.sB0 = B.s0;
   c.sB1 = B.s1;
-  const long long total = (long long)batch * M * ((N + 3) / 4);
-  crt_combine_kernel<<<(unsigned)std::min<long long>((total + 255) / 256, 32LL * num_sms()), 256, 0,
-                       st>>>(c);
+  const int tn = (N + 31) / 32;
+  long long ctas = std::min(((long long)batch * M * tn + 31) / 32, 32LL * num_sms());
+  while (std::gcd(ctas, (long long)tn) != 1) ++ctas;
+  crt_combine_kernel<<<(unsigned)ctas, 256, 0, st>>>(c);
   check_launch("crt_combine_kernel");
 }
 
@@ -685,7 +813,7 @@ void gemm_f64_tensor(Handle& h, bool ta, bool tb, int M, int N, int K, double al
   long long fit = std::max<long long>(1, kWsMax / crt_bytes(Mp, Np, K, 1));
   fit = std::min<long long>(fit, 65535);
   // residue rows are indexed by 32-bit TMA coordinates
-  fit = std::max<long long>(1, std::min(fit, (1LL << 30) / NM / std::max(Mp, Np)));
+  fit = std::max<long long>(1, std::min(fit, (1LL << 30) / (NM + 1) / std::max(Mp, Np)));
   for (int i0 = 0; i0 < M; i0 += Mp)
     for (int j0 = 0; j0 < N; j0 += Np) {
       const int m = std::min(Mp, M - i0), n = std::min(Np, N - j0);

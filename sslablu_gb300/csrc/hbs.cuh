@@ -77,8 +77,9 @@ struct Handle {
 };
 
 // gemm_batched<double> for dense products: on the tensor cores by residue
-// arithmetic where that is faster (crt_gemm.cu; float64-accurate), else the
-// float64 kernel.  C must not overlap A or B.
+// arithmetic where that is faster (crt_gemm.cu, which states its error bound;
+// outputs beyond it are float64 dot products), else the float64 kernel.  C must
+// not overlap A or B.
 void gemm_f64(Handle& h, bool ta, bool tb, int M, int N, int K, double alpha, const double* A,
               int lda, long long sA0, long long sA1, const double* B, int ldb, long long sB0,
               long long sB1, double beta, double* C, int ldc, long long sC0, long long sC1,

@@ -35,9 +35,10 @@ inline double* dp(const DevBuf& b) { return b.as<double>(); }
 inline int* ip(const DevBuf& b) { return b.as<int>(); }
 
 // Products of the factorisations (depth m).  From m = 64 on they run as
-// residue products whatever their size: their error is a tenth of the float64
-// kernel's, and the explicit inverses and composed solve operators inherit it
-// (on 12 copies of a near-resonant 4 x 64 system perturbed by 1e-15, median
+// residue products whatever their size: on blocks without grading their error
+// is a tenth of the float64 kernel's, and the explicit inverses and composed
+// solve operators inherit it (rows, columns and outputs whose operands' scales
+// oppose are float64 dot products there: crt_gemm.cu) (on 12 copies of a near-resonant 4 x 64 system perturbed by 1e-15, median
 // solution residual 8.7e-9 with float64 products and LU-solved inverses, at
 // most 3e-9 in the same test with exact products); at m = 64 both take about
 // 25 us.
