@@ -97,16 +97,16 @@ __device__ __forceinline__ int dp4a_su(uint32_t a, uint32_t b, int c) {
 
 __device__ __forceinline__ uint32_t hi32(double v) { return (uint32_t)__double2hiint(v); }
 
-// A float64 (its bits) whose exponent field is at most F (>= 1) as a t-bit
+// A float64 (its bits) d powers of two below the largest of its row as a t-bit
 // integer (t <= kMaxBits), rounded to nearest and shifted by 2^59 to be non-negative
 // (the tables take the shift off again); ok = false gives zero.
-__device__ __forceinline__ void scaled(uint32_t hi, uint32_t lo, int F, int t, bool ok,
-                                       uint32_t& zlo, uint32_t& zhi) {
+__device__ __forceinline__ void scaled_by(uint32_t hi, uint32_t lo, int d, int t, bool ok,
+                                          uint32_t& zlo, uint32_t& zhi) {
   const int fe = (int)((hi >> 20) & 0x7ff);
   // the mantissa from bit 63 down: |a'| = m 2^-(s + 1), rounded half away
   const uint32_t mh = (__funnelshift_l(lo, hi, 11) & 0x7fffffffu) | (fe ? 0x80000000u : 0u);
   const uint32_t ml = lo << 11;
-  const int s = ok ? 63 - t + F - max(fe, 1) : 64;
+  const int s = ok ? 63 - t + d : 64;
   const uint32_t ql = s < 32 ? __funnelshift_r(ml, mh, s) : (s < 64 ? mh >> (s - 32) : 0u);
   const uint32_t qh = s < 32 ? mh >> s : 0u;
   const unsigned long long q = (((unsigned long long)qh << 32 | ql) + 1) >> 1;
@@ -114,6 +114,11 @@ __device__ __forceinline__ void scaled(uint32_t hi, uint32_t lo, int F, int t, b
   const unsigned long long z = (q ^ sg) + ((1ULL << 59) - sg);
   zlo = (uint32_t)z;
   zhi = (uint32_t)(z >> 32);
+}
+// The same where the largest exponent field of the row is F (>= 1)
+__device__ __forceinline__ void scaled(uint32_t hi, uint32_t lo, int F, int t, bool ok,
+                                       uint32_t& zlo, uint32_t& zhi) {
+  scaled_by(hi, lo, F - max((int)((hi >> 20) & 0x7ff), 1), t, ok, zlo, zhi);
 }
 
 // Balanced residue modulo p (ip = 1 / p) of the shifted integer, from the byte

@@ -8,8 +8,18 @@
 // makes them faster.  Here a step is 16 bfloat16 products modulo the primes of
 // crt.cuh, each exact in float32 (at most 128 terms of at most 2^14), and one
 // reconstruction per output, rounded once: the error is that of rounding S and
-// z at 2^-59 of their row's and column's largest entry, below that of a
-// float64 FMA chain.
+// z to t = 58 or 59 bits of their row's and column's largest entry.  Where the
+// columns of a block of S differ by more than 2^kSpread, they are scaled to one
+// size by powers of two (kx, made with the images) and the entries of z that they
+// meet by the inverse.  So each column of z meets, at its largest entry, an entry
+// of S within 2^-kSpread of its row's largest: the error in a column of outputs,
+// its rows scaled by those of S, is at most w 2^(kSpread - t), below w 2^-53,
+// times the largest sum of |S| |z| there, where a float64 FMA chain's is w 2^-53
+// of the output's own.  Outputs below 2^-32 of the row's and column's largest
+// entries are formed by float64 dot products, so every output keeps 2^-26 of its
+// own size.  (Random cancellation gets there once in 10^9 outputs; at 2^-22 a
+// step of 4 M outputs met two or three, and the 20-40K clocks of each added half
+// to a solve of 261 columns.)
 //
 // One persistent kernel per step.  A tile is a block, up to 128 operator rows
 // and 32, 16 or 8 columns (tiling_of: 16 moduli of 32 columns fill TMEM):
@@ -65,6 +75,7 @@ struct CrtStep {
   sweep::Step<double> s;     // geometry and vectors; s.S for what is not finite
   const __nv_bfloat16* img;  // [Nb][ntile][NM][RT x wP]
   const int* ex;             // exponent field of every row: [Nb][ntile * RT]
+  const short* kx;           // powers of two off S's columns [Nb][wP], or nullptr
   int RT, wP, ntile, t;      // rows and tiles of the images
   int split, RS;             // a tile's rows: RS of RT / split
   int slots, groups;         // image slots, z group buffers
@@ -148,6 +159,19 @@ __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[8]) {
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
         "=r"(r[7])
       : "r"(taddr));
+}
+
+constexpr int kSpread = 4;             // powers of two
+constexpr short kZeroColumn = -8192;   // kx of a column of zeros
+constexpr int kZeroRow = -8192;        // ex of a row of zeros
+
+// v 2^e; infinity (for a float64 dot product) where that or v is not a normal
+// number, zero where v or the column of S is zero.
+__device__ __forceinline__ uint2 times_pow2(uint2 v, int e) {
+  const int fe = (int)(v.y >> 20 & 0x7ff), f = fe + e;
+  if (fe != 0 && fe != 0x7ff && f >= 1 && f <= 2046) return make_uint2(v.x, v.y + ((uint32_t)e << 20));
+  const bool zero = ((v.y & 0x7fffffffu) | v.x) == 0 || (fe != 0x7ff && e == kZeroColumn);
+  return make_uint2(0, zero ? 0u : 0x7ff00000u);
 }
 
 // Row k of block b's z vector (all columns): the step's input ranges in order.
@@ -366,9 +390,19 @@ __global__ void __launch_bounds__(kThreads, 1) crt_step_kernel(const CrtStep o) 
     const int cw = warp - kMma, col = lane % NC;
     const int k0 = (cw * (32 / NC) + lane / NC) * KPT;
     uint2 z[KPT];
+    uint32_t kx[(KPT + 1) / 2];   // two a word
     auto fetch = [&](int i) {
       const Tile T = tile_of(t0 + i, nrt, nct);
       const int c = T.ct * NC + col;
+      if (o.kx) {
+        const short* kp = o.kx + (long long)T.b * wP + (k0 < wP ? k0 : 0);
+        if constexpr (KPT == 1) {
+          kx[0] = (uint16_t)__ldg(kp);
+        } else {
+#pragma unroll
+          for (int u = 0; u < KPT / 2; ++u) kx[u] = __ldg(reinterpret_cast<const uint32_t*>(kp) + u);
+        }
+      }
 #pragma unroll
       for (int u = 0; u < KPT; ++u) {
         z[u] = make_uint2(0, 0);
@@ -383,6 +417,11 @@ __global__ void __launch_bounds__(kThreads, 1) crt_step_kernel(const CrtStep o) 
     const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + CG * g;
     for (int i = 0; i < nt; ++i) {
       const Tile T = tile_of(t0 + i, nrt, nct);
+      if (o.kx) {
+#pragma unroll
+        for (int u = 0; u < KPT; ++u)
+          z[u] = times_pow2(z[u], (int)(short)(kx[u >> 1] >> (16 * (u & 1))));
+      }
       // column exponents
       int mx = 0;
 #pragma unroll
@@ -511,11 +550,12 @@ __global__ void __launch_bounds__(kThreads, 1) crt_step_kernel(const CrtStep o) 
           for (int u = 0; u < EU; ++u) {
             const int e = HALF ? 2 * (e0 + u) + es : e0 + u;
             if (e < nc) {
-              const int fb = cex[i & 1][CG * g + e];
-              out[e] = (fa == 0x7ff || fb == 0x7ff)
-                           ? dot_f64(s, T.b, r0 + r, c0 + e)
-                           : combine(R[u][0], R[u][1], R[u][2], R[u][3],
-                                     max(fa, 1) + max(fb, 1) - 2 * (1022 + o.t));
+              const int fb = cex[i & 1][CG * g + e], f = fa + max(fb, 1);
+              double v = combine(R[u][0], R[u][1], R[u][2], R[u][3], f - 2 * (1022 + o.t));
+              // not finite, or below 2^-32 of the largest entries
+              if (fa == 0x7ff || fb == 0x7ff || (int)(hi32(v) >> 20 & 0x7ff) < f - 1053)
+                v = dot_f64(s, T.b, r0 + r, c0 + e);
+              out[e] = v;
             }
           }
 #pragma unroll
@@ -539,13 +579,54 @@ struct ImageOp {
   const double* S;
   __nv_bfloat16* img;
   int* ex;
+  short* kx;
   int first;   // rows (padded) of the operators before it
+  int firstb;  // blocks of the operators before it
   int rows, w, RT, wP, ntile, t;
 };
 struct ImageOps {
-  int count, total;
+  int count, total, blocks;
+  int* scaled;   // [count], zeroed: operators that have a kx other than 0
   ImageOp op[kMaxOps];
 };
+
+// exponent field of a number, 1 for a subnormal one
+__device__ __forceinline__ int field(uint2 v) { return max((int)(v.y >> 20 & 0x7ff), 1); }
+__device__ __forceinline__ bool is_zero(uint2 v) { return ((v.y & 0x7fffffffu) | v.x) == 0; }
+
+// kx of every column of every block, from its largest finite entry; one CTA per
+// block.
+__global__ void __launch_bounds__(kMaxW) crt_column_kernel(const __grid_constant__ ImageOps a) {
+  __shared__ int lo, hi;
+  const int gb = blockIdx.x, k = threadIdx.x;
+  int i = 0;
+  while (i + 1 < a.count && gb >= a.op[i + 1].firstb) ++i;
+  const ImageOp& o = a.op[i];
+  const int b = gb - o.firstb;
+  if (k == 0) {
+    lo = 0x7fff;
+    hi = 0;
+  }
+  __syncthreads();
+  int e = 0;   // 0: a column of zeros
+  if (k < o.w) {
+    const uint2* S = reinterpret_cast<const uint2*>(o.S + (long long)b * o.rows * o.w + k);
+#pragma unroll 8
+    for (int r = 0; r < o.rows; ++r) {
+      const uint2 v = S[(long long)r * o.w];
+      const int f = field(v);
+      if (f < 0x7ff && !is_zero(v)) e = max(e, f);
+    }
+    if (e) {
+      atomicMin(&lo, e);
+      atomicMax(&hi, e);
+    }
+  }
+  __syncthreads();
+  const short kx = k >= o.w ? 0 : (e == 0 ? kZeroColumn : (hi - lo > kSpread ? (short)(e - 1023) : 0));
+  if (k < o.wP) o.kx[(long long)b * o.wP + k] = kx;
+  if (kx) a.scaled[i] = 1;
+}
 
 // Residue images: one warp per (operator, block, tile row), lane = eight
 // consecutive k; rows beyond the operator's are zero.
@@ -559,19 +640,24 @@ __global__ void __launch_bounds__(256) crt_op_kernel(const __grid_constant__ Ima
   const int bt = gw / RT, rr = gw - bt * RT, b = bt / o.ntile, r = (bt - b * o.ntile) * RT + rr;
   const uint2* row = reinterpret_cast<const uint2*>(o.S + ((long long)b * o.rows + r) * w);
   uint2 v[8];
-  int mx = 0;
+  int ex[8], mx = kZeroRow;
+  bool finite = true;
 #pragma unroll
   for (int u = 0; u < 8; ++u) {
     const int k = 8 * lane + u;
     v[u] = (r < o.rows && k < w) ? row[k] : make_uint2(0, 0);
-    mx = max(mx, (int)(v[u].y & 0x7fffffffu));
+    finite = finite && field(v[u]) < 0x7ff;
+    ex[u] = is_zero(v[u]) ? kZeroRow : field(v[u]) - o.kx[(long long)b * wP + k];
+    mx = max(mx, ex[u]);
   }
-  mx = __reduce_max_sync(0xffffffffu, mx) >> 20;
-  if (lane == 0) o.ex[gw] = mx;
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  finite = __all_sync(0xffffffffu, finite);
+  if (lane == 0) o.ex[gw] = finite ? mx : 0x7ff;
   if (8 * lane >= wP) return;
   uint32_t lo[8], hi[8];
 #pragma unroll
-  for (int u = 0; u < 8; ++u) scaled(v[u].y, v[u].x, max(mx, 1), o.t, mx != 0x7ff, lo[u], hi[u]);
+  for (int u = 0; u < 8; ++u)
+    scaled_by(v[u].y, v[u].x, mx - ex[u], o.t, finite && ex[u] > kZeroRow, lo[u], hi[u]);
   __nv_bfloat16* dst = o.img + (size_t)bt * NM * RT * wP + (size_t)(rr >> 3) * (wP * 8) +
                        lane * 64 + (rr & 7) * 8;
 #pragma unroll
@@ -605,8 +691,8 @@ struct Part {
 bool make_images(cudaStream_t st, const std::vector<Part>& parts, DevBuf& buf) {
   if ((int)parts.size() > kMaxOps) return false;
   ImageOps a{};
-  size_t bytes = 0;
-  long long total = 0;
+  size_t bytes = (4 * parts.size() + 1023) / 1024 * 1024;   // `scaled`
+  long long total = 0, blocks = 0;
   std::vector<size_t> at;
   for (const Part& p : parts) {
     CrtOp& o = *p.op;
@@ -618,7 +704,10 @@ bool make_images(cudaStream_t st, const std::vector<Part>& parts, DevBuf& buf) {
     bytes += (2 * (NM * tr + 8) * o.wP + 1023) / 1024 * 1024;
     at.push_back(bytes);
     bytes += (4 * tr + 1023) / 1024 * 1024;
+    at.push_back(bytes);
+    bytes += (2 * (size_t)o.Nb * o.wP + 1023) / 1024 * 1024;
     total += (long long)tr;
+    blocks += o.Nb;
   }
   if (bytes > kMaxImages || total >= (1LL << 31)) return false;
   try {
@@ -627,13 +716,17 @@ bool make_images(cudaStream_t st, const std::vector<Part>& parts, DevBuf& buf) {
     cudaGetLastError();   // no memory for them: the float64 steps need none
     return false;
   }
+  a.scaled = buf.as<int>();
+  SLU_CHECK_CUDA(cudaMemsetAsync(a.scaled, 0, 4 * parts.size(), st));
   for (size_t i = 0; i < parts.size(); ++i) {
     CrtOp& o = *parts[i].op;
     ImageOp& d = a.op[a.count++];
     d.S = parts[i].S->as<double>();
-    d.img = reinterpret_cast<__nv_bfloat16*>(buf.as<char>() + at[2 * i]);
-    d.ex = reinterpret_cast<int*>(buf.as<char>() + at[2 * i + 1]);
+    d.img = reinterpret_cast<__nv_bfloat16*>(buf.as<char>() + at[3 * i]);
+    d.ex = reinterpret_cast<int*>(buf.as<char>() + at[3 * i + 1]);
+    d.kx = reinterpret_cast<short*>(buf.as<char>() + at[3 * i + 2]);
     d.first = a.total;
+    d.firstb = a.blocks;
     d.rows = o.rows;
     d.w = o.w;
     d.RT = o.RT;
@@ -641,11 +734,21 @@ bool make_images(cudaStream_t st, const std::vector<Part>& parts, DevBuf& buf) {
     d.ntile = o.ntile;
     d.t = bits_for(o.w);
     a.total += o.Nb * o.ntile * o.RT;
+    a.blocks += o.Nb;
     o.img = d.img;
     o.ex = d.ex;
+    o.kx = d.kx;
   }
+  crt_column_kernel<<<(unsigned)blocks, kMaxW, 0, st>>>(a);
+  check_launch("crt_column_kernel");
   crt_op_kernel<<<(unsigned)((a.total + 7) / 8), 256, 0, st>>>(a);
   check_launch("crt_op_kernel");
+  // operators that need no scaling (their steps skip it)
+  std::vector<int> need(parts.size());
+  SLU_CHECK_CUDA(cudaMemcpyAsync(need.data(), a.scaled, 4 * parts.size(), cudaMemcpyDeviceToHost, st));
+  stream_wait(st);   // other streams may use the images from here on, too
+  for (size_t i = 0; i < parts.size(); ++i)
+    if (!need[i]) parts[i].op->kx = nullptr;
   return true;
 }
 
@@ -679,6 +782,7 @@ void launch(cudaStream_t st, const sweep::Step<double>& s, const CrtOp& op, vola
   o.s = s;
   o.img = op.img;
   o.ex = op.ex;
+  o.kx = op.kx;
   o.RT = op.RT;
   o.wP = op.wP;
   o.ntile = op.ntile;
@@ -769,7 +873,7 @@ bool ready(Handle& h, Hbs& H, bool solve, bool trans) {
   }
   const bool made = make_images(st, parts, H.crt_buf[(solve ? 0 : 2) + (trans ? 1 : 0)]);
   if (!made && !compose) return false;
-  stream_wait(st);   // other streams may use the images from here on
+  if (!made) stream_wait(st);   // the composed operators
   if (compose) H.has_apply[trans ? 1 : 0] = true;
   have = made;
   return made;

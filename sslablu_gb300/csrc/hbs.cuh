@@ -113,10 +113,12 @@ struct OzOp {
 
 // A step operator as residue images for the exact tensor-core steps
 // (crt_step.cu): per (block, row tile of RT rows, modulus) one RT x wP bfloat16
-// image in core-matrix order; ex holds every row's largest exponent field.
+// image in core-matrix order; kx the powers of two taken off the columns of every
+// block (nullptr: none), ex every row's largest exponent field after that.
 struct CrtOp {
   const __nv_bfloat16* img = nullptr;   // into Hbs::crt_buf
   const int* ex = nullptr;
+  const short* kx = nullptr;
   int Nb = 0, rows = 0, w = 0;
   int RT = 0, wP = 0, ntile = 0;
 };
