@@ -633,7 +633,7 @@ int slu_lu_factor(slu_handle_t h, int n, double* A, int lda, long long sA, int* 
   return guard(h, [&] {
     SLU_REQUIRE(h && A && piv, "null argument");
     SLU_REQUIRE(n >= 1 && lda >= n && nb >= 1, "bad shape");
-    slu::lu_factor(h->h, n, A, lda, sA, piv, sP, nb, info);
+    slu::lu_factor(h->h, n, A, lda, sA, piv, sP, nb, info, 1);
   });
 }
 

@@ -89,9 +89,11 @@ void gemm_f64_tensor(Handle& h, bool ta, bool tb, int M, int N, int K, double al
                      int ldb, long long sB0, long long sB1, double beta, double* C, int ldc,
                      long long sC0, long long sC1, int batch0, int batch1 = 1);
 // Batched LU with partial pivoting, in place (A_b n x n row-major), pivots
-// piv_b[i] = row swapped with row i (LAPACK getrf convention, 0-based).
+// piv_b[i] = row swapped with row i (LAPACK getrf convention, 0-based).  A zero
+// pivot j of matrix b sets info[istep b] to j + 1 unless it is set: istep 1 with a
+// word per matrix, 0 with one for all (the handle's status word).
 void lu_factor(Handle& h, int n, double* A, int lda, long long sA, int* piv, long long sP,
-               int batch, int* info);
+               int batch, int* info, int istep);
 // Inv_b = A_b^{-1} from the LU factors.
 void lu_inverse(Handle& h, int n, const double* LU, int lda, long long sA, const int* piv,
                 long long sP, double* Inv, int ldi, long long sI, int batch);

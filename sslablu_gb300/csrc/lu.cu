@@ -56,7 +56,8 @@ __device__ inline void argmax_abs_block(double v, int idx, double* sv, int* si, 
 // CTA per matrix.  src[i] = the row that ends at row i.
 __global__ void __launch_bounds__(1024)
 lu_panel_global_kernel(int n, int k0, int kb, double* __restrict__ A, int lda, long long sA,
-                       int* __restrict__ piv, long long sP, int* __restrict__ src, int* info) {
+                       int* __restrict__ piv, long long sP, int* __restrict__ src, int* info,
+                       int istep) {
   A += blockIdx.x * sA;
   piv += blockIdx.x * sP;
   src += (long long)blockIdx.x * n;
@@ -109,7 +110,7 @@ lu_panel_global_kernel(int n, int k0, int kb, double* __restrict__ A, int lda, l
     }
     __syncthreads();
   }
-  if (threadIdx.x == 0 && first_zero && info) atomicCAS(info + blockIdx.x, 0, first_zero);
+  if (threadIdx.x == 0 && first_zero && info) atomicCAS(info + istep * blockIdx.x, 0, first_zero);
 }
 
 // Panel factorisation by one cluster per matrix.  Thread = row, the row's kb
@@ -189,7 +190,7 @@ __device__ __forceinline__ bool panel_wait(uint32_t bar, uint32_t parity) {
 
 __global__ void __launch_bounds__(kPanelRows)
 lu_panel_kernel(int n, int k0, int kb, double* __restrict__ A, int lda, long long sA,
-                int* __restrict__ piv, long long sP, int* __restrict__ src, int* info,
+                int* __restrict__ piv, long long sP, int* __restrict__ src, int* info, int istep,
                 unsigned* err) {
   constexpr int KB = kPanel;
   extern __shared__ __align__(16) unsigned char s_raw[];
@@ -350,7 +351,7 @@ lu_panel_kernel(int n, int k0, int kb, double* __restrict__ A, int lda, long lon
     for (int c = 0; c < kb; ++c) row[c] = fin[c * blockDim.x];
     src[k0 + pos] = k0 + r;
   }
-  if (rank == 0 && threadIdx.x == 0 && first_zero && info) atomicCAS(info + b, 0, first_zero);
+  if (rank == 0 && threadIdx.x == 0 && first_zero && info) atomicCAS(info + istep * b, 0, first_zero);
 }
 
 // The same for up to 1024 rows, four warps per 32 rows: warp g of them holds
@@ -366,7 +367,7 @@ lu_panel_kernel(int n, int k0, int kb, double* __restrict__ A, int lda, long lon
 constexpr int kSplitRows = 1024;
 __global__ void __launch_bounds__(512)
 lu_panel_split_kernel(int n, int k0, int kb, double* __restrict__ A, int lda, long long sA,
-                      int* __restrict__ piv, long long sP, int* __restrict__ src, int* info,
+                      int* __restrict__ piv, long long sP, int* __restrict__ src, int* info, int istep,
                       unsigned* err) {
   constexpr int KB = kPanel, NC = KB / 4;   // columns per warp
   extern __shared__ __align__(16) unsigned char s_raw[];
@@ -549,7 +550,7 @@ lu_panel_split_kernel(int n, int k0, int kb, double* __restrict__ A, int lda, lo
       if (4 * i + g < kb) row[4 * i + g] = fin[(4 * i + g) * rows];
     if (g == 0) src[k0 + pos] = k0 + r;
   }
-  if (rank == 0 && threadIdx.x == 0 && first_zero && info) atomicCAS(info + b, 0, first_zero);
+  if (rank == 0 && threadIdx.x == 0 && first_zero && info) atomicCAS(info + istep * b, 0, first_zero);
 }
 
 // The panel's row swaps on every column outside it, from the net permutation
@@ -661,7 +662,8 @@ lu_block_trsm_kernel(int n, int k0, int nb, int c0, double* __restrict__ A, int 
 }
 
 void launch_panel(cudaStream_t st, int n, int k0, int kb, double* A, int lda, long long sA,
-                  int* piv, long long sP, int* src, int batch, int* info, unsigned* err) {
+                  int* piv, long long sP, int* src, int batch, int* info, int istep,
+                  unsigned* err) {
   const int R = n - k0;
   // 32 rows per CTA (four warps), then up to 128, in clusters of up to eight
   // (the portable size); above 1024 rows a thread per row
@@ -671,7 +673,8 @@ void launch_panel(cudaStream_t st, int n, int k0, int kb, double* A, int lda, lo
   const int warps = ((R + cs - 1) / cs + 31) / 32;   // row groups of 32
   const int threads = 32 * warps * (split ? 4 : 1);
   if (threads > kPanelRows) {
-    lu_panel_global_kernel<<<batch, 1024, 0, st>>>(n, k0, kb, A, lda, sA, piv, sP, src, info);
+    lu_panel_global_kernel<<<batch, 1024, 0, st>>>(n, k0, kb, A, lda, sA, piv, sP, src, info,
+                                                   istep);
     check_launch("lu_panel_global_kernel");
     return;
   }
@@ -693,7 +696,7 @@ void launch_panel(cudaStream_t st, int n, int k0, int kb, double* A, int lda, lo
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   SLU_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, n, k0, kb, A, lda, sA, piv, sP, src,
-                                    info, err));
+                                    info, istep, err));
   check_launch("lu_panel_kernel");
 }
 
@@ -809,7 +812,7 @@ permute_cols_kernel(int n, int np, const double* __restrict__ X, long long sX,
 }  // namespace
 
 void lu_factor(Handle& h, int n, double* A, int lda, long long sA, int* piv, long long sP,
-               int batch, int* info) {
+               int batch, int* info, int istep) {
   if (n <= 0 || batch <= 0) return;
   SLU_REQUIRE(batch <= 65535, "LU batch too large");
   cudaStream_t st = h.stream;
@@ -819,7 +822,8 @@ void lu_factor(Handle& h, int n, double* A, int lda, long long sA, int* piv, lon
     const int K1 = std::min(K0 + kOuter, n);
     for (int k0 = K0; k0 < K1; k0 += kPanel) {
       const int kb = std::min(kPanel, K1 - k0), k1 = k0 + kb;
-      launch_panel(st, n, k0, kb, A, lda, sA, piv, sP, src, batch, info, h.err_word());
+      launch_panel(st, n, k0, kb, A, lda, sA, piv, sP, src, batch, info, istep,
+                   h.err_word());
       if (n > kb) {
         lu_swap_trsm_kernel<<<dim3((n + kSwapCols - 1) / kSwapCols, batch), 32 * kSwapCols, 0, st>>>(
             n, k0, kb, K1, A, lda, sA, piv, sP, src);

@@ -220,7 +220,7 @@ void rb_factor(Handle& h, RbSolver& S, int nblk, int m, const double* SiM, const
     }
     SLU_CHECK_CUDA(cudaMemcpyAsync(dp(L0.T), T, 8 * nblk * mm, cudaMemcpyDeviceToDevice, st));
     SLU_CHECK_CUDA(cudaMemcpyAsync(dp(L0.LU), T, 8 * nblk * mm, cudaMemcpyDeviceToDevice, st));
-    lu_factor(h, m, dp(L0.LU), m, mm, ip(L0.piv), m, nblk, h.info.as<int>());
+    lu_factor(h, m, dp(L0.LU), m, mm, ip(L0.piv), m, nblk, h.info.as<int>(), 0);
     L0.Inv.alloc(8 * nblk * mm, st);
     lu_inverse(h, m, dp(L0.LU), m, mm, ip(L0.piv), m, dp(L0.Inv), m, mm, nblk);
   }
@@ -285,7 +285,7 @@ void rb_factor(Handle& h, RbSolver& S, int nblk, int m, const double* SiM, const
       add_batched<double>(st, m, m, 1.0, dp(N.SiP), m, 0, 0, dp(N.T), m, 0, 0, 1);
     }
     SLU_CHECK_CUDA(cudaMemcpyAsync(dp(N.LU), dp(N.T), 8 * nR * mm, cudaMemcpyDeviceToDevice, st));
-    lu_factor(h, m, dp(N.LU), m, mm, ip(N.piv), m, nR, h.info.as<int>());
+    lu_factor(h, m, dp(N.LU), m, mm, ip(N.piv), m, nR, h.info.as<int>(), 0);
     N.Inv.alloc(8 * nR * mm, st);
     lu_inverse(h, m, dp(N.LU), m, mm, ip(N.piv), m, dp(N.Inv), m, mm, nR);
     S.levels.push_back(std::move(N));
@@ -483,7 +483,7 @@ void thomas_factor(Handle& h, RbSolver& S, int nblk, int m, const double* SiM, c
       gemm_factor(h, m, m, m, -1.0, dp(L.T) + i * mm, m, 0, dp(L.SiP) + (i - 1) * mm, m, 0, 1.0,
                   Bi, m, 0, 1);
     }
-    lu_factor(h, m, Bi, m, 0, ip(L.piv) + i * m, 0, 1, h.info.as<int>());
+    lu_factor(h, m, Bi, m, 0, ip(L.piv) + i * m, 0, 1, h.info.as<int>(), 0);
     lu_inverse(h, m, Bi, m, 0, ip(L.piv) + i * m, 0, dp(L.Inv) + i * mm, m, 0, 1);
   }
   S.fused = false;
