@@ -814,7 +814,13 @@ permute_cols_kernel(int n, int np, const double* __restrict__ X, long long sX,
 void lu_factor(Handle& h, int n, double* A, int lda, long long sA, int* piv, long long sP,
                int batch, int* info, int istep) {
   if (n <= 0 || batch <= 0) return;
-  SLU_REQUIRE(batch <= 65535, "LU batch too large");
+  constexpr int kMaxBatch = 65535;   // matrices of a launch (grid dimensions)
+  if (batch > kMaxBatch) {
+    for (int b0 = 0; b0 < batch; b0 += kMaxBatch)
+      lu_factor(h, n, A + b0 * sA, lda, sA, piv + b0 * sP, sP, std::min(kMaxBatch, batch - b0),
+                info ? info + (long long)istep * b0 : nullptr, istep);
+    return;
+  }
   cudaStream_t st = h.stream;
   h.lu_ws.reserve(sizeof(int) * (size_t)n * batch + 256, st);
   int* src = h.lu_ws.take<int>((size_t)n * batch);
