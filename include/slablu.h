@@ -64,6 +64,16 @@ int slu_set_stream(slu_handle_t h, void* stream);
 /* Synchronises the handle's stream and reports device-side status words
  * (e.g. a Jacobi SVD that did not converge) as SLU_ERR_NOT_CONVERGED. */
 int slu_sync(slu_handle_t h);
+/* Kernels that wait (for their copies, tensor-core products or the other CTAs
+ * of a cluster) do so a bounded number of times; one that gives up leaves its
+ * call's results invalid.  The next call on the same handle then returns
+ * SLU_ERR_TIMEOUT without doing its work, once.  slu_check_waits is such a call
+ * that does nothing else: made after the caller has waited for the handle's
+ * stream, it tells whether what was computed there is valid. */
+int slu_check_waits(slu_handle_t h);
+/* Launches a kernel whose wait runs out after `polls` polls (a diagnostic of
+ * the above). */
+int slu_wait_probe(slu_handle_t h, int polls);
 
 /* ---------------------------------------------------------------- HBS operator
  * Replaces matAssembly/HBS/HBSnew.py:82-118 (HBSMAT.__init__ with a tree):

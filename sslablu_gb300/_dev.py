@@ -31,7 +31,10 @@ def to_dev(x, dtype=F64):
 
 
 def to_host(t):
-    return t.detach().cpu().numpy()
+    h = t.detach().cpu().numpy()
+    if t.is_cuda:
+        L.check_waits()
+    return h
 
 
 def out_like(t, ref):

@@ -27,6 +27,8 @@ SIGNATURES = {
     "slu_destroy": [P],
     "slu_set_stream": [P, P],
     "slu_sync": [P],
+    "slu_check_waits": [P],
+    "slu_wait_probe": [P, c_int],
     "slu_hbs_create": [P, c_int, c_int, c_int, P, ctypes.POINTER(c_void_p)],
     "slu_hbs_destroy": [P],
     "slu_hbs_compress": [P, P, c_int, c_int, c_int, P, P, P, P, c_int],
@@ -194,6 +196,12 @@ def handle():
 
 def sync():
     check(lib().slu_sync(handle()))
+
+
+def check_waits():
+    """Raises where a kernel of the current stream gave up waiting; to be called
+    once the stream's work is done (a result has been copied to the host)."""
+    check(lib().slu_check_waits(handle()))
 
 
 def ptr(t):

@@ -30,9 +30,11 @@ namespace slu {
 std::string& thread_error();
 
 // Runs f, turning exceptions into status codes; no exception crosses the ABI.
+// On a handle one of whose earlier calls gave up waiting, f does not run.
 template <class F>
 int guard_call(slu_handle_t h, F&& f) {
   try {
+    if (h) h->h.check_waits();
     f();
     return SLU_OK;
   } catch (const Error& e) {

@@ -46,6 +46,7 @@ int slu_create(void* stream, slu_handle_t* out) {
     p->h.stream = reinterpret_cast<cudaStream_t>(stream);
     p->h.info.alloc(64 * sizeof(int), p->h.stream);
     SLU_CHECK_CUDA(cudaMemsetAsync(p->h.info.p, 0, 64 * sizeof(int), p->h.stream));
+    p->h.err = slu::mapped_word();
     *out = p.release();
   });
 }
@@ -70,6 +71,7 @@ int slu_sync(slu_handle_t h) {
   int st = guard(h, [&] {
     SLU_REQUIRE(h, "null handle");
     slu::stream_wait(h->h.stream);
+    h->h.check_waits(true);
   });
   if (st != SLU_OK) return st;
   int info[64];
@@ -77,18 +79,6 @@ int slu_sync(slu_handle_t h) {
     SLU_CHECK_CUDA(cudaMemcpy(info, h->h.info.p, sizeof(info), cudaMemcpyDeviceToHost));
   });
   if (st != SLU_OK) return st;
-  bool plan_err = false;
-  for (const auto& w : h->h.plan_err)
-    if (const auto p = w.lock()) {
-      plan_err = plan_err || *p;
-      *p = 0;
-    }
-  if (info[1] != 0 || plan_err) {
-    cudaMemset(h->h.info.p, 0, sizeof(info));
-    g_err = "a tensor-core GEMM gave up waiting on its TMA / MMA pipeline";
-    h->h.last_error = g_err;
-    return SLU_ERR_TIMEOUT;
-  }
   if (info[0] != 0) {
     cudaMemset(h->h.info.p, 0, sizeof(info));
     g_err = "a device-side factorisation reported a failure (zero pivot or Jacobi sweep limit)";
@@ -96,6 +86,13 @@ int slu_sync(slu_handle_t h) {
     return SLU_ERR_NOT_CONVERGED;
   }
   return SLU_OK;
+}
+
+int slu_check_waits(slu_handle_t h) {
+  return guard(h, [&] {
+    SLU_REQUIRE(h, "null handle");
+    h->h.check_waits(true);
+  });
 }
 
 // ------------------------------------------------------------------ HBS
@@ -410,7 +407,7 @@ int slu_ulv_solve_ozaki(slu_handle_t h, slu_hbs_t op, const double* X, int ldx, 
     const size_t bytes = slu::hbs_oz_scratch_bytes(H, nrhs);
     h->h.ws.reserve(bytes + 256, h->h.stream);
     void* scratch = h->h.ws.take<char>(bytes);
-    unsigned* err = reinterpret_cast<unsigned int*>(h->h.info.as<int>()) + 1;
+    volatile unsigned* err = h->h.err_word();
     if (trans)
       slu::ulv_solve_oz_T(h->h.stream, H, X, ldx, Y, ldy, nrhs, scratch, err);
     else
@@ -430,7 +427,7 @@ int slu_hbs_apply_ozaki(slu_handle_t h, slu_hbs_t op, const double* X, int ldx, 
     h->h.ws.reserve(bytes + 256, h->h.stream);
     void* scratch = h->h.ws.take<char>(bytes);
     slu::hbs_apply_oz(h->h.stream, H, X, ldx, Y, ldy, nrhs, scratch,
-                      reinterpret_cast<unsigned int*>(h->h.info.as<int>()) + 1, nullptr, nullptr,
+                      h->h.err_word(), nullptr, nullptr,
                       trans != 0);
   });
 }
@@ -665,7 +662,7 @@ int slu_gemm_split3(slu_handle_t h, int M, int N, int K, double alpha, const dou
     h->h.ws.reserve(slu::tc_gemm_workspace_bytes(M, N, K), h->h.stream);
     void* ws = h->h.ws.take<char>(slu::tc_gemm_workspace_bytes(M, N, K) - 256);
     slu::tc_gemm_split3(h->h.stream, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, ws,
-                        reinterpret_cast<unsigned int*>(h->h.info.as<int>()) + 1);
+                        h->h.err_word());
   });
 }
 

@@ -313,7 +313,7 @@ struct CrtGemm {
   float theta;           // 2^(51 - t)
   int *wa, *wb;          // rows and columns with a sum of theta or more
   int pitch;
-  unsigned int* err;
+  volatile unsigned* err;
 };
 
 // Persistent: each CTA runs every gridDim-th (modulus, batch, tile) item.
@@ -508,14 +508,14 @@ crt_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     }
     if (!ok) {
       s_fail = 1;
-      if (lane == 0 && g.err) atomicOr(g.err, 1u);
+      if (lane == 0 && g.err) *g.err = 1;
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (threadIdx.x == 0 && s_fail) {
     // the copies already issued land before the CTA exits
-    if (g.err) atomicOr(g.err, 1u);
+    if (g.err) *g.err = 1;
     const long long issued = s_issued;
     for (long long j = issued > S ? issued - S : 0; j < issued; ++j)
       mbar_wait(&full_bar[j % S], (uint32_t)(j / S) & 1, nullptr);

@@ -69,10 +69,33 @@ struct Handle {
   Workspace lu_ws;     // permutations and triangles of lu_factor / lu_inverse
   HostStage upload, readback;
   DevBuf info;  // int[64] device status words
-  // set by a tensor-core kernel whose waits ran out (slu_sync reports it)
-  unsigned int* err_word() const { return info.as<unsigned int>() + 1; }
+  // set by a kernel whose bounded waits ran out: mapped host memory, so that
+  // every later call on the handle sees it without waiting
+  std::shared_ptr<volatile unsigned> err;
+  volatile unsigned* err_word() const { return err.get(); }
   // the same words of the solve plans launched on this handle
   std::vector<std::weak_ptr<volatile unsigned>> plan_err;
+  // Throws where a kernel of an earlier call (or, after a wait, of this one)
+  // gave up waiting: that call's results are not valid.  plans: also of the
+  // solve plans (their launches look at their own words).
+  void check_waits(bool plans = false) {
+    bool gave_up = err && *err;
+    if (gave_up) *err = 0;
+    for (size_t i = 0; plans && i < plan_err.size();) {
+      const auto p = plan_err[i].lock();
+      if (!p) {
+        plan_err.erase(plan_err.begin() + i);
+        continue;
+      }
+      gave_up = gave_up || *p;
+      *p = 0;
+      ++i;
+    }
+    if (gave_up)
+      throw Error(SLU_ERR_TIMEOUT,
+                  "a kernel gave up waiting on its copies, tensor-core products or cluster: the "
+                  "results of the call that launched it are not valid");
+  }
   std::string last_error;
 };
 
@@ -413,16 +436,16 @@ size_t hbs_oz_scratch_bytes(const Hbs& H, int c);
 // float64 (distinct buffers), scratch of hbs_oz_scratch_bytes bytes; err a
 // device word set on a device wait timeout.
 void ulv_solve_oz(cudaStream_t st, const Hbs& H, const double* X, int ldx, double* Y, int ldy,
-                  int c, void* scratch, unsigned* err);
+                  int c, void* scratch, volatile unsigned* err);
 // Y <- A^{-T} X on the tensor cores (the transposed steps of the float64
 // mode-T solve, caller ordering through the inverse permutation).
 void ulv_solve_oz_T(cudaStream_t st, const Hbs& H, const double* X, int ldx, double* Y,
-                    int ldy, int c, void* scratch, unsigned* err);
+                    int ldy, int c, void* scratch, volatile unsigned* err);
 // With resb (N x c, leading dimension ldy) the apply returns the residual
 // Y = resb - A X instead, and rnorm2 (c entries, zeroed by the caller)
 // accumulates its squared column norms.
 void hbs_apply_oz(cudaStream_t st, const Hbs& H, const double* X, int ldx, double* Y, int ldy,
-                  int c, void* scratch, unsigned* err, const double* resb = nullptr,
+                  int c, void* scratch, volatile unsigned* err, const double* resb = nullptr,
                   double* rnorm2 = nullptr, bool trans = false);
 
 // Factor pointers of one level by arithmetic type (float64 factors or their

@@ -73,6 +73,22 @@ void stream_wait(cudaStream_t st) {
   SLU_CHECK_CUDA(cudaEventSynchronize(w.ev));
 }
 
+std::shared_ptr<volatile unsigned> mapped_word() {
+  // a handle may be made while its stream is captured: the allocation is no
+  // part of that
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  SLU_CHECK_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+  void* w = nullptr;
+  const cudaError_t e = cudaHostAlloc(&w, 64, cudaHostAllocPortable | cudaHostAllocMapped);
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  SLU_CHECK_CUDA(e);
+  std::shared_ptr<volatile unsigned> p(
+      static_cast<volatile unsigned*>(w),
+      [](volatile unsigned* q) { cudaFreeHost(const_cast<unsigned*>(q)); });
+  *p = 0;
+  return p;
+}
+
 int num_sms() {
   static int n = 0;
   if (!n) {

@@ -191,7 +191,7 @@ __device__ __forceinline__ bool panel_wait(uint32_t bar, uint32_t parity) {
 __global__ void __launch_bounds__(kPanelRows)
 lu_panel_kernel(int n, int k0, int kb, double* __restrict__ A, int lda, long long sA,
                 int* __restrict__ piv, long long sP, int* __restrict__ src, int* info, int istep,
-                unsigned* err) {
+                volatile unsigned* err) {
   constexpr int KB = kPanel;
   extern __shared__ __align__(16) unsigned char s_raw[];
   cg::cluster_group cl = cg::this_cluster();
@@ -283,7 +283,7 @@ lu_panel_kernel(int n, int k0, int kb, double* __restrict__ A, int lda, long lon
     ok = panel_wait(bar, (uint32_t)(j >> 1) & 1);
     if (!__all_sync(0xffffffffu, ok)) {
       ok = false;
-      if (lane == 0 && err) *(volatile unsigned*)err = 1;
+      if (lane == 0 && err) *err = 1;
       break;
     }
     // the winner: largest entry, then the first position
@@ -368,7 +368,7 @@ constexpr int kSplitRows = 1024;
 __global__ void __launch_bounds__(512)
 lu_panel_split_kernel(int n, int k0, int kb, double* __restrict__ A, int lda, long long sA,
                       int* __restrict__ piv, long long sP, int* __restrict__ src, int* info, int istep,
-                      unsigned* err) {
+                      volatile unsigned* err) {
   constexpr int KB = kPanel, NC = KB / 4;   // columns per warp
   extern __shared__ __align__(16) unsigned char s_raw[];
   cg::cluster_group cl = cg::this_cluster();
@@ -485,7 +485,7 @@ lu_panel_split_kernel(int n, int k0, int kb, double* __restrict__ A, int lda, lo
       ok = panel_wait(bar, (uint32_t)(j >> 1) & 1);
       if (!__all_sync(0xffffffffu, ok)) {
         ok = false;
-        if (lane == 0 && err) *(volatile unsigned*)err = 1;
+        if (lane == 0 && err) *err = 1;
         continue;
       }
       // the winner: largest entry, then the first position
@@ -663,7 +663,7 @@ lu_block_trsm_kernel(int n, int k0, int nb, int c0, double* __restrict__ A, int 
 
 void launch_panel(cudaStream_t st, int n, int k0, int kb, double* A, int lda, long long sA,
                   int* piv, long long sP, int* src, int batch, int* info, int istep,
-                  unsigned* err) {
+                  volatile unsigned* err) {
   const int R = n - k0;
   // 32 rows per CTA (four warps), then up to 128, in clusters of up to eight
   // (the portable size); above 1024 rows a thread per row

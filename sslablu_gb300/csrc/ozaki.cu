@@ -94,7 +94,7 @@ struct OzStep {
   // leave scaled by 2^s_j, so every vector between steps stays near unit
   // magnitude, inside the float32 exponent range, whatever the float64 scale
   const unsigned* colbits;
-  unsigned* err;           // device error word (timeouts)
+  volatile unsigned* err;           // device error word (timeouts)
   // residual form of the float64 output (the refinement's last apply step):
   // with resb set, the caller's rows receive resb - (S z) instead of S z
   // (resb in the output's layout and leading dimension), and rnorm2[j]
@@ -509,7 +509,7 @@ __global__ void __launch_bounds__(kThreads, 1) oz_step_kernel(const OzStep o) {
       }
       if (fail) {
         s_fail = 1;
-        if (o.err) atomicOr(o.err, 1u);
+        if (o.err) *o.err = 1;
         __threadfence_block();
         // the last operator copy must land before the CTA exits
         mbar_wait(&op_full, (uint32_t)((nload - 1) & 1));
@@ -563,7 +563,7 @@ __global__ void __launch_bounds__(kThreads, 1) oz_step_kernel(const OzStep o) {
         if (lane == 0) {
           e_fail = 1;
           s_fail = 1;
-          if (o.err) atomicOr(o.err, 1u);
+          if (o.err) *o.err = 1;
         }
         continue;
       }
@@ -804,7 +804,7 @@ __global__ void __launch_bounds__(kThreads, 1) oz_step_kernel(const OzStep o) {
     sweep::launch_dependents();
     if (fail) {
       s_fail = 1;
-      if (o.err) atomicOr(o.err, 1u);
+      if (o.err) *o.err = 1;
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -904,7 +904,7 @@ void make_op(cudaStream_t st, OzOp& o, const double* S, int Nb, int rows, int w)
 }
 
 void launch(cudaStream_t st, const sweep::Step<dfloat>& s, const OzOp& op, bool in_f64,
-            bool out_f64, const unsigned* colbits, unsigned* err, const char* what,
+            bool out_f64, const unsigned* colbits, volatile unsigned* err, const char* what,
             const double* resb = nullptr, double* rnorm2 = nullptr) {
   SLU_REQUIRE(op.dig.p && s.rows == op.rows && s.w == op.w && s.nb == op.Nb,
               "tensor-core sweep: digit operator does not match its step");
@@ -993,7 +993,7 @@ dfloat* oz_vectors(void* scratch, int c) {
 }  // namespace
 
 void ulv_solve_oz(cudaStream_t st, const Hbs& H, const double* X, int ldx, double* Y, int ldy,
-                  int c, void* scratch, unsigned* err) {
+                  int c, void* scratch, volatile unsigned* err) {
   SLU_REQUIRE(H.has_oz, "tensor-core sweep not prepared");
   SLU_REQUIRE(static_cast<const void*>(X) != static_cast<const void*>(Y),
               "tensor-core sweep: input and output must be different buffers");
@@ -1045,7 +1045,7 @@ void ulv_solve_oz(cudaStream_t st, const Hbs& H, const double* X, int ldx, doubl
 // through the inverse permutation), the root^T step, forward^T steps down
 // (Q itself), the result scattered through the inverse permutation.
 void ulv_solve_oz_T(cudaStream_t st, const Hbs& H, const double* X, int ldx, double* Y,
-                    int ldy, int c, void* scratch, unsigned* err) {
+                    int ldy, int c, void* scratch, volatile unsigned* err) {
   SLU_REQUIRE(H.has_ozT, "tensor-core transposed sweep not prepared");
   SLU_REQUIRE(static_cast<const void*>(X) != static_cast<const void*>(Y),
               "tensor-core sweep: input and output must be different buffers");
@@ -1084,7 +1084,7 @@ void ulv_solve_oz_T(cudaStream_t st, const Hbs& H, const double* X, int ldx, dou
 }
 
 void hbs_apply_oz(cudaStream_t st, const Hbs& H, const double* X, int ldx, double* Y, int ldy,
-                  int c, void* scratch, unsigned* err, const double* resb, double* rnorm2,
+                  int c, void* scratch, volatile unsigned* err, const double* resb, double* rnorm2,
                   bool trans) {
   SLU_REQUIRE(trans ? H.has_ozT : H.has_oz, "tensor-core apply not prepared");
   SLU_REQUIRE(static_cast<const void*>(X) != static_cast<const void*>(Y),

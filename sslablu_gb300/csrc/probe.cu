@@ -30,9 +30,37 @@ __global__ void __launch_bounds__(256) fp64_fma_kernel(int iters, double a, doub
   if (s > 1e300) sink[blockIdx.x] = s;
 }
 
+// One thread waits for an mbarrier on which nobody arrives, `polls` times.
+__global__ void wait_probe_kernel(int polls, volatile unsigned* err) {
+  __shared__ __align__(8) unsigned long long bar;
+  const uint32_t addr = static_cast<uint32_t>(__cvta_generic_to_shared(&bar));
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(addr) : "memory");
+  for (int i = 0; i < polls; ++i) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], 0;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(addr)
+        : "memory");
+    if (done) return;
+  }
+  *err = 1;
+}
+
 }  // namespace
 
 extern "C" {
+
+int slu_wait_probe(slu_handle_t h, int polls) {
+  return slu::guard_call(h, [&] {
+    SLU_REQUIRE(h, "null argument");
+    SLU_REQUIRE(polls >= 1 && polls <= (1 << 20), "polls out of range");
+    wait_probe_kernel<<<1, 1, 0, h->h.stream>>>(polls, h->h.err_word());
+    slu::check_launch("wait_probe_kernel");
+  });
+}
 
 int slu_fp64_peak(slu_handle_t h, int iters, double* tflops_out, double* ms_out) {
   return slu::guard_call(h, [&] {

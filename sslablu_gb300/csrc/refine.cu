@@ -63,7 +63,7 @@ void enqueue_iteration(cudaStream_t st, const Hbs& H, RefinePlan& P, bool first,
   if (P.inner == 2) {
     // tensor-core sweep and residual (ozaki.cu): the first solve writes X in
     // float64 directly; corrections come back as double-float pairs
-    unsigned* err = P.ozerr.as<unsigned>();
+    volatile unsigned* err = P.ozerr.as<unsigned>();
     double* d = P.d.as<double>();
     if (first) {
       ulv_solve_oz(st, H, rhs, c, X, c, c, P.solve_ws.p, err);

@@ -203,7 +203,7 @@ void copy_blocks(cudaStream_t st, int nblk, long long width, const void* src, lo
 size_t tc_gemm_workspace_bytes(int M, int N, int K);
 void tc_gemm_split3(cudaStream_t st, int M, int N, int K, double alpha, const double* A, int lda,
                     const double* B, int ldb, double beta, double* C, int ldc, void* ws,
-                    unsigned int* err);
+                    volatile unsigned* err);
 
 int num_sms();
 
@@ -220,6 +220,8 @@ void ensure_smem(const void* kernel, size_t bytes);
 // instead, so many worker threads waiting at once leave the host cores to
 // the threads that are launching work.
 void stream_wait(cudaStream_t st);
+// A word of mapped host memory, zero (one address on host and device).
+std::shared_ptr<volatile unsigned> mapped_word();
 void set_blocking_waits(bool on);
 
 }  // namespace slu

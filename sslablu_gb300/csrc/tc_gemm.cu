@@ -183,7 +183,7 @@ template <int BN>
 __global__ void __maxnreg__(168)
 tc_gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     int M, int N, int Kp, double alpha, double beta, double* __restrict__ C,
-                    int ldc, unsigned int* __restrict__ err) {
+                    int ldc, volatile unsigned* err) {
   using G = TcCfg<BN>;
   constexpr int STAGES = G::kStages;
   extern __shared__ unsigned char smem_raw[];
@@ -389,7 +389,7 @@ tc_gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         : "r"((uint32_t)fail), "r"(32 * kEpiWarps)
         : "memory");
     if (any_fail) {
-      if (lane == 0 && err) atomicOr(err, 1u);
+      if (lane == 0 && err) *err = 1;
     } else {
       // every MMA has completed (the last chunk's commit), so the operand
       // ring is free: the sums are staged there (odd pitch: no bank
@@ -529,7 +529,7 @@ CUtensorMap make_map(const void* base, int rows, long long cols, int box_rows) {
 
 template <int BN>
 void launch_tc(cudaStream_t st, const __nv_bfloat16* Asl, const __nv_bfloat16* Bsl, int M, int N,
-               int Kp, double alpha, double beta, double* C, int ldc, unsigned int* err) {
+               int Kp, double alpha, double beta, double* C, int ldc, volatile unsigned* err) {
   using G = TcCfg<BN>;
   CUtensorMap ma = make_map(Asl, M, 3LL * Kp, BM);
   CUtensorMap mb = make_map(Bsl, N, 3LL * Kp, BN);
@@ -552,7 +552,7 @@ size_t tc_gemm_workspace_bytes(int M, int N, int K) {
 // ws: tc_gemm_workspace_bytes(M, N, K) bytes; err: device word set on a wait timeout.
 void tc_gemm_split3(cudaStream_t st, int M, int N, int K, double alpha, const double* A, int lda,
                     const double* B, int ldb, double beta, double* C, int ldc, void* ws,
-                    unsigned int* err) {
+                    volatile unsigned* err) {
   if (M <= 0 || N <= 0) return;
   SLU_REQUIRE(K >= 1, "K must be positive");
   const int Kp = (K + BK - 1) / BK * BK;

@@ -256,7 +256,7 @@ void rb_factor(Handle& h, RbSolver& S, int nblk, int m, const double* SiM, const
                   (int)m2, 2 * mm, nR);
     } else {
       // Schur products on the tensor cores (split-BF16x3, float32 accumulation)
-      unsigned int* err = reinterpret_cast<unsigned int*>(h.info.as<int>()) + 1;
+      volatile unsigned* err = h.err_word();
       for (int j = 1; j < nR; ++j)
         tc_gemm_split3(st, m, (int)m2, m, 1.0, dp(P.SiM) + 2 * j * mm, m, X + 2 * (j - 1) * mm,
                        (int)m2, 0.0, G1 + 2 * j * mm, (int)m2, tcws.p, err);
@@ -313,7 +313,7 @@ void rb_solve(Handle& h, const RbSolver& S, double* B, int ldb, int c, bool tc) 
   for (int l = 0; l < nL; ++l) v[l] = h.ws.take<double>((size_t)S.levels[l].nS * mc);
   double* z = h.ws.take<double>(std::max<size_t>(1, (size_t)nblk / 2) * mc);
   void* tcws = tc ? h.ws.take<char>(tcb) : nullptr;
-  unsigned int* err = reinterpret_cast<unsigned int*>(h.info.as<int>()) + 1;
+  volatile unsigned* err = h.err_word();
   // C_b = alpha A_b V_b + beta C_b for b < batch (A_b m x m, V_b and C_b m x c):
   // float64 batched GEMM, or with `tc` split-BF16x3 tensor-core products
   auto G = [&](double alpha, const double* A, long long sA, const double* V, long long sV,
@@ -435,6 +435,7 @@ void rb_refine(Handle& h, const RbSolver& S, const double* B, int ldb, double* X
     check_launch("colnorm2_rb");
     SLU_CHECK_CUDA(cudaMemcpyAsync(hr.data(), rn, 8 * c, cudaMemcpyDeviceToHost, st));
     stream_wait(st);
+    h.check_waits();
     worst = 0.0;
     for (int j = 0; j < c; ++j)
       worst = std::max(worst, std::sqrt(hr[j]) / (hb[j] > 0 ? std::sqrt(hb[j]) : 1.0));

@@ -176,14 +176,7 @@ void solve_plan_create(Handle& h, Hbs& H, const double* X, int ldx, double* Y, i
   }
   // the path of a solve call of this shape (residue steps for many columns)
   const bool crt = crt_prepare(h, H, true, trans, c);
-  if (crt) {
-    void* w = nullptr;
-    SLU_CHECK_CUDA(cudaHostAlloc(&w, 64, cudaHostAllocPortable | cudaHostAllocMapped));
-    P.err = std::shared_ptr<volatile unsigned>(
-        static_cast<volatile unsigned*>(w),
-        [](volatile unsigned* p) { cudaFreeHost(const_cast<unsigned*>(p)); });
-    *P.err = 0;
-  }
+  if (crt) P.err = mapped_word();
   for (size_t i = 0; i < steps.size(); ++i)
     sweep::prepare_step(steps[i].s, kn ? (*kn)[i] : PlanKnobs());
   stream_wait(st);   // the scratch exists before the capture

@@ -354,6 +354,7 @@ class HBSMAT:
             L.check(L.lib().slu_ulv_solve_into(L.handle(), self._op, L.ptr(b), c, L.ptr(out), c,
                                                c, int(mode == "T")))
             torch.cuda.current_stream().synchronize()
+            L.check_waits()
             return out
         if (isinstance(b, torch.Tensor) and b.is_cuda and b.dtype == torch.float64
                 and b.dim() == 2 and b.get_device() == L.device()):

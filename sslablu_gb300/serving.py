@@ -52,6 +52,8 @@ import time
 import numpy as np
 import torch
 
+from . import _lib as L
+
 
 class Request:
     __slots__ = ("key", "B", "t_arrival", "t_start", "t_done", "X", "rid", "error")
@@ -260,6 +262,7 @@ class SolveServer:
             Xh = self._staging(stage, "out", N * cols).view(N, cols)
             Xh.copy_(Xd, non_blocking=True)
             stream.synchronize()
+            L.check_waits()
         return [Xh.numpy()]
 
     def _solve_group(self, job, stream, stage):
@@ -279,6 +282,7 @@ class SolveServer:
             Xh = self._staging(stage, "out", off)
             Xh.copy_(Xd, non_blocking=True)
             stream.synchronize()
+            L.check_waits()
         flat = Xh.numpy()
         return [flat[o:o + n * c].reshape(n, c) for o, n, c in layout]
 
