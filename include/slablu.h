@@ -119,6 +119,30 @@ int slu_ulv_factor(slu_handle_t h, slu_hbs_t op);
 int slu_hbs_apply(slu_handle_t h, slu_hbs_t op, int trans, const double* X, int ldx, double* Y,
                   int ldy, int nrhs);
 
+/* slu_hbs_apply, slu_ulv_solve_into and slu_ulv_solve_plan_create for many
+ * right-hand sides: where the operator's shape and nrhs > 32 make it the faster
+ * way (slu_hbs_wide_steps tells), every tree step runs on the tensor cores as an
+ * exact product of its operands rounded to integers of 58 or 59 bits below the
+ * largest entry of their row (step operator) or column (vectors, per block).
+ * An output's error is at most w 2^-54 of the largest |S| |z| in its block's
+ * column (w <= 128 the step's depth; the operator's rows and columns may be
+ * scaled in any way), and 2^-26 of its own; a column of the result does not
+ * depend on the others, but differs from the float64 steps' by rounding.  Other
+ * shapes run the float64 steps, with their bits.  The first call of a direction
+ * (solve or apply, trans) makes images of the step operators, four times their
+ * size (at most 16 GiB; the float64 steps where they cannot be had), kept until the operator changes; inside a stream capture a call
+ * that would have to make them runs the float64 steps.  Beyond upstream. */
+int slu_hbs_apply_wide(slu_handle_t h, slu_hbs_t op, int trans, const double* X, int ldx,
+                       double* Y, int ldy, int nrhs);
+int slu_ulv_solve_wide(slu_handle_t h, slu_hbs_t op, const double* X, int ldx, double* Y,
+                       int ldy, int nrhs, int trans);
+int slu_ulv_solve_wide_plan_create(slu_handle_t h, slu_hbs_t op, const double* X, int ldx,
+                                   double* Y, int ldy, int nrhs, int trans,
+                                   slu_solve_plan_t* out);
+/* *out = 1 where the calls above take the residue steps for a solve (solve = 1)
+ * or an apply of nrhs columns, else 0. */
+int slu_hbs_wide_steps(slu_hbs_t op, int solve, int trans, int nrhs, int* out);
+
 /* Replaces HBSMAT.solve (HBSnew.py:393-416) -> ULVsparse.solve
  * (ULVsparse.py:295-358), in place on B (N x nrhs, unpermuted ordering).
  * trans = 1 reproduces upstream's mode 'T' handling of the permutation. */
@@ -353,7 +377,15 @@ int slu_lu_factor(slu_handle_t h, int n, double* A, int lda, long long sA, int* 
  * X_b n x nrhs (ldx, stride sX).  Replaces scipy.linalg.lu_solve. */
 int slu_lu_solve(slu_handle_t h, int trans, int n, const double* LU, int lda, long long sA,
                  const int* piv, long long sP, double* X, int ldx, long long sX, int nrhs, int nb);
-/* C_b = alpha op(A_b) op(B_b) + beta C_b, strided batch (row-major). */
+/* C_b = alpha op(A_b) op(B_b) + beta C_b, strided batch (row-major).  From
+ * M, N >= 32, K >= 64 and 2 M N K nb >= 2e7 as exact products on the tensor cores
+ * of the operands rounded to 55 bits or more below the largest entry a_i of their
+ * row of op(A) (b_j of their column of op(B)): with s = |op(A)| |op(B)|, the error
+ * of output (i, j) is at most 4 K 2^-53 times the largest s(i', j') (a_i b_j) /
+ * (a_i' b_j') over its row and over its column.  Outputs for which that could not
+ * be had (operands whose scales oppose along k) or whose own s is below
+ * 2^-44 a_i b_j are float64 dot products, as are rows and columns that are not
+ * finite. */
 int slu_gemm_batched(slu_handle_t h, int transa, int transb, int M, int N, int K, double alpha,
                      const double* A, int lda, long long sA, const double* B, int ldb,
                      long long sB, double beta, double* C, int ldc, long long sC, int nb);

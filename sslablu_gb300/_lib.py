@@ -36,6 +36,11 @@ SIGNATURES = {
     "slu_ulv_factor": [P, P],
     "slu_hbs_set_ulv_level": [P, P, c_int, P, P, P, P],
     "slu_hbs_apply": [P, P, c_int, P, c_int, P, c_int, c_int],
+    "slu_hbs_apply_wide": [P, P, c_int, P, c_int, P, c_int, c_int],
+    "slu_ulv_solve_wide": [P, P, P, c_int, P, c_int, c_int, c_int],
+    "slu_ulv_solve_wide_plan_create": [P, P, P, c_int, P, c_int, c_int, c_int,
+                                       ctypes.POINTER(c_void_p)],
+    "slu_hbs_wide_steps": [P, c_int, c_int, c_int, ctypes.POINTER(c_int)],
     "slu_ulv_solve": [P, P, P, c_int, c_int, c_int],
     "slu_ulv_solve_noalloc": [P, P, P, c_int, c_int, c_int],
     "slu_hbs_prepare_f32": [P, P],

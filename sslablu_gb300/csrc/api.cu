@@ -265,6 +265,24 @@ int slu_hbs_apply(slu_handle_t h, slu_hbs_t op, int trans, const double* X, int 
   });
 }
 
+int slu_hbs_apply_wide(slu_handle_t h, slu_hbs_t op, int trans, const double* X, int ldx,
+                       double* Y, int ldy, int nrhs) {
+  return guard(h, [&] {
+    SLU_REQUIRE(h && op && X && Y, "null argument");
+    SLU_REQUIRE(nrhs >= 1 && ldx >= nrhs && ldy >= nrhs, "bad right-hand side shape");
+    slu::Hbs& H = op->H;
+    SLU_REQUIRE(H.has_mats, "HBS factors not loaded");
+    if (!slu::crt_prepare(h->h, H, false, trans != 0, nrhs)) {
+      slu::hbs_apply(h->h, H, trans != 0, X, ldx, Y, ldy, nrhs);
+      return;
+    }
+    const size_t elems = slu::hbs_apply_scratch_elems(H, nrhs);
+    h->h.ws.reserve(8 * elems + 256, h->h.stream);
+    slu::crt_apply(h->h.stream, H, trans != 0, X, ldx, Y, ldy, nrhs, h->h.ws.take<double>(elems),
+                   h->h.err_word());
+  });
+}
+
 int slu_ulv_solve(slu_handle_t h, slu_hbs_t op, double* B, int ldb, int nrhs, int trans) {
   return guard(h, [&] {
     SLU_REQUIRE(h && op && B, "null argument");
@@ -273,15 +291,16 @@ int slu_ulv_solve(slu_handle_t h, slu_hbs_t op, double* B, int ldb, int nrhs, in
   });
 }
 
-int slu_ulv_solve_into(slu_handle_t h, slu_hbs_t op, const double* X, int ldx, double* Y,
-                       int ldy, int nrhs, int trans) {
+namespace {
+int solve_into(slu_handle_t h, slu_hbs_t op, const double* X, int ldx, double* Y, int ldy,
+               int nrhs, int trans, bool wide) {
   return guard(h, [&] {
     SLU_REQUIRE(h && op && X && Y, "null argument");
     SLU_REQUIRE(nrhs >= 1 && ldx >= nrhs && ldy >= nrhs, "bad right-hand side shape");
     slu::Hbs& H = op->H;
     SLU_REQUIRE(H.has_ulv, "HBS operator has no ULV factorisation");
     cudaStream_t st = h->h.stream;
-    const bool crt = slu::crt_prepare(h->h, H, true, trans != 0, nrhs);
+    const bool crt = wide && slu::crt_prepare(h->h, H, true, trans != 0, nrhs);
     const size_t bytes = slu::hbs_solve_scratch_bytes(H, nrhs, sizeof(double));
     h->h.ws.reserve(bytes + 256, st);
     double* scratch = h->h.ws.take<double>(bytes / sizeof(double));
@@ -293,15 +312,46 @@ int slu_ulv_solve_into(slu_handle_t h, slu_hbs_t op, const double* X, int ldx, d
   });
 }
 
-int slu_ulv_solve_plan_create(slu_handle_t h, slu_hbs_t op, const double* X, int ldx, double* Y,
-                              int ldy, int nrhs, int trans, slu_solve_plan_t* out) {
+int plan_create(slu_handle_t h, slu_hbs_t op, const double* X, int ldx, double* Y, int ldy,
+                int nrhs, int trans, bool wide, slu_solve_plan_t* out) {
   return guard(h, [&] {
     SLU_REQUIRE(h && op && X && Y && out, "null argument");
     SLU_REQUIRE(nrhs >= 1 && ldx >= nrhs && ldy >= nrhs, "bad right-hand side shape");
     SLU_REQUIRE(op->H.has_ulv, "HBS operator has no ULV factorisation");
     auto p = std::make_unique<slu_solve_plan_s>();
-    slu::solve_plan_create(h->h, op->H, X, ldx, Y, ldy, nrhs, trans != 0, p->P);
+    slu::solve_plan_create(h->h, op->H, X, ldx, Y, ldy, nrhs, trans != 0, wide, p->P);
     *out = p.release();
+  });
+}
+}  // namespace
+
+int slu_ulv_solve_into(slu_handle_t h, slu_hbs_t op, const double* X, int ldx, double* Y,
+                       int ldy, int nrhs, int trans) {
+  return solve_into(h, op, X, ldx, Y, ldy, nrhs, trans, false);
+}
+
+int slu_ulv_solve_wide(slu_handle_t h, slu_hbs_t op, const double* X, int ldx, double* Y,
+                       int ldy, int nrhs, int trans) {
+  return solve_into(h, op, X, ldx, Y, ldy, nrhs, trans, true);
+}
+
+int slu_ulv_solve_plan_create(slu_handle_t h, slu_hbs_t op, const double* X, int ldx, double* Y,
+                              int ldy, int nrhs, int trans, slu_solve_plan_t* out) {
+  return plan_create(h, op, X, ldx, Y, ldy, nrhs, trans, false, out);
+}
+
+int slu_ulv_solve_wide_plan_create(slu_handle_t h, slu_hbs_t op, const double* X, int ldx,
+                                   double* Y, int ldy, int nrhs, int trans,
+                                   slu_solve_plan_t* out) {
+  return plan_create(h, op, X, ldx, Y, ldy, nrhs, trans, true, out);
+}
+
+int slu_hbs_wide_steps(slu_hbs_t op, int solve, int trans, int nrhs, int* out) {
+  return guard(nullptr, [&] {
+    SLU_REQUIRE(op && out, "null argument");
+    SLU_REQUIRE(nrhs >= 1, "bad right-hand side shape");
+    SLU_REQUIRE(solve ? op->H.has_ulv : op->H.has_mats, "HBS factors not loaded");
+    *out = slu::crt_steps_pay(op->H, solve != 0, trans != 0, nrhs) ? 1 : 0;
   });
 }
 

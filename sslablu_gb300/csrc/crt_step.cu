@@ -889,8 +889,8 @@ bool ready(Handle& h, Hbs& H, bool solve, bool trans) {
 // us, 48: 206 -> 124, 64: 255 -> 126, 300: 1306 -> 292; of 1024 rows with 64
 // columns 79 -> 72 (left to float64), 128: 128 -> 79; with leaves of 16 the
 // float64 steps stay ahead (4096 rows, 300 columns: 297 against 607).
-// Up to 32 columns float64 has the solves that groups and single calls share
-// bit for bit.  One level may be solved in place, which wants whole columns
+// Up to 32 columns a call's bits are those of the float64 steps, which groups and
+// single calls share.  One level may be solved in place, which wants whole columns
 // per CTA.
 bool crt_steps_pay(const Hbs& H, bool solve, bool trans, int c) {
   if (c <= 32 || H.L < 2) return false;

@@ -440,16 +440,11 @@ void hbs_apply(Handle& h, Hbs& H, bool trans, const double* X, int ldx, double* 
                int ldy, int c) {
   cudaStream_t st = h.stream;
   SLU_REQUIRE(H.has_mats, "HBS factors not loaded");
-  const size_t elems = hbs_apply_scratch_elems(H, c);
-  if (crt_prepare(h, H, false, trans, c)) {
-    h.ws.reserve(8 * elems + 256, st);
-    crt_apply(st, H, trans, X, ldx, Yout, ldy, c, h.ws.take<double>(elems), h.err_word());
-    return;
-  }
   if (!H.has_apply[trans ? 1 : 0]) {
     std::lock_guard<std::mutex> lock(H.lazy_mu);
     if (!H.has_apply[trans ? 1 : 0]) hbs_make_apply(h, H, trans);
   }
+  const size_t elems = hbs_apply_scratch_elems(H, c);
   h.ws.reserve(8 * elems + 256, st);
   double* scratch = h.ws.take<double>(elems);
   hbs_apply_fused<double>(st, H, trans, X, ldx, Yout, ldy, c, scratch);
@@ -461,21 +456,9 @@ size_t hbs_solve_scratch_bytes(const Hbs& H, int c, size_t elem) {
 }
 
 template <typename T>
-void hbs_solve(Handle& h, Hbs& H, bool trans, T* B, int ldb, int c) {
-  bool crt = false;
-  if constexpr (sizeof(T) == 8) {
-    SLU_REQUIRE(H.has_ulv, "HBS operator has no ULV factorisation");
-    crt = crt_prepare(h, H, true, trans, c);
-  }
+void hbs_solve(Handle& h, const Hbs& H, bool trans, T* B, int ldb, int c) {
   h.ws.reserve(hbs_solve_scratch_bytes(H, c, sizeof(T)) + 256, h.stream);
   T* scratch = h.ws.take<T>(hbs_solve_scratch_bytes(H, c, sizeof(T)) / sizeof(T));
-  if constexpr (sizeof(T) == 8) {
-    if (crt) {
-      crt_solve(h.stream, H, trans, B, ldb, B, ldb, c, scratch,
-                ((sizeof(T) * (size_t)H.N * c + 255) & ~size_t(255)) / sizeof(T), h.err_word());
-      return;
-    }
-  }
   hbs_solve_scratch<T>(h.stream, H, trans, B, ldb, c, scratch);
 }
 
@@ -495,8 +478,8 @@ void hbs_solve_scratch(cudaStream_t st, const Hbs& H, bool trans, T* B, int ldb,
     ulv_solve_T<T>(st, H, B, ldb, c, scratch, stride);
   }
 }
-template void hbs_solve<double>(Handle&, Hbs&, bool, double*, int, int);
-template void hbs_solve<float>(Handle&, Hbs&, bool, float*, int, int);
+template void hbs_solve<double>(Handle&, const Hbs&, bool, double*, int, int);
+template void hbs_solve<float>(Handle&, const Hbs&, bool, float*, int, int);
 template void hbs_solve_scratch<double>(cudaStream_t, const Hbs&, bool, double*, int, int, double*);
 template void hbs_solve_scratch<float>(cudaStream_t, const Hbs&, bool, float*, int, int, float*);
 

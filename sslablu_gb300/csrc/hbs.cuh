@@ -273,8 +273,9 @@ struct SolvePlan {
     if (exec) cudaGraphExecDestroy(exec);
   }
 };
+// wide: by the residue steps where crt_steps_pay
 void solve_plan_create(Handle& h, Hbs& H, const double* X, int ldx, double* Y, int ldy,
-                       int c, bool trans, SolvePlan& P);
+                       int c, bool trans, bool wide, SolvePlan& P);
 void solve_plan_launch(Handle& h, SolvePlan& P, bool wait);
 // The grouped mode-N solve of hbs_solve_grouped (B[i] <- A_i^{-1} B[i]) for
 // fixed blocks, captured once: step tables built and uploaded at creation.
@@ -316,7 +317,7 @@ void hbs_apply(Handle& h, Hbs& H, bool trans, const double* X, int ldx, double* 
                int ldy, int nrhs);
 // ULV solve, reference semantics of HBSMAT.solve (with the permutation)
 template <typename T>
-void hbs_solve(Handle& h, Hbs& H, bool trans, T* B, int ldb, int nrhs);
+void hbs_solve(Handle& h, const Hbs& H, bool trans, T* B, int ldb, int nrhs);
 // The same solve with caller-provided scratch of hbs_solve_scratch_bytes()
 // bytes (256-byte aligned); it makes no allocation of its own.
 template <typename T>
@@ -413,10 +414,10 @@ void apply_wy(Handle& h, int m, int k, double* W, double* W2, int ldw, long long
 
 // ---------------------------------------------------------------- tensor-core sweep
 // (crt_step.cu) Solves and applies of many right-hand sides as exact residue
-// products, float64 in and out.  crt_steps_pay: by the operator's shape and c
-// alone, so every entry point takes the same path for them.  crt_prepare also
-// makes the residue images on first use (false inside a stream capture that
-// would need it: take the float64 steps).
+// products, float64 in and out, for the entry points whose name says `wide`.
+// crt_steps_pay: by the operator's shape and c alone.  crt_prepare also makes the
+// residue images on first use (false inside a stream capture that would need it,
+// and where they don't fit: take the float64 steps).
 bool crt_steps_pay(const Hbs& H, bool solve, bool trans, int c);
 bool crt_prepare(Handle& h, Hbs& H, bool solve, bool trans, int c);
 void crt_solve(cudaStream_t st, const Hbs& H, bool trans, const double* X, int ldx, double* B,

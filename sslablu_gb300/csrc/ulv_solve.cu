@@ -158,7 +158,7 @@ void ulv_solve_fused(cudaStream_t st, const Hbs& H, T* B, int ldb, int c, T* scr
 }
 
 void solve_plan_create(Handle& h, Hbs& H, const double* X, int ldx, double* Y, int ldy,
-                       int c, bool trans, SolvePlan& P) {
+                       int c, bool trans, bool wide, SolvePlan& P) {
   SLU_REQUIRE(H.has_sweep, "step operators not composed");
   cudaStream_t st = h.stream;
   const size_t stride = ((8 * (size_t)H.N * c + 255) & ~size_t(255)) / 8;
@@ -174,8 +174,7 @@ void solve_plan_create(Handle& h, Hbs& H, const double* X, int ldx, double* Y, i
     auto it = H.tuned.find({type_code<double>(), c});
     if (it != H.tuned.end() && it->second.size() == steps.size()) kn = &it->second;
   }
-  // the path of a solve call of this shape (residue steps for many columns)
-  const bool crt = crt_prepare(h, H, true, trans, c);
+  const bool crt = wide && crt_prepare(h, H, true, trans, c);
   if (crt) P.err = mapped_word();
   for (size_t i = 0; i < steps.size(); ++i)
     sweep::prepare_step(steps[i].s, kn ? (*kn)[i] : PlanKnobs());

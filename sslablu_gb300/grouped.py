@@ -5,8 +5,9 @@ matAssembly/HBS/HBSnew.py:393-416); a batch of slab systems calls it once
 per operator.  ``solve_grouped`` hands the whole batch to the library, which
 runs one kernel launch per tree step for every member together
 (``slu_ulv_solve_grouped`` / ``slu_refine_grouped``).  Each member's result is
-the result of its own ``HBSMAT.solve`` (float64) or ``HBSMAT.solve_refined``
-(mixed precision).
+the result of its own ``HBSMAT.solve`` (float64; bit for bit up to 32 columns,
+beyond to the rounding of that call's tensor-core steps) or
+``HBSMAT.solve_refined`` (mixed precision).
 """
 import ctypes
 

@@ -295,20 +295,24 @@ class HBSMAT:
         return out.value
 
     # ------------------------------------------------------------ apply / solve
-    def _dev_apply(self, X, trans=False):
+    # The calls of the class may run many columns on the tensor cores (the
+    # library's `wide` entry points); wide=False keeps the float64 steps, whose
+    # bits don't depend on the number of columns.
+    def _dev_apply(self, X, trans=False, wide=True):
         X = dv.as_2d(X).contiguous()
         Y = torch.empty_like(X)
-        L.check(L.lib().slu_hbs_apply(L.handle(), self._op, int(trans), L.ptr(X), X.shape[1],
-                                      L.ptr(Y), Y.shape[1], X.shape[1]))
+        f = L.lib().slu_hbs_apply_wide if wide else L.lib().slu_hbs_apply
+        L.check(f(L.handle(), self._op, int(trans), L.ptr(X), X.shape[1], L.ptr(Y), Y.shape[1],
+                  X.shape[1]))
         return Y
 
-    def _dev_solve(self, X, trans=False):
+    def _dev_solve(self, X, trans=False, wide=True):
         # out of place: no copy of the right-hand sides
         X = dv.as_2d(X).contiguous()
         Y = torch.empty_like(X)
         c = X.shape[1]
-        st = L.lib().slu_ulv_solve_into(L.handle(), self._op, X.data_ptr(), c, Y.data_ptr(), c, c,
-                                        1 if trans else 0)
+        f = L.lib().slu_ulv_solve_wide if wide else L.lib().slu_ulv_solve_into
+        st = f(L.handle(), self._op, X.data_ptr(), c, Y.data_ptr(), c, c, 1 if trans else 0)
         if st:
             L.check(st)
         return Y
@@ -351,7 +355,7 @@ class HBSMAT:
             if out.shape != b.shape or not out.is_pinned() or not out.is_contiguous():
                 raise ValueError("out must be a contiguous pinned host tensor of b's shape")
             c = b.shape[1]
-            L.check(L.lib().slu_ulv_solve_into(L.handle(), self._op, L.ptr(b), c, L.ptr(out), c,
+            L.check(L.lib().slu_ulv_solve_wide(L.handle(), self._op, L.ptr(b), c, L.ptr(out), c,
                                                c, int(mode == "T")))
             torch.cuda.current_stream().synchronize()
             L.check_waits()
@@ -395,7 +399,8 @@ class HBSMAT:
     def autotune(self, nrhs, precision="f64", reps=9):
         """Times the launches of a mode-N solve of `nrhs` columns under a set
         of launch-plan caps and keeps the fastest per launch for later solves
-        of that width (results unchanged).  precision 'f64' (solve) or
+        of that width (results unchanged; the tensor-core steps that solve()
+        takes for many columns have no such caps).  precision 'f64' (solve) or
         'dfloat' (solve_dfloat).  Returns the caps chosen per launch as
         (target CTAs per SM, row-slice floor, column cap) triples."""
         code = {"f64": 0, "dfloat": 2}[precision]
@@ -474,8 +479,8 @@ class SolvePlan:
         self._host = host
         self._launch = L.lib().slu_ulv_solve_plan_launch
         p = ctypes.c_void_p()
-        L.check(L.lib().slu_ulv_solve_plan_create(L.handle(), H._op, L.ptr(b), c, L.ptr(out), c,
-                                                  c, int(trans), ctypes.byref(p)))
+        L.check(L.lib().slu_ulv_solve_wide_plan_create(L.handle(), H._op, L.ptr(b), c, L.ptr(out),
+                                                       c, c, int(trans), ctypes.byref(p)))
         self._p = p
 
     def __call__(self):

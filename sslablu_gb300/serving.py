@@ -88,7 +88,7 @@ def hbs_solver(H, precision="f64", tol=1e-10, maxit=10):
     refines the tensor-core sweep (it pays from a few hundred columns per
     batch); 'mixed' the double-float sweep."""
     if precision == "f64":
-        return lambda X: H._dev_solve(X, False)
+        return lambda X: H._dev_solve(X, False, wide=False)   # the bits of a request alone
     inner = "tensor" if precision == "tensor" else "dfloat"
 
     def mixed(X):
