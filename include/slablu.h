@@ -60,6 +60,12 @@ int slu_last_error(char* buf, size_t len);
 /* stream: a cudaStream_t (NULL = legacy default stream). */
 int slu_create(void* stream, slu_handle_t* out);
 int slu_destroy(slu_handle_t h);
+/* A handle keeps its scratch between calls: what solves, applies and compressions
+ * of the largest size so far needed, and up to about 0.5 GB each for dense products
+ * and for LU factors (more for a single matrix that needs it).  slu_trim gives it
+ * back (stream-ordered; no captured graph that holds it may run afterwards); the
+ * next call that needs some allocates it anew. */
+int slu_trim(slu_handle_t h);
 int slu_set_stream(slu_handle_t h, void* stream);
 /* Synchronises the handle's stream and reports device-side status words
  * (e.g. a Jacobi SVD that did not converge) as SLU_ERR_NOT_CONVERGED. */
@@ -130,8 +136,11 @@ int slu_hbs_apply(slu_handle_t h, slu_hbs_t op, int trans, const double* X, int 
  * depend on the others, but differs from the float64 steps' by rounding.  Other
  * shapes run the float64 steps, with their bits.  The first call of a direction
  * (solve or apply, trans) makes images of the step operators, four times their
- * size (at most 16 GiB; the float64 steps where they cannot be had), kept until the operator changes; inside a stream capture a call
- * that would have to make them runs the float64 steps.  Beyond upstream. */
+ * size (slu_hbs_nbytes counts them), kept until the operator changes; where they
+ * are above slu_hbs_set_wide_limit's bytes per direction (16 GiB unless set) or
+ * cannot be allocated, the float64 steps run until operator or limit change;
+ * inside a stream capture a call that would have to make them runs the float64
+ * steps.  Beyond upstream. */
 int slu_hbs_apply_wide(slu_handle_t h, slu_hbs_t op, int trans, const double* X, int ldx,
                        double* Y, int ldy, int nrhs);
 int slu_ulv_solve_wide(slu_handle_t h, slu_hbs_t op, const double* X, int ldx, double* Y,
@@ -142,6 +151,8 @@ int slu_ulv_solve_wide_plan_create(slu_handle_t h, slu_hbs_t op, const double* X
 /* *out = 1 where the calls above take the residue steps for a solve (solve = 1)
  * or an apply of nrhs columns, else 0. */
 int slu_hbs_wide_steps(slu_hbs_t op, int solve, int trans, int nrhs, int* out);
+/* Limit for images not made yet; 0: none, every call runs the float64 steps. */
+int slu_hbs_set_wide_limit(slu_hbs_t op, size_t bytes);
 
 /* Replaces HBSMAT.solve (HBSnew.py:393-416) -> ULVsparse.solve
  * (ULVsparse.py:295-358), in place on B (N x nrhs, unpermuted ordering).
@@ -354,7 +365,7 @@ int slu_hbs_info(slu_hbs_t op, int* L, int* N, int* levels, long long* NNvec, in
 int slu_hbs_export(slu_handle_t h, slu_hbs_t op, int what, int level, double* dst, size_t count,
                    size_t* count_out);
 /* Bytes of stored factors: which = 0 HBS (U, V, D; HBSMAT.nbytes,
- * HBSnew.py:296-302), 1 solve factors. */
+ * HBSnew.py:296-302), 1 solve factors, 2 images of the wide calls. */
 int slu_hbs_nbytes(slu_hbs_t op, int which, size_t* out);
 
 /* Measured float64 FMA throughput of the current device: a register-only

@@ -26,6 +26,7 @@ SIGNATURES = {
     "slu_create": [P, ctypes.POINTER(c_void_p)],
     "slu_destroy": [P],
     "slu_set_stream": [P, P],
+    "slu_trim": [P],
     "slu_sync": [P],
     "slu_check_waits": [P],
     "slu_wait_probe": [P, c_int],
@@ -41,6 +42,7 @@ SIGNATURES = {
     "slu_ulv_solve_wide_plan_create": [P, P, P, c_int, P, c_int, c_int, c_int,
                                        ctypes.POINTER(c_void_p)],
     "slu_hbs_wide_steps": [P, c_int, c_int, c_int, ctypes.POINTER(c_int)],
+    "slu_hbs_set_wide_limit": [P, c_size_t],
     "slu_ulv_solve": [P, P, P, c_int, c_int, c_int],
     "slu_ulv_solve_noalloc": [P, P, P, c_int, c_int, c_int],
     "slu_hbs_prepare_f32": [P, P],

@@ -59,6 +59,13 @@ int slu_destroy(slu_handle_t h) {
   });
 }
 
+int slu_trim(slu_handle_t h) {
+  return guard(h, [&] {
+    SLU_REQUIRE(h, "null handle");
+    for (slu::Workspace* w : {&h->h.ws, &h->h.gemm_ws, &h->h.lu_ws}) w->buf.release();
+  });
+}
+
 int slu_set_stream(slu_handle_t h, void* stream) {
   return guard(h, [&] {
     SLU_REQUIRE(h, "null handle");
@@ -351,7 +358,15 @@ int slu_hbs_wide_steps(slu_hbs_t op, int solve, int trans, int nrhs, int* out) {
     SLU_REQUIRE(op && out, "null argument");
     SLU_REQUIRE(nrhs >= 1, "bad right-hand side shape");
     SLU_REQUIRE(solve ? op->H.has_ulv : op->H.has_mats, "HBS factors not loaded");
-    *out = slu::crt_steps_pay(op->H, solve != 0, trans != 0, nrhs) ? 1 : 0;
+    *out = slu::crt_steps_run(op->H, solve != 0, trans != 0, nrhs) ? 1 : 0;
+  });
+}
+
+int slu_hbs_set_wide_limit(slu_hbs_t op, size_t bytes) {
+  return guard(nullptr, [&] {
+    SLU_REQUIRE(op, "null argument");
+    op->H.crt_limit = bytes;
+    for (auto& n : op->H.no_crt) n = false;
   });
 }
 

@@ -685,9 +685,9 @@ size_t crt_bytes(int M, int N, int K, long long nb) {
          up((size_t)(NM + 1) * nb * M * pitch, 1024) + up((size_t)8 * nb * (M + N), 1024) + 4096;
 }
 
-// Bound on the workspace of one launch set: larger products run in pieces
-// (deeper ones in slices of kDepthMax, accumulated in C).
-constexpr size_t kWsMax = size_t(768) << 20;
+// Larger products than the handle's scratch limit allows run in pieces (deeper
+// ones in slices of kDepthMax, accumulated in C).
+constexpr size_t kWsMax = Handle::kScratchMax;
 constexpr int kDepthMax = 8192;
 
 struct Operand {
@@ -812,6 +812,7 @@ void gemm_f64_tensor(Handle& h, bool ta, bool tb, int M, int N, int K, double al
   const long long nb = (long long)batch0 * batch1;
   long long fit = std::max<long long>(1, kWsMax / crt_bytes(Mp, Np, K, 1));
   fit = std::min<long long>(fit, 65535);
+  fit = (nb + (nb + fit - 1) / fit - 1) / ((nb + fit - 1) / fit);   // pieces of one size
   // residue rows are indexed by 32-bit TMA coordinates
   fit = std::max<long long>(1, std::min(fit, (1LL << 30) / (NM + 1) / std::max(Mp, Np)));
   for (int i0 = 0; i0 < M; i0 += Mp)

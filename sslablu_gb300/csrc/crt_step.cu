@@ -68,7 +68,6 @@ constexpr int kMma = 4;            // warps that copy operator images and issue 
 constexpr int kWarps = 16;         // compute warps, after them
 constexpr int kThreads = 32 * (kMma + kWarps);
 constexpr size_t kSmemMax = 224 * 1024;
-constexpr size_t kMaxImages = 16ULL << 30;   // bytes of a direction's images (4x its operators)
 constexpr long long kWaitLimit = 1LL << 22;
 
 struct CrtStep {
@@ -688,7 +687,7 @@ struct Part {
 
 // Makes the images of `parts` in `buf`; false where they don't fit in the
 // memory they may take.
-bool make_images(cudaStream_t st, const std::vector<Part>& parts, DevBuf& buf) {
+bool make_images(cudaStream_t st, const std::vector<Part>& parts, size_t limit, DevBuf& buf) {
   if ((int)parts.size() > kMaxOps) return false;
   ImageOps a{};
   size_t bytes = (4 * parts.size() + 1023) / 1024 * 1024;   // `scaled`
@@ -709,7 +708,7 @@ bool make_images(cudaStream_t st, const std::vector<Part>& parts, DevBuf& buf) {
     total += (long long)tr;
     blocks += o.Nb;
   }
-  if (bytes > kMaxImages || total >= (1LL << 31)) return false;
+  if (bytes > limit || total >= (1LL << 31)) return false;
   try {
     buf.alloc(bytes, st);
   } catch (const Error&) {
@@ -839,8 +838,10 @@ void each_step(const Hbs& H, bool solve, bool trans, F f) {
 
 // Makes the residue images of a direction unless they are there.
 bool ready(Handle& h, Hbs& H, bool solve, bool trans) {
-  std::atomic<bool>& have = H.has_crt[(solve ? 0 : 2) + (trans ? 1 : 0)];
+  const int dir = (solve ? 0 : 2) + (trans ? 1 : 0);
+  std::atomic<bool>& have = H.has_crt[dir];
   if (have) return true;
+  if (H.no_crt[dir]) return false;
   cudaStream_t st = h.stream;
   // the first use waits for the images: not inside a stream capture
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -848,6 +849,7 @@ bool ready(Handle& h, Hbs& H, bool solve, bool trans) {
   if (cap != cudaStreamCaptureStatusNone) return false;
   std::lock_guard<std::mutex> lock(H.lazy_mu);
   if (have) return true;
+  if (H.no_crt[dir]) return false;
   const bool compose = !solve && !H.has_apply[trans ? 1 : 0];
   if (compose) hbs_make_apply(h, H, trans, false);
   std::vector<Part> parts;
@@ -871,9 +873,12 @@ bool ready(Handle& h, Hbs& H, bool solve, bool trans) {
       add(trans ? l.crDnT : l.crDn, trans ? l.AdnT : l.Adn, nb, l.n, root ? l.n : l.n + l.k);
     }
   }
-  const bool made = make_images(st, parts, H.crt_buf[(solve ? 0 : 2) + (trans ? 1 : 0)]);
-  if (!made && !compose) return false;
-  if (!made) stream_wait(st);   // the composed operators
+  const bool made = make_images(st, parts, H.crt_limit, H.crt_buf[dir]);
+  if (!made) {
+    H.no_crt[dir] = true;
+    if (!compose) return false;
+    stream_wait(st);   // the composed operators
+  }
   if (compose) H.has_apply[trans ? 1 : 0] = true;
   have = made;
   return made;
@@ -907,6 +912,10 @@ bool crt_steps_pay(const Hbs& H, bool solve, bool trans, int c) {
     crt += 3.5 + tile * (double)((g.tiles + sms - 1) / sms);
   });
   return fit && f64 >= crt + 40.0;
+}
+
+bool crt_steps_run(const Hbs& H, bool solve, bool trans, int c) {
+  return !H.no_crt[(solve ? 0 : 2) + (trans ? 1 : 0)] && crt_steps_pay(H, solve, trans, c);
 }
 
 bool crt_prepare(Handle& h, Hbs& H, bool solve, bool trans, int c) {

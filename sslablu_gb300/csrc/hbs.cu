@@ -510,6 +510,10 @@ void hbs_make_f32(Handle& h, Hbs& H) {
 
 size_t hbs_nbytes(const Hbs& H, int which) {
   size_t b = 0;
+  if (which == 2) {
+    for (const DevBuf& i : H.crt_buf) b += i.bytes;
+    return b;
+  }
   for (const Level& l : H.lv) {
     if (which == 0) b += l.U.bytes + l.V.bytes + l.D.bytes;
     else b += l.U.bytes + l.D.bytes + l.Q.bytes + l.W.bytes + l.R.bytes + l.Uu.bytes;

@@ -65,8 +65,11 @@ struct HostStage {
 struct Handle {
   cudaStream_t stream = nullptr;
   Workspace ws;
-  Workspace gemm_ws;   // residues of gemm_f64 (crt_gemm.cu), at most about 1 GB
-  Workspace lu_ws;     // permutations and triangles of lu_factor / lu_inverse
+  // kept between calls (allocating 300 MB takes 0.8 ms, a block solve 0.7); work
+  // that would need more than kScratchMax runs in pieces, down to one matrix
+  Workspace gemm_ws;   // residues of gemm_f64 (crt_gemm.cu)
+  Workspace lu_ws;     // permutations and triangles of lu_factor / lu_inverse / apply_wy
+  static constexpr size_t kScratchMax = size_t(384) << 20;
   HostStage upload, readback;
   DevBuf info;  // int[64] device status words
   // set by a kernel whose bounded waits ran out: mapped host memory, so that
@@ -220,11 +223,16 @@ struct Hbs {
   // residue images (crt_step.cu) of the solve N, T and the apply N, T; made on
   // first use, likewise
   std::atomic<bool> has_crt[4] = {false, false, false, false};
+  // the images could not be had (no memory, or above the limit): not tried again
+  // before the operator or the limit changes
+  std::atomic<bool> no_crt[4] = {false, false, false, false};
+  std::atomic<size_t> crt_limit{16ULL << 30};   // bytes of a direction's images
   DevBuf crt_buf[4];
   // (a new ULV factorisation leaves the applies' operators as they are)
   void drop_crt(bool applies) {
     for (int i = 0; i < (applies ? 4 : 2); ++i) {
       has_crt[i] = false;
+      no_crt[i] = false;
       crt_buf[i].release();
     }
   }
@@ -415,10 +423,12 @@ void apply_wy(Handle& h, int m, int k, double* W, double* W2, int ldw, long long
 // ---------------------------------------------------------------- tensor-core sweep
 // (crt_step.cu) Solves and applies of many right-hand sides as exact residue
 // products, float64 in and out, for the entry points whose name says `wide`.
-// crt_steps_pay: by the operator's shape and c alone.  crt_prepare also makes the
+// crt_steps_pay: by the operator's shape and c alone (crt_steps_run: and its
+// images are there or may be made).  crt_prepare also makes the
 // residue images on first use (false inside a stream capture that would need it,
 // and where they don't fit: take the float64 steps).
 bool crt_steps_pay(const Hbs& H, bool solve, bool trans, int c);
+bool crt_steps_run(const Hbs& H, bool solve, bool trans, int c);
 bool crt_prepare(Handle& h, Hbs& H, bool solve, bool trans, int c);
 void crt_solve(cudaStream_t st, const Hbs& H, bool trans, const double* X, int ldx, double* B,
                int ldb, int c, double* scratch, size_t stride, volatile unsigned* err);

@@ -869,7 +869,7 @@ void lu_inverse(Handle& h, int n, const double* LU, int lda, long long sA, const
   const int w = (n + (1 << q) - 1) >> q, np = w << q;
   const size_t nn = (size_t)np * np;
   const size_t per = 8 * (3 * nn + (size_t)np * n) + sizeof(int) * (size_t)n + 4 * 256;
-  const int fit = (int)std::max<size_t>(1, std::min<size_t>((size_t(1) << 30) / per, 65535 >> (q + 1)));
+  const int fit = (int)std::max<size_t>(1, std::min<size_t>(Handle::kScratchMax / per, 65535 >> (q + 1)));
   for (int b0 = 0; b0 < batch; b0 += fit) {
     const int nb = std::min(fit, batch - b0);
     h.lu_ws.reserve(per * nb + 4096, st);

@@ -128,7 +128,7 @@ void apply_wy(Handle& h, int m, int k, double* W, double* W2, int ldw, long long
   const long long sV = (long long)k * m, sT = (long long)k * k, sX = (long long)nc * k;
   const size_t per = 8 * (size_t)sets * (sV + 2 * sT + 2 * sX) + 5 * 256;
   const int fit = (int)std::max<size_t>(
-      1, std::min<size_t>((size_t(1) << 30) / per, (size_t)65535 / sets));
+      1, std::min<size_t>(Handle::kScratchMax / per, (size_t)65535 / sets));
   const int sm = 8 * (k * (k + 1) + k * k / 2 + 2 * k * 16);
   ensure_smem(reinterpret_cast<const void*>(wy_tri_kernel), sm);
   for (int b0 = 0; b0 < batch; b0 += fit) {
