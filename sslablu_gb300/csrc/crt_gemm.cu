@@ -702,15 +702,17 @@ void crt_piece(Handle& h, int M, int N, int K, double alpha, const Operand& A, c
                int batch) {
   cudaStream_t st = h.stream;
   const int Kp = (int)up(K, BK), pitch = (int)up(N, 16), t = bits_for(K);
-  h.gemm_ws.reserve(crt_bytes(M, N, K, batch), st);
+  Scratch scratch(h.gemm_ws, st);
+  Workspace& ws = scratch.w;
+  ws.reserve(crt_bytes(M, N, K, batch), st);
   constexpr size_t NP = NM + 1;   // planes: residues and magnitudes
-  auto* ra = h.gemm_ws.take<__nv_bfloat16>(NP * batch * M * Kp);
-  auto* rb = h.gemm_ws.take<__nv_bfloat16>(NP * batch * N * Kp);
-  auto* R = h.gemm_ws.take<int8_t>(NP * batch * M * pitch);
-  int* ea = h.gemm_ws.take<int>((size_t)batch * M);
-  int* eb = h.gemm_ws.take<int>((size_t)batch * N);
-  int* wa = h.gemm_ws.take<int>((size_t)batch * M);
-  int* wb = h.gemm_ws.take<int>((size_t)batch * N);
+  auto* ra = ws.take<__nv_bfloat16>(NP * batch * M * Kp);
+  auto* rb = ws.take<__nv_bfloat16>(NP * batch * N * Kp);
+  auto* R = ws.take<int8_t>(NP * batch * M * pitch);
+  int* ea = ws.take<int>((size_t)batch * M);
+  int* eb = ws.take<int>((size_t)batch * N);
+  int* wa = ws.take<int>((size_t)batch * M);
+  int* wb = ws.take<int>((size_t)batch * N);
   const CrtOperand oa{A.x, A.ld, A.s0, A.s1, M, !A.trans, ra, ea, wa};
   const CrtOperand ob{B.x, B.ld, B.s0, B.s1, N, B.trans, rb, eb, wb};
   auto convert = [&](auto kern, int rows) {

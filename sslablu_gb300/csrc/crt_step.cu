@@ -844,9 +844,7 @@ bool ready(Handle& h, Hbs& H, bool solve, bool trans) {
   if (H.no_crt[dir]) return false;
   cudaStream_t st = h.stream;
   // the first use waits for the images: not inside a stream capture
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  SLU_CHECK_CUDA(cudaStreamIsCapturing(st, &cap));
-  if (cap != cudaStreamCaptureStatusNone) return false;
+  if (capturing(st)) return false;
   std::lock_guard<std::mutex> lock(H.lazy_mu);
   if (have) return true;
   if (H.no_crt[dir]) return false;

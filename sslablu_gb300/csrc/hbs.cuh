@@ -29,6 +29,16 @@ struct Workspace {
   }
 };
 
+// The scratch of one call: the handle's own, or, where the call is captured into
+// a graph, memory of that graph (allocated and freed by it at every launch): what
+// the handle keeps may be replaced by a larger one before the graph runs, and what
+// is allocated in a capture does not exist outside its graph.
+struct Scratch {
+  Workspace own;
+  Workspace& w;
+  Scratch(Workspace& kept, cudaStream_t st) : w(capturing(st) ? own : kept) {}
+};
+
 // Pinned host memory for per-call uploads (task tables) and small read-backs
 // (residual norms).  acquire() waits until the copy issued after the previous
 // acquire has completed, so the buffer can be rewritten.

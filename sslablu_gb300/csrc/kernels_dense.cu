@@ -73,6 +73,15 @@ void stream_wait(cudaStream_t st) {
   SLU_CHECK_CUDA(cudaEventSynchronize(w.ev));
 }
 
+bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &s) != cudaSuccess) {
+    cudaGetLastError();   // the legacy stream beside another stream's capture
+    return false;
+  }
+  return s != cudaStreamCaptureStatusNone;
+}
+
 std::shared_ptr<volatile unsigned> mapped_word() {
   // a handle may be made while its stream is captured: the allocation is no
   // part of that

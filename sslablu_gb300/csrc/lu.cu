@@ -822,8 +822,9 @@ void lu_factor(Handle& h, int n, double* A, int lda, long long sA, int* piv, lon
     return;
   }
   cudaStream_t st = h.stream;
-  h.lu_ws.reserve(sizeof(int) * (size_t)n * batch + 256, st);
-  int* src = h.lu_ws.take<int>((size_t)n * batch);
+  Scratch scratch(h.lu_ws, st);
+  scratch.w.reserve(sizeof(int) * (size_t)n * batch + 256, st);
+  int* src = scratch.w.take<int>((size_t)n * batch);
   for (int K0 = 0; K0 < n; K0 += kOuter) {
     const int K1 = std::min(K0 + kOuter, n);
     for (int k0 = K0; k0 < K1; k0 += kPanel) {
@@ -872,11 +873,13 @@ void lu_inverse(Handle& h, int n, const double* LU, int lda, long long sA, const
   const int fit = (int)std::max<size_t>(1, std::min<size_t>(Handle::kScratchMax / per, 65535 >> (q + 1)));
   for (int b0 = 0; b0 < batch; b0 += fit) {
     const int nb = std::min(fit, batch - b0);
-    h.lu_ws.reserve(per * nb + 4096, st);
-    double* T = h.lu_ws.take<double>(2 * nn * nb);
-    double* W = h.lu_ws.take<double>(nn * nb);
-    double* LP = h.lu_ws.take<double>((size_t)np * n * nb);
-    int* perm = h.lu_ws.take<int>((size_t)n * nb);
+    Scratch scratch(h.lu_ws, st);
+    Workspace& ws = scratch.w;
+    ws.reserve(per * nb + 4096, st);
+    double* T = ws.take<double>(2 * nn * nb);
+    double* W = ws.take<double>(nn * nb);
+    double* LP = ws.take<double>((size_t)np * n * nb);
+    int* perm = ws.take<int>((size_t)n * nb);
     const int in_place = 2 * sizeof(int) * (size_t)n > 200 * 1024;
     const size_t sm = in_place ? 0 : 2 * sizeof(int) * (size_t)n;
     ensure_smem(reinterpret_cast<const void*>(tri_pack_kernel), sm);

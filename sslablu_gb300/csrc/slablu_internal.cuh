@@ -220,6 +220,8 @@ void ensure_smem(const void* kernel, size_t bytes);
 // instead, so many worker threads waiting at once leave the host cores to
 // the threads that are launching work.
 void stream_wait(cudaStream_t st);
+// Is a CUDA graph being captured on st?
+bool capturing(cudaStream_t st);
 // A word of mapped host memory, zero (one address on host and device).
 std::shared_ptr<volatile unsigned> mapped_word();
 void set_blocking_waits(bool on);

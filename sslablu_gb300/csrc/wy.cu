@@ -133,12 +133,14 @@ void apply_wy(Handle& h, int m, int k, double* W, double* W2, int ldw, long long
   ensure_smem(reinterpret_cast<const void*>(wy_tri_kernel), sm);
   for (int b0 = 0; b0 < batch; b0 += fit) {
     const int nb = std::min(fit, batch - b0), total = sets * nb;
-    h.lu_ws.reserve(per * nb + 4096, st);
-    double* V = h.lu_ws.take<double>(sV * total);
-    double* G = h.lu_ws.take<double>(sT * total);
-    double* T = h.lu_ws.take<double>(sT * total);
-    double* X1 = h.lu_ws.take<double>(sX * total);
-    double* X2 = h.lu_ws.take<double>(sX * total);
+    Scratch scratch(h.lu_ws, st);
+    Workspace& ws = scratch.w;
+    ws.reserve(per * nb + 4096, st);
+    double* V = ws.take<double>(sV * total);
+    double* G = ws.take<double>(sT * total);
+    double* T = ws.take<double>(sT * total);
+    double* X1 = ws.take<double>(sX * total);
+    double* X2 = ws.take<double>(sX * total);
     double* Wa = W + b0 * sW;
     double* Wb = W2 ? W2 + b0 * sW : Wa;
     const double* ta = tau + b0 * sTau;
