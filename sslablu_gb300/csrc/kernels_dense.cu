@@ -381,9 +381,10 @@ template void gemm_batched<float>(cudaStream_t, bool, bool, int, int, int, float
 // ============================================================== triangular solve
 // Substitution with R or R^T for a chunk of right-hand sides per CTA.
 namespace {
-// y / d with r = 1 / d: the product, corrected once by its exact residual (the
-// last rounding decides, as in a division) where neither leaves the range of
-// normal numbers.  Three dependent operations instead of a division.
+// y / d with r = 1 / d: the product, corrected once by its exact residual (P. W.
+// Markstein, IBM J. Res. Dev. 34, 1990; the last rounding decides, as in a
+// division: within 1 ulp, tested) where neither leaves the range of normal
+// numbers.  Three dependent operations instead of a division.
 __device__ __forceinline__ float quotient(float y, float d, float) { return y / d; }
 __device__ __forceinline__ double quotient(double y, double d, double r) {
   const double q = y * r;
