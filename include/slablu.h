@@ -132,7 +132,7 @@ int slu_hbs_apply(slu_handle_t h, slu_hbs_t op, int trans, const double* X, int 
  * largest entry of their row (step operator) or column (vectors, per block).
  * An output's error is at most w 2^-54 of the largest |S| |z| in its block's
  * column (w <= 128 the step's depth; the operator's rows and columns may be
- * scaled in any way), and 2^-26 of its own; a column of the result does not
+ * scaled in any way), and 2^-14 of its own; a column of the result does not
  * depend on the others, but differs from the float64 steps' by rounding.  Other
  * shapes run the float64 steps, with their bits.  The first call of a direction
  * (solve or apply, trans) makes images of the step operators, four times their

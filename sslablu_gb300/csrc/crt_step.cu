@@ -15,11 +15,13 @@
 // of S within 2^-kSpread of its row's largest: the error in a column of outputs,
 // its rows scaled by those of S, is at most w 2^(kSpread - t), below w 2^-53,
 // times the largest sum of |S| |z| there, where a float64 FMA chain's is w 2^-53
-// of the output's own.  Outputs below 2^-32 of the row's and column's largest
-// entries are formed by float64 dot products, so every output keeps 2^-26 of its
-// own size.  (Random cancellation gets there once in 10^9 outputs; at 2^-22 a
-// step of 4 M outputs met two or three, and the 20-40K clocks of each added half
-// to a solve of 261 columns.)
+// of the output's own.  Outputs below 2^-44 of the row's and column's largest
+// entries are formed by float64 dot products, so every output keeps 2^-14 of its
+// own size.  (The steps of an operator whose couplings have singular values down
+// to 1e-12 have many outputs at 2^-33: with the line at 2^-32 their dot products,
+// 20-40K clocks each, took a solve of 1024 columns from 680 to 832 us; at 2^-22
+// random cancellation alone, two or three outputs a step, added half to a solve of
+// 261 columns.)
 //
 // One persistent kernel per step.  A tile is a block, up to 128 operator rows
 // and 32, 16 or 8 columns (tiling_of: 16 moduli of 32 columns fill TMEM):
@@ -551,8 +553,8 @@ __global__ void __launch_bounds__(kThreads, 1) crt_step_kernel(const CrtStep o) 
             if (e < nc) {
               const int fb = cex[i & 1][CG * g + e], f = fa + max(fb, 1);
               double v = combine(R[u][0], R[u][1], R[u][2], R[u][3], f - 2 * (1022 + o.t));
-              // not finite, or below 2^-32 of the largest entries
-              if (fa == 0x7ff || fb == 0x7ff || (int)(hi32(v) >> 20 & 0x7ff) < f - 1053)
+              // not finite, or below 2^-44 of the largest entries
+              if (fa == 0x7ff || fb == 0x7ff || (int)(hi32(v) >> 20 & 0x7ff) < f - 1065)
                 v = dot_f64(s, T.b, r0 + r, c0 + e);
               out[e] = v;
             }
