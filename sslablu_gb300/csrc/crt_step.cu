@@ -46,8 +46,9 @@
 // tile of 64 x 64 x 32 takes 17K clocks where that work is 8K (the phases of a
 // tile follow one another), the float64 pipe 66K.
 // Measured (us, float64 steps -> these): 8192 rows with leaves of 64 and rank
-// 32, 261 columns: solve 2100 -> 413, transposed 2017 -> 432, apply 1317 ->
-// 377; 4096 rows, 64 columns: 252 -> 118, 275 -> 123, 180 -> 111.  The relative
+// 32, 261 columns: solve 2100 -> 423, transposed 2017 -> 434, apply 1317 ->
+// 381; 4096 rows, 64 columns: 252 -> 117, 275 -> 122, 180 -> 110 (the balanced
+// columns and the look at small outputs 1-3% of it).  The relative
 // error against 64 bits over those shapes: solves 1.2e-15 (float64 steps
 // 1.2e-15), applies 1.1e-15 (1.1e-15): that of the operators, not of the steps.
 // Columns or operator rows that are not finite take float64 dot products.
@@ -890,8 +891,8 @@ bool ready(Handle& h, Hbs& H, bool solve, bool trans) {
 // multiplications at the pipe's rate, 0.87 TFLOP/s of what a step asks for;
 // the residue steps 3.5 us each and a tile's time per wave of tiles (above).
 // They have to win by 40 us, about what the images cost on the first call:
-// solves of 4096 rows (leaves of 64, rank 32) with 33 columns take 166 -> 122
-// us, 48: 206 -> 124, 64: 255 -> 126, 300: 1306 -> 292; of 1024 rows with 64
+// solves of 4096 rows (leaves of 64, rank 32) with 48 columns take 198 -> 116
+// us, 64: 249 -> 117, 300: 1292 -> 293; of 1024 rows with 64
 // columns 79 -> 72 (left to float64), 128: 128 -> 79; with leaves of 16 the
 // float64 steps stay ahead (4096 rows, 300 columns: 297 against 607).
 // Up to 32 columns a call's bits are those of the float64 steps, which groups and
