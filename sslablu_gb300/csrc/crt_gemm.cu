@@ -796,6 +796,7 @@ void gemm_f64_tensor(Handle& h, bool ta, bool tb, int M, int N, int K, double al
                      const double* A, int lda, long long sA0, long long sA1, const double* B,
                      int ldb, long long sB0, long long sB1, double beta, double* C, int ldc,
                      long long sC0, long long sC1, int batch0, int batch1) {
+  if (M <= 0 || N <= 0 || batch0 <= 0 || batch1 <= 0) return;
   if (K > kDepthMax) {
     for (int k0 = 0; k0 < K; k0 += kDepthMax)
       gemm_f64_tensor(h, ta, tb, M, N, std::min(kDepthMax, K - k0), alpha,
@@ -811,29 +812,29 @@ void gemm_f64_tensor(Handle& h, bool ta, bool tb, int M, int N, int K, double al
     if (Mp >= Np) Mp = (int)up((Mp + 1) / 2, 256);
     else Np = (int)up((Np + 1) / 2, 256);
   }
-  const long long nb = (long long)batch0 * batch1;
   long long fit = std::max<long long>(1, kWsMax / crt_bytes(Mp, Np, K, 1));
   fit = std::min<long long>(fit, 65535);
-  fit = (nb + (nb + fit - 1) / fit - 1) / ((nb + fit - 1) / fit);   // pieces of one size
   // residue rows are indexed by 32-bit TMA coordinates
   fit = std::max<long long>(1, std::min(fit, (1LL << 30) / (NM + 1) / std::max(Mp, Np)));
+  // pieces of about one size: whole rows of the batch, else parts of them
+  auto even = [](long long n, long long most) {
+    const long long pieces = (n + most - 1) / most;
+    return (n + pieces - 1) / pieces;
+  };
+  const int n0 = (int)even(batch0, std::min<long long>(fit, batch0));
+  const int n1 = n0 < batch0 ? 1 : (int)even(batch1, std::min<long long>(fit / n0, batch1));
   for (int i0 = 0; i0 < M; i0 += Mp)
     for (int j0 = 0; j0 < N; j0 += Np) {
       const int m = std::min(Mp, M - i0), n = std::min(Np, N - j0);
       const double* a = A + (ta ? (long long)i0 : (long long)i0 * lda);
       const double* b = B + (tb ? (long long)j0 * ldb : (long long)j0);
       double* c = C + (long long)i0 * ldc + j0;
-      if (fit >= nb) {
-        crt_piece(h, m, n, K, alpha, {a, lda, ta, sA0, sA1}, {b, ldb, tb, sB0, sB1}, beta, c, ldc,
-                  sC0, sC1, batch0, (int)nb);
-        continue;
-      }
-      for (int q1 = 0; q1 < batch1; ++q1)
-        for (int q0 = 0; q0 < batch0; q0 += (int)fit) {
-          const int cnt = (int)std::min<long long>(fit, batch0 - q0);
-          crt_piece(h, m, n, K, alpha, {a + q0 * sA0 + q1 * sA1, lda, ta, sA0, 0},
-                    {b + q0 * sB0 + q1 * sB1, ldb, tb, sB0, 0}, beta, c + q0 * sC0 + q1 * sC1, ldc,
-                    sC0, 0, cnt, cnt);
+      for (int q1 = 0; q1 < batch1; q1 += n1)
+        for (int q0 = 0; q0 < batch0; q0 += n0) {
+          const int c0 = std::min(n0, batch0 - q0), c1 = std::min(n1, batch1 - q1);
+          crt_piece(h, m, n, K, alpha, {a + q0 * sA0 + q1 * sA1, lda, ta, sA0, sA1},
+                    {b + q0 * sB0 + q1 * sB1, ldb, tb, sB0, sB1}, beta, c + q0 * sC0 + q1 * sC1, ldc,
+                    sC0, sC1, c0, c0 * c1);
         }
     }
 }
