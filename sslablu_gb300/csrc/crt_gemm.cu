@@ -187,7 +187,8 @@ crt_convert_kernel(CrtOperand a, CrtOperand b, int strips_a, int K, int Kp, int 
     }
     if (!live || kc + 8 * kq >= Kp) continue;
     {
-      const int sub = (max(ex, 187) - 126) << 20;
+      // (not finite: dot products; the others' rows and columns are not to count on it)
+      const int sub = ex == 0x7ff ? 0x7fffffff : (max(ex, 187) - 126) << 20;
       uint32_t w[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u)
