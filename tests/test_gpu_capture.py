@@ -3,7 +3,7 @@ scratch of its own, whatever the handle's does meanwhile."""
 import numpy as np
 import pytest
 
-from tests._gpu import need_gpu
+from tests._gpu import need_gpu, own_stream
 
 pytestmark = pytest.mark.gpu
 
@@ -34,7 +34,7 @@ def test_products_and_factors_in_a_graph():
     C, F = torch.empty((2, 256, 256), dtype=torch.float64, device="cuda"), torch.empty_like(P)
     piv = torch.empty((3, 300), dtype=torch.int32, device="cuda")
     torch.cuda.synchronize()
-    s = torch.cuda.Stream()
+    s = own_stream()
     with torch.cuda.stream(s):
         L.sync()          # the handle of the stream exists; its scratch does not
         graph = torch.cuda.CUDAGraph()
@@ -73,7 +73,7 @@ def test_block_solves_in_a_graph():
           0.2 / np.sqrt(m) * rng.standard_normal((m, m)) if i < nblk - 1 else Z] for i in range(nblk)]
     rb = RedBlackSolver(m)
     rb.factorize(S, None)
-    s = torch.cuda.Stream()
+    s = own_stream()
     with torch.cuda.stream(s):
         B = torch.from_numpy(rng.standard_normal((m * nblk, 64))).cuda()
         X = B.clone()

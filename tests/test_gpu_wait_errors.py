@@ -4,7 +4,7 @@ of a probe kernel with a short limit, on a barrier nobody arrives at."""
 import numpy as np
 import pytest
 
-from tests._gpu import need_gpu
+from tests._gpu import need_gpu, own_stream
 
 pytestmark = pytest.mark.gpu
 
@@ -79,7 +79,7 @@ def test_other_streams_are_not_told(op):
     H, N = op
     b = torch.ones((N, 2), dtype=torch.float64, device="cuda")
     _give_up()
-    s = torch.cuda.Stream()
+    s = own_stream()
     with torch.cuda.stream(s):
         H.solve(b)
     s.synchronize()

@@ -5,7 +5,7 @@ import ctypes
 import numpy as np
 import pytest
 
-from tests._gpu import need_gpu
+from tests._gpu import need_gpu, own_stream
 from tests.test_gpu_crt_steps import _op
 from tests.test_gpu_wide_calls import _rhs, _wide
 
@@ -66,7 +66,7 @@ def test_scratch_is_bounded_and_given_back():
     nb, n = 24, 1024
     A = torch.randn((nb, n, n), dtype=torch.float64, device="cuda")
     C = torch.empty_like(A)
-    s = torch.cuda.Stream()
+    s = own_stream()
     with torch.cuda.stream(s):
         L.sync()
         before = _used()
@@ -80,6 +80,25 @@ def test_scratch_is_bounded_and_given_back():
         assert _used() - before < 64 << 20
     ref = A[23, :3] @ A[23]
     assert float((C[23, :3] - ref).abs().max()) <= 1e-12 * float(ref.abs().max())
+
+
+def test_all_handles_trimmed():
+    """What this thread's handles hold, on whatever streams, is returned; the next
+    call allocates anew."""
+    need_gpu()
+    import torch
+    from sslablu_gb300 import _lib as L
+    H, N = _op(64, 5, 16, False)
+    B = _rhs(N, 40)
+    with torch.cuda.stream(own_stream()):
+        want = H.solve(B)
+        L.sync()
+        torch.cuda.synchronize()
+        for h in L._handles.handles.values():
+            L.check(L.lib().slu_trim(h))
+        got = H.solve(B)
+        L.sync()
+        assert torch.equal(got, want)
 
 
 def test_inverses_in_pieces():
